@@ -291,15 +291,15 @@ int getrs_batched(bem_ctx* ctx, const double2* LU, int64_t lda, int64_t sA, int 
 
 void pivots_to_perm(const std::vector<int>& ipiv, std::vector<int>& perm);
 // grad_geom.cu: the adjoint contractions of the shape gradient.  X, Lam:
-// forward and adjoint solutions (column-major 2N x ncols); RT_dev, hp_dev,
-// rh_dev: the orientations and the far-field adjoint weights h and rhat x h
-// per (column, angle, component) on the device.  grad_v (host, 3 nv, may be
+// forward and adjoint solutions (column-major 2N x ncols); RT_dev, ab_dev: the
+// orientations and the far-field adjoint weight's components along e_par and
+// e_perp per (column, angle) on the device.  grad_v (host, 3 nv, may be
 // null) receives dloss/dv; dpsi_dk (host, 4 doubles) the complex
 // contractions sum S . d(Z D)/dRe k_int and sum S . d(Z D)/dIm k_int,
 // dpsi_deta (2 doubles) sum S . d(Z D)/deta_int.
 int adjoint_geometry(bem_ctx* ctx, const bem_geom* g, std::complex<double> kext, std::complex<double> kint,
                      double eta_e, double eta_i, unsigned flags, const void* X, const void* Lam, int ncols,
-                     const double* RT_dev, int n_orient, const void* hp_dev, const void* rh_dev, int ntheta,
+                     const double* RT_dev, int n_orient, const void* ab_dev, int ntheta,
                      double* grad_v, double* dpsi_dk, double* dpsi_deta);
 // rhs / farfield
 int rhs_dev(bem_ctx* ctx, const bem_geom* g, double k_re, double k_im, double eta,

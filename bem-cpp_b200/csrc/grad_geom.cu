@@ -301,13 +301,16 @@ struct SelfArgs {
 // exp(-Im k R_s) cos(Re k R_s) to 1 (zero, or a step of one unit in the last
 // place) and does not follow Im k, while the imaginary part follows Re k.  So
 // the k derivative is returned for Re k (skr) and Im k (ski) separately.
-__device__ double self_term(const double* v, const HalfInfo& h, const SelfArgs& a, bool extra, cplx* skr, cplx* ski,
-                            cplx* se) {
+template <bool EXTRA>
+__device__ double self_term(const double* v, const HalfInfo& h, const SelfArgs& a, cplx* skr, cplx* ski, cplx* se) {
     const int Nq = a.Nq, N = a.W.N;
     double rp[GQ][3];
     for (int p = 0; p < Nq; p++) bary_point(v, a.q.l1[p], a.q.l2[p], rp[p]);
-    double al[3];
-    for (int t = 0; t < 3; t++) al[t] = h.n[t] >= 0 ? half_alpha(v, h.sign[t], h.jf[t]) : 0.0;
+    double al[3], vF[3][3];
+    for (int t = 0; t < 3; t++) {
+        al[t] = h.n[t] >= 0 ? half_alpha(v, h.sign[t], h.jf[t]) : 0.0;
+        for (int c = 0; c < 3; c++) vF[t][c] = h.n[t] >= 0 ? v[3 * h.jf[t] + c] : 0.0;
+    }
     const double e1x = v[3] - v[0], e1y = v[4] - v[1], e1z = v[5] - v[2];
     const double e2x = v[6] - v[0], e2y = v[7] - v[1], e2z = v[8] - v[2];
     const double nx = e1y * e2z - e1z * e2y, ny = e1z * e2x - e1x * e2z, nz = e1x * e2y - e1y * e2x;
@@ -318,73 +321,86 @@ __device__ double self_term(const double* v, const HalfInfo& h, const SelfArgs& 
     const bool exact = (a.flags & BEM_ASM_GSMOOTH_EXACT) != 0;
     const Medium med[2] = {a.ke, a.ki};
     double psi = 0.0;
-    if (extra) *skr = *ski = *se = {0, 0};
-    for (int t = 0; t < 3; t++) {
-        if (h.n[t] < 0) continue;
-        const double* vFt = v + 3 * h.jf[t];
-        for (int s = 0; s < 3; s++) {
-            if (h.n[s] < 0) continue;
-            const double* vFs = v + 3 * h.jf[s];
-            const double aa = al[t] * al[s];
-            const size_t ix = (size_t)h.n[t] * N + h.n[s];
-            // Graglia sums (without the alpha alpha / A factor)
-            double sA = 0.0, sB = 0.0;
-            for (int p = 0; p < Nq; p++) {
-                sA += a.q.w[p] * P[p];
-                double dot = 0.0;
-                for (int c = 0; c < 3; c++) dot += (rp[p][c] - vFt[c]) * (V[p][c] - vFs[c] * P[p]);
-                sB += a.q.w[p] * dot;
+    if (EXTRA) *skr = *ski = *se = {0, 0};
+    for (int e = 0; e < 2; e++) {
+        const Medium k = med[e];
+        const cplx ik = {-k.ki, k.kr};
+        const double kn = k.kr * k.kr + k.ki * k.ki;
+        const cplx iok = {k.ki / kn, k.kr / kn};  // i/k
+        // the 3 x 3 half pairs share the Green's function of a point pair
+        cplx Ls[3][3], Lkr[EXTRA ? 3 : 1][3], Lki[EXTRA ? 3 : 1][3];
+#pragma unroll
+        for (int t = 0; t < 3; t++)
+#pragma unroll
+            for (int s = 0; s < 3; s++) {
+                Ls[t][s] = {0, 0};
+                if (EXTRA) Lkr[t][s] = Lki[t][s] = {0, 0};
             }
-            const double SA = 4.0 * aa / area * sA * INV4PI_D, SB = aa / area * sB * INV4PI_D;
-            for (int e = 0; e < 2; e++) {
-                const Medium k = med[e];
-                const cplx ik = {-k.ki, k.kr};
-                const double kn = k.kr * k.kr + k.ki * k.ki;
-                const cplx iok = {k.ki / kn, k.kr / kn};  // i/k
-                cplx Ls = {0, 0}, Lkr = {0, 0}, Lki = {0, 0};
-                for (int p = 0; p < Nq; p++)
-                    for (int q = 0; q < Nq; q++) {
-                        const double d0 = rp[p][0] - rp[q][0], d1 = rp[p][1] - rp[q][1], d2 = rp[p][2] - rp[q][2];
-                        const double R2 = fmax(d0 * d0 + d1 * d1 + d2 * d2, 1e-30);
-                        const double invR = rsqrt(R2), Rs = R2 * invR;
-                        const double i4R = __dmul_rn(INV4PI_D, invR);
-                        double sn, cs;
-                        sincos(k.kr * Rs, &sn, &cs);
-                        const double ea = k.ki != 0.0 ? exp_decay(k.ki * Rs) : 1.0;
-                        cplx Gs = {ea * cs * i4R - i4R, ea * sn * i4R};
-                        if (exact) Gs = g_smooth_exact(k, p == q ? 0.0 : Rs);
+        for (int p = 0; p < Nq; p++)
+            for (int q = 0; q < Nq; q++) {
+                const double d0 = rp[p][0] - rp[q][0], d1 = rp[p][1] - rp[q][1], d2 = rp[p][2] - rp[q][2];
+                const double R2 = fmax(d0 * d0 + d1 * d1 + d2 * d2, 1e-30);
+                const double invR = rsqrt(R2), Rs = R2 * invR;
+                const double i4R = __dmul_rn(INV4PI_D, invR);
+                double sn, cs;
+                sincos(k.kr * Rs, &sn, &cs);
+                const double ea = k.ki != 0.0 ? exp_decay(k.ki * Rs) : 1.0;
+                cplx Gs = {ea * cs * i4R - i4R, ea * sn * i4R};
+                if (exact) Gs = g_smooth_exact(k, p == q ? 0.0 : Rs);
+                const double ww = a.q.w[p] * a.q.w[q];
+#pragma unroll
+                for (int t = 0; t < 3; t++)
+#pragma unroll
+                    for (int s = 0; s < 3; s++) {
                         double uu = 0.0;
-                        for (int c = 0; c < 3; c++) uu += (rp[p][c] - vFt[c]) * (rp[q][c] - vFs[c]);
-                        const double ww = a.q.w[p] * a.q.w[q];
+                        for (int c = 0; c < 3; c++) uu += (rp[p][c] - vF[t][c]) * (rp[q][c] - vF[s][c]);
                         // G_s (ik u.u' - 4i/k)
                         const cplx Q = {ik.re * uu - 4.0 * iok.re, ik.im * uu - 4.0 * iok.im};
                         const cplx term = cmul(Gs, Q);
-                        Ls.re += ww * term.re, Ls.im += ww * term.im;
-                        if (extra && e == 1) {
+                        Ls[t][s].re += ww * term.re, Ls[t][s].im += ww * term.im;
+                        if (EXTRA && e == 1) {
                             // dG_s/dk = i exp(ikR)/(4 pi); d Q/dk = i u.u' + 4i/k^2
                             const cplx dGs = {-ea * sn * INV4PI_D, ea * cs * INV4PI_D};
                             const cplx f4k2 = cdiv(cplx{0.0, 4.0}, cmul(cplx{k.kr, k.ki}, cplx{k.kr, k.ki}));
                             const cplx dQ = {f4k2.re, uu + f4k2.im};
                             const cplx dt = cadd(cmul(dGs, Q), cmul(Gs, dQ));
-                            Lkr.re += ww * dt.re, Lkr.im += ww * dt.im;
+                            Lkr[t][s].re += ww * dt.re, Lkr[t][s].im += ww * dt.im;
                             // d/dIm k = i d/dk, except the literal G_s at a coincident point
                             const cplx di = (p == q && !exact) ? cmul(Gs, cmul(cplx{0.0, 1.0}, dQ))
                                                                : cmul(cplx{0.0, 1.0}, dt);
-                            Lki.re += ww * di.re, Lki.im += ww * di.im;
+                            Lki[t][s].re += ww * di.re, Lki[t][s].im += ww * di.im;
                         }
                     }
+            }
+#pragma unroll
+        for (int t = 0; t < 3; t++) {
+            if (h.n[t] < 0) continue;
+#pragma unroll
+            for (int s = 0; s < 3; s++) {
+                if (h.n[s] < 0) continue;
+                const double aa = al[t] * al[s];
+                const size_t ix = (size_t)h.n[t] * N + h.n[s];
+                // Graglia sums (without the alpha alpha / A factor)
+                double sA = 0.0, sB = 0.0;
+                for (int p = 0; p < Nq; p++) {
+                    sA += a.q.w[p] * P[p];
+                    double dot = 0.0;
+                    for (int c = 0; c < 3; c++) dot += (rp[p][c] - vF[t][c]) * (V[p][c] - vF[s][c] * P[p]);
+                    sB += a.q.w[p] * dot;
+                }
+                const double SA = 4.0 * aa / area * sA * INV4PI_D, SB = aa / area * sB * INV4PI_D;
                 // L_e(self) = alpha alpha sum + (-(i/k) SA + ik SB)
                 const cplx corr = {-iok.re * SA + ik.re * SB, -iok.im * SA + ik.im * SB};
-                const cplx Lself = {aa * Ls.re + corr.re, aa * Ls.im + corr.im};
+                const cplx Lself = {aa * Ls[t][s].re + corr.re, aa * Ls[t][s].im + corr.im};
                 const cplx W = c2((e ? a.W.WLi : a.W.WLe)[ix]);
                 psi += W.re * Lself.re - W.im * Lself.im;
-                if (extra && e == 1) {
+                if (EXTRA && e == 1) {
                     // d/dk of the correction: (i/k^2) SA + i SB (holomorphic)
                     const cplx ik2 = cdiv(cplx{0.0, 1.0}, cmul(cplx{k.kr, k.ki}, cplx{k.kr, k.ki}));
                     const cplx dcorr = {ik2.re * SA, ik2.im * SA + SB};
-                    const cplx dLr = {aa * Lkr.re + dcorr.re, aa * Lkr.im + dcorr.im};
+                    const cplx dLr = {aa * Lkr[t][s].re + dcorr.re, aa * Lkr[t][s].im + dcorr.im};
                     const cplx dci = cmul(cplx{0.0, 1.0}, dcorr);
-                    const cplx dLi = {aa * Lki.re + dci.re, aa * Lki.im + dci.im};
+                    const cplx dLi = {aa * Lki[t][s].re + dci.re, aa * Lki[t][s].im + dci.im};
                     *skr = cadd(*skr, cmul(W, dLr));
                     *ski = cadd(*ski, cmul(W, dLi));
                     *se = cadd(*se, cmul(c2(a.W.Weta[ix]), Lself));
@@ -395,34 +411,43 @@ __device__ double self_term(const double* v, const HalfInfo& h, const SelfArgs& 
     return psi;
 }
 
-// One thread per triangle: central differences of its own term in its 9
-// coordinates (step 1e-4 of its longest edge), and the k / eta contractions.
-__global__ void __launch_bounds__(64) grad_self_kernel(SelfArgs a) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= a.nt) return;
-    double v[9];
-    for (int j = 0; j < 9; j++) v[j] = a.tv[9 * t + j];
-    const HalfInfo h = load_halves(a.hinfo, t);
-    double lmax = 0.0;
-    for (int j = 0; j < 3; j++) {
-        const int j1 = (j + 1) % 3;
-        const double dx = v[3 * j] - v[3 * j1], dy = v[3 * j + 1] - v[3 * j1 + 1], dz = v[3 * j + 2] - v[3 * j1 + 2];
-        lmax = fmax(lmax, sqrt(dx * dx + dy * dy + dz * dz));
+// Central differences of a triangle's own term in its 9 coordinates (step
+// 1e-4 of its longest edge), and the k / eta contractions: SELF_EVALS = 19
+// evaluations per triangle, a thread each (18 displaced ones and the
+// undisplaced one with its k derivatives, which sits in a warp of its own
+// kind only by chance: one in 19).  C5: 6.4 ms with one thread per triangle
+// making all 19 in turn (20 blocks) and the Green's function taken per half pair.
+constexpr int SELF_EVALS = 19, SELF_TRI = 6;
+__global__ void __launch_bounds__(SELF_EVALS * SELF_TRI) grad_self_kernel(SelfArgs a) {
+    __shared__ double s_psi[SELF_TRI][SELF_EVALS];
+    const int tl = threadIdx.x % SELF_TRI, ev = threadIdx.x / SELF_TRI, t = blockIdx.x * SELF_TRI + tl;
+    double hstep = 0.0;
+    if (t < a.nt) {
+        double v[9];
+        for (int j = 0; j < 9; j++) v[j] = a.tv[9 * (size_t)t + j];
+        const HalfInfo h = load_halves(a.hinfo, t);
+        double lmax = 0.0;
+        for (int j = 0; j < 3; j++) {
+            const int j1 = (j + 1) % 3;
+            const double dx = v[3 * j] - v[3 * j1], dy = v[3 * j + 1] - v[3 * j1 + 1],
+                         dz = v[3 * j + 2] - v[3 * j1 + 2];
+            lmax = fmax(lmax, sqrt(dx * dx + dy * dy + dz * dz));
+        }
+        hstep = 1e-4 * lmax;
+        if (ev < SELF_EVALS - 1) {
+            const int j = ev >> 1;
+            const double step = (ev & 1) ? -hstep : hstep;
+            for (int i = 0; i < 9; i++) v[i] = i == j ? v[i] + step : v[i];
+            s_psi[tl][ev] = self_term<false>(v, h, a, nullptr, nullptr, nullptr);
+        } else {
+            cplx skr, ski, se;
+            self_term<true>(v, h, a, &skr, &ski, &se);
+            a.sk[4 * t] = skr.re, a.sk[4 * t + 1] = skr.im, a.sk[4 * t + 2] = ski.re, a.sk[4 * t + 3] = ski.im;
+            a.seta[2 * t] = se.re, a.seta[2 * t + 1] = se.im;
+        }
     }
-    const double hstep = 1e-4 * lmax;
-    cplx skr, ski, se;
-    self_term(v, h, a, true, &skr, &ski, &se);
-    for (int j = 0; j < 9; j++) {
-        const double v0 = v[j];
-        v[j] = v0 + hstep;
-        const double fp = self_term(v, h, a, false, nullptr, nullptr, nullptr);
-        v[j] = v0 - hstep;
-        const double fm = self_term(v, h, a, false, nullptr, nullptr, nullptr);
-        v[j] = v0;
-        a.gtri[9 * t + j] = (fp - fm) / (2.0 * hstep);
-    }
-    a.sk[4 * t] = skr.re, a.sk[4 * t + 1] = skr.im, a.sk[4 * t + 2] = ski.re, a.sk[4 * t + 3] = ski.im;
-    a.seta[2 * t] = se.re, a.seta[2 * t + 1] = se.im;
+    __syncthreads();
+    if (t < a.nt && ev < 9) a.gtri[9 * (size_t)t + ev] = (s_psi[tl][2 * ev] - s_psi[tl][2 * ev + 1]) / (2.0 * hstep);
 }
 
 struct HalfArgs {
@@ -503,106 +528,163 @@ __global__ void grad_rhs_kernel(HalfArgs a) {
 }
 
 struct FFArgs2 {
-    const double* tv;
-    const int* htri;
-    const int* hjf;
-    int N, Nq;
+    const double* tv;      // nt x 9
+    const int* hinfo;      // nt x 3 x 3
+    int nt, N, Nq;
     TriQ q;
     double kr, ki, eta;
     const double* RT;      // n_orient x 9
-    int ntheta, ncols;
-    const double2* hp;     // [c][theta][3]: adjoint weight h of the far field
-    const double2* rh;     // [c][theta][3]: rhat x h
-    const double2* X;      // forward solutions, column-major n x ncols
+    int n_orient, ntheta;
+    const double2* ab;     // [c][theta][2]: components A, B of the adjoint weight of the far field
+    const double2* X;      // forward solutions, column-major 2N x 2 n_orient
     int64_t ldx;
-    double* ghalf;         // 2N x 9
+    double* gpart;         // gridDim.y x nt x 9
 };
 
-// Far field at fixed coefficients: Re sum_c sum_theta h . dF_c(theta), per
-// RWG half (thread), F = -ik/(4 pi) [eta J_perp - rhat x M] with
+// Far field at fixed coefficients: Re sum_c sum_theta h . dF_c(theta) in the
+// vertices of every triangle, F = -ik/(4 pi) [eta J_perp - rhat x M] with
 // J = sum_n x_n sum_t alpha_t sum_p w_p (r_p - v_Ft) exp(-ik rhat.r_p)
-// (farfield.cu:100-262); one block walks every column for its halves.
-__global__ void __launch_bounds__(32) grad_ff_kernel(FFArgs2 a) {
+// (farfield.cu:100-262).  With ph = exp(-ik rhat.r_p), Y = eta x_J h +
+// x_M rhat x h and u = r_p - v_Ft a point needs sum ph Y and
+// sum ph (u.Y) rhat.  h = A e_par + B e_perp, rhat x h = A e3 - B e_par,
+// e_par = e1 cos t - e2 sin t, rhat = e1 sin t + e2 cos t (the frame of
+// farfield_adjoint_kernel), so all of it is linear in ten complex sums over
+// the directions that depend on the point and the column alone,
+//   sum ph A (1, cos, sin, cos sin, cos^2) and the same with B.
+// Thread: one quadrature point of a triangle; it takes the phase once for
+// both polarisations and the three RWG halves, and applies coefficients and
+// free vertices after the sum.  Block (x, y): 128 / Nq triangles, every
+// gridDim.y-th orientation.  C5 (2N = 3840, 64 orientations, 181 angles):
+// 45.3 ms with a thread per RWG half that formed Y and u.Y per direction
+// (120 warps on the chip, 3 x the exponentials, 3 x the multiply-adds).
+constexpr int GFF_THREADS = 128, GFF_SPLIT = 32;
+__global__ void __launch_bounds__(GFF_THREADS) grad_ff_kernel(FFArgs2 a) {
     extern __shared__ __align__(16) double sm2[];
-    double* s_r = sm2;                                          // ntheta * 3 (padded to 16 bytes)
-    double2* s_h = (double2*)(sm2 + ((3 * a.ntheta + 1) & ~1));  // ntheta * 3
-    double2* s_x = s_h + 3 * a.ntheta;                          // ntheta * 3
-    const int hn = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool act = hn < 2 * a.N;
-    const int n = act ? hn % a.N : 0, sign = hn < a.N ? 1 : -1;
-    const int t = act ? a.htri[hn] : 0, jf = act ? a.hjf[hn] : 0, Nq = a.Nq;
-    double v[9];
-    for (int j = 0; j < 9; j++) v[j] = a.tv[9 * t + j];
-    const double al = act ? half_alpha(v, sign, jf) : 0.0;
-    const double* vF = v + 3 * jf;
-    double rp[GQ][3];
-    for (int p = 0; p < Nq; p++) bary_point(v, a.q.l1[p], a.q.l2[p], rp[p]);
-    double grp[GQ][3];
-    for (int p = 0; p < Nq; p++) grp[p][0] = grp[p][1] = grp[p][2] = 0.0;
-    double gF[3] = {0, 0, 0}, gal = 0.0;
+    double2* s_t = (double2*)sm2;          // ntheta: sin, cos
+    double2* s_ab = s_t + a.ntheta;        // ntheta x 4: A0 B0 A1 B1
+    double* s_red = sm2;                   // GFF_THREADS x 13, after the sums
+    const int tid = threadIdx.x, Nq = a.Nq, per = GFF_THREADS / Nq;
+    const int tl = tid / Nq, p = tid % Nq, tri = blockIdx.x * per + tl;
+    const bool act = tl < per && tri < a.nt;
+    double v[9], r[3] = {0, 0, 0};
+    HalfInfo h;
+    if (act) {
+        for (int j = 0; j < 9; j++) v[j] = a.tv[9 * (size_t)tri + j];
+        h = load_halves(a.hinfo, tri);
+        bary_point(v, a.q.l1[p], a.q.l2[p], r);
+    }
+    for (int t = tid; t < a.ntheta; t += blockDim.x) {
+        double st, ct;
+        sincos(a.ntheta > 1 ? M_PI * t / (a.ntheta - 1) : 0.0, &st, &ct);
+        s_t[t] = make_double2(st, ct);
+    }
+    double grp[3] = {0, 0, 0}, gF[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}}, gal[3] = {0, 0, 0};
     const cplx pk = {a.ki * INV4PI_D, -a.kr * INV4PI_D};  // -ik/(4 pi)
     const cplx mik = {a.ki, -a.kr};                        // -ik
-    for (int c = 0; c < a.ncols; c++) {
-        const int o = c / 2;
+    for (int o = blockIdx.y; o < a.n_orient; o += gridDim.y) {
         __syncthreads();
-        for (int th = threadIdx.x; th < a.ntheta; th += blockDim.x) {
-            const double ang = a.ntheta > 1 ? M_PI * th / (a.ntheta - 1) : 0.0;
-            double st, ct;
-            sincos(ang, &st, &ct);
-            const double* R = a.RT + 9 * o;
-            for (int i = 0; i < 3; i++) s_r[3 * th + i] = R[3 * i] * st + R[3 * i + 2] * ct;
-            for (int i = 0; i < 3; i++) {
-                s_h[3 * th + i] = a.hp[((size_t)c * a.ntheta + th) * 3 + i];
-                s_x[3 * th + i] = a.rh[((size_t)c * a.ntheta + th) * 3 + i];
-            }
-        }
+        for (int e = tid; e < 4 * a.ntheta; e += blockDim.x)
+            s_ab[e] = a.ab[((size_t)(2 * o + (e & 3) / 2) * a.ntheta + e / 4) * 2 + (e & 1)];
         __syncthreads();
         if (!act) continue;
-        const cplx xJ = c2(a.X[(int64_t)c * a.ldx + n]), xM = c2(a.X[(int64_t)c * a.ldx + a.N + n]);
-        for (int p = 0; p < Nq; p++) {
-            const double u[3] = {rp[p][0] - vF[0], rp[p][1] - vF[1], rp[p][2] - vF[2]};
-            cplx ag[3] = {{0, 0}, {0, 0}, {0, 0}}, aF[3] = {{0, 0}, {0, 0}, {0, 0}}, aa = {0, 0};
-            for (int th = 0; th < a.ntheta; th++) {
-                const double* r = s_r + 3 * th;
-                const double rd = r[0] * rp[p][0] + r[1] * rp[p][1] + r[2] * rp[p][2];
-                double sn, cs;
-                sincos(a.kr * rd, &sn, &cs);
-                const double ea = a.ki != 0.0 ? exp(a.ki * rd) : 1.0;
-                const cplx ph = {ea * cs, -ea * sn};  // exp(-ik rhat.r)
-                cplx Y[3];
-                for (int i = 0; i < 3; i++)
-                    Y[i] = cadd(cscale(cmul(xJ, c2(s_h[3 * th + i])), a.eta), cmul(xM, c2(s_x[3 * th + i])));
-                const cplx uY = cadd(cadd(cscale(Y[0], u[0]), cscale(Y[1], u[1])), cscale(Y[2], u[2]));
-                const cplx pY = cmul(ph, uY);
-                const cplx mp = cmul(mik, pY);
-                for (int i = 0; i < 3; i++) {
-                    const cplx py = cmul(ph, Y[i]);
-                    ag[i] = cadd(ag[i], cadd(py, cscale(mp, r[i])));
-                    aF[i] = cadd(aF[i], py);
+        double e1[3], e2[3], e3[3], x1 = 0.0, x2 = 0.0;
+        const double* R = a.RT + 9 * (size_t)o;
+        for (int i = 0; i < 3; i++) {
+            e1[i] = R[3 * i], e3[i] = R[3 * i + 1], e2[i] = R[3 * i + 2];
+            x1 += e1[i] * r[i], x2 += e2[i] * r[i];
+        }
+        cplx sA[2][5], sB[2][5];  // weights 1, cos, sin, cos sin, cos^2
+#pragma unroll
+        for (int pol = 0; pol < 2; pol++)
+#pragma unroll
+            for (int k = 0; k < 5; k++) sA[pol][k] = sB[pol][k] = {0, 0};
+        for (int t = 0; t < a.ntheta; t++) {
+            const double st = s_t[t].x, ct = s_t[t].y, rd = st * x1 + ct * x2;
+            double sn, cs;
+            sincos(a.kr * rd, &sn, &cs);
+            const double ea = a.ki != 0.0 ? exp(a.ki * rd) : 1.0;
+            const cplx ph = {ea * cs, -ea * sn};
+            const double w[5] = {1.0, ct, st, ct * st, ct * ct};
+#pragma unroll
+            for (int pol = 0; pol < 2; pol++) {
+                const cplx pa = cmul(ph, c2(s_ab[4 * t + 2 * pol])), pb = cmul(ph, c2(s_ab[4 * t + 2 * pol + 1]));
+#pragma unroll
+                for (int k = 0; k < 5; k++) {
+                    sA[pol][k].re += w[k] * pa.re, sA[pol][k].im += w[k] * pa.im;
+                    sB[pol][k].re += w[k] * pb.re, sB[pol][k].im += w[k] * pb.im;
                 }
-                aa = cadd(aa, pY);
             }
-            const double w = a.q.w[p];
-            for (int i = 0; i < 3; i++) {
-                grp[p][i] += al * w * cmul(pk, ag[i]).re;
-                gF[i] -= al * w * cmul(pk, aF[i]).re;
+        }
+        const double wp = a.q.w[p];
+#pragma unroll
+        for (int pol = 0; pol < 2; pol++) {
+            const cplx *A = sA[pol], *B = sB[pol];
+            const cplx Ass = csub(A[0], A[4]), Bss = csub(B[0], B[4]);  // sin^2 = 1 - cos^2
+            const int64_t col = (int64_t)(2 * o + pol) * a.ldx;
+#pragma unroll
+            for (int k = 0; k < 3; k++) {
+                if (h.n[k] < 0) continue;
+                const cplx xJ = cscale(c2(a.X[col + h.n[k]]), a.eta), xM = c2(a.X[col + a.N + h.n[k]]);
+                const double al = half_alpha(v, h.sign[k], h.jf[k]);
+                double u[3], u1 = 0.0, u2 = 0.0, u3 = 0.0;
+                for (int i = 0; i < 3; i++) {
+                    u[i] = r[i] - v[3 * h.jf[k] + i];
+                    u1 += u[i] * e1[i], u2 += u[i] * e2[i], u3 += u[i] * e3[i];
+                }
+                // sum ph Y in the frame (e1, e2, e3)
+                const cplx y1 = csub(cmul(xJ, A[1]), cmul(xM, B[1])), y2 = csub(cmul(xM, B[2]), cmul(xJ, A[2])),
+                           y3 = cadd(cmul(xJ, B[0]), cmul(xM, A[0]));
+                // sum ph (u.Y) sin t and sum ph (u.Y) cos t
+                const cplx js = cadd(csub(cscale(A[3], u1), cscale(Ass, u2)), cscale(B[2], u3)),
+                           ms = cadd(csub(cscale(A[2], u3), cscale(B[3], u1)), cscale(Bss, u2)),
+                           jc = cadd(csub(cscale(A[4], u1), cscale(A[3], u2)), cscale(B[1], u3)),
+                           mc = cadd(csub(cscale(A[1], u3), cscale(B[4], u1)), cscale(B[3], u2));
+                const cplx S = cmul(mik, cadd(cmul(xJ, js), cmul(xM, ms))), Cc = cmul(mik, cadd(cmul(xJ, jc), cmul(xM, mc)));
+                const double f1 = cmul(pk, y1).re, f2 = cmul(pk, y2).re, f3 = cmul(pk, y3).re;
+                const double gs = cmul(pk, S).re, gc = cmul(pk, Cc).re;
+                for (int i = 0; i < 3; i++) {
+                    const double F = al * wp * (e1[i] * f1 + e2[i] * f2 + e3[i] * f3);
+                    gF[k][i] -= F;
+                    grp[i] += F + al * wp * (e1[i] * gs + e2[i] * gc);
+                }
+                gal[k] += wp * (u1 * f1 + u2 * f2 + u3 * f3);
             }
-            gal += w * cmul(pk, aa).re;
         }
     }
-    if (!act) return;
-    double gv[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    for (int p = 0; p < Nq; p++) {
+    __syncthreads();
+    if (act) {
         const double l1 = a.q.l1[p], l2 = a.q.l2[p], l0 = 1.0 - l1 - l2;
-        for (int c = 0; c < 3; c++) {
-            gv[c] += l0 * grp[p][c];
-            gv[3 + c] += l1 * grp[p][c];
-            gv[6 + c] += l2 * grp[p][c];
+        double* out = s_red + (size_t)tid * 13;
+        for (int i = 0; i < 3; i++) {
+            out[i] = l0 * grp[i];
+            out[3 + i] = l1 * grp[i];
+            out[6 + i] = l2 * grp[i];
+        }
+        for (int k = 0; k < 3; k++) {
+            if (h.n[k] >= 0)
+                for (int i = 0; i < 3; i++) out[3 * h.jf[k] + i] += gF[k][i];
+            out[9 + k] = gal[k];
         }
     }
-    for (int c = 0; c < 3; c++) gv[3 * jf + c] += gF[c];
-    alpha_to_vertices(v, sign, jf, gal, gv);
-    for (int j = 0; j < 9; j++) a.ghalf[9 * (size_t)hn + j] = gv[j];
+    __syncthreads();
+    if (act && p == 0) {
+        double gv[12];
+        for (int j = 0; j < 12; j++) gv[j] = 0.0;
+        for (int q = 0; q < Nq; q++)
+            for (int j = 0; j < 12; j++) gv[j] += s_red[(size_t)(tid + q) * 13 + j];
+        for (int k = 0; k < 3; k++)
+            if (h.n[k] >= 0) alpha_to_vertices(v, h.sign[k], h.jf[k], gv[9 + k], gv);
+        for (int j = 0; j < 9; j++) a.gpart[((size_t)blockIdx.y * a.nt + tri) * 9 + j] = gv[j];
+    }
+}
+
+// out[i] = sum over the parts in order
+__global__ void part_sum_kernel(const double* __restrict__ part, int parts, int count, double* __restrict__ out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    double s = 0.0;
+    for (int k = 0; k < parts; k++) s += part[(size_t)k * count + i];
+    out[i] = s;
 }
 
 // S = (Lam Xd^T + Xd Lam^T) / 2 -> the four N x N weight matrices
@@ -654,7 +736,7 @@ unsigned nblocks(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 
 int adjoint_geometry(bem_ctx* ctx, const bem_geom* g, std::complex<double> kext, std::complex<double> kint,
                      double eta_e, double eta_i, unsigned flags, const void* X, const void* Lam, int ncols,
-                     const double* RT_dev, int n_orient, const void* hp_dev, const void* rh_dev, int ntheta,
+                     const double* RT_dev, int n_orient, const void* ab_dev, int ntheta,
                      double* grad_v, double* dpsi_dk, double* dpsi_deta) {
     const int N = g->N, n = 2 * N, nt = g->nt, Nq = g->Nq, nv = g->nv;
     cudaStream_t st = ctx->stream;
@@ -687,8 +769,10 @@ int adjoint_geometry(bem_ctx* ctx, const bem_geom* g, std::complex<double> kext,
     BEM_TRY(dW.alloc(ctx, 4 * NN * sizeof(double2)));
     BEM_TRY(dT.alloc(ctx, 2 * (size_t)n * ncols * sizeof(double2)));
     BEM_TRY(dInfo.alloc(ctx, (hinfo.size() + 4 * (size_t)N) * sizeof(int)));
-    const size_t out_dbl = 2 * (size_t)nt * 9 + 10 * (size_t)nt + 2 * (size_t)n * 9;
-    BEM_TRY(dOut.alloc(ctx, out_dbl * sizeof(double)));
+    // far field: the orientations in up to GFF_SPLIT parts, summed in order
+    const int ff_parts = std::min(n_orient, GFF_SPLIT);
+    const size_t out_dbl = 3 * (size_t)nt * 9 + 10 * (size_t)nt + (size_t)n * 9;
+    BEM_TRY(dOut.alloc(ctx, (out_dbl + (size_t)ff_parts * nt * 9) * sizeof(double)));
     int* d_hinfo = (int*)dInfo.p;
     int* d_htri = d_hinfo + hinfo.size();
     int* d_hjf = d_htri + 2 * N;
@@ -726,18 +810,20 @@ int adjoint_geometry(bem_ctx* ctx, const bem_geom* g, std::complex<double> kext,
     grad_pair_kernel<<<nt, 128, 0, st>>>(pa);
     BEM_LAUNCHED(ctx);
     SelfArgs sa{g->sing.tv, d_hinfo, nt, Nq, tq, ke, ki, flags, gw, o_self, o_sks, o_ses};
-    grad_self_kernel<<<nblocks(nt, 64), 64, 0, st>>>(sa);
+    grad_self_kernel<<<nblocks(nt, SELF_TRI), SELF_EVALS * SELF_TRI, 0, st>>>(sa);
     BEM_LAUNCHED(ctx);
     HalfArgs ha{g->sing.tv, d_htri, d_hjf, N, Nq, tq, kext.real(), kext.imag(), eta_e, RT_dev, n_orient,
                 (const double2*)Lam, n, o_rhs};
     grad_rhs_kernel<<<nblocks(n, 64), 64, 0, st>>>(ha);
     BEM_LAUNCHED(ctx);
-    FFArgs2 fa{g->sing.tv, d_htri, d_hjf, N, Nq, tq, kext.real(), kext.imag(), eta_e, RT_dev, ntheta, ncols,
-               (const double2*)hp_dev, (const double2*)rh_dev, (const double2*)X, n, o_ff};
-    const size_t smem = (size_t)((3 * ntheta + 1) & ~1) * 8 + (size_t)ntheta * 6 * 16;
-    if (smem > 200 * 1024) return fail(ctx, BEM_ERR_INVALID, "ntheta %d too large for the far-field gradient", ntheta);
+    double* d_part = (double*)dOut.p + out_dbl;
+    FFArgs2 fa{g->sing.tv, d_hinfo, nt, N, Nq, tq, kext.real(), kext.imag(), eta_e, RT_dev, n_orient, ntheta,
+               (const double2*)ab_dev, (const double2*)X, n, d_part};
+    const size_t smem = std::max((size_t)ntheta * 5 * 16, (size_t)GFF_THREADS * 13 * 8);
     BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(grad_ff_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    grad_ff_kernel<<<nblocks(n, 32), 32, smem, st>>>(fa);
+    grad_ff_kernel<<<dim3(nblocks(nt, GFF_THREADS / Nq), ff_parts), GFF_THREADS, smem, st>>>(fa);
+    BEM_LAUNCHED(ctx);
+    part_sum_kernel<<<nblocks(9 * (int64_t)nt, 256), 256, 0, st>>>(d_part, ff_parts, 9 * nt, o_ff);
     BEM_LAUNCHED(ctx);
     std::vector<double> out(out_dbl);
     BEM_TRY_CUDA(ctx, cudaMemcpyAsync(out.data(), dOut.p, out_dbl * 8, cudaMemcpyDeviceToHost, st));
@@ -755,13 +841,13 @@ int adjoint_geometry(bem_ctx* ctx, const bem_geom* g, std::complex<double> kext,
         for (int t = 0; t < nt; t++)
             for (int j = 0; j < 3; j++)
                 for (int c = 0; c < 3; c++)
-                    grad_v[3 * (size_t)M.tris[3 * t + j] + c] -= h_pair[9 * t + 3 * j + c] + h_self[9 * t + 3 * j + c];
+                    grad_v[3 * (size_t)M.tris[3 * t + j] + c] +=
+                        h_ff[9 * t + 3 * j + c] - (h_pair[9 * t + 3 * j + c] + h_self[9 * t + 3 * j + c]);
         for (int hn = 0; hn < n; hn++) {
             const int t = htri[hn];
             for (int j = 0; j < 3; j++)
                 for (int c = 0; c < 3; c++)
-                    grad_v[3 * (size_t)M.tris[3 * t + j] + c] +=
-                        h_rhs[9 * (size_t)hn + 3 * j + c] + h_ff[9 * (size_t)hn + 3 * j + c];
+                    grad_v[3 * (size_t)M.tris[3 * t + j] + c] += h_rhs[9 * (size_t)hn + 3 * j + c];
         }
     }
     // pair terms are holomorphic in k: d/dIm k = i d/dRe k

@@ -29,71 +29,125 @@ namespace bem {
 constexpr double INV4PI_G = 0.07957747154594767;  // 1 / (4 pi)
 
 struct AdjFFArgs {
-    DevHalf h;
-    int N, Nq, ntheta, ncols;
+    int nt, N, Nq, ntheta;
     double kr, ki, eta;
-    const double* RT;    // n_orient * 9
-    const double2* hp;   // [c][theta][3]: the transverse adjoint weight h
-    const double2* rh;   // [c][theta][3]: rhat x h
-    double2* G;          // column-major n x ncols
+    const double *c, *u, *jw, *pi;  // triangle data of the assembly (DevTriAsm)
+    const int* tri_half;            // nt x 3 halves h N + n, -1 padded
+    const double* coef;             // 2N: sign l / (2A) of a half
+    const double* RT;               // n_orient * 9
+    const double2* ab;              // [c][theta][2]: the adjoint weight's components A, B
+    double2* G;                     // column-major n x ncols, zeroed before the launch
     int64_t ldg;
 };
 
-// Thread per RWG n, grid (RWG blocks, columns): sums over the directions of
-// the column's orientation and the 2 Nq points of n.
-__global__ void __launch_bounds__(128) farfield_adjoint_kernel(AdjFFArgs a) {
+// Adjoint far field by triangles.  The weight of a direction is transverse,
+// h = A e_par + B e_perp, with e_par = e1 cos t - e2 sin t, e_perp = e3 and
+// rhat = e1 sin t + e2 cos t in the orientation's frame (e1 = R^T x,
+// e2 = R^T z, e3 = R^T y), so rhat x h = A e3 - B e_par and six complex sums
+// over the directions,
+//   sum ph A (1, cos t, sin t) and sum ph B (1, cos t, sin t),
+// ph = exp(-ik rhat.r), give both sum ph h and sum ph rhat x h at a point.
+// Thread: one quadrature point of a triangle, both polarisations of the
+// orientation blockIdx.y; the phase is taken once for them and for the three
+// RWG halves of the triangle, 6 x fewer exponentials than per RWG half and
+// column.  An RWG's entry is the sum of its two halves' terms, added to a
+// zeroed G: 0 + x + y, the same in either order.  C5 (2N = 3840, 64
+// orientations, 181 angles): 2.77 ms per half and column before.
+constexpr int AFF_THREADS = 128;
+__global__ void __launch_bounds__(AFF_THREADS) farfield_adjoint_kernel(AdjFFArgs a) {
     extern __shared__ __align__(16) double sm[];
-    double* s_r = sm;                                        // ntheta * 3 (padded to 16 bytes)
-    double2* s_h = (double2*)(sm + ((3 * a.ntheta + 1) & ~1));  // ntheta * 3
-    double2* s_x = s_h + 3 * a.ntheta;                       // ntheta * 3
-    const int c = blockIdx.y, o = c / 2;
-    for (int t = threadIdx.x; t < a.ntheta; t += blockDim.x) {
-        const double th = a.ntheta > 1 ? M_PI * t / (a.ntheta - 1) : 0.0;
+    double2* s_t = (double2*)sm;           // ntheta: sin, cos
+    double2* s_ab = s_t + a.ntheta;        // ntheta x 4: A0 B0 A1 B1
+    double* s_red = sm;                    // AFF_THREADS x 25, after the sums
+    const int o = blockIdx.y, tid = threadIdx.x, Nq = a.Nq, per = AFF_THREADS / Nq;
+    for (int t = tid; t < a.ntheta; t += blockDim.x) {
         double st, ct;
-        sincos(th, &st, &ct);
-        const double* R = a.RT + 9 * o;
-        for (int i = 0; i < 3; i++) s_r[3 * t + i] = R[3 * i] * st + R[3 * i + 2] * ct;
+        sincos(a.ntheta > 1 ? M_PI * t / (a.ntheta - 1) : 0.0, &st, &ct);
+        s_t[t] = make_double2(st, ct);
+        for (int pol = 0; pol < 2; pol++)
+            for (int k = 0; k < 2; k++) s_ab[4 * t + 2 * pol + k] = a.ab[((size_t)(2 * o + pol) * a.ntheta + t) * 2 + k];
+    }
+    __syncthreads();
+    const int tl = tid / Nq, q = tid % Nq, tri = blockIdx.x * per + tl;
+    const bool act = tl < per && tri < a.nt;
+    double e1[3], e2[3], e3[3];
+    const double* R = a.RT + 9 * o;
+    for (int i = 0; i < 3; i++) e1[i] = R[3 * i], e3[i] = R[3 * i + 1], e2[i] = R[3 * i + 2];
+    double u[3] = {0, 0, 0};
+    double sA[2][3][2], sB[2][3][2];
+#pragma unroll
+    for (int pol = 0; pol < 2; pol++)
+#pragma unroll
+        for (int k = 0; k < 3; k++) sA[pol][k][0] = sA[pol][k][1] = sB[pol][k][0] = sB[pol][k][1] = 0.0;
+    if (act) {
+        double x1 = 0.0, x2 = 0.0;
         for (int i = 0; i < 3; i++) {
-            s_h[3 * t + i] = a.hp[((size_t)c * a.ntheta + t) * 3 + i];
-            s_x[3 * t + i] = a.rh[((size_t)c * a.ntheta + t) * 3 + i];
+            u[i] = a.u[((size_t)tri * Nq + q) * 3 + i];
+            const double r = a.c[3 * (size_t)tri + i] + u[i];
+            x1 += e1[i] * r, x2 += e2[i] * r;
+        }
+        for (int t = 0; t < a.ntheta; t++) {
+            const double st = s_t[t].x, ct = s_t[t].y, rd = st * x1 + ct * x2;
+            double sn, cs;
+            sincos(a.kr * rd, &sn, &cs);
+            const double ea = a.ki != 0.0 ? exp(a.ki * rd) : 1.0;
+            const double er = cs * ea, ei = -sn * ea;
+#pragma unroll
+            for (int pol = 0; pol < 2; pol++) {
+                const double2 A = s_ab[4 * t + 2 * pol], B = s_ab[4 * t + 2 * pol + 1];
+                const double ar = er * A.x - ei * A.y, ai = er * A.y + ei * A.x;
+                const double br = er * B.x - ei * B.y, bi = er * B.y + ei * B.x;
+                sA[pol][0][0] += ar, sA[pol][0][1] += ai;
+                sA[pol][1][0] += ct * ar, sA[pol][1][1] += ct * ai;
+                sA[pol][2][0] += st * ar, sA[pol][2][1] += st * ai;
+                sB[pol][0][0] += br, sB[pol][0][1] += bi;
+                sB[pol][1][0] += ct * br, sB[pol][1][1] += ct * bi;
+                sB[pol][2][0] += st * br, sB[pol][2][1] += st * bi;
+            }
         }
     }
     __syncthreads();
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= a.N) return;
-    double gj[2] = {0, 0}, gm[2] = {0, 0};
-    for (int hh = 0; hh < 2; hh++)
-        for (int q = 0; q < a.Nq; q++) {
-            const size_t p = ((size_t)hh * a.N + n) * a.Nq + q;
-            const double px = a.h.px[p], py = a.h.py[p], pz = a.h.pz[p], w = a.h.jw[p];
-            const double fx = a.h.fx[p] * w, fy = a.h.fy[p] * w, fz = a.h.fz[p] * w;
-            for (int t = 0; t < a.ntheta; t++) {
-                const double rd = s_r[3 * t] * px + s_r[3 * t + 1] * py + s_r[3 * t + 2] * pz;
-                double sn, cs;
-                sincos(a.kr * rd, &sn, &cs);
-                const double ea = a.ki != 0.0 ? exp(a.ki * rd) : 1.0;
-                const double er = cs * ea, ei = -sn * ea;  // exp(-i k rhat.r)
-                const double2* hv = s_h + 3 * t;
-                const double2* xv = s_x + 3 * t;
-                const double dr = fx * hv[0].x + fy * hv[1].x + fz * hv[2].x;
-                const double di = fx * hv[0].y + fy * hv[1].y + fz * hv[2].y;
-                const double mr = fx * xv[0].x + fy * xv[1].x + fz * xv[2].x;
-                const double mi = fx * xv[0].y + fy * xv[1].y + fz * xv[2].y;
-                gj[0] += er * dr - ei * di;
-                gj[1] += er * di + ei * dr;
-                gm[0] += er * mr - ei * mi;
-                gm[1] += er * mi + ei * mr;
+    // the point's term of every (half, polarisation, J / M): f w . sum ph h and f w . sum ph (rhat x h)
+    if (act) {
+        const double w = a.jw[(size_t)tri * Nq + q];
+        for (int k = 0; k < 3; k++) {
+            const int hn = a.tri_half[3 * (size_t)tri + k];
+            double f1 = 0, f2 = 0, f3 = 0;
+            if (hn >= 0) {
+                const double s = a.coef[hn] * w;
+                for (int i = 0; i < 3; i++) {
+                    const double f = s * (u[i] - a.pi[3 * (size_t)hn + i]);
+                    f1 += f * e1[i], f2 += f * e2[i], f3 += f * e3[i];
+                }
             }
+#pragma unroll
+            for (int pol = 0; pol < 2; pol++)
+#pragma unroll
+                for (int c = 0; c < 2; c++) {
+                    double* out = s_red + (size_t)tid * 25 + (k * 2 + pol) * 4 + c;
+                    out[0] = f1 * sA[pol][1][c] - f2 * sA[pol][2][c] + f3 * sB[pol][0][c];
+                    out[2] = f3 * sA[pol][0][c] - f1 * sB[pol][1][c] + f2 * sB[pol][2][c];
+                }
         }
+    }
+    __syncthreads();
     // -ik/(4 pi) = (k_im - i k_re)/(4 pi); the J part also carries eta
-    const double pr = a.ki * INV4PI_G, pi_ = -a.kr * INV4PI_G;
-    double2 vj, vm;
-    vj.x = a.eta * (pr * gj[0] - pi_ * gj[1]);
-    vj.y = a.eta * (pr * gj[1] + pi_ * gj[0]);
-    vm.x = pr * gm[0] - pi_ * gm[1];
-    vm.y = pr * gm[1] + pi_ * gm[0];
-    a.G[(int64_t)c * a.ldg + n] = vj;
-    a.G[(int64_t)c * a.ldg + a.N + n] = vm;
+    const double pr = a.ki * INV4PI_G, pim = -a.kr * INV4PI_G;
+    for (int e = tid; e < per * 12; e += blockDim.x) {
+        const int t = blockIdx.x * per + e / 12, v = e % 12, k = v / 4, pol = (v / 2) % 2, jm = v % 2;
+        if (t >= a.nt) break;
+        const int hn = a.tri_half[3 * (size_t)t + k];
+        if (hn < 0) continue;
+        double gr = 0.0, gi = 0.0;
+        for (int p = 0; p < Nq; p++) {
+            const double* in = s_red + (size_t)((e / 12) * Nq + p) * 25 + (k * 2 + pol) * 4 + 2 * jm;
+            gr += in[0], gi += in[1];
+        }
+        const double sc = jm == 0 ? a.eta : 1.0;
+        double2* out = &a.G[(int64_t)(2 * o + pol) * a.ldg + (int64_t)jm * a.N + hn % a.N];
+        atomicAdd(&out->x, sc * (pr * gr - pim * gi));
+        atomicAdd(&out->y, sc * (pr * gi + pim * gr));
+    }
 }
 
 // partial[b] = sum over this block's entries of L[i] R[i] (complex, no conjugate)
@@ -232,65 +286,62 @@ static int adjoint_core(bem_ctx* ctx, const bem_problem* p, const double* target
     const double loss = misfit(M.data());
     std::vector<double> coef(nt);
     for (int t = 0; t < nt; t++) coef[t] = 2.0 * (wt ? wt[t] : 1.0) * (M[t] - target[t]);
-    // adjoint weights: h_c(theta) = coef w_o sum_{e in (e_par, e_perp)} conj(F.e) e, and rhat x h
-    std::vector<double> hp((size_t)nc * nt * 3 * 2), rh((size_t)nc * nt * 3 * 2);
+    // adjoint weights h_c(theta) = coef w_o sum_{e in (e_par, e_perp)} conj(F.e) e: their two components
+    std::vector<double> ab((size_t)nc * nt * 2 * 2);
     for (int c = 0; c < nc; c++) {
         const int o = c / 2;
         const double* R = RT.data() + 9 * o;
         for (int t = 0; t < nt; t++) {
             const double th = M_PI * t / (nt - 1), st = std::sin(th), ct = std::cos(th);
-            double r[3], ep[3], ee[3];
-            for (int i = 0; i < 3; i++) {
-                r[i] = R[3 * i] * st + R[3 * i + 2] * ct;
-                ep[i] = R[3 * i] * ct - R[3 * i + 2] * st;
-                ee[i] = R[3 * i + 1];
-            }
             const double* F = Fv.data() + ((size_t)c * nt + t) * 6;
-            std::complex<double> Fc[3] = {{F[0], F[1]}, {F[2], F[3]}, {F[4], F[5]}};
-            std::complex<double> a = std::conj(Fc[0] * ep[0] + Fc[1] * ep[1] + Fc[2] * ep[2]);
-            std::complex<double> b = std::conj(Fc[0] * ee[0] + Fc[1] * ee[1] + Fc[2] * ee[2]);
             const double s = coef[t] * w[o];
-            std::complex<double> h[3];
-            for (int i = 0; i < 3; i++) h[i] = s * (a * ep[i] + b * ee[i]);
-            std::complex<double> x[3] = {r[1] * h[2] - r[2] * h[1], r[2] * h[0] - r[0] * h[2],
-                                         r[0] * h[1] - r[1] * h[0]};
-            double* hq = hp.data() + ((size_t)c * nt + t) * 6;
-            double* xq = rh.data() + ((size_t)c * nt + t) * 6;
+            double ar = 0, ai = 0, br = 0, bi = 0;
             for (int i = 0; i < 3; i++) {
-                hq[2 * i] = h[i].real(), hq[2 * i + 1] = h[i].imag();
-                xq[2 * i] = x[i].real(), xq[2 * i + 1] = x[i].imag();
+                const double ep = R[3 * i] * ct - R[3 * i + 2] * st, ee = R[3 * i + 1];
+                ar += F[2 * i] * ep, ai += F[2 * i + 1] * ep;
+                br += F[2 * i] * ee, bi += F[2 * i + 1] * ee;
             }
+            double* q = ab.data() + ((size_t)c * nt + t) * 4;
+            q[0] = s * ar, q[1] = -s * ai, q[2] = s * br, q[3] = -s * bi;
         }
     }
-    DevMem dH, dRh, dRT, dPart;
-    const size_t hb = hp.size() * 8;
-    if (cudaMalloc(&dH.p, hb) != cudaSuccess || cudaMalloc(&dRh.p, hb) != cudaSuccess ||
-        cudaMalloc(&dRT.p, RT.size() * 8) != cudaSuccess || cudaMalloc(&dPart.p, 1024 * 16) != cudaSuccess) {
+    DevMem dAB, dRT, dPart;
+    const size_t hb = ab.size() * 8;
+    if (cudaMalloc(&dAB.p, hb) != cudaSuccess || cudaMalloc(&dRT.p, RT.size() * 8) != cudaSuccess ||
+        cudaMalloc(&dPart.p, 1024 * 16) != cudaSuccess) {
         cudaGetLastError();
         return fail(ctx, BEM_ERR_OOM, "gradient weights");
     }
-    BEM_TRY_CUDA(ctx, cudaMemcpyAsync(dH.p, hp.data(), hb, cudaMemcpyHostToDevice, ctx->stream));
-    BEM_TRY_CUDA(ctx, cudaMemcpyAsync(dRh.p, rh.data(), hb, cudaMemcpyHostToDevice, ctx->stream));
+    BEM_TRY_CUDA(ctx, cudaMemcpyAsync(dAB.p, ab.data(), hb, cudaMemcpyHostToDevice, ctx->stream));
     BEM_TRY_CUDA(ctx, cudaMemcpyAsync(dRT.p, RT.data(), RT.size() * 8, cudaMemcpyHostToDevice, ctx->stream));
     AdjFFArgs aa{};
-    aa.h = g->half;
+    aa.nt = g->nt;
     aa.N = N;
     aa.Nq = g->Nq;
     aa.ntheta = nt;
-    aa.ncols = nc;
     aa.kr = kext.real();
     aa.ki = kext.imag();
     aa.eta = eta_e;
+    aa.c = g->tri.c;
+    aa.u = g->tri.u;
+    aa.jw = g->tri.jw;
+    aa.pi = g->tri.pi;
+    aa.tri_half = g->tri.tri_half;
+    aa.coef = g->sing_coef;
     aa.RT = (const double*)dRT.p;
-    aa.hp = (const double2*)dH.p;
-    aa.rh = (const double2*)dRh.p;
+    aa.ab = (const double2*)dAB.p;
     aa.G = (double2*)dY.p;  // g
     aa.ldg = n;
-    const size_t smem = (size_t)((3 * nt + 1) & ~1) * 8 + (size_t)nt * 6 * 16;
-    if (smem > 200 * 1024) return fail(ctx, BEM_ERR_INVALID, "ntheta %d too large for the adjoint far field", nt);
+    // ntheta x (1 + 4) complex, reused by the 25 values of a thread.  The
+    // limit on ntheta is that of the reassembly path's buffers of old (120 B an angle).
+    if ((size_t)((3 * nt + 1) & ~1) * 8 + (size_t)nt * 6 * 16 > 200 * 1024)
+        return fail(ctx, BEM_ERR_INVALID, "ntheta %d too large for the adjoint far field", nt);
+    const size_t smem = std::max((size_t)nt * 5 * 16, (size_t)AFF_THREADS * 25 * 8);
     BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(farfield_adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)smem));
-    farfield_adjoint_kernel<<<dim3((N + 127) / 128, nc), 128, smem, ctx->stream>>>(aa);
+    BEM_TRY_CUDA(ctx, cudaMemsetAsync(dY.p, 0, xb, ctx->stream));
+    const int per = AFF_THREADS / g->Nq;
+    farfield_adjoint_kernel<<<dim3((g->nt + per - 1) / per, no), AFF_THREADS, smem, ctx->stream>>>(aa);
     BEM_LAUNCHED(ctx);
     // lambda = D Z^-1 D g
     const int64_t half = (int64_t)(n - N) * nc;
@@ -318,7 +369,7 @@ static int adjoint_core(bem_ctx* ctx, const bem_problem* p, const double* target
         const double am = std::abs(m), am3 = am * am * am;
         double dk[4] = {0, 0, 0, 0}, deta[2] = {0, 0};
         BEM_TRY(adjoint_geometry(ctx, g, kext, kext * m, eta_e, 1.0 / am, p->asm_flags, dX.p, dL.p, nc,
-                                 (const double*)dRT.p, no, dH.p, dRh.p, nt, grad_v, dk, deta));
+                                 (const double*)dRT.p, no, dAB.p, nt, grad_v, dk, deta));
         if (grad_out) {
             // k_i = k_e m with k_e real: d/dRe m = k_e d/dRe k_i, d/dIm m = k_e d/dIm k_i;
             // eta_i = 1/|m|
