@@ -22,6 +22,44 @@ struct Medium {
     double kr, ki;  // k = kr + i ki
 };
 
+// sin and cos without a branch, for |x| below SINCOS_MAX: n = round(2 x / pi),
+// the remainder x - n pi/2 in two fused steps (the first is exact: both
+// operands are multiples of the remainder's last place), the Taylor
+// polynomials of degree 15 and 16 on [-pi/4, pi/4] (their first omitted terms
+// are below 5e-17 and 3e-18) and the quadrant's exchange and signs.  Within
+// 2e-16 of the exact values (tests).  The library's function takes a branch
+// for large arguments at every call, which keeps the compiler from
+// interleaving the independent evaluations of a quadrature loop: the kernels
+// here are bound by the latency of these chains at 8 to 16 warps per SM.
+constexpr double SINCOS_MAX = 1048576.0;
+__device__ __forceinline__ void sincos_bounded(double x, double* sn, double* cs) {
+    const double shift = 6755399441055744.0;  // 1.5 * 2^52: the sum's low bits are the rounded integer
+    const double t = __fma_rn(x, 0.63661977236758134308, shift);
+    const int n = __double2loint(t);
+    const double fn = t - shift;
+    double r = __fma_rn(-fn, 1.5707963267948965580, x);
+    r = __fma_rn(-fn, 6.1232339957367660359e-17, r);
+    const double z = r * r;
+    double p = __fma_rn(z, -1.0 / 1307674368000.0, 1.0 / 6227020800.0);
+    p = __fma_rn(z, p, -1.0 / 39916800.0);
+    p = __fma_rn(z, p, 1.0 / 362880.0);
+    p = __fma_rn(z, p, -1.0 / 5040.0);
+    p = __fma_rn(z, p, 1.0 / 120.0);
+    p = __fma_rn(z, p, -1.0 / 6.0);
+    const double s = __fma_rn(r * z, p, r);
+    double q = __fma_rn(z, 1.0 / 20922789888000.0, -1.0 / 87178291200.0);
+    q = __fma_rn(z, q, 1.0 / 479001600.0);
+    q = __fma_rn(z, q, -1.0 / 3628800.0);
+    q = __fma_rn(z, q, 1.0 / 40320.0);
+    q = __fma_rn(z, q, -1.0 / 720.0);
+    q = __fma_rn(z, q, 1.0 / 24.0);
+    q = __fma_rn(z, q, -0.5);
+    const double c = __fma_rn(z, q, 1.0);
+    const double a = (n & 1) ? c : s, b = (n & 1) ? s : c;
+    *sn = __hiloint2double(__double2hiint(a) ^ (int)((unsigned)(n & 2) << 30), __double2loint(a));
+    *cs = __hiloint2double(__double2hiint(b) ^ (int)((unsigned)((n + 1) & 2) << 30), __double2loint(b));
+}
+
 // e^-x for x >= 0.  Below 2^-54 the correctly rounded value is exactly 1;
 // the literal G_smooth at coincident points (R_s = 1e-15) subtracts
 // 1/(4 pi R_s) from e^-x cos(k R_s)/(4 pi R_s), so one unit in the last

@@ -125,8 +125,15 @@ static void position_arrays(const bem_geom* g, PosArrays& A) {
         }
 }
 
+static double largest_vertex(const HostMesh& m) {
+    double r2 = 0.0;
+    for (const V3& v : m.verts) r2 = std::max(r2, v.x * v.x + v.y * v.y + v.z * v.z);
+    return std::sqrt(r2);
+}
+
 int geom_upload(bem_ctx* ctx, bem_geom* g) {
     const HostMesh& m = g->mesh;
+    g->rmax = largest_vertex(m);
     const HostRWG& r = g->rwg;
     const Quad& q = g->quad;
     const int N = r.N, Nq = q.n, nt = m.nt();
@@ -314,6 +321,7 @@ int geom_set_vertices(bem_ctx* ctx, bem_geom* g, const double* verts) {
         return fail(ctx, BEM_ERR_INVALID, "vertex update needs a geometry built from its mesh");
     for (int i = 0; i < m.nv(); i++) m.verts[i] = {verts[3 * i], verts[3 * i + 1], verts[3 * i + 2]};
     rwg_refresh(m, r);
+    g->rmax = largest_vertex(m);
     PosArrays A;
     position_arrays(g, A);
     const int N = r.N;

@@ -242,6 +242,7 @@ struct bem_geom {
     bem_ctx* ctx = nullptr;  // creating context (not used after bem_geom_free starts)
     int device = 0;
     int N = 0, Nq = 0, nv = 0, nt = 0, quad_order = 7;
+    double rmax = 0.0;     // largest |vertex|: bounds every quadrature point's
     bem::HostMesh mesh;
     bem::HostRWG rwg;
     bem::Quad quad;

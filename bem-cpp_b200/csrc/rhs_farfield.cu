@@ -14,6 +14,7 @@
 #include <mutex>
 #include <vector>
 
+#include "asm_device.cuh"
 #include "bem_internal.h"
 
 namespace bem {
@@ -445,12 +446,272 @@ __global__ void __launch_bounds__(256) farfield_tri_kernel(FFArgs a, DevTriAsm t
     ff_epilogue(a, o, d, r, acc);
 }
 
+// ------------------------------------------- far field from a band limit
+// On the circle rhat(t) = R^T x sin t + R^T z cos t of an orientation the
+// coefficient sums J(t), M(t) of a particle within rmax of the origin are
+// trigonometric polynomials to rounding: exp(-ik rhat.r) =
+// sum_n (-i)^n J_n(k rho) e^(in(t - phi)) with rho <= rmax (Jacobi-Anger), and
+// J_n(x) falls below 1e-17 a few tens of orders past n = x.  So the sums are
+// taken at 2 H equally spaced nodes of the whole circle, H that order, and
+// the ntheta directions of the Mueller matrix interpolate them exactly
+// (trigonometric interpolation at equispaced nodes: condition ~ log H).  For
+// a real k the node t + pi costs nothing: the phase is the conjugate one and
+// everything it multiplies is real or a coefficient, so E(t + pi) = conj E(t)
+// per triangle, and with P = sum alpha Re Eu + gamma Re E0, Q the same with
+// Im, the two nodes are P + iQ and P - iQ.  H phases per point instead of
+// ntheta: 47 instead of 181 at k rmax = 16, 18 at k rmax = 1.
+//
+// farfield_nodes_kernel is bound by the FP64 pipe: per (node pair, triangle)
+// Nq (23 for the sine and cosine, 10) + 96 operations.  Block: FN_PAIRS node
+// pairs x FN_LANES triangle lanes of one orientation, and every gridDim.z-th
+// chunk of FN_CHUNK triangles; the parts are added in order by
+// farfield_interp_kernel.
+constexpr int FN_PAIRS = 16, FN_LANES = 8, FN_CHUNK = 64;
+constexpr int FN_REC = 17;  // a triangle's 4 alpha and 12 gamma, padded: odd, so the lanes' records do not conflict
+
+template <int NQ>
+__global__ void __launch_bounds__(FN_PAIRS* FN_LANES, 3)
+farfield_nodes_kernel(FFArgs a, DevTriAsm ta, int nt, const double* __restrict__ coef, int H,
+                      double* __restrict__ nodes) {
+    extern __shared__ __align__(16) double sm[];
+    const int Nq = NQ > 0 ? NQ : a.Nq;
+    double2* s_p = (double2*)sm;                      // FN_CHUNK * Nq * 3: (x1, x2) (w, w u_x) (w u_y, w u_z)
+    double2* s_ag = s_p + FN_CHUNK * Nq * 3;          // FN_CHUNK * FN_REC: per column k alpha, gamma
+    const int o = blockIdx.y, tid = threadIdx.x, lane = tid % FN_LANES;
+    const int j = blockIdx.x * FN_PAIRS + tid / FN_LANES;  // node pair: t_j = pi j / H and t_j + pi
+    const int c0 = 2 * o, c1 = 2 * o + 1, N = a.N;
+    const double* R = a.RT + 9 * (size_t)o;
+    double st, ct;
+    sincospi((double)j / H, &st, &ct);
+    st *= a.kr, ct *= a.kr;
+    double P[12][2], Q[12][2];
+#pragma unroll
+    for (int i = 0; i < 12; i++) P[i][0] = P[i][1] = Q[i][0] = Q[i][1] = 0.0;
+    for (int t0 = blockIdx.z * FN_CHUNK; t0 < nt; t0 += gridDim.z * FN_CHUNK) {
+        const int cnt = min(FN_CHUNK, nt - t0);
+        __syncthreads();
+        for (int e = tid; e < cnt * Nq; e += FN_PAIRS * FN_LANES) {
+            const size_t src = (size_t)t0 * Nq + e;
+            const double* c = ta.c + 3 * (size_t)(t0 + e / Nq);
+            const double ux = ta.u[src * 3], uy = ta.u[src * 3 + 1], uz = ta.u[src * 3 + 2], w = ta.jw[src];
+            // R^T x . r and R^T z . r, the centroid's part first
+            const double x1 = (R[0] * c[0] + R[3] * c[1] + R[6] * c[2]) + (R[0] * ux + R[3] * uy + R[6] * uz);
+            const double x2 = (R[2] * c[0] + R[5] * c[1] + R[8] * c[2]) + (R[2] * ux + R[5] * uy + R[8] * uz);
+            s_p[3 * e] = make_double2(x1, x2);
+            s_p[3 * e + 1] = make_double2(w, w * ux);
+            s_p[3 * e + 2] = make_double2(w * uy, w * uz);
+        }
+        for (int e = tid; e < cnt * 4; e += FN_PAIRS * FN_LANES) {
+            const int tt = e / 4, k = e % 4;  // k: J0 M0 J1 M1
+            const double2* src = ((k & 1) ? a.cM : a.cJ) + (int64_t)(k < 2 ? c0 : c1) * a.cs;
+            double2 al = make_double2(0, 0), ga[3] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
+            for (int h = 0; h < 3; h++) {
+                const int hn = ta.tri_half[(size_t)(t0 + tt) * 3 + h];
+                if (hn < 0) break;
+                const double2 cc = src[hn >= N ? hn - N : hn];
+                const double sg = coef[hn];
+                al.x += cc.x * sg, al.y += cc.y * sg;
+                for (int x = 0; x < 3; x++) {
+                    const double sp = sg * ta.pi[(size_t)hn * 3 + x];
+                    ga[x].x -= cc.x * sp, ga[x].y -= cc.y * sp;
+                }
+            }
+            double2* rec = s_ag + tt * FN_REC + 4 * k;
+            rec[0] = al;
+            for (int x = 0; x < 3; x++) rec[1 + x] = ga[x];
+        }
+        __syncthreads();
+        for (int tt = lane; tt < cnt; tt += FN_LANES) {
+            double E0r = 0, E0i = 0, Eu[3][2] = {{0, 0}, {0, 0}, {0, 0}};
+            const double2* pt = s_p + (size_t)tt * Nq * 3;
+#pragma unroll
+            for (int q = 0; q < Nq; q++) {
+                const double2 x = pt[3 * q], wx = pt[3 * q + 1], yz = pt[3 * q + 2];
+                double sn, cs;
+                sincos_bounded(st * x.x + ct * x.y, &sn, &cs);
+                // exp(-i k rhat.r) = cs - i sn
+                E0r += cs * wx.x, E0i -= sn * wx.x;
+                Eu[0][0] += cs * wx.y, Eu[0][1] -= sn * wx.y;
+                Eu[1][0] += cs * yz.x, Eu[1][1] -= sn * yz.x;
+                Eu[2][0] += cs * yz.y, Eu[2][1] -= sn * yz.y;
+            }
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const double2 *rec = s_ag + tt * FN_REC + 4 * k, al = rec[0];
+#pragma unroll
+                for (int x = 0; x < 3; x++) {
+                    const double2 ga = rec[1 + x];
+                    P[3 * k + x][0] += al.x * Eu[x][0] + ga.x * E0r;
+                    P[3 * k + x][1] += al.y * Eu[x][0] + ga.y * E0r;
+                    Q[3 * k + x][0] += al.x * Eu[x][1] + ga.x * E0i;
+                    Q[3 * k + x][1] += al.y * Eu[x][1] + ga.y * E0i;
+                }
+            }
+        }
+    }
+    // the lanes of a node pair are neighbours in a warp
+#pragma unroll
+    for (int i = 0; i < 12; i++)
+#pragma unroll
+        for (int c = 0; c < 2; c++)
+            for (int off = FN_LANES / 2; off > 0; off >>= 1) {
+                P[i][c] += __shfl_down_sync(0xffffffffu, P[i][c], off);
+                Q[i][c] += __shfl_down_sync(0xffffffffu, Q[i][c], off);
+            }
+    if (lane != 0 || j >= H) return;
+    double* out = nodes + (((size_t)blockIdx.z * a.n_orient + o) * 2 * H + j) * 24;
+#pragma unroll
+    for (int i = 0; i < 12; i++) {
+        out[2 * i] = P[i][0] - Q[i][1];
+        out[2 * i + 1] = P[i][1] + Q[i][0];
+        out[(size_t)H * 24 + 2 * i] = P[i][0] + Q[i][1];
+        out[(size_t)H * 24 + 2 * i + 1] = P[i][1] - Q[i][0];
+    }
+}
+
+// W[j][d] of the trigonometric interpolation from the 2 H nodes t_j = pi j / H
+// to t_d = pi d / (ndir - 1): sin(H x) cot(x / 2) / (2 H) with x = t_d - t_j =
+// pi m / (H (ndir - 1)), m an integer, so both arguments reduce exactly
+// (2 H (ndir - 1) < 2^31: H is at most ndir and its sums fit shared memory).
+__global__ void ff_weights_kernel(int H, int ndir, double* __restrict__ W) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= 2 * H * ndir) return;
+    const int j = i / ndir, d = i % ndir, nd = ndir - 1;
+    // x modulo 2 pi in (-pi, pi], and sin(H x) = sin(pi m / nd) from the
+    // fraction nearest to its zeros: quotients near 0 keep their relative accuracy
+    const int per = 2 * H * nd;
+    int m = (int)(((long long)d * H - (long long)j * nd) % per);
+    if (m > per / 2) m -= per;
+    if (m <= -per / 2) m += per;
+    double w = 1.0;
+    if (m != 0) {
+        double s, c;
+        sincospi((double)m / (double)per, &s, &c);  // x / 2
+        int k = m % (2 * nd);
+        if (k > nd) k -= 2 * nd;
+        if (k < -nd) k += 2 * nd;
+        if (2 * k > nd) k = nd - k;
+        if (2 * k < -nd) k = -nd - k;
+        w = sinpi((double)k / nd) * c / (s * 2.0 * H);
+    }
+    W[i] = w;
+}
+
+// Thread: one direction of the orientation blockIdx.x; the node sums (all
+// parts, in order) in shared memory.
+__global__ void __launch_bounds__(192) farfield_interp_kernel(FFArgs a, const double* __restrict__ nodes, int parts,
+                                                              int H, const double* __restrict__ W) {
+    extern __shared__ __align__(16) double sm[];  // 2 H x 24
+    const int o = blockIdx.x, cnt = 2 * H * 24;
+    for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
+        double s = 0.0;
+        for (int z = 0; z < parts; z++) s += nodes[((size_t)z * a.n_orient + o) * cnt + e];
+        sm[e] = s;
+    }
+    __syncthreads();
+    const int d = blockIdx.y * blockDim.x + threadIdx.x;
+    if (d >= a.ndir) return;
+    double acc[12][2];
+#pragma unroll
+    for (int i = 0; i < 12; i++) acc[i][0] = acc[i][1] = 0.0;
+    for (int j = 0; j < 2 * H; j++) {
+        const double w = W[(size_t)j * a.ndir + d];
+        const double2* v = (const double2*)(sm + (size_t)j * 24);
+#pragma unroll
+        for (int i = 0; i < 12; i++) {
+            const double2 x = v[i];
+            acc[i][0] += w * x.x, acc[i][1] += w * x.y;
+        }
+    }
+    double st, ct, r[3];
+    sincos(theta_of(a, d), &st, &ct);
+    const double* R = a.RT + 9 * (size_t)o;
+    for (int i = 0; i < 3; i++) r[i] = R[3 * i] * st + R[3 * i + 2] * ct;
+    ff_epilogue(a, o, d, r, acc);
+}
+
+// Node pairs for the band limit: one past the first order n > x at which
+// J_n(x) <= exp(n (tanh b - b)) / sqrt(2 pi n tanh b), cosh b = n / x (Debye),
+// is below 1e-17.  0: more than `limit`.
+static int ff_node_pairs(double x, int limit) {
+    x = std::max(x, 1e-3);
+    for (int n = (int)x + 2; n < limit; n++) {
+        const double b = std::acosh(n / x), t = std::tanh(b);
+        if (std::exp(n * (t - b)) < 1e-17 * std::sqrt(2.0 * M_PI * n * t)) return n + 1;
+    }
+    return 0;
+}
+
+// Plan of the band-limited far field of a call, H = 0 where the direct kernel
+// takes it: a complex k (no conjugate nodes), directions of the caller,
+// arguments beyond the sine's range, or so few directions that H node pairs
+// and the interpolation cost more (operations per direction: Nq 33 + 96 per
+// triangle either way; per node pair and direction 48 of interpolation).
+// RT (host) need not be orthonormal: |rhat(t).r| <= smax |r| with smax the
+// largest singular value of (R^T x, R^T z).
+struct FFPlan {
+    int H = 0, parts = 1;
+    size_t node_bytes = 0, weight_bytes = 0;
+};
+static FFPlan plan_ff(const bem_ctx* ctx, const bem_geom* g, const double* RT, int n_orient, int ndir, double k_re,
+                      double k_im) {
+    FFPlan p;
+    if (ctx->ff_kernel != 0 || k_im != 0.0 || ndir < 8 || g->Nq > FF_MAXQ) return p;
+    double s2 = 0.0;
+    for (int o = 0; o < n_orient; o++) {
+        const double* R = RT + 9 * (size_t)o;
+        double aa = 0, bb = 0, ab = 0;
+        for (int i = 0; i < 3; i++)
+            aa += R[3 * i] * R[3 * i], bb += R[3 * i + 2] * R[3 * i + 2], ab += R[3 * i] * R[3 * i + 2];
+        s2 = std::max(s2, 0.5 * (aa + bb) + std::sqrt(0.25 * (aa - bb) * (aa - bb) + ab * ab));
+    }
+    const double x = std::fabs(k_re) * g->rmax * std::sqrt(s2);
+    if (!(x < SINCOS_MAX)) return p;
+    const int H = ff_node_pairs(x, ndir);
+    const double per_dir = (g->Nq * 33.0 + 96.0) * g->nt;
+    // the interpolation's shared memory bounds H as well
+    if (H < 1 || H * (per_dir + 48.0 * ndir) > per_dir * ndir || (size_t)2 * H * 24 * 8 > 200 * 1024) return p;
+    p.H = H;
+    const int chunks = (H + FN_PAIRS - 1) / FN_PAIRS, tchunks = (g->nt + FN_CHUNK - 1) / FN_CHUNK;
+    // three blocks of 128 threads fit an SM: enough parts for about four waves
+    const int64_t want = 12LL * ctx->sm_count, have = (int64_t)chunks * n_orient;
+    p.parts = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(tchunks, 64), (want + have - 1) / have));
+    p.node_bytes = (size_t)p.parts * n_orient * 2 * H * 24 * 8;
+    p.weight_bytes = (size_t)2 * H * ndir * 8;
+    return p;
+}
+
+static int launch_ff_nodes(bem_ctx* ctx, const bem_geom* g, const FFArgs& a, const FFPlan& p, double* nodes,
+                           double* weights) {
+    cudaEvent_t ev = ctx->prof_begin(PROF_FARFIELD);
+    ff_weights_kernel<<<(2 * p.H * a.ndir + 255) / 256, 256, 0, ctx->stream>>>(p.H, a.ndir, weights);
+    BEM_LAUNCHED(ctx);
+    auto kern = g->Nq == 7 ? farfield_nodes_kernel<7> : g->Nq == 4 ? farfield_nodes_kernel<4> : farfield_nodes_kernel<0>;
+    const size_t smem = (size_t)FN_CHUNK * (g->Nq * 3 + FN_REC) * 16;
+    BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<dim3((p.H + FN_PAIRS - 1) / FN_PAIRS, a.n_orient, p.parts), FN_PAIRS * FN_LANES, smem, ctx->stream>>>(
+        a, g->tri, g->nt, g->sing_coef, p.H, nodes);
+    BEM_LAUNCHED(ctx);
+    const size_t ismem = (size_t)2 * p.H * 24 * 8;
+    BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(farfield_interp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)ismem));
+    farfield_interp_kernel<<<dim3(a.n_orient, (a.ndir + 191) / 192), 192, ismem, ctx->stream>>>(a, nodes, p.parts, p.H,
+                                                                                             weights);
+    BEM_LAUNCHED(ctx);
+    // the unit of launch_ff: (orientation, direction, point) terms
+    if (ev)
+        ctx->prof_end(PROF_FARFIELD, ev, 110.0 * a.n_orient * (double)a.ndir * 2.0 * a.N * a.Nq,
+                      (double)a.n_orient * a.ndir * 16 * 8);
+    return BEM_OK;
+}
+
 // M_avg[i*ndir + d] = sum over o in order of Mo[o][i][d]
 __global__ void mueller_sum_kernel(const double* __restrict__ Mo, int n_orient, int nel,
                                    double* __restrict__ out) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nel) return;
     double s = 0.0;
+#pragma unroll 8
     for (int o = 0; o < n_orient; o++) s += Mo[(size_t)o * nel + i];
     out[i] = s;
 }
@@ -530,8 +791,15 @@ int mueller_dev(bem_ctx* ctx, const bem_geom* g, const void* X, int64_t ldx, con
            fvb = Fv_host ? (size_t)2 * n_orient * ntheta * 3 * 16 : 0;
     size_t off = 0;
     auto take = [&](size_t b) { size_t o = off; off += (b + 255) & ~(size_t)255; return o; };
+    FFPlan plan = plan_ff(ctx, g, RT, n_orient, ntheta, k_re, k_im);
     size_t oRT = take(rtb), oW = take(wb), oT = take(tb), oMo = take(mob), oMa = take(mab), oFv = take(fvb);
-    BEM_TRY(ctx->ensure_ws(off));
+    const size_t direct = off;
+    size_t oNd = take(plan.node_bytes), oWt = take(plan.weight_bytes);
+    if (ctx->ensure_ws(off) != BEM_OK) {
+        if (plan.H == 0) return BEM_ERR_OOM;
+        plan = FFPlan{};  // without room for the node sums: every direction on its own
+        BEM_TRY(ctx->ensure_ws(direct));
+    }
     char* ws = (char*)ctx->ws;
     std::vector<double> th(ntheta);
     for (int i = 0; i < ntheta; i++) th[i] = ntheta > 1 ? M_PI * i / (ntheta - 1) : 0.0;
@@ -557,9 +825,12 @@ int mueller_dev(bem_ctx* ctx, const bem_geom* g, const void* X, int64_t ldx, con
     a.Mo = M_orient_dev ? M_orient_dev : (double*)(ws + oMo);
     a.gamma_mirror = gamma_mirror;
     a.Fv = Fv_host ? (double2*)(ws + oFv) : nullptr;
-    BEM_TRY(launch_ff(ctx, g, a));
+    if (plan.H > 0)
+        BEM_TRY(launch_ff_nodes(ctx, g, a, plan, (double*)(ws + oNd), (double*)(ws + oWt)));
+    else
+        BEM_TRY(launch_ff(ctx, g, a));
     int nel = 16 * ntheta;
-    mueller_sum_kernel<<<(nel + 255) / 256, 256, 0, ctx->stream>>>(a.Mo, n_orient, nel, (double*)(ws + oMa));
+    mueller_sum_kernel<<<(nel + 63) / 64, 64, 0, ctx->stream>>>(a.Mo, n_orient, nel, (double*)(ws + oMa));
     BEM_LAUNCHED(ctx);
     BEM_TRY_CUDA(ctx, cudaMemcpyAsync(M_avg, ws + oMa, mab, cudaMemcpyDeviceToHost, ctx->stream));
     if (Fv_host) BEM_TRY_CUDA(ctx, cudaMemcpyAsync(Fv_host, ws + oFv, fvb, cudaMemcpyDeviceToHost, ctx->stream));
@@ -630,7 +901,7 @@ int mueller_noalloc(bem_ctx* ctx, const bem_geom* g, const void* X, int64_t ldx,
     a.gamma_mirror = gamma_mirror;
     BEM_TRY(launch_ff(ctx, g, a));
     int nel = 16 * ntheta;
-    mueller_sum_kernel<<<(nel + 255) / 256, 256, 0, ctx->stream>>>(d_Mo, n_orient, nel, M_out_dev);
+    mueller_sum_kernel<<<(nel + 63) / 64, 64, 0, ctx->stream>>>(d_Mo, n_orient, nel, M_out_dev);
     BEM_LAUNCHED(ctx);
     return BEM_OK;
 }
