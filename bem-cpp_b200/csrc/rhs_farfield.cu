@@ -22,7 +22,8 @@ namespace bem {
 #define INV4PI_FF 0.079577471545947667884
 
 struct RhsArgs {
-    DevHalf h;
+    DevTriAsm ta;
+    const double* coef;  // 2N: sign l / (2A) of a half
     int N, Nq, n_orient;
     double kr, ki, eta;
     const double* RT;  // n_orient * 9, row-major R^T
@@ -31,64 +32,121 @@ struct RhsArgs {
     int64_t ldb;
 };
 
-// One thread per (RWG n, orientation o): both polarisations.
-__global__ void rhs_kernel(RhsArgs a) {
-    int n = blockIdx.x * blockDim.x + threadIdx.x;
-    int o = blockIdx.y;
-    if (n >= a.N || o >= a.n_orient) return;
-    double kh[3], ep[3][3];
-    int npol;
-    if (a.E0) {
-        // explicit single wave: E0 = a.E0[0..2], k_hat = a.E0[3..5]
-        npol = 1;
-        for (int i = 0; i < 3; i++) ep[0][i] = a.E0[i], kh[i] = a.E0[3 + i];
-    } else {
-        npol = 2;
-        const double* R = a.RT + 9 * o;
-        for (int i = 0; i < 3; i++) {
-            kh[i] = R[3 * i + 2];
-            ep[0][i] = R[3 * i + 0];  // R^T x
-            ep[1][i] = R[3 * i + 1];  // R^T y
+// Both polarisations of RHS_ORI orientations at a time for the 16 RWGs of an
+// assembly tile, by triangles: the phase at a quadrature point is shared by
+// the RWG halves of its triangle, f_h = s_h (u - pi_h), so the tile's ~16
+// triangles are taken once per orientation (thread: triangle and
+// orientation; E0 = sum ph w, Eu = sum ph w u into shared memory) and each RWG
+// then adds s_h (Eu.e - (pi_h.e) E0) of its two halves for the four field
+// vectors e (thread: RWG and orientation).  2 x fewer exponentials than per
+// RWG half, and the fields are dotted once per half instead of per point.
+// Bound by the FP64 pipe; the output is 4 x 16 B per (RWG, orientation).
+// GENERAL: complex k or arguments beyond sincos_bounded (library functions).
+constexpr int RHS_ORI = 16, RHS_THREADS = 288;  // 18 triangles x 16 orientations a pass
+constexpr int RHS_FLD = 15;                     // k_hat and (E, H) of two polarisations
+constexpr int RHS_E = 9;                        // E0, Eu of an orientation: 8, padded to an odd pitch
+constexpr int RHS_TRI = RHS_ORI * RHS_E + 1;    // a triangle's, odd as well: the RWGs of a warp read without conflicts
+template <bool GENERAL, int NQ>
+__global__ void __launch_bounds__(RHS_THREADS, 3) rhs_kernel(RhsArgs a) {
+    extern __shared__ __align__(16) double sm[];
+    const int tile = blockIdx.x, tid = threadIdx.x, Nq = NQ > 0 ? NQ : a.Nq, N = a.N;
+    const int ntri = a.ta.tile_ntri[tile], npol = a.E0 ? 1 : 2;
+    double* s_pt = sm;                                  // ntri x Nq x 4: u, w
+    double* s_c = s_pt + ASM_TRI_MAX * Nq * 4;          // ntri x 3
+    double* s_f = s_c + ASM_TRI_MAX * 3;                // RHS_ORI x RHS_FLD
+    double* s_E = s_f + RHS_ORI * RHS_FLD;              // ntri x RHS_TRI
+    __shared__ int s_loc[ASM_TILE * 2];
+    for (int e = tid; e < ntri * Nq; e += RHS_THREADS) {
+        const size_t src = (size_t)a.ta.tile_tri[(size_t)tile * ASM_TRI_MAX + e / Nq] * Nq + e % Nq;
+        for (int x = 0; x < 3; x++) s_pt[4 * e + x] = a.ta.u[src * 3 + x];
+        s_pt[4 * e + 3] = a.ta.jw[src];
+    }
+    for (int e = tid; e < ntri * 3; e += RHS_THREADS) {
+        s_c[e] = a.ta.c[(size_t)a.ta.tile_tri[(size_t)tile * ASM_TRI_MAX + e / 3] * 3 + e % 3];
+        const int ent = a.ta.tile_ent[(size_t)tile * ASM_TRI_MAX * 3 + e];
+        if (ent != 0xff) s_loc[ent] = e / 3;
+    }
+    // the RWG of this thread in the second phase (RHS_THREADS is a multiple of ASM_TILE)
+    static_assert(RHS_THREADS % ASM_TILE == 0, "a thread keeps its RWG");
+    const int sl = tid % ASM_TILE, n = a.ta.tile_rwg[(size_t)tile * ASM_TILE + sl];
+    double sg[2] = {0, 0}, pi[2][3] = {{0, 0, 0}, {0, 0, 0}};
+    if (n >= 0)
+        for (int h = 0; h < 2; h++) {
+            sg[h] = a.coef[h * N + n];
+            for (int i = 0; i < 3; i++) pi[h][i] = a.ta.pi[3 * (size_t)(h * N + n) + i];
         }
-    }
-    double H[2][3];
-    for (int p = 0; p < npol; p++) {
-        // H0 = k_hat x E0 / eta
-        H[p][0] = (kh[1] * ep[p][2] - kh[2] * ep[p][1]) * (1.0 / a.eta);
-        H[p][1] = (kh[2] * ep[p][0] - kh[0] * ep[p][2]) * (1.0 / a.eta);
-        H[p][2] = (kh[0] * ep[p][1] - kh[1] * ep[p][0]) * (1.0 / a.eta);
-    }
-    double bE[2][2] = {{0, 0}, {0, 0}}, bH[2][2] = {{0, 0}, {0, 0}};
-    for (int h = 0; h < 2; h++) {
-        double sE[2][2] = {{0, 0}, {0, 0}}, sH[2][2] = {{0, 0}, {0, 0}};
-        for (int q = 0; q < a.Nq; q++) {
-            size_t i = ((size_t)(h * a.N + n)) * a.Nq + q;
-            double px = a.h.px[i], py = a.h.py[i], pz = a.h.pz[i];
-            double fx = a.h.fx[i], fy = a.h.fy[i], fz = a.h.fz[i];
-            double jw = a.h.jw[i];
-            double s = kh[0] * px + kh[1] * py + kh[2] * pz;
-            double sn, cs;
-            sincos(a.kr * s, &sn, &cs);
-            double ea = exp(-a.ki * s);
-            double phr = ea * cs, phi = ea * sn;
-            for (int p = 0; p < npol; p++) {
-                double fe = fx * ep[p][0] + fy * ep[p][1] + fz * ep[p][2];
-                double fh = fx * H[p][0] + fy * H[p][1] + fz * H[p][2];
-                sE[p][0] += fe * phr * jw;
-                sE[p][1] += fe * phi * jw;
-                sH[p][0] += fh * phr * jw;
-                sH[p][1] += fh * phi * jw;
+    const double ieta = 1.0 / a.eta;
+    for (int g0 = blockIdx.y * RHS_ORI; g0 < a.n_orient; g0 += gridDim.y * RHS_ORI) {
+        const int go = min(RHS_ORI, a.n_orient - g0);
+        __syncthreads();
+        if (tid < go) {
+            double* f = s_f + tid * RHS_FLD;
+            const double* R = a.E0 ? nullptr : a.RT + 9 * (size_t)(g0 + tid);
+            double kh[3];
+            for (int i = 0; i < 3; i++) f[i] = kh[i] = a.E0 ? a.E0[3 + i] : R[3 * i + 2];
+            for (int p = 0; p < 2; p++) {
+                double* e = f + 3 + 6 * p;
+                for (int i = 0; i < 3; i++) e[i] = a.E0 ? a.E0[i] : R[3 * i + p];  // R^T x, R^T y
+                // H0 = k_hat x E0 / eta
+                e[3] = (kh[1] * e[2] - kh[2] * e[1]) * ieta;
+                e[4] = (kh[2] * e[0] - kh[0] * e[2]) * ieta;
+                e[5] = (kh[0] * e[1] - kh[1] * e[0]) * ieta;
             }
         }
-        for (int p = 0; p < npol; p++) {
-            bE[p][0] += sE[p][0], bE[p][1] += sE[p][1];
-            bH[p][0] += sH[p][0], bH[p][1] += sH[p][1];
+        __syncthreads();
+        for (int it = tid; it < ntri * RHS_ORI; it += RHS_THREADS) {
+            const int li = it / RHS_ORI, ol = it % RHS_ORI;
+            if (ol >= go) continue;
+            const double* kh = s_f + ol * RHS_FLD;
+            const double kx = kh[0], ky = kh[1], kz = kh[2];
+            const double* c = s_c + 3 * li;
+            const double sc = kx * c[0] + ky * c[1] + kz * c[2];
+            double E[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+            for (int q = 0; q < Nq; q++) {
+                const double2 uxy = *(const double2*)(s_pt + 4 * (li * Nq + q)),
+                              uzw = *(const double2*)(s_pt + 4 * (li * Nq + q) + 2);
+                const double sq = sc + (kx * uxy.x + ky * uxy.y + kz * uzw.x);
+                double sn, cs;
+                if constexpr (GENERAL) {
+                    sincos(a.kr * sq, &sn, &cs);
+                    const double ea = exp(-a.ki * sq);
+                    sn *= ea, cs *= ea;
+                } else {
+                    sincos_bounded(a.kr * sq, &sn, &cs);
+                }
+                const double pr = cs * uzw.y, pm = sn * uzw.y;
+                E[0] += pr, E[1] += pm;
+                E[2] += pr * uxy.x, E[3] += pm * uxy.x;
+                E[4] += pr * uxy.y, E[5] += pm * uxy.y;
+                E[6] += pr * uzw.x, E[7] += pm * uzw.x;
+            }
+            for (int i = 0; i < 8; i++) s_E[li * RHS_TRI + ol * RHS_E + i] = E[i];
         }
-    }
-    for (int p = 0; p < npol; p++) {
-        double2* col = a.B + (int64_t)(npol * o + p) * a.ldb;
-        col[n] = make_double2(bE[p][0], bE[p][1]);
-        col[a.N + n] = make_double2(bH[p][0], bH[p][1]);
+        __syncthreads();
+        if (n < 0) continue;
+        for (int ol = tid / ASM_TILE; ol < go; ol += RHS_THREADS / ASM_TILE) {
+            const double* f = s_f + ol * RHS_FLD + 3;
+            const double *Ep = s_E + s_loc[2 * sl] * RHS_TRI + ol * RHS_E,
+                         *Em = s_E + s_loc[2 * sl + 1] * RHS_TRI + ol * RHS_E;
+#pragma unroll
+            for (int p = 0; p < 2; p++) {
+                if (p >= npol) break;
+                double2* col = a.B + (int64_t)(npol * (g0 + ol) + p) * a.ldb;
+#pragma unroll
+                for (int k = 0; k < 2; k++) {
+                    const double* v = f + 6 * p + 3 * k;
+                    const double pp = pi[0][0] * v[0] + pi[0][1] * v[1] + pi[0][2] * v[2];
+                    const double pm = pi[1][0] * v[0] + pi[1][1] * v[1] + pi[1][2] * v[2];
+                    double2 out;
+                    out.x = sg[0] * ((Ep[2] * v[0] + Ep[4] * v[1] + Ep[6] * v[2]) - pp * Ep[0]) +
+                            sg[1] * ((Em[2] * v[0] + Em[4] * v[1] + Em[6] * v[2]) - pm * Em[0]);
+                    out.y = sg[0] * ((Ep[3] * v[0] + Ep[5] * v[1] + Ep[7] * v[2]) - pp * Ep[1]) +
+                            sg[1] * ((Em[3] * v[0] + Em[5] * v[1] + Em[7] * v[2]) - pm * Em[1]);
+                    col[(int64_t)k * N + n] = out;
+                }
+            }
+        }
     }
 }
 
@@ -108,7 +166,8 @@ int rhs_dev(bem_ctx* ctx, const bem_geom* g, double k_re, double k_im, double et
     }
     BEM_TRY_CUDA(ctx, cudaMemcpyAsync(ctx->ws, src, bytes, cudaMemcpyHostToDevice, ctx->stream));
     RhsArgs a;
-    a.h = g->half;
+    a.ta = g->tri;
+    a.coef = g->sing_coef;
     a.N = g->N;
     a.Nq = g->Nq;
     a.n_orient = RT_host ? n_orient : 1;
@@ -119,8 +178,24 @@ int rhs_dev(bem_ctx* ctx, const bem_geom* g, double k_re, double k_im, double et
     a.E0 = RT_host ? nullptr : (const double*)ctx->ws;
     a.B = (double2*)B;
     a.ldb = ldb;
-    dim3 grid((g->N + 127) / 128, a.n_orient);
-    rhs_kernel<<<grid, 128, 0, ctx->stream>>>(a);
+    // the largest |k_hat| of the call bounds the phases k k_hat.r
+    double kh2 = 0.0;
+    for (int o = 0; o < a.n_orient; o++) {
+        double h2 = 0.0;
+        for (int i = 0; i < 3; i++) {
+            const double v = RT_host ? RT_host[9 * (size_t)o + 3 * i + 2] : khat_host[i];
+            h2 += v * v;
+        }
+        kh2 = std::max(kh2, h2);
+    }
+    const bool general = k_im != 0.0 || !(std::fabs(k_re) * g->rmax * std::sqrt(kh2) < SINCOS_MAX);
+    // about four waves of blocks (two a SM), each taking several groups of orientations
+    const int groups = (a.n_orient + RHS_ORI - 1) / RHS_ORI;
+    const int gy = std::max(1, std::min(groups, (int)((8LL * ctx->sm_count + g->tri.ntile - 1) / g->tri.ntile)));
+    const size_t smem = ((size_t)ASM_TRI_MAX * (g->Nq * 4 + 3) + RHS_ORI * RHS_FLD + (size_t)ASM_TRI_MAX * RHS_TRI) * 8;
+    auto kern = general ? rhs_kernel<true, 0> : g->Nq == 7 ? rhs_kernel<false, 7> : g->Nq == 4 ? rhs_kernel<false, 4> : rhs_kernel<false, 0>;
+    BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<dim3(g->tri.ntile, gy), RHS_THREADS, smem, ctx->stream>>>(a);
     BEM_LAUNCHED(ctx);
     // the workspace is reused by later calls: finish before returning
     BEM_TRY_CUDA(ctx, cudaStreamSynchronize(ctx->stream));

@@ -1,8 +1,9 @@
-"""Band-limited far field on the device, against the direct form."""
+"""Band-limited far field and by-triangle right-hand sides on the device, against the direct forms."""
 import numpy as np
 import pytest
 
 from conftest import rel
+from oracle import bem_oracle as bo
 
 pytestmark = pytest.mark.gpu
 
@@ -56,3 +57,17 @@ def test_complex_wavenumber_and_few_directions_match_oracle(ctx):
         D = bb.mueller_from_solutions_dev(g, X, RT, w, k, 1.0, ntheta=nth)
         bb.set_option(ctx, "farfield_kernel", 0)
         assert rel(M, D) < 1e-13
+
+
+# one orientation, one short of, exactly and one over a group of 16, several groups; every rule; a complex k
+@pytest.mark.parametrize("mesh,q,no,k", [("ico", 7, 1, 2.0), ("ico", 4, 15, 2.0), ("hex", 13, 16, 3.0), ("ico", 7, 17, 0.01),
+                                         ("hex", 7, 50, 5.0), ("ico", 7, 3, 2.0 + 0.3j)])
+def test_plane_waves_by_triangles_match_oracle(ctx, mesh, q, no, k):
+    import bem_b200 as bb
+    v, t = bb.icosphere(1.0, 2) if mesh == "ico" else bb.hex_prism(0.7, 1)
+    g = bb.Geometry(ctx, v, t, q)
+    RT = _rotations(no, no)
+    B = bb.rhs_planewave_dev(g, complex(k), 1.2, RT).cpu().numpy().T
+    tt = t.astype(np.int64)
+    Bo = bo.orientation_rhs(bo.build_rwg(v, tt, "cpp"), v, tt, [(r, 1.0) for r in RT], complex(k), 1.2, q)
+    assert rel(B, Bo) < 1e-13
