@@ -66,6 +66,42 @@ __device__ __forceinline__ void sincos_bounded(double x, double* sn, double* cs)
 // place of e^-x there would become 0.0156 in G.
 __device__ __forceinline__ double exp_decay(double x) { return x < 5.551115123125783e-17 ? 1.0 : exp(-x); }
 
+// e^-x without a branch, x clamped to [0, 708] (e^-0 = 1 exactly; below e^-708
+// the value does not count): x = -(n ln 2 + r), |r| <= ln 2 / 2, in two fused
+// steps, the Taylor polynomial of degree 13 (first omitted term below 5e-18)
+// and 2^n added to the exponent.
+__device__ __forceinline__ double exp_decay_bounded(double x) {
+    x = fmin(fmax(x, 0.0), 708.0);
+    const double shift = 6755399441055744.0;
+    const double t = __fma_rn(x, -1.4426950408889634074, shift);
+    const double fn = t - shift;
+    double r = __fma_rn(fn, -0.69314718055994530942, -x);
+    r = __fma_rn(fn, -2.3190468138462995585e-17, r);
+    double p = __fma_rn(r, 1.0 / 6227020800.0, 1.0 / 479001600.0);
+    p = __fma_rn(r, p, 1.0 / 39916800.0);
+    p = __fma_rn(r, p, 1.0 / 3628800.0);
+    p = __fma_rn(r, p, 1.0 / 362880.0);
+    p = __fma_rn(r, p, 1.0 / 40320.0);
+    p = __fma_rn(r, p, 1.0 / 5040.0);
+    p = __fma_rn(r, p, 1.0 / 720.0);
+    p = __fma_rn(r, p, 1.0 / 120.0);
+    p = __fma_rn(r, p, 1.0 / 24.0);
+    p = __fma_rn(r, p, 1.0 / 6.0);
+    p = __fma_rn(r, p, 0.5);
+    p = __fma_rn(r, p, 1.0);
+    p = __fma_rn(r, p, 1.0);
+    return __hiloint2double(__double2hiint(p) + (int)((unsigned)__double2loint(t) << 20), __double2loint(p));
+}
+
+// 1 / sqrt(x) for a normal x > 0: the hardware's approximation (about 2^-20)
+// and one cubically convergent step, y (1 + e / 2 + 3 e^2 / 8) with e = 1 - x y^2.
+__device__ __forceinline__ double rsqrt_normal(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = __fma_rn(-x * y, y, 1.0);
+    return __fma_rn(y * e, __fma_rn(e, 0.375, 0.5), y);
+}
+
 // G_smooth = (exp(ikR) - 1)/(4 pi R) without cancellation (limit ik/(4 pi)).
 __device__ __forceinline__ cplx g_smooth_exact(Medium k, double R) {
     if (R == 0.0) return {-k.ki * INV4PI_D, k.kr * INV4PI_D};

@@ -566,20 +566,128 @@ __global__ void __launch_bounds__(256) assemble_kernel(AsmArgs a) {
 // f_n = s_n (v - nu_n):
 //   sum G f_m.f_n  = s_m s_n (Muv - pi.Mv - nu.Mu + pi.nu M0)
 //   sum g f_m.(d x f_n) = s_m s_n (P1 - nu.Q2 - pi.Q3 + pi.(Q4 x nu))
+// The quadrature sum over the points of b is formed first, sum_q G w_q (1, v)
+// and sum_q g w_q (1, v): four complex sums per point of a and kernel, from
+// which the moments take u once per point of a instead of once per pair of
+// points (16 multiply-adds per point pair and medium fewer).  One thread does
+// both media of a triangle pair: they share the distance and the K moments
+// (only K_e + K_i is needed).
 // Each (RWG pair, half pair) term lands in its own shared-memory slot and the
 // four half pairs of an entry are summed in a fixed order, so the result does
 // not depend on the tiling.  RWGs are tiled in the Morton order of their
-// triangles (geom_upload), ~17 distinct triangles per 16 RWGs: ~3.5x fewer
-// Green's function evaluations than per RWG pair.
-constexpr size_t tri_smem_bytes(int nmed) {
-    return (size_t)2 * nmed * 1024 * sizeof(double2) +
-           sizeof(double) * (2 * ASM_TRI_MAX * 3 + 2 * ASM_TRI_MAX * MAXQ * 3 + 2 * ASM_TRI_MAX * MAXQ +
-                             2 * TILE * 2 * 5) +
+// triangles (geom_upload), ~17 distinct triangles per 16 RWGs.
+//
+// Bound by the FP64 pipe, ~100 operations per point pair for two lossless
+// media, ~120 with one absorbing, which is 58 % busy: the 52 accumulators of a
+// thread leave room for two blocks of four warps an SM.  2N = 18432, one
+// medium absorbing: 28.6 ms, 64.3 ms before (moments per point pair and medium,
+// 17.1 triangles a tile).  Measured against it: three blocks at 168 registers
+// spill (45 ms), 96 or 160 threads 35 ms, the inner loop unrolled 7 times
+// 29.3 ms.  A tile pair's ~240 triangle pairs are two rounds of 128 threads.
+constexpr int ASM_THREADS = 128;
+// points of a triangle in shared memory: Nq x (u, weight), padded to an odd
+// number of 16-byte units so that the triangles of neighbouring lanes do not conflict
+__host__ __device__ constexpr int asm_pt_pitch(int Nq) { return 4 * Nq + 2; }
+constexpr size_t tri_smem_bytes(int Nq) {
+    return (size_t)256 * 4 * 3 * sizeof(double2) +
+           sizeof(double) * (2 * ASM_TRI_MAX * asm_pt_pitch(Nq) + 2 * ASM_TRI_MAX * 3 + 2 * TILE * 2 * 5) +
            sizeof(int) * (2 * ASM_TRI_MAX + 2) + 2 * ASM_TRI_MAX * 3;
 }
 
+__device__ __forceinline__ void cfma(cplx& a, cplx b, double s) { a.re += b.re * s, a.im += b.im * s; }
+
+// One medium's or the media's combined outputs of the half pairs of a
+// triangle pair, from the moments.  LM: L moments per medium (M0, Muv, Mu,
+// Mv); KM: K moments (S0, A, B, C); null LM[e].k: no K (the same triangle).
+struct LMoments {
+    cplx M0, Muv, Mu[3], Mv[3];
+};
+struct KMoments {
+    cplx S0, A[3], B[3], C[3];
+};
+
+// term(x, y) of the half pairs into their slots: (TL, BR, K) for Z, (L, K) for one operator.
 template <int NMED>
-__global__ void __launch_bounds__(256, 2) assemble_tri_kernel(AsmArgs a, DevTriAsm ta) {
+__device__ __forceinline__ void store_half_pairs(const AsmArgs& a, const LMoments* L, const KMoments& K, double Dx,
+                                                 double Dy, double Dz, const unsigned char* ea,
+                                                 const unsigned char* eb, const double* ssig, const double* sdiv,
+                                                 const double* spi, double2* slots) {
+    // scalar part: sum_e c_e (i / k_e) M0_e; vector part's factor c_e i k_e; c_e = eta_e (TL), 1 / eta_e (BR)
+    cplx s1 = {0, 0}, s2 = {0, 0}, v1[NMED], v2[NMED];
+#pragma unroll
+    for (int e = 0; e < NMED; e++) {
+        const Medium k = a.med[e];
+        const double c1 = a.Z ? (e ? a.eta_i : a.eta_e) : 1.0, c2 = 1.0 / c1, k2 = k.kr * k.kr + k.ki * k.ki;
+        const cplx t = cmul(cplx{k.ki / k2, k.kr / k2}, L[e].M0);
+        cfma(s1, t, c1), cfma(s2, t, c2);
+        v1[e] = {-k.ki * c1, k.kr * c1}, v2[e] = {-k.ki * c2, k.kr * c2};
+    }
+    // P1 = -D.C, Q2 = A x D - C, Q3 = D x B + C, Q4 = D S0 + A - B
+    const double DD[3] = {Dx, Dy, Dz};
+    cplx P1 = {0, 0}, Q2[3], Q3[3], Q4[3];
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+        const int j1 = (j + 1) % 3, j2 = (j + 2) % 3;
+        cfma(P1, K.C[j], -DD[j]);
+        Q2[j] = {K.A[j1].re * DD[j2] - K.A[j2].re * DD[j1] - K.C[j].re,
+                 K.A[j1].im * DD[j2] - K.A[j2].im * DD[j1] - K.C[j].im};
+        Q3[j] = {DD[j1] * K.B[j2].re - DD[j2] * K.B[j1].re + K.C[j].re,
+                 DD[j1] * K.B[j2].im - DD[j2] * K.B[j1].im + K.C[j].im};
+        Q4[j] = {DD[j] * K.S0.re + K.A[j].re - K.B[j].re, DD[j] * K.S0.im + K.A[j].im - K.B[j].im};
+    }
+    for (int x = 0; x < 3; x++) {
+        const int er = ea[x];
+        if (er == 0xff) break;
+        const int r = er >> 1;
+        const double sr = ssig[er], dr = sdiv[er];
+        const double p[3] = {spi[er * 3], spi[er * 3 + 1], spi[er * 3 + 2]};
+        // over the test half: Muv - p.Mv, Mu - p M0; P1 - p.Q3, Q2 - p x Q4
+        cplx qx[NMED], ux[NMED][3], kx = P1, wx[3];
+#pragma unroll
+        for (int e = 0; e < NMED; e++) {
+            qx[e] = L[e].Muv;
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                cfma(qx[e], L[e].Mv[j], -p[j]);
+                ux[e][j] = L[e].Mu[j];
+                cfma(ux[e][j], L[e].M0, -p[j]);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const int j1 = (j + 1) % 3, j2 = (j + 2) % 3;
+            cfma(kx, Q3[j], -p[j]);
+            wx[j] = {Q2[j].re - (p[j1] * Q4[j2].re - p[j2] * Q4[j1].re),
+                     Q2[j].im - (p[j1] * Q4[j2].im - p[j2] * Q4[j1].im)};
+        }
+        for (int y = 0; y < 3; y++) {
+            const int ec = eb[y];
+            if (ec == 0xff) break;
+            const int c = ec >> 1;
+            const double ss = sr * ssig[2 * TILE + ec], dd = dr * sdiv[2 * TILE + ec];
+            const double* nu = spi + (2 * TILE + ec) * 3;
+            cplx o1 = {0, 0}, o2 = {0, 0}, kv = kx;
+#pragma unroll
+            for (int e = 0; e < NMED; e++) {
+                cplx lv = qx[e];
+#pragma unroll
+                for (int j = 0; j < 3; j++) cfma(lv, ux[e][j], -nu[j]);
+                const cplx t1 = cmul(v1[e], lv), t2 = cmul(v2[e], lv);
+                o1.re += t1.re, o1.im += t1.im, o2.re += t2.re, o2.im += t2.im;
+            }
+#pragma unroll
+            for (int j = 0; j < 3; j++) cfma(kv, wx[j], -nu[j]);
+            double2* out = slots + ((r * TILE + c) * 4 + (er & 1) * 2 + (ec & 1)) * 3;
+            out[0] = make_double2(ss * o1.re - dd * s1.re, ss * o1.im - dd * s1.im);
+            out[1] = make_double2(ss * o2.re - dd * s2.re, ss * o2.im - dd * s2.im);
+            out[2] = make_double2(ss * kv.re, ss * kv.im);
+        }
+    }
+}
+
+// DAMP: bit e set when medium e absorbs (k_im != 0).  NQ: points of the rule (0: a.Nq).
+template <int NMED, int DAMP, int NQ>
+__global__ void __launch_bounds__(ASM_THREADS, 2) assemble_tri_kernel(AsmArgs a, DevTriAsm ta) {
     int64_t lin = blockIdx.x;
     const int T = a.ntile;
     int bi = (int)floor((2.0 * T + 1.0 - sqrt((2.0 * T + 1.0) * (2.0 * T + 1.0) - 8.0 * (double)lin)) * 0.5);
@@ -588,38 +696,36 @@ __global__ void __launch_bounds__(256, 2) assemble_tri_kernel(AsmArgs a, DevTriA
     while ((int64_t)(bi + 1) * T - (int64_t)(bi + 1) * bi / 2 <= lin) bi++;
     const int bj = bi + (int)(lin - ((int64_t)bi * T - (int64_t)bi * (bi - 1) / 2));
     if (a.tile_flag && !a.tile_flag[bi] && !a.tile_flag[bj]) return;  // a tile the caller keeps
-    const int N = a.N, Nq = a.Nq, tid = threadIdx.x;
+    const int N = a.N, Nq = NQ > 0 ? NQ : a.Nq, tid = threadIdx.x, pitch = asm_pt_pitch(Nq);
 
     extern __shared__ __align__(16) unsigned char tri_smem[];
-    double2* sL = reinterpret_cast<double2*>(tri_smem);  // [NMED][256 entries][4 half pairs]
-    double2* sK = sL + NMED * 1024;
-    double* sc = reinterpret_cast<double*>(sK + NMED * 1024);  // [2][TRI_MAX][3]
-    double* su = sc + 2 * ASM_TRI_MAX * 3;                      // [2][TRI_MAX][MAXQ][3]
-    double* sjw = su + 2 * ASM_TRI_MAX * MAXQ * 3;              // [2][TRI_MAX][MAXQ]
-    double* ssig = sjw + 2 * ASM_TRI_MAX * MAXQ;                // [2][TILE][2]
-    double* sdiv = ssig + 2 * TILE * 2;                         // [2][TILE][2]
-    double* spi = sdiv + 2 * TILE * 2;                          // [2][TILE][2][3]
-    int* stri = reinterpret_cast<int*>(spi + 2 * TILE * 2 * 3);  // [2][TRI_MAX]
-    int* sntri = stri + 2 * ASM_TRI_MAX;                         // [2]
-    unsigned char* sent = reinterpret_cast<unsigned char*>(sntri + 2);  // [2][TRI_MAX][3]
+    double2* slots = reinterpret_cast<double2*>(tri_smem);         // [256 entries][4 half pairs][3]
+    double* spt = reinterpret_cast<double*>(slots + 256 * 4 * 3);  // [2][TRI_MAX][pitch]: u, weight per point
+    double* sc = spt + 2 * ASM_TRI_MAX * pitch;                    // [2][TRI_MAX][3]
+    double* ssig = sc + 2 * ASM_TRI_MAX * 3;                       // [2][TILE][2]
+    double* sdiv = ssig + 2 * TILE * 2;                            // [2][TILE][2]
+    double* spi = sdiv + 2 * TILE * 2;                             // [2][TILE][2][3]
+    int* stri = reinterpret_cast<int*>(spi + 2 * TILE * 2 * 3);    // [2][TRI_MAX]
+    unsigned char* sent = reinterpret_cast<unsigned char*>(stri + 2 * ASM_TRI_MAX);  // [2][TRI_MAX][3]
 
-    for (int i = tid; i < 2 * ASM_TRI_MAX; i += blockDim.x) {
-        const int side = i / ASM_TRI_MAX, li = i % ASM_TRI_MAX;
-        const int t = ta.tile_tri[(size_t)(side ? bj : bi) * ASM_TRI_MAX + li];
-        stri[i] = t;
-        for (int j = 0; j < 3; j++) sc[i * 3 + j] = t >= 0 ? ta.c[(size_t)t * 3 + j] : 0.0;
+    const int na = ta.tile_ntri[bi], nb = ta.tile_ntri[bj];
+    for (int i = tid; i < na + nb; i += ASM_THREADS) {
+        const int sl = i < na ? i : ASM_TRI_MAX + i - na;
+        const int t = ta.tile_tri[(size_t)(i < na ? bi : bj) * ASM_TRI_MAX + sl % ASM_TRI_MAX];
+        stri[sl] = t;
+        for (int j = 0; j < 3; j++) sc[sl * 3 + j] = ta.c[(size_t)t * 3 + j];
     }
-    for (int i = tid; i < 2 * ASM_TRI_MAX * Nq; i += blockDim.x) {
-        const int q = i % Nq, sl = i / Nq;  // sl = side * TRI_MAX + li
-        const int t = ta.tile_tri[(size_t)(sl >= ASM_TRI_MAX ? bj : bi) * ASM_TRI_MAX + sl % ASM_TRI_MAX];
-        for (int j = 0; j < 3; j++) su[(sl * MAXQ + q) * 3 + j] = t >= 0 ? ta.u[((size_t)t * Nq + q) * 3 + j] : 0.0;
-        sjw[sl * MAXQ + q] = t >= 0 ? ta.jw[(size_t)t * Nq + q] : 0.0;
+    for (int i = tid; i < (na + nb) * Nq; i += ASM_THREADS) {
+        const int q = i % Nq, l = i / Nq, sl = l < na ? l : ASM_TRI_MAX + l - na;
+        const int t = ta.tile_tri[(size_t)(l < na ? bi : bj) * ASM_TRI_MAX + sl % ASM_TRI_MAX];
+        const size_t src = (size_t)t * Nq + q;
+        double* d = spt + sl * pitch + 4 * q;
+        for (int j = 0; j < 3; j++) d[j] = ta.u[src * 3 + j];
+        d[3] = ta.jw[src];
     }
-    for (int i = tid; i < 2 * ASM_TRI_MAX * 3; i += blockDim.x) {
-        const int side = i / (ASM_TRI_MAX * 3);
-        sent[i] = ta.tile_ent[(size_t)(side ? bj : bi) * ASM_TRI_MAX * 3 + i % (ASM_TRI_MAX * 3)];
-    }
-    for (int i = tid; i < 2 * TILE * 2; i += blockDim.x) {
+    for (int i = tid; i < 2 * ASM_TRI_MAX * 3; i += ASM_THREADS)
+        sent[i] = ta.tile_ent[(size_t)(i >= ASM_TRI_MAX * 3 ? bj : bi) * ASM_TRI_MAX * 3 + i % (ASM_TRI_MAX * 3)];
+    for (int i = tid; i < 2 * TILE * 2; i += ASM_THREADS) {
         const int side = i / (TILE * 2), slot = (i / 2) % TILE, h = i % 2;
         const int n = ta.tile_rwg[(size_t)(side ? bj : bi) * TILE + slot];
         const int hn = h * N + (n >= 0 ? n : 0);
@@ -627,169 +733,181 @@ __global__ void __launch_bounds__(256, 2) assemble_tri_kernel(AsmArgs a, DevTriA
         sdiv[i] = n >= 0 ? a.h.div[hn] : 0.0;
         for (int j = 0; j < 3; j++) spi[i * 3 + j] = n >= 0 ? ta.pi[(size_t)hn * 3 + j] : 0.0;
     }
-    if (tid < 2) sntri[tid] = ta.tile_ntri[tid ? bj : bi];
     __syncthreads();
 
-    const int na = sntri[0], nb = sntri[1];
-    const bool exact = (a.flags & BEM_ASM_GSMOOTH_EXACT) != 0;
-    const int items = na * nb * NMED;
-    for (int it = tid; it < items; it += blockDim.x) {
-        // medium-major: the lanes of a warp take the same branches (the
-        // exterior medium is lossless, the interior one takes exp)
-        const int e = it / (na * nb), pr = it % (na * nb), ia = pr / nb, ib = ASM_TRI_MAX + pr % nb;
-        const bool same = stri[ia] == stri[ib];
-        const Medium k = a.med[e];
+    for (int it = tid; it < na * nb; it += ASM_THREADS) {
+        const int ia = it / nb, ib = ASM_TRI_MAX + it - ia * nb;
+        if (stri[ia] == stri[ib]) continue;  // the same triangle: below
         const double Dx = sc[ia * 3] - sc[ib * 3], Dy = sc[ia * 3 + 1] - sc[ib * 3 + 1],
                      Dz = sc[ia * 3 + 2] - sc[ib * 3 + 2];
-        cplx M0 = {0, 0}, Muv = {0, 0}, S0 = {0, 0};
-        cplx Mu[3], Mv[3], A[3], B[3], C[3];
+        LMoments L[NMED];
+        KMoments K;
 #pragma unroll
-        for (int j = 0; j < 3; j++) Mu[j] = Mv[j] = A[j] = B[j] = C[j] = {0, 0};
+        for (int e = 0; e < NMED; e++) {
+            L[e].M0 = L[e].Muv = {0, 0};
+#pragma unroll
+            for (int j = 0; j < 3; j++) L[e].Mu[j] = L[e].Mv[j] = {0, 0};
+        }
+        K.S0 = {0, 0};
+#pragma unroll
+        for (int j = 0; j < 3; j++) K.A[j] = K.B[j] = K.C[j] = {0, 0};
+#pragma unroll 1
         for (int qa = 0; qa < Nq; qa++) {
-            const double* up = &su[(ia * MAXQ + qa) * 3];
-            const double ux = up[0], uy = up[1], uz = up[2], wa = sjw[ia * MAXQ + qa];
+            const double2 uxy = *(const double2*)(spt + ia * pitch + 4 * qa),
+                          uzw = *(const double2*)(spt + ia * pitch + 4 * qa + 2);
+            const double ex = Dx + uxy.x, ey = Dy + uxy.y, ez = Dz + uzw.x, wa = uzw.y * INV4PI_D;
+            cplx T0[NMED], Tv[NMED][3], s0 = {0, 0}, sv[3];
+#pragma unroll
+            for (int j = 0; j < 3; j++) sv[j] = {0, 0};
+#pragma unroll
+            for (int e = 0; e < NMED; e++) {
+                T0[e] = {0, 0};
+#pragma unroll
+                for (int j = 0; j < 3; j++) Tv[e][j] = {0, 0};
+            }
+#pragma unroll 2
             for (int qb = 0; qb < Nq; qb++) {
-                const double* vp = &su[(ib * MAXQ + qb) * 3];
-                const double vx = vp[0], vy = vp[1], vz = vp[2], w = wa * sjw[ib * MAXQ + qb];
-                const double dx = Dx + (ux - vx), dy = Dy + (uy - vy), dz = Dz + (uz - vz);
-                // 1/R from one reciprocal square root (R clamped at 1e-15 as
-                // R^2 at 1e-30); R = R^2 / R
+                const double2 vxy = *(const double2*)(spt + ib * pitch + 4 * qb),
+                              vzw = *(const double2*)(spt + ib * pitch + 4 * qb + 2);
+                const double dx = ex - vxy.x, dy = ey - vxy.y, dz = ez - vzw.x;
+                const double R2 = fmax(dx * dx + dy * dy + dz * dz, 1e-30);  // R clamped at 1e-15
+                const double invR = rsqrt_normal(R2), R = R2 * invR, iw = invR * vzw.y;
+                cplx g = {0, 0};  // sum_e G_e (i k_e - 1/R)
+#pragma unroll
+                for (int e = 0; e < NMED; e++) {
+                    const Medium k = a.med[e];
+                    double sn, cs;
+                    sincos_bounded(k.kr * R, &sn, &cs);
+                    double am = iw;
+                    if ((DAMP >> e) & 1) am *= exp_decay_bounded(k.ki * R);
+                    const cplx G = {am * cs, am * sn};
+                    T0[e].re += G.re, T0[e].im += G.im;
+                    cfma(Tv[e][0], G, vxy.x), cfma(Tv[e][1], G, vxy.y), cfma(Tv[e][2], G, vzw.x);
+                    const double f = ((DAMP >> e) & 1) ? -k.ki - invR : -invR;
+                    g.re += G.re * f - G.im * k.kr;
+                    g.im += G.im * f + G.re * k.kr;
+                }
+                const double gr = R2 > 1e-24 ? invR : 0.0;  // coincident points of distinct triangles: no K
+                g.re *= gr, g.im *= gr;
+                s0.re += g.re, s0.im += g.im;
+                cfma(sv[0], g, vxy.x), cfma(sv[1], g, vxy.y), cfma(sv[2], g, vzw.x);
+            }
+            const double wu[3] = {wa * uxy.x, wa * uxy.y, wa * uzw.x};
+#pragma unroll
+            for (int e = 0; e < NMED; e++) {
+                cfma(L[e].M0, T0[e], wa);
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    cfma(L[e].Mu[j], T0[e], wu[j]);
+                    cfma(L[e].Mv[j], Tv[e][j], wa);
+                    cfma(L[e].Muv, Tv[e][j], wu[j]);
+                }
+            }
+            cfma(K.S0, s0, wa);
+#pragma unroll
+            for (int j = 0; j < 3; j++) {
+                const int j1 = (j + 1) % 3, j2 = (j + 2) % 3;
+                cfma(K.A[j], s0, wu[j]);
+                cfma(K.B[j], sv[j], wa);
+                K.C[j].re += wu[j1] * sv[j2].re - wu[j2] * sv[j1].re;
+                K.C[j].im += wu[j1] * sv[j2].im - wu[j2] * sv[j1].im;
+            }
+        }
+        store_half_pairs<NMED>(a, L, K, Dx, Dy, Dz, sent + ia * 3, sent + ib * 3, ssig, sdiv, spi, slots);
+    }
+    // the same triangle on both sides: G_smooth in the literal or the exact
+    // form with the library's functions, no K (few per tile pair: thread per
+    // row triangle)
+    const bool exact = (a.flags & BEM_ASM_GSMOOTH_EXACT) != 0;
+    for (int ia = tid; ia < na; ia += ASM_THREADS) {
+        int ib = -1;
+        for (int l = 0; l < nb; l++)
+            if (stri[ASM_TRI_MAX + l] == stri[ia]) ib = ASM_TRI_MAX + l;
+        if (ib < 0) continue;
+        LMoments L[NMED];
+        KMoments K;
+        K.S0 = {0, 0};
+        for (int j = 0; j < 3; j++) K.A[j] = K.B[j] = K.C[j] = {0, 0};
+#pragma unroll 1
+        for (int e = 0; e < NMED; e++) {
+            const Medium k = a.med[e];
+            LMoments S;
+            S.M0 = S.Muv = {0, 0};
+            for (int j = 0; j < 3; j++) S.Mu[j] = S.Mv[j] = {0, 0};
+#pragma unroll 1
+            for (int p = 0; p < Nq * Nq; p++) {
+                const double* u = spt + ia * pitch + 4 * (p / Nq);
+                const double* v = spt + ib * pitch + 4 * (p % Nq);
+                const double w = u[3] * v[3];
+                const double dx = u[0] - v[0], dy = u[1] - v[1], dz = u[2] - v[2];
                 const double R2 = fmax(dx * dx + dy * dy + dz * dz, 1e-30);
-                const double invR = rsqrt(R2), Rs = R2 * invR, R = Rs;
+                const double invR = rsqrt(R2), Rs = R2 * invR;
                 const double i4R = __dmul_rn(INV4PI_D, invR);  // rounded alone, as in assemble_kernel
                 double sn, cs;
                 sincos(k.kr * Rs, &sn, &cs);
-                const double ea = (k.ki != 0.0) ? exp_decay(k.ki * Rs) : 1.0;
-                const cplx G = {ea * cs * i4R, ea * sn * i4R};
-                cplx Gu = G;
-                if (same) {
-                    if (exact) Gu = g_smooth_exact(k, R);
-                    else Gu.re -= i4R;
-                }
-                const cplx Gj = {Gu.re * w, Gu.im * w};
-                const double uv = ux * vx + uy * vy + uz * vz;
-                M0.re += Gj.re, M0.im += Gj.im;
-                Muv.re += Gj.re * uv, Muv.im += Gj.im * uv;
-                Mu[0].re += Gj.re * ux, Mu[0].im += Gj.im * ux;
-                Mu[1].re += Gj.re * uy, Mu[1].im += Gj.im * uy;
-                Mu[2].re += Gj.re * uz, Mu[2].im += Gj.im * uz;
-                Mv[0].re += Gj.re * vx, Mv[0].im += Gj.im * vx;
-                Mv[1].re += Gj.re * vy, Mv[1].im += Gj.im * vy;
-                Mv[2].re += Gj.re * vz, Mv[2].im += Gj.im * vz;
-                if (!same && R > 1e-12) {
-                    const cplx gc = cmul(G, cplx{(-k.ki - invR) * invR, k.kr * invR});
-                    const cplx gw = {gc.re * w, gc.im * w};
-                    const double uu[3] = {ux, uy, uz}, vv[3] = {vx, vy, vz};
-                    const double cr[3] = {uy * vz - uz * vy, uz * vx - ux * vz, ux * vy - uy * vx};
-                    S0.re += gw.re, S0.im += gw.im;
-#pragma unroll
-                    for (int j = 0; j < 3; j++) {
-                        A[j].re += gw.re * uu[j], A[j].im += gw.im * uu[j];
-                        B[j].re += gw.re * vv[j], B[j].im += gw.im * vv[j];
-                        C[j].re += gw.re * cr[j], C[j].im += gw.im * cr[j];
-                    }
-                }
+                const double eav = (k.ki != 0.0) ? exp_decay(k.ki * Rs) : 1.0;
+                cplx G = {eav * cs * i4R, eav * sn * i4R};
+                if (exact) G = g_smooth_exact(k, Rs);
+                else G.re -= i4R;
+                G.re *= w, G.im *= w;
+                S.M0.re += G.re, S.M0.im += G.im;
+                cfma(S.Muv, G, u[0] * v[0] + u[1] * v[1] + u[2] * v[2]);
+                for (int j = 0; j < 3; j++) cfma(S.Mu[j], G, u[j]), cfma(S.Mv[j], G, v[j]);
             }
-        }
-        // P1 = -D.C, Q2 = A x D - C, Q3 = D x B + C, Q4 = D S0 + A - B
-        const double DD[3] = {Dx, Dy, Dz};
-        cplx P1 = {0, 0}, Q2[3], Q3[3], Q4[3];
 #pragma unroll
-        for (int j = 0; j < 3; j++) {
-            const int j1 = (j + 1) % 3, j2 = (j + 2) % 3;
-            P1.re -= DD[j] * C[j].re, P1.im -= DD[j] * C[j].im;
-            Q2[j] = {A[j1].re * DD[j2] - A[j2].re * DD[j1] - C[j].re, A[j1].im * DD[j2] - A[j2].im * DD[j1] - C[j].im};
-            Q3[j] = {DD[j1] * B[j2].re - DD[j2] * B[j1].re + C[j].re, DD[j1] * B[j2].im - DD[j2] * B[j1].im + C[j].im};
-            Q4[j] = {DD[j] * S0.re + A[j].re - B[j].re, DD[j] * S0.im + A[j].im - B[j].im};
+            for (int e2 = 0; e2 < NMED; e2++)
+                if (e2 == e) L[e2] = S;
         }
-        const cplx ik = {-k.ki, k.kr};
-        const double k2 = k.kr * k.kr + k.ki * k.ki;
-        const cplx iok = {k.ki / k2, k.kr / k2};  // i/k
-        for (int x = 0; x < 3; x++) {
-            const int er = sent[ia * 3 + x];
-            if (er == 0xff) break;
-            const int r = er >> 1, hr = er & 1;
-            const double sr = ssig[(r)*2 + hr], dr = sdiv[(r)*2 + hr];
-            const double* pp = &spi[((r)*2 + hr) * 3];
-            for (int y = 0; y < 3; y++) {
-                const int ec = sent[ib * 3 + y];
-                if (ec == 0xff) break;
-                const int c = ec >> 1, hc = ec & 1;
-                const double scn = ssig[(TILE + c) * 2 + hc], dc = sdiv[(TILE + c) * 2 + hc];
-                const double* nn = &spi[((TILE + c) * 2 + hc) * 3];
-                const double ss = sr * scn, pn = pp[0] * nn[0] + pp[1] * nn[1] + pp[2] * nn[2];
-                cplx lv = {Muv.re + pn * M0.re, Muv.im + pn * M0.im};
-#pragma unroll
-                for (int j = 0; j < 3; j++) {
-                    lv.re -= pp[j] * Mv[j].re + nn[j] * Mu[j].re;
-                    lv.im -= pp[j] * Mv[j].im + nn[j] * Mu[j].im;
-                }
-                lv.re *= ss, lv.im *= ss;
-                const double dd = dr * dc;
-                const cplx ls = {dd * M0.re, dd * M0.im};
-                const cplx t1 = cmul(ik, lv), t2 = cmul(iok, ls);
-                cplx kv = P1;
-                // pi . (Q4 x nu)
-                const cplx qx[3] = {{Q4[1].re * nn[2] - Q4[2].re * nn[1], Q4[1].im * nn[2] - Q4[2].im * nn[1]},
-                                    {Q4[2].re * nn[0] - Q4[0].re * nn[2], Q4[2].im * nn[0] - Q4[0].im * nn[2]},
-                                    {Q4[0].re * nn[1] - Q4[1].re * nn[0], Q4[0].im * nn[1] - Q4[1].im * nn[0]}};
-#pragma unroll
-                for (int j = 0; j < 3; j++) {
-                    kv.re += pp[j] * qx[j].re - nn[j] * Q2[j].re - pp[j] * Q3[j].re;
-                    kv.im += pp[j] * qx[j].im - nn[j] * Q2[j].im - pp[j] * Q3[j].im;
-                }
-                const int slot = (r * TILE + c) * 4 + hr * 2 + hc;
-                sL[e * 1024 + slot] = make_double2(t1.re - t2.re, t1.im - t2.im);
-                sK[e * 1024 + slot] = make_double2(ss * kv.re, ss * kv.im);
-            }
-        }
+        store_half_pairs<NMED>(a, L, K, 0.0, 0.0, 0.0, sent + ia * 3, sent + ib * 3, ssig, sdiv, spi, slots);
     }
     __syncthreads();
 
-    const int r = tid / TILE, c = tid % TILE;
-    const int mm = ta.tile_rwg[(size_t)bi * TILE + r], n = ta.tile_rwg[(size_t)bj * TILE + c];
-    if (mm < 0 || n < 0) return;
-    if (bi == bj && c < r) return;  // diagonal tile pair: the upper entry writes both positions
-    cplx Lf[NMED], Kk[NMED];
+    for (int en = tid; en < TILE * TILE; en += ASM_THREADS) {
+        const int r = en / TILE, c = en % TILE;
+        const int mm = ta.tile_rwg[(size_t)bi * TILE + r], n = ta.tile_rwg[(size_t)bj * TILE + c];
+        if (mm < 0 || n < 0) continue;
+        if (bi == bj && c < r) continue;  // diagonal tile pair: the upper entry writes both positions
+        double2 o[3];
 #pragma unroll
-    for (int e = 0; e < NMED; e++) {
-        const double2* l = &sL[e * 1024 + (r * TILE + c) * 4];
-        const double2* kk = &sK[e * 1024 + (r * TILE + c) * 4];
-        Lf[e] = {((l[0].x + l[1].x) + l[2].x) + l[3].x, ((l[0].y + l[1].y) + l[2].y) + l[3].y};
-        Kk[e] = {((kk[0].x + kk[1].x) + kk[2].x) + kk[3].x, ((kk[0].y + kk[1].y) + kk[2].y) + kk[3].y};
-    }
-    const bool mirror = (n != mm);
-    if (a.Z) {
-        cplx TL, BR, Ks;
-        if constexpr (NMED == 2) {
-            TL = {a.eta_e * Lf[0].re + a.eta_i * Lf[1].re, a.eta_e * Lf[0].im + a.eta_i * Lf[1].im};
-            BR = {Lf[0].re / a.eta_e + Lf[1].re / a.eta_i, Lf[0].im / a.eta_e + Lf[1].im / a.eta_i};
-            Ks = {Kk[0].re + Kk[1].re, Kk[0].im + Kk[1].im};
+        for (int k = 0; k < 3; k++) {
+            const double2* sl = slots + en * 12 + k;
+            o[k] = make_double2(((sl[0].x + sl[3].x) + sl[6].x) + sl[9].x, ((sl[0].y + sl[3].y) + sl[6].y) + sl[9].y);
+        }
+        const bool mirror = (n != mm);
+        if (a.Z) {
+            const double2 TL = o[0], BR = o[1], Ks = o[2], Km = make_double2(-o[2].x, -o[2].y);
+            double2* Z = a.Z;
+            const int64_t ld = a.ldz;
+            Z[(int64_t)mm * ld + n] = TL;
+            Z[(int64_t)mm * ld + N + n] = Km;
+            Z[(int64_t)(N + mm) * ld + n] = Ks;
+            Z[(int64_t)(N + mm) * ld + N + n] = BR;
+            if (mirror) {
+                Z[(int64_t)n * ld + mm] = TL;
+                Z[(int64_t)n * ld + N + mm] = Km;
+                Z[(int64_t)(N + n) * ld + mm] = Ks;
+                Z[(int64_t)(N + n) * ld + N + mm] = BR;
+            }
         } else {
-            TL = {a.eta_e * Lf[0].re, a.eta_e * Lf[0].im};
-            BR = {Lf[0].re / a.eta_e, Lf[0].im / a.eta_e};
-            Ks = Kk[0];
-        }
-        double2* Z = a.Z;
-        const int64_t ld = a.ldz;
-        Z[(int64_t)mm * ld + n] = make_double2(TL.re, TL.im);
-        Z[(int64_t)mm * ld + N + n] = make_double2(-Ks.re, -Ks.im);
-        Z[(int64_t)(N + mm) * ld + n] = make_double2(Ks.re, Ks.im);
-        Z[(int64_t)(N + mm) * ld + N + n] = make_double2(BR.re, BR.im);
-        if (mirror) {
-            Z[(int64_t)n * ld + mm] = make_double2(TL.re, TL.im);
-            Z[(int64_t)n * ld + N + mm] = make_double2(-Ks.re, -Ks.im);
-            Z[(int64_t)(N + n) * ld + mm] = make_double2(Ks.re, Ks.im);
-            Z[(int64_t)(N + n) * ld + N + mm] = make_double2(BR.re, BR.im);
-        }
-    } else {
-        a.L[(int64_t)mm * a.ld + n] = make_double2(Lf[0].re, Lf[0].im);
-        a.K[(int64_t)mm * a.ld + n] = make_double2(Kk[0].re, Kk[0].im);
-        if (mirror) {
-            a.L[(int64_t)n * a.ld + mm] = make_double2(Lf[0].re, Lf[0].im);
-            a.K[(int64_t)n * a.ld + mm] = make_double2(Kk[0].re, Kk[0].im);
+            a.L[(int64_t)mm * a.ld + n] = o[0];
+            a.K[(int64_t)mm * a.ld + n] = o[2];
+            if (mirror) {
+                a.L[(int64_t)n * a.ld + mm] = o[0];
+                a.K[(int64_t)n * a.ld + mm] = o[2];
+            }
         }
     }
+}
+
+template <int NMED, int DAMP>
+static int launch_assemble_tri(bem_ctx* ctx, const bem_geom* g, const AsmArgs& a, unsigned ntiles) {
+    auto kern = g->Nq == 7   ? assemble_tri_kernel<NMED, DAMP, 7>
+                : g->Nq == 4 ? assemble_tri_kernel<NMED, DAMP, 4>
+                             : assemble_tri_kernel<NMED, DAMP, 0>;
+    const size_t smem = tri_smem_bytes(g->Nq);
+    BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<ntiles, ASM_THREADS, smem, ctx->stream>>>(a, g->tri);
+    return BEM_OK;
 }
 
 // Tiles to recompute from an RWG mask (tile_rwg null: tiles of 16
@@ -944,7 +1062,10 @@ int assemble_dev(bem_ctx* ctx, const bem_geom* g, double ke_re, double ke_im, do
     a.ld = ldz;
     a.coef = g->sing_coef;
     a.tile_flag = nullptr;
-    const bool tri = ctx->asm_kernel == 0;
+    // triangle pairs, unless a phase could leave the range of sincos_bounded
+    // (|r - r'| <= 2 rmax): then the per-RWG kernel with the library's sine and cosine
+    const double kmax = std::max(std::fabs(ke_re), mode == 2 ? std::fabs(ki_re) : 0.0);
+    const bool tri = ctx->asm_kernel == 0 && kmax * 2.0 * g->rmax < SINCOS_MAX;
     const unsigned char* rec = nullptr;
     if (rwg_mask) {
         // tiles holding a flagged RWG, and the RWGs of those tiles
@@ -962,20 +1083,14 @@ int assemble_dev(bem_ctx* ctx, const bem_geom* g, double ke_re, double ke_im, do
     if (g->Nq > MAXQ) return fail(ctx, BEM_ERR_INVALID, "quadrature of %d points (at most %d)", g->Nq, MAXQ);
     cudaEvent_t ev = ctx->prof_begin(PROF_ASSEMBLY);
     if (tri) {
-        // dynamic shared memory beyond 48 KB: set once per device
-        static unsigned attr_done = 0;
-        const unsigned bit = 1u << (ctx->device & 31);
-        if (!(__atomic_load_n(&attr_done, __ATOMIC_ACQUIRE) & bit)) {
-            BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(assemble_tri_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)tri_smem_bytes(2)));
-            BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(assemble_tri_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)tri_smem_bytes(1)));
-            __atomic_fetch_or(&attr_done, bit, __ATOMIC_RELEASE);
-        }
+        const int damp = (ke_im != 0.0 ? 1 : 0) | (mode == 2 && ki_im != 0.0 ? 2 : 0);
+        const unsigned nb = (unsigned)ntiles;
         if (mode == 2)
-            assemble_tri_kernel<2><<<(unsigned)ntiles, 256, tri_smem_bytes(2), st>>>(a, g->tri);
+            BEM_TRY(damp == 0   ? (launch_assemble_tri<2, 0>(ctx, g, a, nb))
+                    : damp == 2 ? (launch_assemble_tri<2, 2>(ctx, g, a, nb))
+                                : (launch_assemble_tri<2, 3>(ctx, g, a, nb)));
         else
-            assemble_tri_kernel<1><<<(unsigned)ntiles, 256, tri_smem_bytes(1), st>>>(a, g->tri);
+            BEM_TRY(damp == 0 ? (launch_assemble_tri<1, 0>(ctx, g, a, nb)) : (launch_assemble_tri<1, 1>(ctx, g, a, nb)));
     } else if (mode == 2) {
         assemble_kernel<2><<<(unsigned)ntiles, 256, 0, st>>>(a);
     } else {
