@@ -131,6 +131,81 @@ static double largest_vertex(const HostMesh& m) {
     return std::sqrt(r2);
 }
 
+// RWG order of the assembly tiles (ASM_TILE consecutive ones each): patches
+// grown over shared triangles.  A tile starts at the first triangle along the
+// Morton order that still has RWGs to place, and takes in turn an RWG whose
+// two triangles it already has, else the one whose other triangle has the
+// fewest RWGs left outside the patch (it would be left behind otherwise), the
+// nearest to the patch's centre among equals.  15.5-15.8 distinct triangles
+// per 16 RWGs on spheres and prisms against 17.1 along the Morton curve
+// itself: 18 % fewer triangle pairs in the assembly.
+static std::vector<int> patch_order(const HostRWG& r, int nt, const std::vector<double>& tc,
+                                    const std::vector<int>& torder) {
+    const int N = r.N;
+    std::vector<int> first(nt + 1, 0), on(2 * (size_t)N), left(nt, 0);
+    for (int n = 0; n < N; n++) first[r.tri_p[n] + 1]++, first[r.tri_m[n] + 1]++;
+    for (int t = 0; t < nt; t++) left[t] = first[t + 1], first[t + 1] += first[t];
+    {
+        std::vector<int> at(first.begin(), first.end() - 1);
+        for (int n = 0; n < N; n++) on[at[r.tri_p[n]]++] = n, on[at[r.tri_m[n]]++] = n;
+    }
+    std::vector<char> used(N, 0);
+    std::vector<int> in_cand(N, -1), in_tile(nt, -1), cand, perm;
+    perm.reserve(N);
+    int ptr = 0, tile = 0, cnt = 0, ntri = 0;
+    double sum[3] = {0, 0, 0};
+    auto add_tri = [&](int t) {
+        in_tile[t] = tile;
+        ntri++;
+        for (int j = 0; j < 3; j++) sum[j] += tc[3 * (size_t)t + j];
+        for (int i = first[t]; i < first[t + 1]; i++)
+            if (!used[on[i]] && in_cand[on[i]] != tile) in_cand[on[i]] = tile, cand.push_back(on[i]);
+    };
+    while ((int)perm.size() < N) {
+        if (cand.empty()) {
+            while (left[torder[ptr]] == 0) ptr++;
+            add_tri(torder[ptr]);
+        }
+        size_t best = 0;
+        int best_key = 1 << 30;
+        double best_d = 0.0;
+        for (size_t i = 0; i < cand.size(); i++) {
+            const int n = cand[i], ta = r.tri_p[n], tb = r.tri_m[n];
+            const bool ha = in_tile[ta] == tile, hb = in_tile[tb] == tile;
+            if (ha && hb) {
+                best = i;
+                break;
+            }
+            const int t = ha ? tb : ta;
+            int key = 0;
+            for (int k = first[t]; k < first[t + 1]; k++)
+                if (!used[on[k]]) key += in_cand[on[k]] == tile ? -1 : 1;
+            if (key > best_key) continue;
+            double d = 0.0;
+            for (int j = 0; j < 3; j++) {
+                const double x = tc[3 * (size_t)t + j] - sum[j] / ntri;
+                d += x * x;
+            }
+            if (key < best_key || d < best_d) best = i, best_key = key, best_d = d;
+        }
+        const int n = cand[best];
+        cand.erase(cand.begin() + best);
+        used[n] = 1;
+        perm.push_back(n);
+        for (int t : {r.tri_p[n], r.tri_m[n]}) {
+            left[t]--;
+            if (in_tile[t] != tile) add_tri(t);
+        }
+        if (++cnt == ASM_TILE) {
+            cnt = ntri = 0;
+            sum[0] = sum[1] = sum[2] = 0.0;
+            tile++;
+            cand.clear();
+        }
+    }
+    return perm;
+}
+
 int geom_upload(bem_ctx* ctx, bem_geom* g) {
     const HostMesh& m = g->mesh;
     g->rmax = largest_vertex(m);
@@ -169,9 +244,7 @@ int geom_upload(bem_ctx* ctx, bem_geom* g) {
     g->sing.npairs = (int)pair_mn.size() / 2;
     g->sing.nitems = (int)item.size() / 3;
 
-    // RWGs in the Morton order of their triangles' centroids: each triangle
-    // in turn appends its RWGs not placed yet, so a tile of 16 consecutive
-    // RWGs touches ~17 distinct triangles instead of ~21-32
+    // triangles in the Morton order of their centroids, along which patch_order starts the tiles
     std::vector<int> torder(nt);
     {
         double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
@@ -202,14 +275,10 @@ int geom_upload(bem_ctx* ctx, bem_geom* g) {
             if (j == 3) return fail(ctx, BEM_ERR_INVALID, "triangle %d carries more than 3 RWG halves", t);
             tri_half[3 * (size_t)t + j] = h * N + n;
         }
-    std::vector<std::vector<int>> rwg_of_tri(nt);
-    for (int n = 0; n < N; n++) rwg_of_tri[r.tri_p[n]].push_back(n), rwg_of_tri[r.tri_m[n]].push_back(n);
     const int ntile = (N + ASM_TILE - 1) / ASM_TILE;
-    std::vector<int> perm, pos(N, -1);
-    perm.reserve(N);
-    for (int t : torder)
-        for (int n : rwg_of_tri[t])
-            if (pos[n] < 0) pos[n] = (int)perm.size(), perm.push_back(n);
+    const std::vector<int> perm = patch_order(r, nt, tc, torder);
+    std::vector<int> pos(N);
+    for (int i = 0; i < N; i++) pos[perm[i]] = i;
     std::vector<int> tile_rwg((size_t)ntile * ASM_TILE, -1), tile_tri((size_t)ntile * ASM_TRI_MAX, -1), tile_ntri(ntile, 0);
     std::vector<unsigned char> tile_ent((size_t)ntile * ASM_TRI_MAX * 3, 0xff);
     for (int tl = 0; tl < ntile; tl++) {
@@ -574,8 +643,8 @@ __global__ void __launch_bounds__(256) assemble_kernel(AsmArgs a) {
 // (only K_e + K_i is needed).
 // Each (RWG pair, half pair) term lands in its own shared-memory slot and the
 // four half pairs of an entry are summed in a fixed order, so the result does
-// not depend on the tiling.  RWGs are tiled in the Morton order of their
-// triangles (geom_upload), ~17 distinct triangles per 16 RWGs.
+// not depend on the tiling.  RWGs are tiled in patches grown over shared
+// triangles (geom_upload), ~15.5 distinct triangles per 16 RWGs.
 //
 // Bound by the FP64 pipe, ~100 operations per point pair for two lossless
 // media, ~120 with one absorbing, which is 58 % busy: the 52 accumulators of a

@@ -138,7 +138,7 @@ void devmem_cache_enable(int device, bool on);
 bool devmem_cache_enabled(int device);
 
 // Triangle-pair assembly: per-triangle quadrature data relative to the
-// centroid, and the RWGs in tiles of ASM_TILE ordered along a Morton curve of
+// centroid, and the RWGs in tiles of ASM_TILE grown over shared triangles along a Morton curve of
 // their triangles' centroids, so that the RWGs of a tile share triangles.
 constexpr int ASM_TRI_MAX = 32;  // distinct triangles of one tile (2 halves x 16 RWGs at most)
 struct DevTriAsm {
