@@ -9,11 +9,11 @@
 //       panel_kernel  -- cooperative kernel, whole sub-panel held in shared
 //                        memory across all SMs, one grid barrier per column
 //                        (pivot search, swap, scale, rank-1 update); panels
-//                        that fit the shared memory of one cluster of at
-//                        most 8 CTAs run panel_cluster_kernel instead, with
-//                        a cluster barrier per column
-//       laswp + small TRSM + thin GEMM for the rest of the block column
-//     laswp of the block's pivots on the other columns
+//                        of up to 8192 rows run panel_reg_kernel instead,
+//                        rows in registers, on one cluster of at most 16
+//                        CTAs with a cluster barrier per column
+//       interchanges + U12 + thin GEMM for the rest of the block column
+//     interchanges of the block's pivots on the other columns
 //     U12 = L11^-1 A12  (blocked TRSM)
 //     A22 -= L21 U12    (the trailing update: FP64 on the FP64 tensor path,
 //                        mma.sync f64, three real products per complex
@@ -151,6 +151,24 @@ template <typename R> __device__ __forceinline__ R cabs1(typename C2T<R>::type v
 }
 
 // ------------------------------------------------------------ panel kernel
+// 1 / p of a pivot: conj(p) times the reciprocal of |p|^2, which the hardware
+// approximates to about 2^-20 and two Newton steps finish (the division's
+// branches were ~100 cycles of every panel column); conj(p) / |p|^2 by
+// divisions outside that approximation's range.
+__device__ __forceinline__ double2 pivot_recip(double2 p) {
+    const double den = p.x * p.x + p.y * p.y;
+    if (!(den > 1e-290 && den < 1e290)) return make_double2(p.x / den, -p.y / den);
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(den));
+    y = __fma_rn(y, __fma_rn(-den, y, 1.0), y);
+    y = __fma_rn(y, __fma_rn(-den, y, 1.0), y);
+    return make_double2(p.x * y, -p.y * y);
+}
+__device__ __forceinline__ float2 pivot_recip(float2 p) {
+    const float den = p.x * p.x + p.y * p.y;
+    return make_float2(p.x / den, -p.y / den);
+}
+
 // The two per-element operations of a panel column, with explicit fused
 // multiply-adds so that every panel kernel rounds them alike:
 // l = a inv and x - l u (complex).
@@ -325,12 +343,7 @@ panel_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int r0, int nro
         __syncthreads();
         // 5. scale column jj below the diagonal, rank-1 update of the rest
         if (!zero) {
-            C2 p = s_piv[jj];
-            R den = p.x * p.x + p.y * p.y;
-            C2 inv;
-            inv.x = p.x / den;
-            inv.y = -p.y / den;
-            panel_eliminate<R>(tile, w, nloc, lo, jj, s_piv, inv);
+            panel_eliminate<R>(tile, w, nloc, lo, jj, s_piv, pivot_recip(s_piv[jj]));
         }
         __syncthreads();
     }
@@ -340,30 +353,36 @@ panel_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int r0, int nro
     }
 }
 
-// ----------------------------------------------------- cluster panel kernel
-// The sub-panel of panel_kernel on one thread-block cluster per matrix.  The
-// C CTAs of a cluster hold the panel rows in shared memory (CTA b: rows
-// [b Rp, (b+1) Rp), Rp >= w, so the w pivot rows live in CTA 0); each
-// thread owns whole rows (row pitch WT + 1 complex: no bank conflicts) and is
-// the only one to update them.  Per column jj:
-//   A. every thread updates its rows for the pivot of column jj (row jj
-//      takes the pivot row u, the pivot row takes the former row jj, rows
-//      below jj are scaled by 1/u_jj in column jj and take the rank-1 update
-//      x -= l u right of it) and keeps the largest |re| + |im| of column
-//      jj + 1 among them (smallest row on ties);
-//   B. every warp publishes its candidate with that row's values in its
-//      CTA's shared memory, CTA 0's owner of row jj + 1 publishes that row;
-//   C. cluster barrier;
-//   D. warp 0 of every CTA reads the C x 8 candidates through distributed
-//      shared memory and reduces them alike: pivot row, its values u, row
-//      jj + 1's values, 1/u_jj+1 -- into its own shared memory;
-//   E. block barrier.
-// One cluster barrier and one block barrier per column, no spin loop.  The
-// candidate buffers alternate between two parities: a CTA in column jj + 2
-// cannot have passed barrier C of jj + 1 before every CTA has finished step
-// D of jj.  Same pivot rule and per-element arithmetic (panel_mul,
-// panel_msub) as panel_kernel, so the same pivots and factors.
-constexpr int PC_THREADS = 256, PC_WARPS = PC_THREADS / 32;
+// ---------------------------------------------------- register panel kernel
+// The sub-panel of panel_kernel with every row in the registers of one
+// thread, on one thread-block cluster per matrix: thread t of CTA b owns
+// panel row b T + t.  No row is moved while the columns are eliminated:
+// interchanging rows jj and p only exchanges their positions (one integer per
+// thread, which is also the tie break), and each row is written to its final
+// position at the end.  Per column jj:
+//   1. every warp finds its largest |re| + |im| of column jj among rows not
+//      yet taken (smallest position on ties); the winning lane leaves its
+//      columns jj.. in shared memory; block barrier;
+//   2. warp k reduces the CTA's candidates, forms 1 / pivot and writes value,
+//      position, reciprocal and row into CTA k's shared memory; cluster
+//      barrier;
+//   3. every warp reduces the C candidates from its own shared memory, and
+//      every row still active is scaled and takes the rank-1 update
+//      x -= l u, u read as a broadcast.
+// So a column costs one block and one cluster barrier and no load from
+// another SM: 60 us per 16 columns at 2300 rows with the rows in shared
+// memory, their interchange there and the candidates gathered from the
+// peers after the barrier.  Buffers alternate between two parities: a CTA
+// writing a peer's buffer in column jj + 2 has passed the barrier of jj + 1,
+// which that peer reaches after its reads of column jj.
+// Same pivot rule and per-element arithmetic (panel_mul, panel_msub) as
+// panel_kernel, so the same pivots and factors.
+// moves (2 n integers per matrix): for the w top positions k of the panel,
+// moves[r0 + k] is the row now at position k and moves[n + r0 + k] the
+// position of the row formerly there: the interchanges as one gather.
+template <typename R> struct PanelW { static constexpr int v = 64 / (2 * (int)sizeof(R) / 4); };  // 64 registers a row
+constexpr int PR_THREADS = 512, PR_WARPS = PR_THREADS / 32, PR_CLUSTER = 16, PG = 4;
+constexpr int PR_PITCH = 256 + 16;  // bytes of a row in shared memory
 
 // The warp's largest bv, the smallest br among the lanes holding it and that
 // lane's bk, in every lane.  bv >= 0 (a lane without a candidate holds 0 with
@@ -372,12 +391,17 @@ constexpr int PC_THREADS = 256, PC_WARPS = PC_THREADS / 32;
 __device__ __forceinline__ void warp_argmax_bits(unsigned hi, unsigned lo, int& br, int& bk, unsigned& mhi,
                                                  unsigned& mlo) {
     mhi = __reduce_max_sync(0xffffffffu, hi);
-    mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
-    const bool top = hi == mhi && lo == mlo;
-    const unsigned mrow = __reduce_min_sync(0xffffffffu, top ? (unsigned)br : 0xffffffffu);
-    const unsigned win = __ballot_sync(0xffffffffu, top && (unsigned)br == mrow);
-    bk = __shfl_sync(0xffffffffu, bk, __ffs(win) - 1);
-    br = (int)mrow;
+    unsigned win = __ballot_sync(0xffffffffu, hi == mhi);
+    if (win & (win - 1)) {  // several lanes share the upper word: the lower one and the row decide
+        mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
+        const bool top = hi == mhi && lo == mlo;
+        const unsigned mrow = __reduce_min_sync(0xffffffffu, top ? (unsigned)br : 0xffffffffu);
+        win = __ballot_sync(0xffffffffu, top && (unsigned)br == mrow);
+    }
+    const int w = __ffs(win) - 1;
+    mlo = __shfl_sync(0xffffffffu, lo, w);
+    br = __shfl_sync(0xffffffffu, br, w);
+    bk = __shfl_sync(0xffffffffu, bk, w);
 }
 __device__ __forceinline__ void warp_argmax(double& bv, int& br, int& bk) {
     const unsigned long long b = (unsigned long long)__double_as_longlong(bv);
@@ -391,255 +415,242 @@ __device__ __forceinline__ void warp_argmax(float& bv, int& br, int& bk) {
     bv = __uint_as_float(mhi);
 }
 
-template <typename R, int WT>
-__global__ void __launch_bounds__(PC_THREADS)
-panel_cluster_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int r0, int nrows, int w, int Rp,
-                     int* __restrict__ ipiv, int* __restrict__ info, int64_t sA, int sPiv) {
+template <typename R>
+__global__ void __launch_bounds__(PR_THREADS, 1)
+panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int r0, int nrows, int w,
+                 int* __restrict__ ipiv, int* __restrict__ info, int* __restrict__ moves, int64_t sA) {
     using C2 = typename C2T<R>::type;
     namespace cg = cooperative_groups;
-    constexpr int PITCH = WT + 1;
+    constexpr int W = PanelW<R>::v;
     cg::cluster_group cluster = cg::this_cluster();
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    C2* tile = (C2*)smem_raw;                          // Rp * PITCH
-    C2* pub_data = tile + (size_t)Rp * PITCH;          // [2][PC_WARPS][32]: candidate rows
-    C2* disp = pub_data + 2 * PC_WARPS * 32;           // [2][32]: the next pivot row's former values (CTA 0)
-    __shared__ R pub_v[2][PC_WARPS];
-    __shared__ int pub_row[2][PC_WARPS];
-    __shared__ C2 s_u[32], s_dv[32];
-    __shared__ C2 s_inv;
-    __shared__ int s_piv, s_zero;
+    __shared__ __align__(16) C2 s_row[2][PR_WARPS][W];    // a warp's candidate row
+    __shared__ __align__(16) C2 r_row[2][PR_CLUSTER][W];  // a CTA's candidate row (written by the peers)
+    __shared__ C2 r_inv[2][PR_CLUSTER];
+    __shared__ R s_v[2][PR_WARPS], r_v[2][PR_CLUSTER];
+    __shared__ int s_pos[2][PR_WARPS], r_pos[2][PR_CLUSTER], s_at[PR_THREADS];
+    // the rows on their way in and out, 256 B each: 16 lanes a row in global
+    // memory, a thread a row here (an odd number of 16-byte units apart)
+    extern __shared__ __align__(16) unsigned char pr_smem[];
 
-    const int C = (int)cluster.num_blocks(), b = (int)cluster.block_rank(), tid = threadIdx.x;
-    const int mi = blockIdx.x / C;
+    const int C = (int)cluster.num_blocks(), b = (int)cluster.block_rank(), tid = threadIdx.x, T = blockDim.x;
+    const int mi = blockIdx.x / C, lane = tid & 31, warp = tid >> 5, nw = T >> 5;
     A += mi * sA;
-    ipiv += mi * sPiv;
+    ipiv += (int64_t)mi * n;
     info += mi;
-    const int lane = tid & 31, q = tid >> 5;
-    const int lo = b * Rp;
-    const int nloc = max(0, min(Rp, nrows - lo));
-    const int K = C * PC_WARPS;  // candidates per column
-    C2 zero;
-    zero.x = 0;
-    zero.y = 0;
-
-    for (int e = tid; e < nloc * w; e += blockDim.x) {
-        const int i = e / w, c = e % w;
-        tile[i * PITCH + c] = A[(int64_t)(r0 + lo + i) * lda + r0 + c];
+    moves += (int64_t)mi * 2 * n;
+    const int gr = b * T + tid;
+    const bool valid = gr < nrows;
+    bool act = valid;
+    int pos = gr;
+    C2 x[W];
+    C2* mine = reinterpret_cast<C2*>(pr_smem + (size_t)tid * PR_PITCH);
+    C2* base = A + (int64_t)(r0 + b * T) * lda + r0;  // the CTA's first row
+    const int rows = max(0, min(T, nrows - b * T));
+    // whole 16-byte units (FP32: even lda and r0), else element by element
+    const bool wide = w == W && ((reinterpret_cast<uintptr_t>(base) | ((uintptr_t)lda * sizeof(C2))) & 15) == 0;
+    if (wide) {
+        for (int e = tid; e < rows * 16; e += T)
+            dmma::cp16(pr_smem + (size_t)(e >> 4) * PR_PITCH + 16 * (e & 15),
+                       reinterpret_cast<const unsigned char*>(base + (int64_t)(e >> 4) * lda) + 16 * (e & 15), true);
+        dmma::cp_commit();
+        dmma::cp_wait<0>();
+    } else {
+        for (int e = tid; e < rows * w; e += T)
+            reinterpret_cast<C2*>(pr_smem + (size_t)(e / w) * PR_PITCH)[e % w] = base[(int64_t)(e / w) * lda + e % w];
     }
     __syncthreads();
-
-    // candidate for column 0: every row
-    R bv = (R)0;
-    int br = 0x7fffffff, bk = 0;
-    for (int i = tid; i < nloc; i += PC_THREADS) {
-        const R v = cabs1<R>(tile[i * PITCH]);
-        if (v > bv || (v == bv && lo + i < br)) bv = v, br = lo + i;
+#pragma unroll
+    for (int c = 0; c < W; c++) {
+        x[c].x = x[c].y = 0;
+        if (valid && c < w) x[c] = mine[c];
     }
-
-    for (int jn = 0; jn <= w; jn++) {
-        // jn >= 1: step A for column jj = jn - 1 (its pivot is in s_*), with
-        // the candidate for column jn
-        if (jn >= 1) {
-            const int jj = jn - 1, piv = s_piv;
-            const bool zp = s_zero != 0;
-            const C2 inv = s_inv;
-            bv = (R)0;
-            br = 0x7fffffff;
-            for (int i = tid; i < nloc; i += PC_THREADS) {
-                const int gr = lo + i;
-                C2* row = tile + (size_t)i * PITCH;
-                if (gr == jj) {
-                    for (int c = 0; c < w; c++) row[c] = s_u[c];
-                } else if (gr > jj) {
-                    const bool isp = gr == piv && piv != jj;  // takes the former row jj
-                    if (isp)
-                        for (int c = 0; c < w; c++) row[c] = s_dv[c];
-                    if (!zp) {
-                        const C2 l = panel_mul(row[jj], inv);
-                        row[jj] = l;
-                        for (int c = jj + 1; c < w; c++) row[c] = panel_msub(row[c], l, s_u[c]);
-                    }
-                    if (jn < w) {
-                        const R v = cabs1<R>(row[jn]);
-                        if (v > bv || (v == bv && gr < br)) bv = v, br = gr;
-                    }
-                }
-            }
+    if (C > 1) cluster.sync();  // every CTA runs before its shared memory is written
+    // PG columns at a time: x[0 .. PG) are the current ones, x[rem .. W) the
+    // finished ones; the row rotates left by PG after each group, so W / PG
+    // groups bring it back.  One loop over the groups instead of W unrolled
+    // columns: those were 13 k instructions that every launch fetched anew.
+    for (int g0 = 0; g0 < W; g0 += PG) {
+      const int rem = W - g0;
+#pragma unroll
+      for (int q = 0; q < PG; q++) {
+        const int jj = g0 + q;
+        if (jj >= w) break;
+        const int par = q & 1;  // PG is even: the parity of jj
+        // 1. this warp's candidate (v = 0: none; a NaN is none either)
+        R v = act ? cabs1<R>(x[q]) : (R)0;
+        if (!(v > (R)0)) v = (R)0;
+        int br = v > (R)0 ? pos : 0x7fffffff, bk = lane;
+        warp_argmax(v, br, bk);
+        if (lane == bk && v > (R)0) {
+#pragma unroll
+            for (int c = q; c < W; c++)
+                if (c < rem) s_row[par][warp][c] = x[c];
         }
-        if (jn == w) break;
-        const int par = jn & 1;
-        // B. publish this warp's candidate for column jn with its row, and row jn
-        warp_argmax(bv, br, bk);  // in every lane
-        __syncwarp();
-        if (lane == 0) {
-            pub_v[par][q] = bv;
-            pub_row[par][q] = br;
-        }
-        if (br != 0x7fffffff && lane < w) pub_data[(par * PC_WARPS + q) * 32 + lane] = tile[(br - lo) * PITCH + lane];
-        if (b == 0 && (jn % PC_THREADS) / 32 == q && lane < w) disp[par * 32 + lane] = tile[jn * PITCH + lane];
-        // C. every candidate of the cluster published (a one-CTA cluster:
-        // the block barrier)
-        if (C > 1)
-            cluster.sync();
-        else
-            __syncthreads();
-        // D. the pivot of column jn, in warp 0 of every CTA
-        if (q == 0) {
-            R gv = (R)0;
-            int grw = 0x7fffffff, gk = -1;
-            for (int k = lane; k < K; k += 32) {
-                const int rk = k / PC_WARPS, sk = k % PC_WARPS;
-                const int r = C > 1 ? *cluster.map_shared_rank(&pub_row[par][sk], rk) : pub_row[par][sk];
-                const R v = C > 1 ? *cluster.map_shared_rank(&pub_v[par][sk], rk) : pub_v[par][sk];
-                if (r != 0x7fffffff && (v > gv || (v == gv && r < grw))) gv = v, grw = r, gk = k;
-            }
-            warp_argmax(gv, grw, gk);  // in every lane
-            const bool zp = !(gv > (R)0);
-            if (zp) {
-                grw = jn;  // no interchange; LAPACK records info and skips the scaling
-                gk = -1;
-            }
-            C2 u = zero;
-            if (lane < w) {
-                const C2* dsrc = C > 1 ? cluster.map_shared_rank(disp, 0) : disp;
-                const C2* usrc = C > 1 ? cluster.map_shared_rank(pub_data, gk >= 0 ? gk / PC_WARPS : 0) : pub_data;
-                const C2 dv = dsrc[par * 32 + lane];
-                u = gk >= 0 ? usrc[(par * PC_WARPS + gk % PC_WARPS) * 32 + lane] : dv;
-                s_dv[lane] = dv;
-                s_u[lane] = u;
-            }
-            C2 p;
-            p.x = __shfl_sync(0xffffffffu, u.x, jn);
-            p.y = __shfl_sync(0xffffffffu, u.y, jn);
-            if (lane == 0) {
-                C2 inv = zero;
-                if (!zp) {
-                    const R den = p.x * p.x + p.y * p.y;
-                    inv.x = p.x / den;
-                    inv.y = -p.y / den;
-                }
-                s_inv = inv;
-                s_piv = grw;
-                s_zero = zp ? 1 : 0;
-                if (b == 0) {
-                    if (zp) atomicCAS(info, 0, r0 + jn + 1);
-                    ipiv[r0 + jn] = r0 + grw;
-                }
-            }
-        }
-        // E. the pivot known to every thread of this CTA
+        if (lane == 0) s_v[par][warp] = v, s_pos[par][warp] = br;
         __syncthreads();
+        const C2* u;
+        C2 inv;
+        if (C > 1) {
+            // 2. the CTA's candidate into every CTA of the cluster
+            for (int k = warp; k < C; k += nw) {
+                R cv = lane < nw ? s_v[par][lane] : (R)0;
+                int cr = lane < nw ? s_pos[par][lane] : 0x7fffffff, ck = lane;
+                warp_argmax(cv, cr, ck);
+                if (cv > (R)0) {
+                    const C2 iv = pivot_recip(s_row[par][ck][q]);
+                    if (lane >= q && lane < rem) cluster.map_shared_rank(&r_row[par][b][0], k)[lane] = s_row[par][ck][lane];
+                    if (lane == 0) *cluster.map_shared_rank(&r_inv[par][b], k) = iv;
+                }
+                if (lane == 0) {
+                    *cluster.map_shared_rank(&r_v[par][b], k) = cv;
+                    *cluster.map_shared_rank(&r_pos[par][b], k) = cv > (R)0 ? cr : 0x7fffffff;
+                }
+            }
+            cluster.sync();
+            v = lane < C ? r_v[par][lane] : (R)0;
+            br = lane < C ? r_pos[par][lane] : 0x7fffffff;
+            bk = lane;
+            warp_argmax(v, br, bk);
+            u = r_row[par][bk];
+            inv = r_inv[par][bk];
+        } else {
+            v = lane < nw ? s_v[par][lane] : (R)0;
+            br = lane < nw ? s_pos[par][lane] : 0x7fffffff;
+            bk = lane;
+            warp_argmax(v, br, bk);
+            u = s_row[par][bk];
+            inv = pivot_recip(u[q]);
+        }
+        // 3. v = 0: a zero column, no interchange and no scaling (LAPACK records it)
+        const bool zp = !(v > (R)0);
+        const int piv = zp ? jj : br;
+        if (b == 0 && tid == 0) {
+            ipiv[r0 + jj] = r0 + piv;
+            if (zp) atomicCAS(info, 0, r0 + jj + 1);
+        }
+        if (pos == piv) {
+            pos = jj;
+            act = false;
+        } else if (pos == jj) {
+            pos = piv;
+        }
+        if (act && !zp) {
+            const C2 l = panel_mul(x[q], inv);
+            x[q] = l;
+#pragma unroll
+            for (int c0 = 0; c0 < W; c0 += PG)
+                if (c0 < rem) {
+#pragma unroll
+                    for (int c = c0; c < c0 + PG; c++)
+                        if (c > q) x[c] = panel_msub(x[c], l, u[c]);
+                }
+        }
+      }
+      C2 done[PG];
+#pragma unroll
+      for (int c = 0; c < PG; c++) done[c] = x[c];
+#pragma unroll
+      for (int c = 0; c + PG < W; c++) x[c] = x[c + PG];
+#pragma unroll
+      for (int c = 0; c < PG; c++) x[W - PG + c] = done[c];
+    }
+    // rows to their positions (every row of the panel was read before the first barrier)
+    if (valid) {
+#pragma unroll
+        for (int c = 0; c < W; c++)
+            if (c < w) mine[c] = x[c];
+        s_at[tid] = pos;
     }
     __syncthreads();
-    for (int e = tid; e < nloc * w; e += blockDim.x) {
-        const int i = e / w, c = e % w;
-        A[(int64_t)(r0 + lo + i) * lda + r0 + c] = tile[i * PITCH + c];
+    C2* top = A + (int64_t)r0 * lda + r0;
+    if (wide) {
+        for (int e = tid; e < rows * 16; e += T)
+            *reinterpret_cast<uint4*>(reinterpret_cast<unsigned char*>(top + (int64_t)s_at[e >> 4] * lda) + 16 * (e & 15)) =
+                *reinterpret_cast<const uint4*>(pr_smem + (size_t)(e >> 4) * PR_PITCH + 16 * (e & 15));
+    } else {
+        for (int e = tid; e < rows * w; e += T)
+            top[(int64_t)s_at[e / w] * lda + e % w] = reinterpret_cast<const C2*>(pr_smem + (size_t)(e / w) * PR_PITCH)[e % w];
     }
-    // no CTA leaves while another may still read its shared memory
-    cluster.sync();
-}
-
-constexpr int PANEL_CLUSTER_MAX = 8;                // portable cluster size
-constexpr size_t PANEL_CLUSTER_SMEM = 200 * 1024;   // shared memory per CTA
-
-// CTAs per cluster for a sub-panel of nrows x w (elements of `esz` bytes):
-// about 384 rows per CTA, every CTA holding at least w rows, at most 8 CTAs
-// whose rows fit their shared memory; 0 when the panel does not fit one
-// cluster (panel_kernel takes it).
-static int panel_cluster_pitch(int w) { return (w <= 8 ? 8 : w <= 16 ? 16 : 32) + 1; }
-static size_t panel_cluster_smem(int Rp, int w, size_t esz) {
-    return ((size_t)Rp * panel_cluster_pitch(w) + 2 * PC_WARPS * 32 + 2 * 32) * esz;
-}
-static int panel_cluster_size(int nrows, int w, size_t esz) {
-    if (w < 1 || w > 32) return 0;
-    int C = std::min(PANEL_CLUSTER_MAX, std::max(1, (nrows + 383) / 384));
-    C = std::max(1, std::min(C, nrows / w));
-    for (; C <= PANEL_CLUSTER_MAX; C++) {
-        const int Rp = (nrows + C - 1) / C;
-        if (Rp < w) return 0;
-        if (panel_cluster_smem(Rp, w, esz) <= PANEL_CLUSTER_SMEM) return C;
+    if (valid) {
+        if (pos < w) moves[r0 + pos] = r0 + gr;
+        if (gr < w) moves[n + r0 + gr] = r0 + pos;
     }
-    return 0;
 }
 
-// panel_cluster_size, kept only where a cluster of that size and shared
-// memory can be resident on this device (cudaOccupancyMaxActiveClusters,
-// asked once per shape and remembered); 0: the cooperative panel.
+// CTAs per cluster and threads per CTA for a sub-panel of nrows rows, 0 when
+// it does not fit one cluster (panel_kernel takes it): 256 rows a CTA up to 8
+// CTAs (the portable size), then up to 512 rows a CTA, then 16 CTAs -- 8192
+// rows.  Few rows a CTA keep the rank-1 update short (64 registers a row, the
+// FP64 pipe of one SM), few CTAs the cluster barrier.
+struct PanelShape {
+    int C = 0, T = 0;
+};
+static PanelShape panel_reg_shape(int nrows) {
+    PanelShape p;
+    if (nrows > PR_CLUSTER * PR_THREADS) return p;
+    p.C = nrows <= 8 * PR_THREADS ? std::min(8, (nrows + 255) / 256) : PR_CLUSTER;
+    p.T = ((nrows + p.C - 1) / p.C + 31) / 32 * 32;
+    return p;
+}
+
+// panel_reg_shape, kept only where a cluster of that shape can be resident on
+// this device (asked once per shape and remembered).
 template <typename R>
-static int panel_cluster_choice(bem_ctx* ctx, int nrows, int iw) {
-    using C2 = typename C2T<R>::type;
-    if (!ctx->panel_clusters) return 0;
-    const int C = panel_cluster_size(nrows, iw, sizeof(C2));
-    if (C < 1) return 0;
-    const int Rp = (nrows + C - 1) / C;
-    const size_t smem = panel_cluster_smem(Rp, iw, sizeof(C2));
-    auto kern = iw <= 8 ? panel_cluster_kernel<R, 8> : iw <= 16 ? panel_cluster_kernel<R, 16> : panel_cluster_kernel<R, 32>;
+static PanelShape panel_reg_choice(bem_ctx* ctx, int nrows, int iw) {
+    PanelShape p;
+    if (!ctx->panel_clusters || iw > PanelW<R>::v) return p;
+    p = panel_reg_shape(nrows);
+    if (p.C == 0) return p;
     static std::mutex mu;
-    static std::map<std::tuple<int, const void*, int, size_t>, bool> ok;
-    const auto key = std::make_tuple(ctx->device, (const void*)kern, C, (smem + 4095) / 4096);
-    {
-        std::lock_guard<std::mutex> lk(mu);
-        auto it = ok.find(key);
-        if (it != ok.end()) return it->second ? C : 0;
-    }
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PANEL_CLUSTER_SMEM) != cudaSuccess) {
-        cudaGetLastError();
-        return 0;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)C);
-    cfg.blockDim = dim3(PC_THREADS);
-    cfg.dynamicSmemBytes = ((smem + 4095) / 4096) * 4096 < PANEL_CLUSTER_SMEM ? ((smem + 4095) / 4096) * 4096 : smem;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)C;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    int ncl = 0;
-    const bool fits = cudaOccupancyMaxActiveClusters(&ncl, (const void*)kern, &cfg) == cudaSuccess && ncl >= 1;
-    if (!fits) cudaGetLastError();
+    static std::map<std::tuple<int, int, int>, bool> ok;
+    const auto key = std::make_tuple(ctx->device, p.C, p.T);
     std::lock_guard<std::mutex> lk(mu);
-    ok[key] = fits;
-    return fits ? C : 0;
+    auto it = ok.find(key);
+    if (it == ok.end()) {
+        auto kern = panel_reg_kernel<R>;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)p.C);
+        cfg.blockDim = dim3((unsigned)p.T);
+        cfg.dynamicSmemBytes = (size_t)p.T * PR_PITCH;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = (unsigned)p.C;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = 1;
+        int ncl = 0;
+        const bool fits =
+            cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, PR_THREADS * PR_PITCH) == cudaSuccess &&
+            (p.C <= 8 || cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
+            cudaOccupancyMaxActiveClusters(&ncl, (const void*)kern, &cfg) == cudaSuccess && ncl >= 1;
+        if (!fits) cudaGetLastError();
+        it = ok.emplace(key, fits).first;
+    }
+    if (!it->second) p = PanelShape{};
+    return p;
 }
 
-// One launch of panel_cluster_kernel: `batch` matrices (A + i sA, pivots
-// ipiv + i sPiv, info + i), C CTAs per matrix.
+// One launch of panel_reg_kernel: `batch` matrices (A + i sA, pivots
+// ipiv + i n, info + i, moves + 2 i n), one cluster each.
 template <typename R>
-static int launch_panel_cluster(bem_ctx* ctx, typename C2T<R>::type* A, int64_t lda, int i0, int nrows, int iw,
-                                int* d_ipiv, int* d_info, int batch, int64_t sA, int sPiv, int C) {
+static int launch_panel_reg(bem_ctx* ctx, typename C2T<R>::type* A, int64_t lda, int n, int i0, int nrows, int iw,
+                            int* d_ipiv, int* d_info, int* d_moves, int batch, int64_t sA, PanelShape p) {
     using C2 = typename C2T<R>::type;
-    static std::atomic<unsigned long long> attr_set{0};
-    const unsigned long long bit = 1ull << (ctx->device & 63);
-    if (!(attr_set.load() & bit)) {
-        BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(panel_cluster_kernel<R, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)PANEL_CLUSTER_SMEM));
-        BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(panel_cluster_kernel<R, 16>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PANEL_CLUSTER_SMEM));
-        BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(panel_cluster_kernel<R, 32>,
-                                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PANEL_CLUSTER_SMEM));
-        attr_set.fetch_or(bit);
-    }
-    auto kern = iw <= 8 ? panel_cluster_kernel<R, 8> : iw <= 16 ? panel_cluster_kernel<R, 16> : panel_cluster_kernel<R, 32>;
-    const int Rp = (nrows + C - 1) / C;
-    const size_t smem = panel_cluster_smem(Rp, iw, sizeof(C2));
-    if (smem > PANEL_CLUSTER_SMEM || Rp < iw || iw > 32) return fail(ctx, BEM_ERR_INVALID, "cluster panel bound violated");
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(C * batch));
-    cfg.blockDim = dim3(PC_THREADS);
-    cfg.dynamicSmemBytes = smem;
+    cfg.gridDim = dim3((unsigned)(p.C * batch));
+    cfg.blockDim = dim3((unsigned)p.T);
+    cfg.dynamicSmemBytes = (size_t)p.T * PR_PITCH;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = (unsigned)C;
+    at[0].val.clusterDim.x = (unsigned)p.C;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
     cudaEvent_t ev = ctx->prof_begin(PROF_PANEL);
-    BEM_TRY_CUDA(ctx, cudaLaunchKernelEx(&cfg, kern, A, lda, i0, nrows, iw, Rp, d_ipiv, d_info, sA, sPiv));
+    BEM_TRY_CUDA(ctx, cudaLaunchKernelEx(&cfg, panel_reg_kernel<R>, A, lda, n, i0, nrows, iw, d_ipiv, d_info, d_moves, sA));
     BEM_LAUNCHED(ctx);
     if (ev)
         ctx->prof_end(PROF_PANEL, ev, 8.0 * (double)nrows * iw * iw / 2 * batch,
@@ -647,27 +658,100 @@ static int launch_panel_cluster(bem_ctx* ctx, typename C2T<R>::type* A, int64_t 
     return BEM_OK;
 }
 
+// moves of a sub-panel (see panel_reg_kernel) from its interchanges, for the
+// panels of panel_kernel.  One thread per matrix: w <= 32 steps.
+__global__ void moves_kernel(const int* __restrict__ ipiv, int n, int r0, int w, int* __restrict__ moves, int batch) {
+    const int mi = blockIdx.x * blockDim.x + threadIdx.x;
+    if (mi >= batch) return;
+    ipiv += (int64_t)mi * n;
+    moves += (int64_t)mi * 2 * n;
+    // a position below the top is only ever exchanged with a top row, and only top rows go there
+    int top[32], out_row[32], out_of[32], cnt = 0;
+    for (int k = 0; k < w; k++) top[k] = r0 + k;
+    for (int k = 0; k < w; k++) {
+        const int p = ipiv[r0 + k];
+        if (p < r0 + w) {
+            const int t = top[k];
+            top[k] = top[p - r0];
+            top[p - r0] = t;
+            continue;
+        }
+        int e = 0;
+        while (e < cnt && out_row[e] != p) e++;
+        if (e == cnt) out_row[cnt] = p, out_of[cnt] = p, cnt++;
+        const int t = top[k];
+        top[k] = out_of[e];
+        out_of[e] = t;
+    }
+    for (int k = 0; k < w; k++) {
+        moves[r0 + k] = top[k];
+        if (top[k] < r0 + w) moves[n + top[k]] = r0 + k;
+    }
+    for (int e = 0; e < cnt; e++)
+        if (out_of[e] < r0 + w) moves[n + out_of[e]] = out_row[e];
+}
+
 // ------------------------------------------------------------------ laswp
-// Row interchanges k = k0..k1-1 (rows k <-> ipiv[k]) on the columns of up to
-// two ranges [c0a, c1a) and [c0b, c1b); one thread per column.
-template <typename R>
-__global__ void laswp_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, const int* __restrict__ ipiv,
-                             int k0, int k1, int c0a, int c1a, int c0b, int c1b, int64_t sA = 0, int sPiv = 0) {
+// The interchanges of the sub-panels [k0, k1) (w rows each, in order) on the
+// columns of up to two ranges, one thread per column: a sub-panel's rows are
+// all loaded before any is stored (moves names each top position's new row
+// and each displaced row's new position), so its latency is one load instead
+// of one per interchange -- 16 of them per sub-panel, 60 us for the 256 of a
+// block column before.  SOLVE (one sub-panel): the columns of the second
+// range are then solved with the panel's unit lower triangle (U12 of the
+// sub-panel), saving that kernel's launch and its pass over the rows.
+template <typename R, bool SOLVE>
+__global__ void __launch_bounds__(64)
+move_rows_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, const int* __restrict__ moves, int n, int k0,
+                 int k1, int w, int c0a, int c1a, int c0b, int c1b, int64_t sA = 0) {
     using C2 = typename C2T<R>::type;
+    constexpr int W = PanelW<R>::v;
     A += blockIdx.y * sA;  // batched: blockIdx.y selects the matrix
-    ipiv += blockIdx.y * sPiv;
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    int na = c1a - c0a;
-    int c;
-    if (t < na) c = c0a + t;
-    else if (t < na + (c1b - c0b)) c = c0b + (t - na);
-    else return;
-    for (int k = k0; k < k1; k++) {
-        int p = ipiv[k];
-        if (p == k) continue;
-        C2 x = A[(int64_t)k * lda + c];
-        A[(int64_t)k * lda + c] = A[(int64_t)p * lda + c];
-        A[(int64_t)p * lda + c] = x;
+    moves += (int64_t)blockIdx.y * 2 * n;
+    __shared__ C2 sT[SOLVE ? W : 1][W + 1];
+    __shared__ int s_src[W], s_dst[W];
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, na = c1a - c0a;
+    const bool in = t < na + (c1b - c0b), second = t >= na;
+    const int c = second ? c0b + (t - na) : c0a + t;
+    for (int r0 = k0; r0 < k1; r0 += w) {
+        const int iw = min(w, k1 - r0);
+        __syncthreads();
+        if (threadIdx.x < iw) {
+            s_src[threadIdx.x] = moves[r0 + threadIdx.x];
+            s_dst[threadIdx.x] = moves[n + r0 + threadIdx.x];
+        }
+        if (SOLVE)
+            for (int e = threadIdx.x; e < iw * iw; e += blockDim.x)
+                sT[e / iw][e % iw] = A[(int64_t)(r0 + e / iw) * lda + r0 + e % iw];
+        __syncthreads();
+        if (!in) continue;
+        C2 x[W], y[W];
+#pragma unroll
+        for (int k = 0; k < W; k++) {
+            x[k].x = x[k].y = y[k].x = y[k].y = 0;
+            if (k >= iw) continue;
+            if (SOLVE || s_src[k] != r0 + k) x[k] = A[(int64_t)s_src[k] * lda + c];
+            if (s_dst[k] >= r0 + iw) y[k] = A[(int64_t)(r0 + k) * lda + c];
+        }
+        if (SOLVE && second) {
+#pragma unroll
+            for (int k = 0; k < W; k++) {
+                if (k >= iw) break;
+#pragma unroll
+                for (int i = k + 1; i < W; i++) {
+                    if (i >= iw) break;
+                    const C2 l = sT[i][k];
+                    x[i].x -= l.x * x[k].x - l.y * x[k].y;
+                    x[i].y -= l.x * x[k].y + l.y * x[k].x;
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < W; k++) {
+            if (k >= iw) continue;
+            if (s_dst[k] >= r0 + iw) A[(int64_t)s_dst[k] * lda + c] = y[k];
+            if (s_src[k] != r0 + k || (SOLVE && second)) A[(int64_t)(r0 + k) * lda + c] = x[k];
+        }
     }
 }
 
@@ -684,73 +768,6 @@ __global__ void permute_rows_kernel(const typename C2T<R>::type* __restrict__ B,
     int r = (int)(i % n), c = (int)(i / n);
     X[(int64_t)c * ldx + r] = B[(int64_t)c * ldb + (perm ? perm[r] : r)];
 }
-
-// ------------------------------------------------------------ small TRSM
-// Solves T x = b for one TB x TB diagonal block T = A[r0.., r0..] of the
-// row-major factor (UPPER: non-unit upper, backward; else unit lower,
-// forward), for every column in [c0, c1) of the right-hand side held either
-// row-major in the same matrix (B_ROWMAJOR: element (i, c) at
-// B[(r0+i)*ldb + c]) or column-major (B[c*ldb + r0 + i]).  kb <= TB rows.
-template <typename R, int TB, bool UPPER, bool B_ROWMAJOR>
-__global__ void __launch_bounds__(128)
-trsm_small_kernel(const typename C2T<R>::type* __restrict__ T, int64_t ldt, int r0, int kb,
-                  typename C2T<R>::type* __restrict__ B, int64_t ldb, int c0, int c1) {
-    using C2 = typename C2T<R>::type;
-    __shared__ C2 sT[TB][TB + 1];
-    for (int e = threadIdx.x; e < kb * kb; e += blockDim.x) {
-        int i = e / kb, j = e % kb;
-        sT[i][j] = T[(int64_t)(r0 + i) * ldt + r0 + j];
-    }
-    __syncthreads();
-    int c = c0 + blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= c1) return;
-    C2 x[TB];
-#pragma unroll
-    for (int i = 0; i < TB; i++)
-        if (i < kb) x[i] = B_ROWMAJOR ? B[(int64_t)(r0 + i) * ldb + c] : B[(int64_t)c * ldb + r0 + i];
-    if (!UPPER) {
-#pragma unroll
-        for (int i = 1; i < TB; i++) {
-            if (i >= kb) break;
-            C2 s = x[i];
-#pragma unroll
-            for (int k = 0; k < TB; k++) {
-                if (k >= i) break;
-                C2 l = sT[i][k];
-                s.x -= l.x * x[k].x - l.y * x[k].y;
-                s.y -= l.x * x[k].y + l.y * x[k].x;
-            }
-            x[i] = s;
-        }
-    } else {
-#pragma unroll
-        for (int ii = TB - 1; ii >= 0; ii--) {
-            if (ii >= kb) continue;
-            C2 s = x[ii];
-#pragma unroll
-            for (int k = 0; k < TB; k++) {
-                if (k <= ii || k >= kb) continue;
-                C2 u = sT[ii][k];
-                s.x -= u.x * x[k].x - u.y * x[k].y;
-                s.y -= u.x * x[k].y + u.y * x[k].x;
-            }
-            C2 d = sT[ii][ii];
-            R den = d.x * d.x + d.y * d.y;
-            C2 q;
-            q.x = (s.x * d.x + s.y * d.y) / den;
-            q.y = (s.y * d.x - s.x * d.y) / den;
-            x[ii] = q;
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < TB; i++)
-        if (i < kb) {
-            if (B_ROWMAJOR) B[(int64_t)(r0 + i) * ldb + c] = x[i];
-            else B[(int64_t)c * ldb + r0 + i] = x[i];
-        }
-}
-
-template <typename R> struct TBsel { static constexpr int v = 16; };
 
 // ------------------------------------------------------------ block TRSM
 // Solves T X = X for a whole diagonal block T = A[r0.., r0..] (kb <= 256 rows;
@@ -996,7 +1013,7 @@ int getrf(bem_ctx* ctx, typename C2T<R>::type* A, int64_t lda, int n, int* d_ipi
     auto take = [&](size_t b) { size_t o = ws_bytes; ws_bytes += (b + 255) & ~(size_t)255; return o; };
     size_t o_cval = take(2 * (size_t)Gcap * sizeof(R)), o_crow = take(2 * (size_t)Gcap * 4),
            o_cdata = take(2 * (size_t)Gcap * W * sizeof(C2)), o_disp = take(2 * W * sizeof(C2)),
-           o_bar = take(256);
+           o_bar = take(256), o_mv = take(2 * (size_t)n * sizeof(int));
     BEM_TRY(ctx->ensure_ws(ws_bytes));
     char* ws = (char*)ctx->ws;
     PanelWS pw;
@@ -1006,6 +1023,7 @@ int getrf(bem_ctx* ctx, typename C2T<R>::type* A, int64_t lda, int n, int* d_ipi
     pw.disp = ws + o_disp;
     pw.bar = (unsigned*)(ws + o_bar);
     pw.status = ctx->d_status;
+    int* d_moves = (int*)(ws + o_mv);
     BEM_TRY_CUDA(ctx, cudaMemsetAsync(d_info, 0, sizeof(int), ctx->stream));
     BEM_TRY_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
     // FP64: U12 = L11^-1 A12 by 64-row slabs with GEMM updates between them
@@ -1016,9 +1034,9 @@ int getrf(bem_ctx* ctx, typename C2T<R>::type* A, int64_t lda, int n, int* d_ipi
         for (int i0 = j0; i0 < j0 + jb; i0 += W) {
             const int iw = std::min(W, j0 + jb - i0);
             const int nrows = n - i0;
-            const int Cl = panel_cluster_choice<R>(ctx, nrows, iw);
-            if (Cl > 0) {
-                BEM_TRY(launch_panel_cluster<R>(ctx, A, lda, i0, nrows, iw, d_ipiv, d_info, 1, 0, 0, Cl));
+            const PanelShape ps = panel_reg_choice<R>(ctx, nrows, iw);
+            if (ps.C > 0) {
+                BEM_TRY(launch_panel_reg<R>(ctx, A, lda, n, i0, nrows, iw, d_ipiv, d_info, d_moves, 1, 0, ps));
             } else {
                 int G = std::min(Gcap, std::max(1, nrows / iw));
                 G = std::min(G, Gmax_sm);
@@ -1038,19 +1056,20 @@ int getrf(bem_ctx* ctx, typename C2T<R>::type* A, int64_t lda, int n, int* d_ipi
                 if (ev)
                     ctx->prof_end(PROF_PANEL, ev, 8.0 * (double)nrows * iw * iw / 2,
                                   (double)nrows * iw * 2 * sizeof(C2));
+                moves_kernel<<<1, 32, 0, ctx->stream>>>(d_ipiv, n, i0, iw, d_moves, 1);
+                BEM_LAUNCHED(ctx);
             }
-            // interchanges on the rest of this block column
+            // interchanges on the rest of this block column, and the sub-panel's U12
             int ca0 = j0, ca1 = i0, cb0 = i0 + iw, cb1 = j0 + jb;
             int ncol = (ca1 - ca0) + (cb1 - cb0);
             if (ncol > 0) {
                 cudaEvent_t ev = ctx->prof_begin(PROF_PIVOT);
-                laswp_kernel<R><<<(ncol + 255) / 256, 256, 0, ctx->stream>>>(A, lda, d_ipiv, i0, i0 + iw,
-                                                                          ca0, ca1, cb0, cb1);
+                move_rows_kernel<R, true><<<(ncol + 63) / 64, 64, 0, ctx->stream>>>(A, lda, d_moves, n, i0, i0 + iw, iw,
+                                                                                  ca0, ca1, cb0, cb1);
                 BEM_LAUNCHED(ctx);
                 if (ev) ctx->prof_end(PROF_PIVOT, ev, 0.0, 4.0 * sizeof(C2) * iw * (double)ncol);
             }
             if (cb1 > cb0) {
-                BEM_TRY(trsm_rows_lower_unit<R>(ctx, A, lda, i0, iw, cb0, cb1));
                 BEM_TRY(cgemm<R>(ctx, n - i0 - iw, cb1 - cb0, iw, A + (int64_t)(i0 + iw) * lda + i0, lda,
                                  A + (int64_t)i0 * lda + cb0, lda, false,
                                  A + (int64_t)(i0 + iw) * lda + cb0, lda, false, mk<C2>(-1, 0),
@@ -1061,8 +1080,8 @@ int getrf(bem_ctx* ctx, typename C2T<R>::type* A, int64_t lda, int n, int* d_ipi
         int ncol = j0 + (n - j0 - jb);
         if (ncol > 0) {
             cudaEvent_t ev = ctx->prof_begin(PROF_PIVOT);
-            laswp_kernel<R><<<(ncol + 255) / 256, 256, 0, ctx->stream>>>(A, lda, d_ipiv, j0, j0 + jb, 0,
-                                                                      j0, j0 + jb, n);
+            move_rows_kernel<R, false><<<(ncol + 63) / 64, 64, 0, ctx->stream>>>(A, lda, d_moves, n, j0, j0 + jb, W, 0, j0,
+                                                                               j0 + jb, n);
             BEM_LAUNCHED(ctx);
             if (ev) ctx->prof_end(PROF_PIVOT, ev, 0.0, 4.0 * sizeof(C2) * jb * (double)ncol);
         }
@@ -1141,12 +1160,12 @@ int getrf_batched(bem_ctx* ctx, double2* A, int64_t lda, int64_t sA, int n, int 
     using C2 = double2;
     const int NB = shape.NB, W = shape.W;
     if (n < 1 || batch < 1) return fail(ctx, BEM_ERR_INVALID, "batched LU: n=%d batch=%d", n, batch);
-    if (W < 1 || W > 32 || NB < W || NB > TRSM_KB || NB % W != 0)
+    if (W < 1 || W > PanelW<R>::v || NB < W || NB > TRSM_KB || NB % W != 0)
         return fail(ctx, BEM_ERR_INVALID, "batched LU shape NB=%d W=%d", NB, W);
     const size_t smem_max = 220 * 1024;
     // every sub-panel fits one cluster (the first is the tallest): no
     // cooperative grid, no chunking of the batch
-    const bool all_clusters = panel_cluster_choice<R>(ctx, n, W) > 0;
+    const bool all_clusters = panel_reg_choice<R>(ctx, n, W).C > 0;
     const int Rp_max = (int)std::min<int64_t>(n, ((int64_t)smem_max / (int64_t)sizeof(C2) - W) / W);
     if (Rp_max < 2 * W) return fail(ctx, BEM_ERR_INVALID, "batched LU: panel does not fit");
     const int Gm_min = (n + Rp_max - 1) / Rp_max;
@@ -1180,7 +1199,8 @@ int getrf_batched(bem_ctx* ctx, double2* A, int64_t lda, int64_t sA, int n, int 
     auto take = [&](size_t b) { size_t o = ws_bytes; ws_bytes += (b + 255) & ~(size_t)255; return o; };
     const size_t per = (size_t)batch * 2 * Gm;
     size_t o_cval = take(per * sizeof(R)), o_crow = take(per * 4), o_cdata = take(per * W * sizeof(C2)),
-           o_disp = take((size_t)batch * 2 * W * sizeof(C2)), o_bar = take(256);
+           o_disp = take((size_t)batch * 2 * W * sizeof(C2)), o_bar = take(256),
+           o_mv = take((size_t)batch * 2 * n * sizeof(int));
     BEM_TRY(ctx->ensure_ws(ws_bytes));
     char* ws = (char*)ctx->ws;
     PanelWS pw;
@@ -1190,6 +1210,7 @@ int getrf_batched(bem_ctx* ctx, double2* A, int64_t lda, int64_t sA, int n, int 
     pw.disp = ws + o_disp;
     pw.bar = (unsigned*)(ws + o_bar);
     pw.status = ctx->d_status;
+    int* d_moves = (int*)(ws + o_mv);
     BEM_TRY_CUDA(ctx, cudaMemsetAsync(d_info, 0, batch * sizeof(int), ctx->stream));
     BEM_TRY_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
     const C2 m1 = mk<C2>(-1, 0), p1 = mk<C2>(1, 0);
@@ -1200,9 +1221,9 @@ int getrf_batched(bem_ctx* ctx, double2* A, int64_t lda, int64_t sA, int n, int 
         for (int i0 = j0; i0 < j0 + jb; i0 += W) {
             const int iw = std::min(W, j0 + jb - i0);
             const int nrows = n - i0;
-            const int Cl = panel_cluster_choice<R>(ctx, nrows, iw);
-            if (Cl > 0) {
-                BEM_TRY(launch_panel_cluster<R>(ctx, A, lda, i0, nrows, iw, d_ipiv, d_info, batch, sA, n, Cl));
+            const PanelShape ps = panel_reg_choice<R>(ctx, nrows, iw);
+            if (ps.C > 0) {
+                BEM_TRY(launch_panel_reg<R>(ctx, A, lda, n, i0, nrows, iw, d_ipiv, d_info, d_moves, batch, sA, ps));
             } else {
                 int G = std::min(Gm, std::max(1, nrows / iw));
                 const int Rp = (nrows + G - 1) / G;
@@ -1220,18 +1241,19 @@ int getrf_batched(bem_ctx* ctx, double2* A, int64_t lda, int64_t sA, int n, int 
                 if (ev)
                     ctx->prof_end(PROF_PANEL, ev, 8.0 * (double)nrows * iw * iw / 2 * batch,
                                   (double)nrows * iw * 2 * sizeof(C2) * batch);
+                moves_kernel<<<(batch + 31) / 32, 32, 0, ctx->stream>>>(d_ipiv, n, i0, iw, d_moves, batch);
+                BEM_LAUNCHED(ctx);
             }
             const int ca0 = j0, ca1 = i0, cb0 = i0 + iw, cb1 = j0 + jb;
             const int ncol = (ca1 - ca0) + (cb1 - cb0);
             if (ncol > 0) {
                 cudaEvent_t ev = ctx->prof_begin(PROF_PIVOT);
-                laswp_kernel<R><<<dim3((ncol + 255) / 256, batch), 256, 0, ctx->stream>>>(
-                    A, lda, d_ipiv, i0, i0 + iw, ca0, ca1, cb0, cb1, sA, n);
+                move_rows_kernel<R, true><<<dim3((ncol + 63) / 64, batch), 64, 0, ctx->stream>>>(
+                    A, lda, d_moves, n, i0, i0 + iw, iw, ca0, ca1, cb0, cb1, sA);
                 BEM_LAUNCHED(ctx);
                 if (ev) ctx->prof_end(PROF_PIVOT, ev, 0.0, 4.0 * sizeof(C2) * iw * (double)ncol * batch);
             }
             if (cb1 > cb0) {
-                BEM_TRY(trsm_rows_lower_unit<R>(ctx, A, lda, i0, iw, cb0, cb1, batch, sA));
                 BEM_TRY(cgemm<R>(ctx, n - i0 - iw, cb1 - cb0, iw, A + (int64_t)(i0 + iw) * lda + i0, lda,
                                  A + (int64_t)i0 * lda + cb0, lda, false, A + (int64_t)(i0 + iw) * lda + cb0, lda,
                                  false, m1, p1, PROF_PANEL_UPDATE, batch, sA, sA, sA));
@@ -1240,8 +1262,8 @@ int getrf_batched(bem_ctx* ctx, double2* A, int64_t lda, int64_t sA, int n, int 
         const int ncol = j0 + (n - j0 - jb);
         if (ncol > 0) {
             cudaEvent_t ev = ctx->prof_begin(PROF_PIVOT);
-            laswp_kernel<R><<<dim3((ncol + 255) / 256, batch), 256, 0, ctx->stream>>>(A, lda, d_ipiv, j0, j0 + jb, 0,
-                                                                                      j0, j0 + jb, n, sA, n);
+            move_rows_kernel<R, false><<<dim3((ncol + 63) / 64, batch), 64, 0, ctx->stream>>>(A, lda, d_moves, n, j0, j0 + jb,
+                                                                                            W, 0, j0, j0 + jb, n, sA);
             BEM_LAUNCHED(ctx);
             if (ev) ctx->prof_end(PROF_PIVOT, ev, 0.0, 4.0 * sizeof(C2) * jb * (double)ncol * batch);
         }
@@ -1317,7 +1339,7 @@ int tune_lu_shape(bem_ctx* ctx, int n, int batch, LuShape* out) {
         *out = it->second;
         return BEM_OK;
     }
-    const LuShape cands[] = {{256, 16}, {128, 16}, {256, 32}, {128, 32}, {256, 8}, {64, 16}};
+    const LuShape cands[] = {{256, 16}, {128, 16}, {256, 8}, {128, 8}, {64, 16}};
     const size_t nn = (size_t)n * n;
     void* A = devmem_alloc(ctx->device, nn * tb * sizeof(double2), ctx);
     void* ip = devmem_alloc(ctx->device, (size_t)n * tb * sizeof(int) + (size_t)tb * sizeof(int), ctx);
