@@ -55,13 +55,28 @@ int cgemm(bem_ctx* ctx, int M, int N, int K, const typename C2T<R>::type* A, int
     }
     if (batch > 1 && sizeof(R) != 8) return fail(ctx, BEM_ERR_INVALID, "batched GEMM is FP64 only");
     dim3 grid((N + 63) / 64, (M + 63) / 64, batch);
+    // the 3M kernel's tile: the least time of its rounds over the SMs.  A
+    // tile's time goes with its outputs; the smaller tiles reach about 0.8 and
+    // 0.5 of the big one's rate.
+    int tile = 0;
+    if (sizeof(R) == 8 && ctx->dmma_3m) {
+        const int bm[3] = {64, 32, 32}, bn[3] = {64, 32, 8};
+        const double rate[3] = {1.0, 0.8, 0.5};
+        double best = 0.0;
+        for (int t = 0; t < 3; t++) {
+            const int64_t tiles = (int64_t)((M + bm[t] - 1) / bm[t]) * ((N + bn[t] - 1) / bn[t]) * batch;
+            const double cost = (double)((tiles + ctx->sm_count - 1) / ctx->sm_count) * bm[t] * bn[t] / rate[t];
+            if (t == 0 || (cost < best && (M + 31) / 32 <= 65535)) best = cost, tile = t;
+        }
+        grid = dim3((N + bn[tile] - 1) / bn[tile], (M + bm[tile] - 1) / bm[tile], batch);
+    }
     if (grid.y > 65535) return fail(ctx, BEM_ERR_INVALID, "gemm M too large");
     cudaEvent_t ev = prof_cls >= 0 ? ctx->prof_begin(prof_cls) : nullptr;
     if (sizeof(R) == 8) {
         // FP64: the m8n8k4 f64 tensor path (zgemm_dmma.cuh)
         // the attribute is per device: one bit per (kernel variant, device id)
         // (three real products per complex one unless the context asks for four)
-        static std::atomic<unsigned long long> attr[8];
+        static std::atomic<unsigned long long> attr[16];
         const double2* Ad = reinterpret_cast<const double2*>(A);
         const double2* Bd = reinterpret_cast<const double2*>(B);
         double2* Cd = reinterpret_cast<double2*>(C);
@@ -75,15 +90,18 @@ int cgemm(bem_ctx* ctx, int M, int N, int K, const typename C2T<R>::type* A, int
             kern<<<grid, threads, smem, ctx->stream>>>(M, N, K, Ad, lda, Bd, ldb, Cd, ldc, al, be, sA, sB, sC);
             return BEM_OK;
         };
-        const int t4 = 128, s4 = dmma::SMEM_BYTES, t3 = dmma::M3_THREADS, s3 = dmma::M3_SMEM_BYTES;
+        auto go3 = [&](auto tl, int slot) -> int {
+            using T = decltype(tl);
+            if (b_kmajor)
+                return c_colmajor ? go(dmma::zgemm3m_kernel<T, true, true>, slot, T::THREADS, T::SMEM_BYTES)
+                                  : go(dmma::zgemm3m_kernel<T, true, false>, slot + 1, T::THREADS, T::SMEM_BYTES);
+            return c_colmajor ? go(dmma::zgemm3m_kernel<T, false, true>, slot + 2, T::THREADS, T::SMEM_BYTES)
+                              : go(dmma::zgemm3m_kernel<T, false, false>, slot + 3, T::THREADS, T::SMEM_BYTES);
+        };
+        const int t4 = 128, s4 = dmma::SMEM_BYTES;
         int s;
         if (ctx->dmma_3m) {
-            if (b_kmajor)
-                s = c_colmajor ? go(dmma::zgemm3m_kernel<true, true>, 4, t3, s3)
-                               : go(dmma::zgemm3m_kernel<true, false>, 5, t3, s3);
-            else
-                s = c_colmajor ? go(dmma::zgemm3m_kernel<false, true>, 6, t3, s3)
-                               : go(dmma::zgemm3m_kernel<false, false>, 7, t3, s3);
+            s = tile == 0 ? go3(dmma::M3Big{}, 4) : tile == 1 ? go3(dmma::M3Small{}, 8) : go3(dmma::M3Thin{}, 12);
         } else if (b_kmajor) {
             s = c_colmajor ? go(dmma::zgemm_kernel<true, true>, 0, t4, s4) : go(dmma::zgemm_kernel<true, false>, 1, t4, s4);
         } else {

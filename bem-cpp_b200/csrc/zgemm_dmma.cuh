@@ -195,66 +195,77 @@ zgemm_kernel(int M, int N, int K, const double2* __restrict__ A, int64_t lda, co
 
 
 // ----------------------------------------------------------------- 3M form
-constexpr int M3_WM = 2, M3_WN = 4, M3_NJ = 2;  // warps along M / N, 8-column tiles per warp
-constexpr int M3_THREADS = 32 * M3_WM * M3_WN;
-constexpr int M3_AROW = 2 * BKC + 8;   // doubles: 20 16-byte units, 4 mod 8 (conflict-free 128-bit reads)
-constexpr int M3_BROW_K = 2 * BKC + 8;
-constexpr int M3_BROW_N = 2 * BN + 4;  // 66 16-byte units, 2 mod 8
-constexpr int M3_A_STAGE = BM * M3_AROW;
-constexpr int M3_B_STAGE = BN * M3_BROW_K > BKC * M3_BROW_N ? BN * M3_BROW_K : BKC * M3_BROW_N;
-constexpr int M3_SMEM_BYTES = STAGES * (M3_A_STAGE + M3_B_STAGE) * 8;
-static_assert(32 * M3_WM == BM && 8 * M3_NJ * M3_WN == BN, "3M tile");
+// Tile of the 3M kernel: BM x BN complex outputs, WM x WN warps (each
+// BM / WM x BN / WN).  An SM gives ~125 G FP64 multiply-adds a second, so a
+// 64 x 64 tile of K = 256 takes 50 us on it: products with fewer such tiles
+// than SMs (the block updates of a solve with few right-hand sides) run on
+// smaller tiles that reach every SM.  An output's sums run over k in the same
+// order in every tile, so the tiles give the same bits.
+template <int BM_, int BN_, int WM_, int WN_, int MINB_> struct M3Tile {
+    static constexpr int BM = BM_, BN = BN_, WM = WM_, WN = WN_, MINB = MINB_;
+    static constexpr int THREADS = 32 * WM * WN, IM = BM / WM / 8, NJ = BN / WN / 8;
+    static constexpr int AROW = 2 * BKC + 8;    // doubles: 20 16-byte units, 4 mod 8 (conflict-free 128-bit reads)
+    static constexpr int BROW_K = 2 * BKC + 8;
+    static constexpr int BROW_N = 2 * BN + 4;   // 2 mod 8 16-byte units
+    static constexpr int A_STAGE = BM * AROW;
+    static constexpr int B_STAGE = BN * BROW_K > BKC * BROW_N ? BN * BROW_K : BKC * BROW_N;
+    static constexpr int SMEM_BYTES = STAGES * (A_STAGE + B_STAGE) * 8;
+    static_assert(BM % (8 * WM) == 0 && BN % (8 * WN) == 0, "3M tile");
+    static_assert(BM * BKC % THREADS == 0 && BN * BKC % THREADS == 0, "3M tile loads");
+};
+using M3Big = M3Tile<64, 64, 2, 4, 2>;
+using M3Small = M3Tile<32, 32, 2, 2, 4>;
+using M3Thin = M3Tile<32, 8, 4, 1, 4>;
 
-template <bool B_KMAJOR, bool C_COLMAJOR>
-__global__ void __launch_bounds__(M3_THREADS, 2)
+template <class T, bool B_KMAJOR, bool C_COLMAJOR>
+__global__ void __launch_bounds__(T::THREADS, T::MINB)
 zgemm3m_kernel(int M, int N, int K, const double2* __restrict__ A, int64_t lda, const double2* __restrict__ B,
                int64_t ldb, double2* __restrict__ C, int64_t ldc, double2 alpha, double2 beta, int64_t sA = 0,
                int64_t sB = 0, int64_t sC = 0) {
-    constexpr int NJ = M3_NJ;
+    constexpr int NJ = T::NJ, IM = T::IM;
     A += blockIdx.z * sA;
     B += blockIdx.z * sB;
     C += blockIdx.z * sC;
     extern __shared__ __align__(16) double sm[];
-    double* As = sm;                          // STAGES x M3_A_STAGE
-    double* Bs = sm + STAGES * M3_A_STAGE;    // STAGES x M3_B_STAGE
+    double* As = sm;                          // STAGES x A_STAGE
+    double* Bs = sm + STAGES * T::A_STAGE;    // STAGES x B_STAGE
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = (warp / M3_WN) * 32, wn = (warp % M3_WN) * 8 * NJ;  // warp tile origin (complex)
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+    const int wm = (warp / T::WN) * 8 * IM, wn = (warp % T::WN) * 8 * NJ;  // warp tile origin (complex)
+    const int m0 = blockIdx.y * T::BM, n0 = blockIdx.x * T::BN;
     const int nst = (K + BKC - 1) / BKC;
 
     auto load_stage = [&](int st, int buf) {
         const int k0 = st * BKC;
-        double* as = As + buf * M3_A_STAGE;
-        double* bs = Bs + buf * M3_B_STAGE;
-        // A and B: 64 rows x 16 complex each = 1024 copies of 16 B, 4 per thread
+        double* as = As + buf * T::A_STAGE;
+        double* bs = Bs + buf * T::B_STAGE;
 #pragma unroll
-        for (int l = 0; l < BM * BKC / M3_THREADS; l++) {
-            const int e = tid + M3_THREADS * l;
+        for (int l = 0; l < T::BM * BKC / T::THREADS; l++) {
+            const int e = tid + T::THREADS * l;
             const int r = e >> 4, kc = e & 15;
             const int gi = m0 + r, gk = k0 + kc;
             const bool ok = gi < M && gk < K;
-            cp16(as + r * M3_AROW + 2 * kc, A + (ok ? (int64_t)gi * lda + gk : 0), ok);
+            cp16(as + r * T::AROW + 2 * kc, A + (ok ? (int64_t)gi * lda + gk : 0), ok);
         }
 #pragma unroll
-        for (int l = 0; l < BN * BKC / M3_THREADS; l++) {
-            const int e = tid + M3_THREADS * l;
+        for (int l = 0; l < T::BN * BKC / T::THREADS; l++) {
+            const int e = tid + T::THREADS * l;
             if (B_KMAJOR) {
                 const int j = e >> 4, kc = e & 15;
                 const int gj = n0 + j, gk = k0 + kc;
                 const bool ok = gj < N && gk < K;
-                cp16(bs + j * M3_BROW_K + 2 * kc, B + (ok ? (int64_t)gj * ldb + gk : 0), ok);
+                cp16(bs + j * T::BROW_K + 2 * kc, B + (ok ? (int64_t)gj * ldb + gk : 0), ok);
             } else {
-                const int kr = e >> 6, j = e & 63;
+                const int kr = e / T::BN, j = e % T::BN;
                 const int gj = n0 + j, gk = k0 + kr;
                 const bool ok = gj < N && gk < K;
-                cp16(bs + kr * M3_BROW_N + 2 * j, B + (ok ? (int64_t)gk * ldb + gj : 0), ok);
+                cp16(bs + kr * T::BROW_N + 2 * j, B + (ok ? (int64_t)gk * ldb + gj : 0), ok);
             }
         }
     };
 
-    double t1[4][NJ][2], t2[4][NJ][2], t3[4][NJ][2];
+    double t1[IM][NJ][2], t2[IM][NJ][2], t3[IM][NJ][2];
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+    for (int i = 0; i < IM; i++)
 #pragma unroll
         for (int j = 0; j < NJ; j++)
 #pragma unroll
@@ -275,15 +286,15 @@ zgemm3m_kernel(int M, int N, int K, const double2* __restrict__ A, int64_t lda, 
             cp_commit();
         }
         const int buf = st % STAGES;
-        const double* as = As + buf * M3_A_STAGE;
-        const double* bs = Bs + buf * M3_B_STAGE;
+        const double* as = As + buf * T::A_STAGE;
+        const double* bs = Bs + buf * T::B_STAGE;
 #pragma unroll
         for (int kk = 0; kk < BKC / 4; kk++) {  // complex K steps of 4
             const int kc = 4 * kk + fk;
-            double ar[4], ai[4], asum[4], br[NJ], bi[NJ], bsum[NJ];
+            double ar[IM], ai[IM], asum[IM], br[NJ], bi[NJ], bsum[NJ];
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-                const double2 v = *reinterpret_cast<const double2*>(as + (wm + 8 * i + fr) * M3_AROW + 2 * kc);
+            for (int i = 0; i < IM; i++) {
+                const double2 v = *reinterpret_cast<const double2*>(as + (wm + 8 * i + fr) * T::AROW + 2 * kc);
                 ar[i] = v.x;
                 ai[i] = v.y;
                 asum[i] = v.x + v.y;
@@ -291,14 +302,14 @@ zgemm3m_kernel(int M, int N, int K, const double2* __restrict__ A, int64_t lda, 
 #pragma unroll
             for (int j = 0; j < NJ; j++) {
                 const int n = wn + 8 * j + fr;
-                const double2 v = B_KMAJOR ? *reinterpret_cast<const double2*>(bs + n * M3_BROW_K + 2 * kc)
-                                           : *reinterpret_cast<const double2*>(bs + kc * M3_BROW_N + 2 * n);
+                const double2 v = B_KMAJOR ? *reinterpret_cast<const double2*>(bs + n * T::BROW_K + 2 * kc)
+                                           : *reinterpret_cast<const double2*>(bs + kc * T::BROW_N + 2 * n);
                 br[j] = v.x;
                 bi[j] = v.y;
                 bsum[j] = v.x + v.y;
             }
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < IM; i++)
 #pragma unroll
                 for (int j = 0; j < NJ; j++) {
                     dmma(t1[i][j][0], t1[i][j][1], ar[i], br[j]);
@@ -311,7 +322,7 @@ zgemm3m_kernel(int M, int N, int K, const double2* __restrict__ A, int64_t lda, 
     // epilogue: thread holds C(row 8i + lane/4, cols 8j + 2(lane%4) + {0,1})
     const bool has_beta = beta.x != 0.0 || beta.y != 0.0;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
+    for (int i = 0; i < IM; i++) {
         const int gi = m0 + wm + 8 * i + fr;
         if (gi >= M) continue;
 #pragma unroll
