@@ -1012,50 +1012,8 @@ __global__ void pack_b_row_kernel(const float2* __restrict__ B, int64_t ldb, int
 
 // ---------------------------------------------------------------- FP16 split
 // Scale of one operand row (A') or complex column (B): the power of two s
-// with s * max(|Re|, |Im|) in [2^14, 2^15), stored with its inverse as
-// sc[t] = (s, 1/s).  Element k of item t is X[t * si + k * sk], times
-// dsc[k * dstride] when dsc is given (the D of an L D L^T update, applied as
-// the pack kernel applies it).  per_warp: one warp per item, lanes over k
-// (k contiguous); else 32 items per block of 256 threads (items contiguous
-// across the lanes of a warp), the 8 warps over interleaved k, reduced in
-// shared memory.
-__global__ void f16_scale_kernel(const float2* __restrict__ X, int64_t si, int64_t sk, int n, int K,
-                                 const float2* __restrict__ dsc, int64_t dstride, int per_warp,
-                                 float2* __restrict__ sc) {
-    float m = 0.f;
-    int t;
-    int k0 = 0, kstep = 1;
-    if (per_warp) {
-        t = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-        k0 = threadIdx.x & 31;
-        kstep = 32;
-    } else {
-        t = (int)blockIdx.x * 32 + (int)(threadIdx.x & 31);
-        k0 = (int)(threadIdx.x >> 5);
-        kstep = (int)(blockDim.x >> 5);
-    }
-    if (t < n) {
-        for (int k = k0; k < K; k += kstep) {
-            float2 x = X[(int64_t)t * si + (int64_t)k * sk];
-            if (dsc) {
-                const float2 d = dsc[(int64_t)k * dstride];
-                x = make_float2(x.x * d.x - x.y * d.y, x.x * d.y + x.y * d.x);
-            }
-            m = fmaxf(m, fmaxf(fabsf(x.x), fabsf(x.y)));
-        }
-    }
-    if (per_warp) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if ((threadIdx.x & 31) != 0) return;
-    } else {
-        __shared__ float part[32][33];
-        part[threadIdx.x >> 5][threadIdx.x & 31] = m;
-        __syncthreads();
-        if (threadIdx.x >= 32) return;
-        for (int w = 1; w < (int)(blockDim.x >> 5); w++) m = fmaxf(m, part[w][threadIdx.x]);
-    }
-    if (t >= n) return;
+// with s * max(|Re|, |Im|) in [2^14, 2^15), stored with its inverse as (s, 1/s).
+__device__ __forceinline__ float2 f16_scale(float m) {
     float sv = 1.f, inv = 1.f;
     if (m > 0.f && m <= 3.0e38f) {
         int e;
@@ -1064,7 +1022,33 @@ __global__ void f16_scale_kernel(const float2* __restrict__ X, int64_t si, int64
         sv = ldexpf(1.f, 15 - e);
         inv = ldexpf(1.f, e - 15);
     }
-    sc[t] = make_float2(sv, inv);
+    return make_float2(sv, inv);
+}
+
+// Scales of 32 items t0.. whose elements are strided (element k of item t at
+// X[k * sk + t]): lanes over the items, the block's 8 warps over interleaved k.
+__device__ __forceinline__ void f16_scale_strided(const float2* __restrict__ X, int64_t sk, int n, int K, int t0,
+                                                  float2* __restrict__ sc) {
+    __shared__ float part[8][33];
+    const int t = t0 + (int)(threadIdx.x & 31), w = (int)(threadIdx.x >> 5);
+    float m = 0.f;
+    if (t < n) {
+#pragma unroll 8
+        for (int k = w; k < K; k += 8) {
+            const float2 x = X[(int64_t)k * sk + t];
+            m = fmaxf(m, fmaxf(fabsf(x.x), fabsf(x.y)));
+        }
+    }
+    part[w][threadIdx.x & 31] = m;
+    __syncthreads();
+    if (threadIdx.x >= 32 || t >= n) return;
+    for (int v = 1; v < 8; v++) m = fmaxf(m, part[v][threadIdx.x]);
+    sc[t] = f16_scale(m);
+}
+
+__global__ void __launch_bounds__(256) f16_scale_kernel(const float2* __restrict__ X, int64_t sk, int n, int K,
+                                                        float2* __restrict__ sc) {
+    f16_scale_strided(X, sk, n, K, (int)blockIdx.x * 32, sc);
 }
 
 __device__ __forceinline__ void split_h(float x, __half& h, __half& l) {
@@ -1072,21 +1056,117 @@ __device__ __forceinline__ void split_h(float x, __half& h, __half& l) {
     l = __float2half_rn(x - __half2float(h));
 }
 
-// The FP16 counterparts of the four pack kernels above: same layouts, each
-// value multiplied by its row's (A) or column's (B) scale first.
-__global__ void pack_a_h_kernel(const float2* __restrict__ A, int64_t lda, int M, int K, __half* __restrict__ hi,
-                                __half* __restrict__ lo, int ld, const float2* __restrict__ sc) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int64_t tot = (int64_t)M * (ld / 2);
-    if (t >= tot) return;
-    int i = (int)(t / (ld / 2)), k = (int)(t % (ld / 2));
-    float2 a = k < K ? A[(int64_t)i * lda + k] : make_float2(0.f, 0.f);
-    const float s = sc[i].x;
-    __half h0, h1, l0, l1;
-    split_h(a.x * s, h0, l0);
-    split_h(a.y * s, h1, l1);
-    reinterpret_cast<__half2*>(hi + (int64_t)i * ld)[k] = __halves2half2(h0, h1);
-    reinterpret_cast<__half2*>(lo + (int64_t)i * ld)[k] = __halves2half2(l0, l1);
+// The FP16 counterparts of the pack kernels above: same layouts, each value
+// multiplied by its row's (A) or column's (B) scale first.
+//
+// Operands with contiguous k, A's rows and B's columns, in one launch: a warp
+// takes an item, finds its largest part, and writes its scale and its planes
+// from the registers that hold it (CACHED, K <= PACK_K) or from a second read.
+// Items [0, na) are rows of A, [na, na + N) columns of B.  dsc (B only, the D
+// of an L D L^T update): element k is multiplied by dsc[k * dstride] first.
+// Blocks past the items scale a transposed A, 32 rows each (ts > 0), for
+// pack_a_trans_h_kernel.  A GEMM of the L D L^T solves is ~60 us between four
+// launches of 4 to 8 us each with the scale and the pack of each operand apart.
+constexpr int PACK_K = 1024;
+struct PackRows {
+    const float2 *A, *B, *dsc;
+    int64_t lda, ldb, dstride;
+    int na, N, K, ld, row_blocks, ts;
+    __half *ah, *al, *bh, *bl;
+    float2 *sc_a, *sc_b;
+};
+
+template <bool CACHED>
+__global__ void __launch_bounds__(256) pack_rows_h_kernel(PackRows p) {
+    if ((int)blockIdx.x >= p.row_blocks) {
+        f16_scale_strided(p.A, p.lda, p.ts, p.K, ((int)blockIdx.x - p.row_blocks) * 32, p.sc_a);
+        return;
+    }
+    extern __shared__ __align__(16) float2 s_d[];  // dsc, K values
+    if (p.dsc) {
+        for (int k = threadIdx.x; k < p.K; k += blockDim.x) s_d[k] = p.dsc[(int64_t)k * p.dstride];
+        __syncthreads();
+    }
+    const int item = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (item >= p.na + p.N) return;
+    const bool isb = item >= p.na;
+    const int t = isb ? item - p.na : item;
+    const float2* src = isb ? p.B + (int64_t)t * p.ldb : p.A + (int64_t)t * p.lda;
+    const bool vec = (reinterpret_cast<uintptr_t>(src) & 15) == 0;
+    const int K = p.K, Kp = p.ld / 2;
+    // complex elements k, k + 1 of the item
+    auto load = [&](int k) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (vec && k + 1 < K) {
+            v = *reinterpret_cast<const float4*>(src + k);
+        } else {
+            if (k < K) { const float2 x = src[k]; v.x = x.x, v.y = x.y; }
+            if (k + 1 < K) { const float2 x = src[k + 1]; v.z = x.x, v.w = x.y; }
+        }
+        if (isb && p.dsc && k < K) {
+            const float2 d0 = s_d[k];
+            const float2 x = make_float2(v.x * d0.x - v.y * d0.y, v.x * d0.y + v.y * d0.x);
+            v.x = x.x, v.y = x.y;
+            if (k + 1 < K) {
+                const float2 d1 = s_d[k + 1];
+                const float2 y = make_float2(v.z * d1.x - v.w * d1.y, v.z * d1.y + v.w * d1.x);
+                v.z = y.x, v.w = y.y;
+            }
+        }
+        return v;
+    };
+    constexpr int NV = CACHED ? PACK_K / 64 : 1;
+    float4 c[NV];
+    float m = 0.f;
+    if (CACHED) {
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+            const int k = 2 * lane + 64 * i;
+            c[i] = k < K ? load(k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int i = 0; i < NV; i++)
+            m = fmaxf(fmaxf(m, fmaxf(fabsf(c[i].x), fabsf(c[i].y))), fmaxf(fabsf(c[i].z), fabsf(c[i].w)));
+    } else {
+        for (int k = 2 * lane; k < K; k += 64) {
+            const float4 v = load(k);
+            m = fmaxf(fmaxf(m, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    const float2 sc = f16_scale(m);
+    if (lane == 0) (isb ? p.sc_b : p.sc_a)[t] = sc;
+    auto store = [&](int k, float4 v) {
+        __half h[4], l[4];
+        split_h(v.x * sc.x, h[0], l[0]);
+        split_h(v.y * sc.x, h[1], l[1]);
+        split_h(v.z * sc.x, h[2], l[2]);
+        split_h(v.w * sc.x, h[3], l[3]);
+        auto put = [&](__half* plane, int64_t row, __half a0, __half a1, __half a2, __half a3) {
+            __half2 q[2] = {__halves2half2(a0, a1), __halves2half2(a2, a3)};
+            *reinterpret_cast<uint2*>(plane + row * p.ld + 2 * k) = *reinterpret_cast<const uint2*>(q);
+        };
+        if (isb) {
+            put(p.bh, 2 * (int64_t)t, h[0], __hneg(h[1]), h[2], __hneg(h[3]));
+            put(p.bh, 2 * (int64_t)t + 1, h[1], h[0], h[3], h[2]);
+            put(p.bl, 2 * (int64_t)t, l[0], __hneg(l[1]), l[2], __hneg(l[3]));
+            put(p.bl, 2 * (int64_t)t + 1, l[1], l[0], l[3], l[2]);
+        } else {
+            put(p.ah, t, h[0], h[1], h[2], h[3]);
+            put(p.al, t, l[0], l[1], l[2], l[3]);
+        }
+    };
+    // the planes' rows are padded with zeros to ld (a multiple of 64 halves)
+    if (CACHED) {
+#pragma unroll
+        for (int i = 0; i < NV; i++) {
+            const int k = 2 * lane + 64 * i;
+            if (k < Kp) store(k, c[i]);
+        }
+    } else {
+        for (int k = 2 * lane; k < Kp; k += 64) store(k, k < K ? load(k) : make_float4(0.f, 0.f, 0.f, 0.f));
+    }
 }
 
 __global__ void pack_a_trans_h_kernel(const float2* __restrict__ At, int64_t lda, int M, int K,
@@ -1111,28 +1191,6 @@ __global__ void pack_a_trans_h_kernel(const float2* __restrict__ At, int64_t lda
         reinterpret_cast<__half2*>(hi + (int64_t)i * ld)[k] = __halves2half2(h0, h1);
         reinterpret_cast<__half2*>(lo + (int64_t)i * ld)[k] = __halves2half2(l0, l1);
     }
-}
-
-__global__ void pack_b_col_h_kernel(const float2* __restrict__ B, int64_t ldb, int N, int K, __half* __restrict__ hi,
-                                    __half* __restrict__ lo, int ld, const float2* __restrict__ dsc,
-                                    int64_t dstride, const float2* __restrict__ sc) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    int64_t tot = (int64_t)N * (ld / 2);
-    if (t >= tot) return;
-    int j = (int)(t / (ld / 2)), k = (int)(t % (ld / 2));
-    float2 b = k < K ? B[(int64_t)j * ldb + k] : make_float2(0.f, 0.f);
-    if (dsc && k < K) {
-        const float2 d = dsc[(int64_t)k * dstride];
-        b = make_float2(b.x * d.x - b.y * d.y, b.x * d.y + b.y * d.x);
-    }
-    const float s = sc[j].x;
-    __half hr, hm, lr, lm;
-    split_h(b.x * s, hr, lr);
-    split_h(b.y * s, hm, lm);
-    reinterpret_cast<__half2*>(hi + (int64_t)(2 * j) * ld)[k] = __halves2half2(hr, __hneg(hm));
-    reinterpret_cast<__half2*>(hi + (int64_t)(2 * j + 1) * ld)[k] = __halves2half2(hm, hr);
-    reinterpret_cast<__half2*>(lo + (int64_t)(2 * j) * ld)[k] = __halves2half2(lr, __hneg(lm));
-    reinterpret_cast<__half2*>(lo + (int64_t)(2 * j + 1) * ld)[k] = __halves2half2(lm, lr);
 }
 
 __global__ void pack_b_row_h_kernel(const float2* __restrict__ B, int64_t ldb, int N, int K, __half* __restrict__ hi,
@@ -1231,38 +1289,35 @@ int tc_gemm_ex(bem_ctx* ctx, int M, int N, int K, const float2* A, int64_t lda, 
     float2* sc_b = f16 ? sc_a + M : nullptr;
     cudaEvent_t ev = prof_cls >= 0 ? ctx->prof_begin(prof_cls) : nullptr;
     if (f16) {
-        // scales: rows of A (k contiguous unless A comes transposed), complex columns of B
-        if (o.a_trans)
-            tc::f16_scale_kernel<<<(M + 31) / 32, 256, 0, ctx->stream>>>(A, 1, lda, M, K, nullptr, 0, 0, sc_a);
-        else
-            tc::f16_scale_kernel<<<(unsigned)(((int64_t)M * 32 + 255) / 256), 256, 0, ctx->stream>>>(
-                A, lda, 1, M, K, nullptr, 0, 1, sc_a);
-        BEM_LAUNCHED(ctx);
-        if (b_rowmajor)
-            tc::f16_scale_kernel<<<(N + 31) / 32, 256, 0, ctx->stream>>>(B, 1, ldb, N, K, nullptr, 0, 0, sc_b);
-        else
-            tc::f16_scale_kernel<<<(unsigned)(((int64_t)N * 32 + 255) / 256), 256, 0, ctx->stream>>>(
-                B, ldb, 1, N, K, o.bscale, o.bscale_stride, 1, sc_b);
-        BEM_LAUNCHED(ctx);
         __half *ah = (__half*)a_hi, *al = (__half*)a_lo, *bh = (__half*)b_hi, *bl = (__half*)b_lo;
+        // operands with contiguous k: scaled and packed in one launch, with the scales of a transposed A
+        tc::PackRows pr;
+        pr.A = A, pr.lda = lda, pr.B = B, pr.ldb = ldb, pr.dsc = o.bscale, pr.dstride = o.bscale_stride;
+        pr.na = o.a_trans ? 0 : M, pr.N = b_rowmajor ? 0 : N, pr.K = K, pr.ld = ld;
+        pr.ah = ah, pr.al = al, pr.bh = bh, pr.bl = bl, pr.sc_a = sc_a, pr.sc_b = sc_b;
+        pr.row_blocks = (pr.na + pr.N + 7) / 8;
+        pr.ts = o.a_trans ? M : 0;
+        const int blocks = pr.row_blocks + (pr.ts + 31) / 32;
+        const size_t dsm = o.bscale ? (size_t)K * sizeof(float2) : 0;
+        if (blocks > 0) {
+            auto kern = K <= tc::PACK_K ? tc::pack_rows_h_kernel<true> : tc::pack_rows_h_kernel<false>;
+            if (dsm > 48 * 1024)
+                BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm));
+            kern<<<blocks, 256, dsm, ctx->stream>>>(pr);
+            BEM_LAUNCHED(ctx);
+        }
         if (o.a_trans) {
             dim3 g((M + 31) / 32, (ld / 2 + 31) / 32);
             tc::pack_a_trans_h_kernel<<<g, 256, 0, ctx->stream>>>(A, lda, M, K, ah, al, ld, sc_a);
-        } else {
-            int64_t tot = (int64_t)M * (ld / 2);
-            tc::pack_a_h_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, ctx->stream>>>(A, lda, M, K, ah, al, ld,
-                                                                                       sc_a);
+            BEM_LAUNCHED(ctx);
         }
-        BEM_LAUNCHED(ctx);
         if (b_rowmajor) {
+            tc::f16_scale_kernel<<<(N + 31) / 32, 256, 0, ctx->stream>>>(B, ldb, N, K, sc_b);
+            BEM_LAUNCHED(ctx);
             dim3 g((N + 31) / 32, (ld / 2 + 31) / 32);
             tc::pack_b_row_h_kernel<<<g, 256, 0, ctx->stream>>>(B, ldb, N, K, bh, bl, ld, sc_b);
-        } else {
-            int64_t tot = (int64_t)N * (ld / 2);
-            tc::pack_b_col_h_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, ctx->stream>>>(
-                B, ldb, N, K, bh, bl, ld, o.bscale, o.bscale_stride, sc_b);
+            BEM_LAUNCHED(ctx);
         }
-        BEM_LAUNCHED(ctx);
     } else {
         float *ah = (float*)a_hi, *al = (float*)a_lo, *bh = (float*)b_hi, *bl = (float*)b_lo;
         if (o.a_trans) {
