@@ -758,9 +758,7 @@ move_rows_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, const int* 
 #pragma unroll
                 for (int i = k + 1; i < W; i++) {
                     if (i >= iw) break;
-                    const C2 l = sT[i][k];
-                    x[i].x -= l.x * x[k].x - l.y * x[k].y;
-                    x[i].y -= l.x * x[k].y + l.y * x[k].x;
+                    x[i] = panel_msub(x[i], sT[i][k], x[k]);
                 }
             }
         }
@@ -827,9 +825,8 @@ __device__ __forceinline__ float2 shfl_c(float2 v, int k) {
 __device__ __forceinline__ double2 shfl_c(double2 v, int k) {
     return make_double2(__shfl_sync(0xffffffffu, v.x, k), __shfl_sync(0xffffffffu, v.y, k));
 }
-template <typename C2> __device__ __forceinline__ void csub_mul(C2& x, C2 a, C2 b) {  // x -= a b
-    x.x -= a.x * b.x - a.y * b.y;
-    x.y -= a.x * b.y + a.y * b.x;
+template <typename C2> __device__ __forceinline__ void csub_mul(C2& x, C2 a, C2 b) {  // x -= a b, four fused operations
+    x = panel_msub(x, a, b);
 }
 
 template <typename R, bool UPPER, bool B_ROWMAJOR, int RB, int MODE = 0>
@@ -1517,16 +1514,12 @@ ldlt_diag_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int j0, int
                 one.x = 1;
                 one.y = 0;
                 const C2 inv = zp ? zero : cdiv(one, d);
-                C2 l;
-                l.x = x[0].x * inv.x - x[0].y * inv.y;
-                l.y = x[0].x * inv.y + x[0].y * inv.x;
+                const C2 l = panel_mul(x[0], inv);
                 // a[i][c] -= l_i (d l_c), d l_c being the unscaled a[c][jj]
 #pragma unroll
                 for (int c = 1; c < LDLT_SP; c++) {
                     if (jj + c < w) {
-                        const C2 u = s_col[par][jj + c];
-                        x[c].x -= l.x * u.x - l.y * u.y;
-                        x[c].y -= l.x * u.y + l.y * u.x;
+                        x[c] = panel_msub(x[c], l, s_col[par][jj + c]);
                     }
                 }
                 x[0] = l;
@@ -1548,10 +1541,7 @@ ldlt_diag_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int j0, int
             for (int e = tid; e < w * rest; e += LDLT_THREADS) {
                 const int k = e / rest, c = e % rest;
                 const C2 dk = P[k * LDLT_PITCH + k], lc = P[(w + c) * LDLT_PITCH + k];
-                C2 t;
-                t.x = dk.x * lc.x - dk.y * lc.y;
-                t.y = dk.x * lc.y + dk.y * lc.x;
-                T[k * LDLT_TP + c] = t;
+                T[k * LDLT_TP + c] = panel_mul(dk, lc);
             }
             __syncthreads();
             // 128 x 64 output blocks of the lower triangle, 8 x 4 per thread
@@ -1581,10 +1571,7 @@ ldlt_diag_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int j0, int
 #pragma unroll
                         for (int r = 0; r < 8; r++)
 #pragma unroll
-                            for (int c = 0; c < 4; c++) {
-                                acc[r][c].x -= a[r].x * b[c].x - a[r].y * b[c].y;
-                                acc[r][c].y -= a[r].x * b[c].y + a[r].y * b[c].x;
-                            }
+                            for (int c = 0; c < 4; c++) acc[r][c] = panel_msub(acc[r][c], a[r], b[c]);
                     }
 #pragma unroll
                     for (int r = 0; r < 8; r++)
@@ -1603,11 +1590,14 @@ ldlt_diag_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int j0, int
 // block kept in distributed shared memory: CTA q holds block rows
 // 32q..32q+31, columns 0..32q+31, so no entry makes a round trip through
 // L2 between sub-panels.  Per 32-column sub-panel p:
-//   A. CTA p factors the 32 x 32 diagonal sub-block with one warp (lane i:
-//      row i, column by column), keeping the unscaled column entries in U;
+//   A. CTA p factors the 32 x 32 diagonal sub-block, column by column with
+//      a block barrier each: its 8 warps hold four rows each, a lane per
+//      column, so a column is one multiply-add per row and lane instead of 31 (277 us per block with one warp holding a row per lane,
+//      here and in B); the unscaled column entries go to U;
 //   cluster barrier;
 //   B. every CTA q > p copies U and the pivots from CTA p and eliminates
-//      the sub-panel columns of its own rows (one thread per row);
+//      the sub-panel columns of its own rows (four rows per warp, a lane per
+//      column);
 //   cluster barrier;
 //   C. every CTA q > p updates its rows' lower triangle right of the
 //      sub-panel: T = D L^T of block rows 32(p+1)..32q+31 is gathered from
@@ -1661,40 +1651,46 @@ ldlt_diag_cluster_kernel(float2* __restrict__ A, int64_t lda, int j0, int jb, in
     const int np = (jb + LDC_ROWS - 1) / LDC_ROWS;
     for (int p = 0; p < np; p++) {
         const int c0 = p * LDC_ROWS, w = min(LDC_ROWS, jb - c0);
-        // A. the diagonal sub-block (rows c0.. of the block are this CTA's rows 0..w-1)
-        if (q == p && wid == 0) {
-            const int i = lane;
-            const bool act = i < w;
-            float2 x[LDC_ROWS];  // x[c] = a[i][jj + c], shifted left as columns retire
+        // A. the diagonal sub-block (rows c0.. of the block are this CTA's rows 0..w-1):
+        // warp: four rows, lane: column (the lower triangle counts); a column's
+        // unscaled entries are published by the lane that holds it
+        if (q == p) {
+            float2 x[4];
 #pragma unroll
-            for (int c = 0; c < LDC_ROWS; c++) x[c] = (act && c < w) ? S[i * LDC_PITCH + c0 + c] : zero;
+            for (int r = 0; r < 4; r++) {
+                const int i = wid * 4 + r;
+                x[r] = zero;
+                if (i < w && lane <= i) x[r] = S[i * LDC_PITCH + c0 + lane];
+            }
             for (int jj = 0; jj < w; jj++) {
-                const int par = jj & 1;
-                if (act) s_col[par * LDC_ROWS + i] = x[0];
-                __syncwarp();
-                const float2 d = s_col[par * LDC_ROWS + jj];
-                const bool zp = (d.x == 0 && d.y == 0);
-                if (zp && i == jj) atomicCAS(info, 0, j0 + c0 + jj + 1);
-                if (act && i > jj) {
-                    const float2 inv = zp ? zero : cdiv(one, d);
-                    float2 l;
-                    l.x = x[0].x * inv.x - x[0].y * inv.y;
-                    l.y = x[0].x * inv.y + x[0].y * inv.x;
+                float2* col = s_col + (jj & 1) * LDC_ROWS;
+                if (lane == jj) {
 #pragma unroll
-                    for (int c = 1; c < LDC_ROWS; c++) {
-                        if (jj + c < w) {
-                            const float2 u = s_col[par * LDC_ROWS + jj + c];
-                            x[c].x -= l.x * u.x - l.y * u.y;
-                            x[c].y -= l.x * u.y + l.y * u.x;
+                    for (int r = 0; r < 4; r++) col[wid * 4 + r] = x[r];
+                }
+                __syncthreads();
+                const float2 d = col[jj], u = col[lane];
+                const bool zp = (d.x == 0 && d.y == 0);
+                if (zp && tid == 0) atomicCAS(info, 0, j0 + c0 + jj + 1);
+                const float2 inv = zp ? zero : cdiv(one, d);
+#pragma unroll
+                for (int r = 0; r < 4; r++) {
+                    const int i = wid * 4 + r;
+                    const float2 a = col[i];
+                    const float2 l = panel_mul(a, inv);
+                    if (i > jj) {
+                        if (lane > jj) csub_mul(x[r], l, u);
+                        if (lane == jj) {
+                            U[i * LDC_UP + jj] = a;
+                            x[r] = l;
                         }
                     }
-                    U[i * LDC_UP + jj] = x[0];
-                    x[0] = l;
                 }
-                if (act && jj <= i) S[i * LDC_PITCH + c0 + jj] = x[0];
+            }
 #pragma unroll
-                for (int c = 0; c + 1 < LDC_ROWS; c++) x[c] = x[c + 1];
-                x[LDC_ROWS - 1] = zero;
+            for (int r = 0; r < 4; r++) {
+                const int i = wid * 4 + r;
+                if (i < w && lane <= i) S[i * LDC_PITCH + c0 + lane] = x[r];
             }
         }
         cluster.sync();
@@ -1712,29 +1708,28 @@ ldlt_diag_cluster_kernel(float2* __restrict__ A, int64_t lda, int j0, int jb, in
                 dinv[tid] = (d.x == 0 && d.y == 0) ? zero : cdiv(one, d);
             }
             __syncthreads();
-            if (wid == 0 && lane < nr) {
-                const int i = lane;
-                float2 x[LDC_ROWS];
+            // warp: four rows, lane: column
+            float2 x[4];
 #pragma unroll
-                for (int c = 0; c < LDC_ROWS; c++) x[c] = c < w ? S[i * LDC_PITCH + c0 + c] : zero;
-                for (int jj = 0; jj < w; jj++) {
-                    const float2 inv = dinv[jj];
-                    float2 l;
-                    l.x = x[0].x * inv.x - x[0].y * inv.y;
-                    l.y = x[0].x * inv.y + x[0].y * inv.x;
+            for (int r = 0; r < 4; r++) {
+                const int i = wid * 4 + r;
+                x[r] = (i < nr && lane < w) ? S[i * LDC_PITCH + c0 + lane] : zero;
+            }
+#pragma unroll 4
+            for (int jj = 0; jj < w; jj++) {
+                const float2 inv = dinv[jj], u = UL[lane * LDC_UP + jj];
 #pragma unroll
-                    for (int c = 1; c < LDC_ROWS; c++) {
-                        if (jj + c < w) {
-                            const float2 u = UL[(jj + c) * LDC_UP + jj];
-                            x[c].x -= l.x * u.x - l.y * u.y;
-                            x[c].y -= l.x * u.y + l.y * u.x;
-                        }
-                    }
-                    S[i * LDC_PITCH + c0 + jj] = l;
-#pragma unroll
-                    for (int c = 0; c + 1 < LDC_ROWS; c++) x[c] = x[c + 1];
-                    x[LDC_ROWS - 1] = zero;
+                for (int r = 0; r < 4; r++) {
+                    const float2 a = shfl_c(x[r], jj);
+                    const float2 l = panel_mul(a, inv);
+                    if (lane > jj) csub_mul(x[r], l, u);
+                    if (lane == jj) x[r] = l;
                 }
+            }
+#pragma unroll
+            for (int r = 0; r < 4; r++) {
+                const int i = wid * 4 + r;
+                if (i < nr && lane < w) S[i * LDC_PITCH + c0 + lane] = x[r];
             }
         }
         cluster.sync();
@@ -1756,10 +1751,7 @@ ldlt_diag_cluster_kernel(float2* __restrict__ A, int64_t lda, int j0, int jb, in
                     const int e = e0 + u * LDLT_THREADS + tid, c = e / w, k = e % w;
                     if (e < w * nc) {
                         const float2 d = dk[k];
-                        float2 t;
-                        t.x = d.x * lc[u].x - d.y * lc[u].y;
-                        t.y = d.x * lc[u].y + d.y * lc[u].x;
-                        T[k * LDC_TP + c] = t;
+                        T[k * LDC_TP + c] = panel_mul(d, lc[u]);
                     }
                 }
             }
@@ -1784,10 +1776,7 @@ ldlt_diag_cluster_kernel(float2* __restrict__ A, int64_t lda, int j0, int jb, in
                     if (g < ng) {  // the column groups this CTA has at this sub-panel
                         const float2 b = T[k * LDC_TP + lane + 32 * g];
 #pragma unroll
-                        for (int r = 0; r < 4; r++) {
-                            acc[r][g].x -= a[r].x * b.x - a[r].y * b.y;
-                            acc[r][g].y -= a[r].x * b.y + a[r].y * b.x;
-                        }
+                        for (int r = 0; r < 4; r++) csub_mul(acc[r][g], a[r], b);
                     }
             }
 #pragma unroll
