@@ -684,8 +684,12 @@ __device__ __forceinline__ void mbar_arrive_remote(uint32_t bar_cluster) {
 // by column.  Lower (square row-major C): a group's columns stop at its last
 // row's diagonal, and tiles wholly above the diagonal (nt >= 2 mt + 2) are
 // skipped by every role alike.
+// Triangular A (tri 1 lower, 2 upper, blocks of a tile's rows): a row tile
+// takes only the K stages of its non-zero blocks, the longest ones first.
 struct PairTiles {
-    int num_m, num_n, gm, lower;
+    int num_m, num_n, gm, lower, tri;
+    __device__ __forceinline__ int k_begin(int mt, int per) const { return tri == 2 ? mt * per : 0; }
+    __device__ __forceinline__ int k_end(int mt, int per, int nk) const { return tri == 1 ? min(nk, (mt + 1) * per) : nk; }
     __device__ __forceinline__ int gwidth(int g) const {
         const int first = g * gm, gs = min(gm, num_m - first);
         return lower ? min(num_n, 2 * (first + gs)) : num_n;
@@ -696,6 +700,11 @@ struct PairTiles {
         return c;
     }
     __device__ __forceinline__ bool tile(int t, int& mt, int& nt) const {
+        if (tri) {
+            mt = tri == 1 ? num_m - 1 - t / num_n : t / num_n;
+            nt = t % num_n;
+            return true;
+        }
         int g = 0;
         for (;; g++) {
             const int c = min(gm, num_m - g * gm) * gwidth(g);
@@ -713,7 +722,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(P_THREADS, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tA_hi, const __grid_constant__ CUtensorMap tA_lo,
                  const __grid_constant__ CUtensorMap tB_hi, const __grid_constant__ CUtensorMap tB_lo,
                  float2* __restrict__ C, int64_t ldc, int c_colmajor, int M, int Nc, int K2, int lower, int store,
-                 int group_m, int* status, const float2* __restrict__ sa, const float2* __restrict__ sb) {
+                 int tri, int group_m, int* status, const float2* __restrict__ sa, const float2* __restrict__ sb) {
     constexpr int BKE = 2 * BK;  // halves of K per stage (one 128-byte row)
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -735,6 +744,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tA_hi, const __grid_constan
     tm.num_n = (2 * Nc + 2 * P_BROWS - 1) / (2 * P_BROWS);
     tm.gm = group_m > 0 ? group_m : 8;
     tm.lower = lower;
+    tm.tri = tri;
+    constexpr int KT_ROWS = 2 * (2 * P_ROWS) / BKE;  // K stages that a tile's rows span as columns of a square A
     const int ntiles = tm.count();
     const int cid = (int)cl_idx(), ncl = (int)cl_count();
 
@@ -769,7 +780,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tA_hi, const __grid_constan
                 if (!tm.tile(t, mt, nt)) continue;
                 const int ya = mt * 2 * P_ROWS + (int)rank * P_ROWS;
                 const int yb = nt * 2 * P_BROWS + (int)rank * P_BROWS;
-                for (int kt = 0; kt < nk; kt++, it++) {
+                const int ke = tm.k_end(mt, KT_ROWS, nk);
+                for (int kt = tm.k_begin(mt, KT_ROWS); kt < ke; kt++, it++) {
                     const int s = it % P_STAGES;
                     if (!mbar_wait(smem_u32(&empty[s]), ((it / P_STAGES) & 1) ^ 1, status, &abort_flag)) break;
                     unsigned char* st = smem + s * P_STAGE_BYTES;
@@ -795,7 +807,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tA_hi, const __grid_constan
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t acc = tmem + (uint32_t)(b * 256);
                 bool ok = true;
-                for (int kt = 0; kt < nk; kt++, it++) {
+                const int kb = tm.k_begin(mt, KT_ROWS), ke = tm.k_end(mt, KT_ROWS, nk);
+                for (int kt = kb; kt < ke; kt++, it++) {
                     const int s = it % P_STAGES;
                     if (!mbar_wait(smem_u32(&full[s]), (it / P_STAGES) & 1, status, &abort_flag)) {
                         ok = false;
@@ -810,7 +823,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tA_hi, const __grid_constan
                         const uint32_t off = ks * 32;
                         const uint64_t dah = smem_desc(a_hi + off), dal = smem_desc(a_lo + off);
                         const uint64_t dbh = smem_desc(b_hi + off), dbl = smem_desc(b_lo + off);
-                        mma_f16_pair(acc, dah, dbh, (kt > 0 || ks > 0) ? 1u : 0u);
+                        mma_f16_pair(acc, dah, dbh, (kt > kb || ks > 0) ? 1u : 0u);
                         mma_f16_pair(acc, dah, dbl, 1u);
                         mma_f16_pair(acc, dal, dbh, 1u);
                     }
@@ -1258,6 +1271,7 @@ int tc_gemm_ex(bem_ctx* ctx, int M, int N, int K, const float2* A, int64_t lda, 
     const int prof_cls = o.prof_cls;
     if (M <= 0 || N <= 0 || K <= 0) return BEM_OK;
     if (o.lower && (M != N || c_colmajor)) return fail(ctx, BEM_ERR_INVALID, "tc gemm: lower needs square row-major C");
+    if (o.a_tri && (M != K || o.lower)) return fail(ctx, BEM_ERR_INVALID, "tc gemm: triangular A needs a square A");
     if (o.bscale && b_rowmajor) return fail(ctx, BEM_ERR_INVALID, "tc gemm: B scaling needs column-major B");
     BEM_TRY(tc_encode_init(ctx));
     // FP16 parts need the persistent kernel; the one-CTA-per-tile kernel keeps TF32
@@ -1367,7 +1381,7 @@ int tc_gemm_ex(bem_ctx* ctx, int M, int N, int K, const float2* A, int64_t lda, 
         const int ntiles = o.lower ? nm * std::min(nn, 2 * nm) : nm * nn;  // an upper bound for the lower raster
         const int grid = 2 * std::max(1, std::min(ntiles, ctx->sm_count / 2));
         tc::gemm_pair_kernel<<<grid, tc::P_THREADS, tc::P_SMEM_BYTES, ctx->stream>>>(
-            mah, mal, pbh, pbl, C, ldc, c_colmajor ? 1 : 0, M, N, ld, o.lower ? 1 : 0, o.store ? 1 : 0,
+            mah, mal, pbh, pbl, C, ldc, c_colmajor ? 1 : 0, M, N, ld, o.lower ? 1 : 0, o.store ? 1 : 0, o.a_tri,
             std::max(1, ctx->tc_group_m / 2), ctx->d_status, sc_a, sc_b);
     } else if (ctx->tc_persistent) {
         const int nm = (M + tc::BM - 1) / tc::BM;

@@ -1886,22 +1886,21 @@ __global__ void neg_eye_kernel(float2* __restrict__ W, int jb) {
 // inverse factor W = L11^-T D^-1 comes from a block TRSM on -I; the panel
 // below becomes L21 = S21 W in one tensor-core GEMM (in place: the operands
 // are packed before the product is written); then the lower-triangle update.
-// L[c * 256 + r] = W[c * 256 + r] d_r for r, c < jb (W = -L11^-1 D^-1 of the
-// diagonal block at j0, d_r its pivots), 0 elsewhere: -L11^-1 itself.
+// L[c * ldl + r] = W[c * 256 + r] d_r for c <= r < jb (W = -L11^-1 D^-1 of the
+// diagonal block at j0, d_r its pivots): -L11^-1 itself.  The rest of L is zero already.
 __global__ void linv_from_w_kernel(const float2* __restrict__ W, const float2* __restrict__ A, int64_t lda, int j0,
-                                   int jb, float2* __restrict__ L) {
+                                   int jb, float2* __restrict__ L, int ldl) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= TRSM_KB * TRSM_KB) return;
     const int c = t / TRSM_KB, r = t % TRSM_KB;
-    float2 v = make_float2(0.f, 0.f);
-    if (r < jb && c < jb) {
+    if (c <= r && r < jb) {
         const float2 w = W[t], d = A[(int64_t)(j0 + r) * lda + j0 + r];
-        v = make_float2(w.x * d.x - w.y * d.y, w.x * d.y + w.y * d.x);
+        const float2 v = make_float2(w.x * d.x - w.y * d.y, w.x * d.y + w.y * d.x);
+        L[(size_t)c * ldl + r] = v;
     }
-    L[t] = v;
 }
 
-int sytrf_nopiv(bem_ctx* ctx, float2* A, int64_t lda, int n, int* d_info, float2* Linv) {
+int sytrf_nopiv(bem_ctx* ctx, float2* A, int64_t lda, int n, int* d_info, float2* Linv, int linv_sb) {
     using C2 = float2;
     const int NB = TRSM_KB;
     const size_t smem = ldlt_smem_bytes(sizeof(C2));
@@ -1918,7 +1917,10 @@ int sytrf_nopiv(bem_ctx* ctx, float2* A, int64_t lda, int n, int* d_info, float2
             if (p) cudaFree(p);
         }
     } W;
-    BEM_TRY_CUDA(ctx, cudaMalloc(&W.p, (size_t)NB * NB * sizeof(float2)));
+    const int SI = NB * linv_sb;  // rows of an inverse block
+    BEM_TRY_CUDA(ctx, cudaMalloc(&W.p, (size_t)NB * (NB + SI) * sizeof(float2)));
+    float2* T = W.p + (size_t)NB * NB;  // 256 x SI, column-major
+    if (Linv) BEM_TRY_CUDA(ctx, cudaMemsetAsync(Linv, 0, linv_count(n, linv_sb) * sizeof(float2), ctx->stream));
     // the diagonal block at j0 and its panel below: L D L^T of the block,
     // then L21 = S21 L11^-T D^-1 for the rows [j0 + jb, n)
     auto factor_block = [&](int j0, int jb) -> int {
@@ -1939,9 +1941,22 @@ int sytrf_nopiv(bem_ctx* ctx, float2* A, int64_t lda, int n, int* d_info, float2
             BEM_TRY((trsm_block<float, false, false, TRSM_DIVDIAG>(ctx, A, lda, j0, jb, W.p, NB, 0, jb, 0)));
         }
         if (Linv) {
-            linv_from_w_kernel<<<NB * NB / 256, 256, 0, ctx->stream>>>(W.p, A, lda, j0, jb,
-                                                                     Linv + (size_t)(j0 / NB) * NB * NB);
+            // into its place in the SI x SI inverse block at I0, then the rows left of it:
+            // -[[A, 0], [C, B]]^-1 = [[Ma, 0], [Mb C Ma, Mb]] with Ma = -A^-1, Mb = -B^-1
+            const int I0 = j0 / SI * SI, k = j0 - I0;
+            float2* Mi = Linv + (size_t)(I0 / SI) * SI * SI;
+            float2* Mb = Mi + (size_t)k * SI + k;
+            linv_from_w_kernel<<<NB * NB / 256, 256, 0, ctx->stream>>>(W.p, A, lda, j0, jb, Mb, SI);
             BEM_LAUNCHED(ctx);
+            if (k > 0) {
+                TcOpts o;
+                o.c_colmajor = true;
+                o.store = true;
+                o.prof_cls = PROF_PANEL_UPDATE;
+                BEM_TRY(tc_gemm_ex(ctx, jb, k, k, A + (int64_t)j0 * lda + I0, lda, Mi, SI, T, NB, o));  // T = -C Ma
+                o.a_trans = true;
+                BEM_TRY(tc_gemm_ex(ctx, jb, k, jb, Mb, SI, T, NB, Mi + k, SI, o));                      // -Mb T
+            }
         }
         if (below > 0) {
             // L21 = S21 L11^-T D^-1: B given row-major (K x N) is
@@ -2005,7 +2020,7 @@ __global__ void diag_div_kernel(const float2* __restrict__ A, int64_t lda, float
 
 // X = S^-1 B with S = L D L^T (B, X column-major complex64; X may alias B).
 int sytrs_nopiv(bem_ctx* ctx, const float2* A, int64_t lda, int n, const float2* B, int64_t ldb, float2* X,
-                int64_t ldx, int nrhs, const float2* Linv, float2* tmp) {
+                int64_t ldx, int nrhs, const float2* Linv, int linv_sb) {
     const int NB = TRSM_KB;
     if (nrhs <= 0) return BEM_OK;
     int64_t tot = (int64_t)n * nrhs;
@@ -2017,8 +2032,13 @@ int sytrs_nopiv(bem_ctx* ctx, const float2* A, int64_t lda, int n, const float2*
     // Super-blocks of solve_sb 256-row diagonal blocks: the blocks of a
     // super-block update one another with thin GEMMs, so the update of all
     // rows beyond runs with K = 256 solve_sb (fewer launches and fewer
-    // read-modify-writes of X).
-    const int SB = std::max(1, std::min(4, ctx->solve_sb)) * NB;
+    // read-modify-writes of X).  With the inverses of whole super-blocks a
+    // super-block's own part is one product of M = K = 1024 over its
+    // non-zero blocks: 20 ms -> 10 ms of a 161 ms solve (2N = 15360, 2790
+    // columns) against products with 256-row inverses and K = 256 updates
+    // between them, whose 22 tiles left two thirds of the SMs idle.
+    const int SB = Linv ? linv_sb * NB : std::max(1, std::min(4, ctx->solve_sb)) * NB;
+    const int DB = Linv ? SB : NB;  // rows of a diagonal block
     auto update = [&](int M, int K, const float2* Ablk, bool trans, float2* Bx, float2* Cx) {
         TcOpts o;
         o.c_colmajor = true;
@@ -2027,28 +2047,27 @@ int sytrs_nopiv(bem_ctx* ctx, const float2* A, int64_t lda, int n, const float2*
         return tc_gemm_ex(ctx, M, nrhs, K, Ablk, lda, Bx, ldx, Cx, ldx, o);
     };
     // the diagonal block at J0 (jb rows): X_blk = L11^-1 X_blk (back: L11^-T),
-    // as -(-L11^-1) tmp with tmp a copy of X_blk, or a block triangular solve
+    // as -(-L11^-1) X_blk (in place: the product packs X_blk before it writes), or a block triangular solve
     auto diag = [&](int J0, int jb, bool back) -> int {
-        if (!Linv || !tmp) {
+        if (!Linv) {
             if (back)
                 return trsm_block<float, true, false, TRSM_TRANS | TRSM_UNIT>(ctx, A, lda, J0, jb, X, ldx, 0, nrhs);
             return trsm_block<float, false, false>(ctx, A, lda, J0, jb, X, ldx, 0, nrhs);
         }
-        BEM_TRY_CUDA(ctx, cudaMemcpy2DAsync(tmp, NB * sizeof(float2), X + J0, ldx * sizeof(float2),
-                                            jb * sizeof(float2), nrhs, cudaMemcpyDeviceToDevice, ctx->stream));
         TcOpts o;
         o.c_colmajor = true;
         o.store = true;
-        o.a_trans = !back;  // forward: A[r][c] = Li[c * 256 + r]; back: A[r][c] = Li[r * 256 + c]
+        o.a_trans = !back;  // forward: A[r][c] = Li[c * SB + r]; back: A[r][c] = Li[r * SB + c]
+        o.a_tri = back ? 2 : 1;
         o.prof_cls = PROF_TRSM;
-        const float2* Li = Linv + (size_t)(J0 / NB) * NB * NB;
-        return tc_gemm_ex(ctx, jb, nrhs, jb, Li, NB, tmp, NB, X + J0, ldx, o);
+        const float2* Li = Linv + (size_t)(J0 / SB) * SB * SB;
+        return tc_gemm_ex(ctx, jb, nrhs, jb, Li, SB, X + J0, ldx, X + J0, ldx, o);
     };
     // L z = b
     for (int J0 = 0; J0 < n; J0 += SB) {
         const int JB = std::min(SB, n - J0);
-        for (int j = J0; j < J0 + JB; j += NB) {
-            const int jb = std::min(NB, J0 + JB - j), nc = J0 + JB - j - jb;
+        for (int j = J0; j < J0 + JB; j += DB) {
+            const int jb = std::min(DB, J0 + JB - j), nc = J0 + JB - j - jb;
             BEM_TRY(diag(j, jb, false));
             // the super-block's later rows: X[j+jb:J0+JB] -= L[j+jb:J0+JB, j:j+jb] X[j:j+jb]
             if (nc > 0) BEM_TRY(update(nc, jb, A + (int64_t)(j + jb) * lda + j, false, X + j, X + j + jb));
@@ -2063,8 +2082,8 @@ int sytrs_nopiv(bem_ctx* ctx, const float2* A, int64_t lda, int n, const float2*
     const int nsb = (n + SB - 1) / SB;
     for (int bi = nsb - 1; bi >= 0; bi--) {
         const int J0 = bi * SB, JB = std::min(SB, n - J0);
-        for (int j = J0 + ((JB - 1) / NB) * NB; j >= J0; j -= NB) {
-            const int jb = std::min(NB, J0 + JB - j);
+        for (int j = J0 + ((JB - 1) / DB) * DB; j >= J0; j -= DB) {
+            const int jb = std::min(DB, J0 + JB - j);
             BEM_TRY(diag(j, jb, true));
             // the super-block's earlier rows: X[J0:j] -= (L[j:j+jb, J0:j])^T X[j:j+jb]
             if (j > J0) BEM_TRY(update(j - J0, jb, A + (int64_t)j * lda + J0, true, X + j, X + J0));

@@ -29,6 +29,8 @@ struct TcOpts {
     bool a_trans = false;     // A given as its transpose: K x M row-major
     bool lower = false;       // square row-major C: only the tiles on or below the diagonal
     bool store = false;       // C = -op(A) op(B) (C is not read)
+    int a_tri = 0;            // op(A) square, 1 lower / 2 upper triangular by 256-row blocks: its zero blocks
+                              // (stored as zeros) need not be multiplied
     const float2* bscale = nullptr;  // column-major B: B[k][j] *= bscale[k * bscale_stride]
     int64_t bscale_stride = 0;
     int prof_cls = -1;
@@ -68,14 +70,18 @@ void pivots_to_perm(const std::vector<int>& ipiv, std::vector<int>& perm);
 // tensor-core updates) and its multi-RHS solve.
 int sym_structure(bem_ctx* ctx, const double2* Z, int64_t ldz, int n, bool* sym, bool* sym_half);
 constexpr int TRSM_BLOCK = 256;  // rows of the diagonal blocks of the blocked factorisations and solves
-// Linv (optional, ceil(n / 256) blocks of 256 x 256): the factorisation
-// also stores -L11^-1 of every 256-row diagonal block b at Linv + b 256^2,
-// element (r, c) at [c * 256 + r]; the solve then applies the diagonal
-// blocks as tensor-core products with these inverses (tmp: 256 x nrhs
-// complex64 scratch) instead of block triangular solves.
-int sytrf_nopiv(bem_ctx* ctx, float2* A, int64_t lda, int n, int* d_info, float2* Linv = nullptr);
+// Linv (optional, linv_count(n, linv_sb) complex64): the factorisation also
+// stores -L11^-1 of every diagonal block b of S = 256 linv_sb rows at
+// Linv + b S^2, element (r, c) at [c * S + r]; the solve then applies the
+// diagonal blocks as tensor-core products with these inverses instead of
+// block triangular solves.
+inline size_t linv_count(int n, int linv_sb) {
+    const size_t S = (size_t)TRSM_BLOCK * linv_sb;
+    return ((size_t)n + S - 1) / S * S * S;
+}
+int sytrf_nopiv(bem_ctx* ctx, float2* A, int64_t lda, int n, int* d_info, float2* Linv = nullptr, int linv_sb = 1);
 int sytrs_nopiv(bem_ctx* ctx, const float2* A, int64_t lda, int n, const float2* B, int64_t ldb, float2* X,
-                int64_t ldx, int nrhs, const float2* Linv = nullptr, float2* tmp = nullptr);
+                int64_t ldx, int nrhs, const float2* Linv = nullptr, int linv_sb = 1);
 
 // Factorisation without the int8 digit planes of Z (residual_digits false:
 // a factorisation used only as a preconditioner), its order, and one
