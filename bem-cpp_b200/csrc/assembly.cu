@@ -16,7 +16,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <map>
 #include <vector>
 
 #include "asm_device.cuh"
@@ -221,26 +220,52 @@ int geom_upload(bem_ctx* ctx, bem_geom* g) {
     auto& tri = A.tri; auto& tv = A.tv; auto& tc = A.tc; auto& tu = A.tu; auto& tjw = A.tjw; auto& hpi = A.hpi;
     // singular pairs: halves per triangle, ordered (test, source) items per
     // unordered RWG pair
-    std::vector<std::vector<int>> on_tri(nt);
-    for (int h = 0; h < 2; h++)
-        for (int n = 0; n < N; n++) on_tri[h == 0 ? r.tri_p[n] : r.tri_m[n]].push_back(h * N + n);
-    std::map<std::pair<int, int>, std::vector<int>> slot;  // (m<=n) -> items (t, a, b)
-    for (int t = 0; t < nt; t++)
-        for (int a : on_tri[t])
-            for (int b : on_tri[t]) {
-                int mm = a % N, nn = b % N;
-                auto& v = slot[{std::min(mm, nn), std::max(mm, nn)}];
-                v.push_back(t);
-                v.push_back(a);
-                v.push_back(b);
-            }
-    std::vector<int> pair_mn, item_ptr{0}, item;
-    for (auto& kv : slot) {
-        pair_mn.push_back(kv.first.first);
-        pair_mn.push_back(kv.first.second);
-        item.insert(item.end(), kv.second.begin(), kv.second.end());
-        item_ptr.push_back((int)item.size() / 3);
+    // (half h N + n of each triangle in that order, triangle by triangle)
+    std::vector<int> tfirst((size_t)nt + 1, 0), on_tri(2 * (size_t)N);
+    for (int n = 0; n < N; n++) tfirst[r.tri_p[n] + 1]++, tfirst[r.tri_m[n] + 1]++;
+    for (int t = 0; t < nt; t++) tfirst[t + 1] += tfirst[t];
+    {
+        std::vector<int> at(tfirst.begin(), tfirst.end() - 1);
+        for (int n = 0; n < N; n++) on_tri[at[r.tri_p[n]]++] = n;
+        for (int n = 0; n < N; n++) on_tri[at[r.tri_m[n]]++] = N + n;
     }
+    // one entry per (triangle, test, source), sorted by (m <= n) and, for one
+    // pair, in the order above: a bucket per m and an insertion sort by n in it
+    struct Item {
+        int n, t, a, b;
+    };
+    std::vector<int> mfirst((size_t)N + 1, 0);
+    auto each = [&](auto&& f) {
+        for (int t = 0; t < nt; t++)
+            for (int i = tfirst[t]; i < tfirst[t + 1]; i++)
+                for (int k = tfirst[t]; k < tfirst[t + 1]; k++) {
+                    const int mm = on_tri[i] % N, nn = on_tri[k] % N;
+                    f(std::min(mm, nn), Item{std::max(mm, nn), t, on_tri[i], on_tri[k]});
+                }
+    };
+    each([&](int mm, const Item&) { mfirst[mm + 1]++; });
+    for (int i = 0; i < N; i++) mfirst[i + 1] += mfirst[i];
+    std::vector<Item> items(mfirst[N]);
+    {
+        std::vector<int> at(mfirst.begin(), mfirst.end() - 1);
+        each([&](int mm, const Item& x) {
+            int i = at[mm]++;
+            for (; i > mfirst[mm] && items[i - 1].n > x.n; i--) items[i] = items[i - 1];
+            items[i] = x;
+        });
+    }
+    std::vector<int> pair_mn, item_ptr{0}, item;
+    item.reserve(3 * items.size());
+    for (int mm = 0; mm < N; mm++)
+        for (int i = mfirst[mm]; i < mfirst[mm + 1]; i++) {
+            if (i == mfirst[mm] || items[i].n != items[i - 1].n) {
+                if (!pair_mn.empty()) item_ptr.push_back((int)item.size() / 3);
+                pair_mn.push_back(mm);
+                pair_mn.push_back(items[i].n);
+            }
+            item.insert(item.end(), {items[i].t, items[i].a, items[i].b});
+        }
+    if (!pair_mn.empty()) item_ptr.push_back((int)item.size() / 3);
     g->sing.npairs = (int)pair_mn.size() / 2;
     g->sing.nitems = (int)item.size() / 3;
 
@@ -324,33 +349,36 @@ int geom_upload(bem_ctx* ctx, bem_geom* g) {
     if (!g->dmem) return fail(ctx, BEM_ERR_OOM, "geometry arrays (%zu bytes)", off);
     g->dmem_bytes = off;
     char* base = (char*)g->dmem;
+    // the arrays side by side on the host as on the device, in one copy
+    std::vector<char> stage(off, 0);
+    auto put = [&](void* dst, const void* src, size_t bytes) { std::memcpy(stage.data() + ((char*)dst - base), src, bytes); };
     double** pts[10] = {&g->half.px, &g->half.py, &g->half.pz, &g->half.fx, &g->half.fy,
                         &g->half.fz, &g->half.cx, &g->half.cy, &g->half.cz, &g->half.jw};
     std::vector<double>* src[10] = {&px, &py, &pz, &fx, &fy, &fz, &cx, &cy, &cz, &jw};
     for (int i = 0; i < 10; i++) {
         *pts[i] = (double*)(base + o_pt[i]);
-        BEM_TRY(h2d(ctx, *pts[i], src[i]->data(), P * 8));
+        put(*pts[i], src[i]->data(), P * 8);
     }
     g->half.div = (double*)(base + o_div);
     g->half.tri = (int*)(base + o_tri);
     double* d_coef = (double*)(base + o_coef);
     double* d_fr = (double*)(base + o_fr);
-    BEM_TRY(h2d(ctx, g->half.div, div.data(), 2 * N * 8));
-    BEM_TRY(h2d(ctx, d_coef, coef.data(), 2 * N * 8));
-    BEM_TRY(h2d(ctx, d_fr, frx.data(), 2 * N * 8));
-    BEM_TRY(h2d(ctx, d_fr + 2 * N, fry.data(), 2 * N * 8));
-    BEM_TRY(h2d(ctx, d_fr + 4 * N, frz.data(), 2 * N * 8));
-    BEM_TRY(h2d(ctx, g->half.tri, tri.data(), 2 * N * 4));
+    put(g->half.div, div.data(), 2 * N * 8);
+    put(d_coef, coef.data(), 2 * N * 8);
+    put(d_fr, frx.data(), 2 * N * 8);
+    put(d_fr + 2 * N, fry.data(), 2 * N * 8);
+    put(d_fr + 4 * N, frz.data(), 2 * N * 8);
+    put(g->half.tri, tri.data(), 2 * N * 4);
     g->sing.pair_mn = (int*)(base + o_pmn);
     g->sing.item_ptr = (int*)(base + o_iptr);
     g->sing.item = (int*)(base + o_item);
     g->sing.P = (double*)(base + o_P);
     g->sing.V = (double*)(base + o_V);
     g->sing.tv = (double*)(base + o_tv);
-    BEM_TRY(h2d(ctx, g->sing.pair_mn, pair_mn.data(), pair_mn.size() * 4));
-    BEM_TRY(h2d(ctx, g->sing.item_ptr, item_ptr.data(), item_ptr.size() * 4));
-    BEM_TRY(h2d(ctx, g->sing.item, item.data(), item.size() * 4));
-    BEM_TRY(h2d(ctx, g->sing.tv, tv.data(), tv.size() * 8));
+    put(g->sing.pair_mn, pair_mn.data(), pair_mn.size() * 4);
+    put(g->sing.item_ptr, item_ptr.data(), item_ptr.size() * 4);
+    put(g->sing.item, item.data(), item.size() * 4);
+    put(g->sing.tv, tv.data(), tv.size() * 8);
     DevTriAsm& ta = g->tri;
     ta.c = (double*)(base + o_tc);
     ta.u = (double*)(base + o_tu);
@@ -365,16 +393,17 @@ int geom_upload(bem_ctx* ctx, bem_geom* g) {
     ta.rwg_rec = (unsigned char*)(base + o_rrec);
     ta.ntile = ntile;
     ta.tri_half = (int*)(base + o_thalf);
-    BEM_TRY(h2d(ctx, ta.tri_half, tri_half.data(), tri_half.size() * 4));
-    BEM_TRY(h2d(ctx, ta.c, tc.data(), tc.size() * 8));
-    BEM_TRY(h2d(ctx, ta.u, tu.data(), tu.size() * 8));
-    BEM_TRY(h2d(ctx, ta.jw, tjw.data(), tjw.size() * 8));
-    BEM_TRY(h2d(ctx, ta.pi, hpi.data(), hpi.size() * 8));
-    BEM_TRY(h2d(ctx, ta.tile_rwg, tile_rwg.data(), tile_rwg.size() * 4));
-    BEM_TRY(h2d(ctx, ta.pos, pos.data(), (size_t)N * 4));
-    BEM_TRY(h2d(ctx, ta.tile_tri, tile_tri.data(), tile_tri.size() * 4));
-    BEM_TRY(h2d(ctx, ta.tile_ntri, tile_ntri.data(), (size_t)ntile * 4));
-    BEM_TRY(h2d(ctx, ta.tile_ent, tile_ent.data(), tile_ent.size()));
+    put(ta.tri_half, tri_half.data(), tri_half.size() * 4);
+    put(ta.c, tc.data(), tc.size() * 8);
+    put(ta.u, tu.data(), tu.size() * 8);
+    put(ta.jw, tjw.data(), tjw.size() * 8);
+    put(ta.pi, hpi.data(), hpi.size() * 8);
+    put(ta.tile_rwg, tile_rwg.data(), tile_rwg.size() * 4);
+    put(ta.pos, pos.data(), (size_t)N * 4);
+    put(ta.tile_tri, tile_tri.data(), tile_tri.size() * 4);
+    put(ta.tile_ntri, tile_ntri.data(), (size_t)ntile * 4);
+    put(ta.tile_ent, tile_ent.data(), tile_ent.size());
+    BEM_TRY(h2d(ctx, base, stage.data(), off));
     // half coefficient and free vertex live right after div (see fixup kernel)
     (void)d_coef;
     (void)d_fr;

@@ -87,6 +87,7 @@ HostMesh make_icosphere(double radius, int refinements);
 HostMesh make_hex_prism(double aspect_ratio, int refinements);
 HostMesh subdivide_flat(const HostMesh& m);
 HostRWG build_rwg(const HostMesh& m);
+int count_rwg(const HostMesh& m);  // its N alone
 // Free vertices, edge lengths and areas of a mesh-built basis after the
 // vertices moved (same formulas as build_rwg).
 void rwg_refresh(const HostMesh& m, HostRWG& r);

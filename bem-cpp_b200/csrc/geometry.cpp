@@ -101,32 +101,65 @@ HostMesh make_hex_prism(double ar, int refinements) {
     return m;
 }
 
+// Edge j of triangle t: key vertices lo < hi, sorted by (lo, hi) and, for one
+// edge, in the order of the triangles.  A bucket per lower vertex (a handful
+// of edges each) and an insertion sort in it.
+namespace {
+struct TriEdge {
+    int lo, hi, tri, opp;
+};
+std::vector<TriEdge> sorted_edges(const HostMesh& m) {
+    const int nt = m.nt(), nv = m.nv();
+    std::vector<int> first((size_t)nv + 1, 0);
+    for (int t = 0; t < nt; t++)
+        for (int j = 0; j < 3; j++) first[std::min(m.tris[3 * t + j], m.tris[3 * t + (j + 1) % 3]) + 1]++;
+    for (int v = 0; v < nv; v++) first[v + 1] += first[v];
+    std::vector<int> at(first.begin(), first.end() - 1);
+    std::vector<TriEdge> e(3 * (size_t)nt);
+    for (int t = 0; t < nt; t++)
+        for (int j = 0; j < 3; j++) {
+            const int a = m.tris[3 * t + j], b = m.tris[3 * t + (j + 1) % 3];
+            const TriEdge x{std::min(a, b), std::max(a, b), t, m.tris[3 * t + (j + 2) % 3]};
+            int i = at[x.lo]++;
+            for (; i > first[x.lo] && e[i - 1].hi > x.hi; i--) e[i] = e[i - 1];
+            e[i] = x;
+        }
+    return e;
+}
+}  // namespace
+
+// Number of RWG functions of a mesh (edges shared by exactly two triangles).
+int count_rwg(const HostMesh& m) {
+    const std::vector<TriEdge> e = sorted_edges(m);
+    int n = 0;
+    for (size_t i = 0, k; i < e.size(); i = k) {
+        for (k = i + 1; k < e.size() && e[k].lo == e[i].lo && e[k].hi == e[i].hi;) k++;
+        n += k - i == 2;
+    }
+    return n;
+}
+
 // build_rwg -- rwg.cpp:5-43.  Interior edges (shared by exactly two
 // triangles) in (min,max) key order; the first visiting triangle is '+'.
 HostRWG build_rwg(const HostMesh& m) {
-    std::map<std::pair<int, int>, std::vector<std::pair<int, int>>> edges;
-    for (int t = 0; t < m.nt(); t++)
-        for (int j = 0; j < 3; j++) {
-            int a = m.tris[3 * t + j], b = m.tris[3 * t + (j + 1) % 3];
-            int opp = m.tris[3 * t + (j + 2) % 3];
-            edges[{std::min(a, b), std::max(a, b)}].push_back({t, opp});
-        }
+    const std::vector<TriEdge> e = sorted_edges(m);
     HostRWG r;
-    for (auto& kv : edges) {
-        if (kv.second.size() != 2) continue;
-        int tp = kv.second[0].first, vp = kv.second[0].second;
-        int tm = kv.second[1].first, vm = kv.second[1].second;
+    for (size_t i = 0, k; i < e.size(); i = k) {
+        for (k = i + 1; k < e.size() && e[k].lo == e[i].lo && e[k].hi == e[i].hi;) k++;
+        if (k - i != 2) continue;
+        int tp = e[i].tri, vp = e[i].opp;
+        int tm = e[i + 1].tri, vm = e[i + 1].opp;
         r.tri_p.push_back(tp);
         r.tri_m.push_back(tm);
         r.vfree_p.push_back(vp);
         r.vfree_m.push_back(vm);
         r.free_p.push_back(m.verts[vp]);
         r.free_m.push_back(m.verts[vm]);
-        r.length.push_back(norm(sub(m.verts[kv.first.second], m.verts[kv.first.first])));
+        r.length.push_back(norm(sub(m.verts[e[i].hi], m.verts[e[i].lo])));
         r.area_p.push_back(tri_area(m, tp));
         r.area_m.push_back(tri_area(m, tm));
-        r.edge_lo.push_back(kv.first.first);
-        r.edge_hi.push_back(kv.first.second);
+        r.edge_lo.push_back(e[i].lo);
+        r.edge_hi.push_back(e[i].hi);
     }
     r.N = (int)r.tri_p.size();
     return r;

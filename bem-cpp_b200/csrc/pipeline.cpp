@@ -462,7 +462,7 @@ int bem_batch_run(bem_ctx* ctx, const bem_problem* problems, int count, bem_resu
                 continue;
             HostMesh hm;
             if (!host_mesh_from(p.verts, p.nv, p.tris, p.nt, &hm)) continue;
-            buckets[build_rwg(hm).N].push_back(i);
+            buckets[count_rwg(hm)].push_back(i);
         }
         for (auto& kv : buckets) {
             if (kv.second.size() < 2) continue;
