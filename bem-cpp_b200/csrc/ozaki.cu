@@ -376,19 +376,18 @@ residual_kernel(const __grid_constant__ CUtensorMap tA, const __grid_constant__ 
 }
 
 // ---------------------------------------------------------------- slicing
-// e[i] = ilogb(max_k |Z'[i,k]|) + 2 (so |Z'[i,k] 2^-e| < 1/2); 0 for a zero row.
-__global__ void row_exp_kernel(const double2* __restrict__ Z, int64_t ldz, int n, int* __restrict__ e) {
-    __shared__ double s[256];
-    const double2* row = Z + (int64_t)blockIdx.x * ldz;
-    double m = 0.0;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) m = fmax(m, fmax(fabs(row[k].x), fabs(row[k].y)));
-    s[threadIdx.x] = m;
+// Exponent of a row of Z or a column of X from its largest part: ilogb + 2, so
+// that |v 2^-e| < 1/2; 0 for zeros only.  The block's threads hold partial
+// maxima.
+__device__ __forceinline__ int block_exponent(double m) {
+    __shared__ double part[32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = m;
     __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o) s[threadIdx.x] = fmax(s[threadIdx.x], s[threadIdx.x + o]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) e[blockIdx.x] = s[0] > 0.0 ? ilogb(s[0]) + 2 : 0;
+    m = part[0];
+    for (int w = 1; w < (int)(blockDim.x >> 5); w++) m = fmax(m, part[w]);
+    return m > 0.0 ? ilogb(m) + 2 : 0;
 }
 
 // The right-hand operand: X itself (complex128), or a refinement correction
@@ -407,98 +406,152 @@ struct ColSrc {
     }
 };
 
-// f[j] for column j of X (column-major): both X' rows 2j, 2j+1 hold the same
-// magnitudes, so one exponent per complex column.
-__global__ void col_exp_kernel(ColSrc src, int n, int* __restrict__ f) {
-    __shared__ double s[256];
-    double m = 0.0;
-    for (int k = threadIdx.x; k < n; k += blockDim.x) {
-        const double2 v = src.get(blockIdx.x, k);
-        m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
-    }
-    s[threadIdx.x] = m;
-    __syncthreads();
-    for (int o = 128; o > 0; o >>= 1) {
-        if (threadIdx.x < o) s[threadIdx.x] = fmax(s[threadIdx.x], s[threadIdx.x + o]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) f[blockIdx.x] = s[0] > 0.0 ? ilogb(s[0]) + 2 : 0;
-}
-
+// Signed digits q_s = rint(128^(s+1) v) of |v| < 1/2, most significant first.
+// Adding 1.5 2^52 leaves the rounded integer in the sum's low word, so a digit
+// is three FP64 operations and no conversion.
+template <int S>
 __device__ __forceinline__ void digits(double v, int8_t* q) {
+    const double shift = 6755399441055744.0;
 #pragma unroll
-    for (int s = 0; s < S_MAX; s++) {
-        double t = v * 128.0;
-        double r = rint(t);
-        q[s] = (int8_t)(int)r;
-        v = t - r;
-    }
-}
-
-// A digit planes: A[s][i][k'] int8, k' = 2k + {0: Re, 1: Im}, row pitch ldk bytes.
-__global__ void slice_rows_kernel(const double2* __restrict__ Z, int64_t ldz, int n, const int* __restrict__ e,
-                                  int8_t* __restrict__ A, int64_t ldk, int64_t plane, int S) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t kc = ldk / 2;  // complex slots per row (zero padded)
-    if (t >= (int64_t)n * kc) return;
-    const int i = (int)(t / kc), k = (int)(t % kc);
-    double2 z = k < n ? Z[(int64_t)i * ldz + k] : make_double2(0.0, 0.0);
-    const int ex = e[i];
-    int8_t qr[S_MAX], qi[S_MAX];
-    const double sc = pow2i(-ex);
-    digits(z.x * sc, qr);
-    digits(z.y * sc, qi);
     for (int s = 0; s < S; s++) {
-        char2 c;
-        c.x = qr[s];
-        c.y = qi[s];
-        reinterpret_cast<char2*>(A + s * plane + (int64_t)i * ldk)[k] = c;
+        const double t = __fma_rn(v, 128.0, shift);
+        q[s] = (int8_t)__double2loint(t);
+        v = __fma_rn(v, 128.0, shift - t);  // exact: a multiple of the last place below 1/2
     }
 }
 
-// B digit planes: B[t][2j + p][k'] for X' rows (Re, -Im) / (Im, Re).
+// 4 consecutive complex digits as one 8-byte word: (a0, b0, a1, b1, ..).
+__device__ __forceinline__ uint2 pack8(const int8_t* a, const int8_t* b) {
+    auto u = [](int8_t v) { return (unsigned)(uint8_t)v; };
+    uint2 w;
+    w.x = u(a[0]) | u(b[0]) << 8 | u(a[1]) << 16 | u(b[1]) << 24;
+    w.y = u(a[2]) | u(b[2]) << 8 | u(a[3]) << 16 | u(b[3]) << 24;
+    return w;
+}
+
+// Exponent and digit planes of one row of Z per block: A[s][i][k'] int8,
+// k' = 2k + {0: Re, 1: Im}, row pitch ldk bytes (a multiple of 128, zero
+// padded).  The second read of the row comes from L2; a thread takes four
+// entries and stores 8 bytes per plane.  Bound by HBM: 2N = 15360, 7 digits
+// 1.55 ms (4.6 TB/s of 16 + 14 bytes an entry); 3.9 ms with the exponents in a
+// kernel of their own, one entry and a 2-byte store per thread and a
+// conversion per digit.
+constexpr int SLICE_THREADS = 1024;
+template <int S>
+__global__ void __launch_bounds__(SLICE_THREADS) slice_rows_kernel(const double2* __restrict__ Z, int64_t ldz, int n,
+                                                                  int* __restrict__ e, int8_t* __restrict__ A,
+                                                                  int64_t ldk, int64_t plane) {
+    const int i = blockIdx.x;
+    const double2* row = Z + (int64_t)i * ldz;
+    double m = 0.0;
+#pragma unroll 4
+    for (int k = threadIdx.x; k < n; k += SLICE_THREADS) {
+        const double2 z = row[k];
+        m = fmax(m, fmax(fabs(z.x), fabs(z.y)));
+    }
+    const int ex = block_exponent(m);
+    if (threadIdx.x == 0) e[i] = ex;
+    const double sc = pow2i(-ex);
+    int8_t* out = A + (int64_t)i * ldk;
+    for (int k = 4 * threadIdx.x; k < (int)(ldk / 2); k += 4 * SLICE_THREADS) {
+        int8_t qr[4][S], qi[4][S];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const double2 z = k + c < n ? row[k + c] : make_double2(0.0, 0.0);
+            digits<S>(z.x * sc, qr[c]);
+            digits<S>(z.y * sc, qi[c]);
+        }
+#pragma unroll
+        for (int s = 0; s < S; s++) {
+            const int8_t a[4] = {qr[0][s], qr[1][s], qr[2][s], qr[3][s]}, b[4] = {qi[0][s], qi[1][s], qi[2][s], qi[3][s]};
+            *reinterpret_cast<uint2*>(out + s * plane + 2 * k) = pack8(a, b);
+        }
+    }
+}
+
+// Exponent and digit planes of one column of X per block: B[t][2j + p][k'] for
+// X' rows (Re, -Im) / (Im, Re), which hold the same magnitudes.
 // fix (optional): the value the S digits represent, x~ = 2^ex sum_s q_s
 // 128^-(s+1) (exact in FP64 for S <= 7: 49 bits), replaces x there (src.X)
 // or corrects it (src.D: fix += x~ - x).
-__global__ void slice_cols_kernel(ColSrc src, int n, int nrhs, const int* __restrict__ f, int8_t* __restrict__ B,
-                                  int64_t ldk, int64_t plane, int S, double2* __restrict__ fix, int64_t ldfix) {
-    int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const int64_t kc = ldk / 2;
-    if (t >= (int64_t)nrhs * kc) return;
-    const int j = (int)(t / kc), k = (int)(t % kc);
-    double2 x = k < n ? src.get(j, k) : make_double2(0.0, 0.0);
-    const int ex = f[j];
-    int8_t qr[S_MAX], qi[S_MAX];
-    const double sc = pow2i(-ex);
-    digits(x.x * sc, qr);
-    digits(x.y * sc, qi);
-    if (fix && k < n) {
-        double rr = 0.0, ri = 0.0;
-        for (int s = S - 1; s >= 0; s--) {  // Horner in base 128: exact
-            rr = (rr + (double)qr[s]) * (1.0 / 128.0);
-            ri = (ri + (double)qi[s]) * (1.0 / 128.0);
-        }
-        const double up = pow2i(ex);
-        rr *= up;
-        ri *= up;
-        double2* p = fix + (int64_t)j * ldfix + k;
-        if (src.X) {
-            *p = make_double2(rr, ri);
-        } else {
-            const double2 v = *p;
-            *p = make_double2(v.x + (rr - x.x), v.y + (ri - x.y));
-        }
+constexpr int SLICE_COL_THREADS = 512;
+template <int S>
+__global__ void __launch_bounds__(SLICE_COL_THREADS)
+slice_cols_kernel(ColSrc src, int n, int* __restrict__ f, int8_t* __restrict__ B, int64_t ldk, int64_t plane,
+                  double2* __restrict__ fix, int64_t ldfix) {
+    const int j = blockIdx.x;
+    double m = 0.0;
+#pragma unroll 4
+    for (int k = threadIdx.x; k < n; k += SLICE_COL_THREADS) {
+        const double2 v = src.get(j, k);
+        m = fmax(m, fmax(fabs(v.x), fabs(v.y)));
     }
-    for (int s = 0; s < S; s++) {
-        char2 r0, r1;
-        r0.x = qr[s];
-        r0.y = (int8_t)(-qi[s]);
-        r1.x = qi[s];
-        r1.y = qr[s];
-        reinterpret_cast<char2*>(B + s * plane + (int64_t)(2 * j) * ldk)[k] = r0;
-        reinterpret_cast<char2*>(B + s * plane + (int64_t)(2 * j + 1) * ldk)[k] = r1;
+    const int ex = block_exponent(m);
+    if (threadIdx.x == 0) f[j] = ex;
+    const double sc = pow2i(-ex), up = pow2i(ex);
+    int8_t* out = B + (int64_t)(2 * j) * ldk;
+    for (int k = 4 * threadIdx.x; k < (int)(ldk / 2); k += 4 * SLICE_COL_THREADS) {
+        int8_t qr[4][S], qi[4][S];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            const double2 x = k + c < n ? src.get(j, k + c) : make_double2(0.0, 0.0);
+            digits<S>(x.x * sc, qr[c]);
+            digits<S>(x.y * sc, qi[c]);
+            if (fix && k + c < n) {
+                double rr = 0.0, ri = 0.0;
+#pragma unroll
+                for (int s = S - 1; s >= 0; s--) {  // Horner in base 128: exact
+                    rr = (rr + (double)qr[c][s]) * (1.0 / 128.0);
+                    ri = (ri + (double)qi[c][s]) * (1.0 / 128.0);
+                }
+                rr *= up;
+                ri *= up;
+                double2* p = fix + (int64_t)j * ldfix + k + c;
+                if (src.X) {
+                    *p = make_double2(rr, ri);
+                } else {
+                    const double2 v = *p;
+                    *p = make_double2(v.x + (rr - x.x), v.y + (ri - x.y));
+                }
+            }
+        }
+#pragma unroll
+        for (int s = 0; s < S; s++) {
+            const int8_t a[4] = {qr[0][s], qr[1][s], qr[2][s], qr[3][s]}, b[4] = {qi[0][s], qi[1][s], qi[2][s], qi[3][s]};
+            const int8_t nb[4] = {(int8_t)-b[0], (int8_t)-b[1], (int8_t)-b[2], (int8_t)-b[3]};
+            *reinterpret_cast<uint2*>(out + s * plane + 2 * k) = pack8(a, nb);
+            *reinterpret_cast<uint2*>(out + s * plane + ldk + 2 * k) = pack8(b, a);
+        }
     }
 }
+
+// The instance of a kernel template for S digits (1 .. S_MAX).
+template <template <int> class Launch, typename... Args> static int by_digits(int S, Args&&... args) {
+    switch (S) {
+        case 1: return Launch<1>::go(args...);
+        case 2: return Launch<2>::go(args...);
+        case 3: return Launch<3>::go(args...);
+        case 4: return Launch<4>::go(args...);
+        case 5: return Launch<5>::go(args...);
+        case 6: return Launch<6>::go(args...);
+        case 7: return Launch<7>::go(args...);
+        default: return Launch<8>::go(args...);
+    }
+}
+static_assert(S_MAX == 8, "digit instances");
+template <int S> struct SliceRows {
+    static int go(bem_ctx* ctx, const OzakiZ* o, const double2* Z, int64_t ldz, int n) {
+        slice_rows_kernel<S><<<n, SLICE_THREADS, 0, ctx->stream>>>(Z, ldz, n, o->e, o->A, o->ldk, o->plane);
+        return BEM_OK;
+    }
+};
+template <int S> struct SliceCols {
+    static int go(bem_ctx* ctx, ColSrc src, int n, int nrhs, int* f, int8_t* B, int64_t ldk, int64_t plane, double2* fix,
+                  int64_t ldfix) {
+        slice_cols_kernel<S><<<nrhs, SLICE_COL_THREADS, 0, ctx->stream>>>(src, n, f, B, ldk, plane, fix, ldfix);
+        return BEM_OK;
+    }
+};
 
 }  // namespace oz
 
@@ -544,11 +597,7 @@ int ozaki_prepare_z(bem_ctx* ctx, OzakiZ* oz_, const double2* Z, int64_t ldz, in
         ozaki_free(oz_);
         return fail(ctx, BEM_ERR_OOM, "ozaki digit planes (%zu bytes)", bytes);
     }
-    oz::row_exp_kernel<<<n, 256, 0, ctx->stream>>>(Z, ldz, n, oz_->e);
-    BEM_LAUNCHED(ctx);
-    int64_t tot = (int64_t)n * (oz_->ldk / 2);
-    oz::slice_rows_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, ctx->stream>>>(Z, ldz, n, oz_->e, oz_->A, oz_->ldk,
-                                                                                 oz_->plane, S);
+    BEM_TRY(oz::by_digits<oz::SliceRows>(S, ctx, oz_, Z, ldz, n));
     BEM_LAUNCHED(ctx);
     return BEM_OK;
 }
@@ -589,11 +638,7 @@ static int ozaki_apply(bem_ctx* ctx, const OzakiZ* oz_, oz::ColSrc src, double2*
     int8_t* Bd = (int8_t*)ctx->oz_buf;
     int* f = (int*)((char*)ctx->oz_buf + (((size_t)Sx * bplane + 255) & ~(size_t)255));
     cudaEvent_t ev = ctx->prof_begin(PROF_RESIDUAL);
-    oz::col_exp_kernel<<<nrhs, 256, 0, ctx->stream>>>(src, n, f);
-    BEM_LAUNCHED(ctx);
-    int64_t tot = (int64_t)nrhs * (ldk / 2);
-    oz::slice_cols_kernel<<<(unsigned)((tot + 255) / 256), 256, 0, ctx->stream>>>(src, n, nrhs, f, Bd, ldk, bplane,
-                                                                                  Sx, fix, ldfix);
+    BEM_TRY(oz::by_digits<oz::SliceCols>(Sx, ctx, src, n, nrhs, f, Bd, ldk, bplane, fix, ldfix));
     BEM_LAUNCHED(ctx);
     CUtensorMap tA, tB;
     BEM_TRY(encode_i8(ctx, &tA, oz_->A, (int64_t)oz_->S * n, ldk, oz::BM));
