@@ -129,7 +129,39 @@ __device__ void block_sum(double* vals, double* smem, double* out) {
 }
 
 // One block per triangle a; its threads take the triangles b != a.
-__global__ void __launch_bounds__(128) grad_pair_kernel(PairArgs a) {
+// In b's frame, r_q = v0 + l1 e1 + l2 e2 and rho = r_p - v0, the halves of b
+// enter through three weights per matrix, c = sum_s c_s, c1 and c2 (those of
+// the halves whose free vertex is v1, v2):
+//   sum_s c_s (r_q - v_Fs) = (l1 c - c1) e1 + (l2 c - c2) e2,
+// and d x W, W the same sum with the K weights, is linear in (l1, l2) as well.
+// So a point p needs of its point pairs the moments of G and G'/R in
+// (1, l1, l2) and of g = G'/R and g'/R in (1, l1, l2, l1^2, l1 l2, l2^2) (for
+// the derivatives along d = rho - l1 e1 - l2 e2), and the three halves of a
+// are contracted with these moments instead of with each point pair.
+// Bound by the FP64 pipe: ~10 k operations of point pairs and ~8 k of
+// contractions a triangle pair (~100 k with three evaluations of both
+// Green's functions and six complex cross products per point pair).
+// 1280 triangles, 7 points, an absorbing interior: 8.94 -> 3.09 ms.
+// DAMP: bit e, Im k_e != 0; BOUNDED: a real exterior k, Im k >= 0 inside and
+// phases below SINCOS_MAX, the range of the branch-free functions (else the
+// library's functions).
+constexpr int GP_THREADS = 128, GP_W = 24;  // weights per half of a: (c, c1, c2) of WLe, WLi, WK, Weta
+
+// c m_1 - c_1 m_0 and the like: Re(x y - z w)
+__device__ __forceinline__ double re_msub(cplx x, cplx y, cplx z, cplx w) {
+    return x.re * y.re - x.im * y.im - z.re * w.re + z.im * w.im;
+}
+__device__ __forceinline__ cplx cmsub(cplx x, cplx y, cplx z, cplx w) {
+    return {x.re * y.re - x.im * y.im - z.re * w.re + z.im * w.im, x.re * y.im + x.im * y.re - z.re * w.im - z.im * w.re};
+}
+__device__ __forceinline__ void cfma(cplx& a, cplx b, double f) { a.re += b.re * f, a.im += b.im * f; }
+__device__ __forceinline__ double dot3(const double* a, const double* b) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; }
+__device__ __forceinline__ void cross3(const double* a, const double* b, double* c) {
+    c[0] = a[1] * b[2] - a[2] * b[1], c[1] = a[2] * b[0] - a[0] * b[2], c[2] = a[0] * b[1] - a[1] * b[0];
+}
+
+template <int DAMP, bool BOUNDED> __global__ void __launch_bounds__(GP_THREADS, 2) grad_pair_kernel(PairArgs a) {
+    extern __shared__ double s_w[];  // [3 GP_W][GP_THREADS]: each thread's weights
     const int ta = blockIdx.x, tid = threadIdx.x, Nq = a.Nq, N = a.W.N;
     __shared__ double s_va[9], s_rp[GQ][3], s_alpha[3];
     __shared__ double s_red[4 * 13];
@@ -145,116 +177,184 @@ __global__ void __launch_bounds__(128) grad_pair_kernel(PairArgs a) {
     cplx Sk = {0, 0}, Se = {0, 0};
     const Medium med[2] = {a.ke, a.ki};
 
-    for (int tb = tid; tb < a.nt; tb += blockDim.x) {
+    for (int tb = tid; tb < a.nt; tb += GP_THREADS) {
         if (tb == ta) continue;
-        double vb[9];
-        for (int j = 0; j < 9; j++) vb[j] = a.tv[9 * tb + j];
-        const HalfInfo hb = load_halves(a.hinfo, tb);
-        double as[3];
-        for (int s = 0; s < 3; s++) as[s] = hb.n[s] >= 0 ? half_alpha(vb, hb.sign[s], hb.jf[s]) : 0.0;
-        for (int t = 0; t < 3; t++) {
-            const int nt_ = ha.n[t];
-            if (nt_ < 0) continue;
-            // weights of half t against the halves of b, aggregated over s:
-            // sum_s c_ts (r_q - v_Fs) = A r_q - B
-            cplx A0 = {0, 0}, A1 = {0, 0}, C = {0, 0}, Ae = {0, 0};
-            cplx B0[3], B1[3], D[3], Be[3];
-            for (int c = 0; c < 3; c++) B0[c] = B1[c] = D[c] = Be[c] = {0, 0};
-            for (int s = 0; s < 3; s++) {
-                const int ns = hb.n[s];
-                if (ns < 0) continue;
-                const double aa = s_alpha[t] * as[s];
-                const size_t ix = (size_t)nt_ * N + ns;
-                const cplx w0 = cscale(c2(a.W.WLe[ix]), aa), w1 = cscale(c2(a.W.WLi[ix]), aa),
-                           wk = cscale(c2(a.W.WK[ix]), aa), we = cscale(c2(a.W.Weta[ix]), aa);
-                A0 = cadd(A0, w0), A1 = cadd(A1, w1), C = cadd(C, wk), Ae = cadd(Ae, we);
-                const double* vf = vb + 3 * hb.jf[s];
-                for (int c = 0; c < 3; c++) {
-                    B0[c] = cadd(B0[c], cscale(w0, vf[c]));
-                    B1[c] = cadd(B1[c], cscale(w1, vf[c]));
-                    D[c] = cadd(D[c], cscale(wk, vf[c]));
-                    Be[c] = cadd(Be[c], cscale(we, vf[c]));
-                }
-            }
-            const double* vFt = s_va + 3 * ha.jf[t];
-            for (int p = 0; p < Nq; p++) {
-                const double rp[3] = {s_rp[p][0], s_rp[p][1], s_rp[p][2]};
-                const double u[3] = {rp[0] - vFt[0], rp[1] - vFt[1], rp[2] - vFt[2]};
-                double grp[3] = {0, 0, 0};
-                for (int q = 0; q < Nq; q++) {
-                    double rq[3];
-                    bary_point(vb, a.q.l1[q], a.q.l2[q], rq);
-                    const double d[3] = {rp[0] - rq[0], rp[1] - rq[1], rp[2] - rq[2]};
-                    const double R2 = d[0] * d[0] + d[1] * d[1] + d[2] * d[2];
-                    const double invR = rsqrt(R2), R = R2 * invR;
-                    const double dh[3] = {d[0] * invR, d[1] * invR, d[2] * invR};
-                    const double ww = a.q.w[p] * a.q.w[q];
+        double v0[3], e1[3], e2[3], nv[3];
+        {
+            double vb[9], as[3];
+            for (int j = 0; j < 9; j++) vb[j] = a.tv[9 * tb + j];
+            const HalfInfo hb = load_halves(a.hinfo, tb);
 #pragma unroll
-                    for (int e = 0; e < 2; e++) {
-                        const Medium k = med[e];
-                        double sn, cs;
-                        sincos(k.kr * R, &sn, &cs);
-                        const double ea = k.ki != 0.0 ? exp(-k.ki * R) : 1.0;
-                        const double i4R = INV4PI_D * invR;
-                        const cplx G = {ea * cs * i4R, ea * sn * i4R};
-                        const cplx ik = {-k.ki, k.kr};
-                        const cplx dG = cmul(G, cplx{-k.ki - invR, k.kr});  // G' = G (ik - 1/R)
-                        const cplx gc = cscale(dG, invR);
-                        // g' = -G (k^2 R^2 + 3 i k R - 3) / R^3
-                        const cplx kk = cmul(cplx{k.kr, k.ki}, cplx{k.kr, k.ki});
-                        const cplx pg = {kk.re * R2 - 3.0 * k.ki * R - 3.0, kk.im * R2 + 3.0 * k.kr * R};
-                        const cplx dgc = cscale(cmul(G, pg), -invR * invR * invR);
-                        const double kn = k.kr * k.kr + k.ki * k.ki;
-                        const cplx fik = {4.0 * k.ki / kn, 4.0 * k.kr / kn};  // 4i/k
-                        const cplx Aw = e ? A1 : A0;
-                        const cplx* Bw = e ? B1 : B0;
-                        cplx Vt[3], Wt[3];
-                        for (int c = 0; c < 3; c++) {
-                            Vt[c] = csub(cscale(Aw, rq[c]), Bw[c]);
-                            Wt[c] = csub(cscale(C, rq[c]), D[c]);
-                        }
-                        const cplx uv = cadd(cadd(cscale(Vt[0], u[0]), cscale(Vt[1], u[1])), cscale(Vt[2], u[2]));
-                        const cplx QL = csub(cmul(ik, uv), cmul(fik, Aw));
-                        cplx dxW[3], Wxu[3];
-                        for (int c = 0; c < 3; c++) {
-                            const int c1 = (c + 1) % 3, c2_ = (c + 2) % 3;
-                            dxW[c] = csub(cscale(Wt[c2_], d[c1]), cscale(Wt[c1], d[c2_]));
-                            Wxu[c] = csub(cscale(Wt[c1], u[c2_]), cscale(Wt[c2_], u[c1]));
-                        }
-                        const cplx tau =
-                            cadd(cadd(cscale(dxW[0], u[0]), cscale(dxW[1], u[1])), cscale(dxW[2], u[2]));
-                        const cplx fL = cscale(cmul(G, QL), ww), fK = cscale(cmul(gc, tau), ww);
-                        gal[t] += fL.re + fK.re;
-                        const cplx cd = cscale(cadd(cmul(dG, QL), cmul(dgc, tau)), ww);
-                        const cplx Gik = cscale(cmul(G, ik), ww), gcw = cscale(gc, ww);
-                        for (int c = 0; c < 3; c++) {
-                            const cplx a1 = cmul(Gik, Vt[c]), a2 = cmul(gcw, dxW[c]), a3 = cmul(gcw, Wxu[c]);
-                            grp[c] += cd.re * dh[c] + a1.re + a2.re + a3.re;
-                            gF[t][c] -= a1.re + a2.re;
-                        }
-                        if (e == 1) {
-                            // d/dk: dG/dk = i R G, d(gc)/dk = -k G
-                            const cplx iRG = cmul(cplx{0.0, R}, G);
-                            const cplx kn2 = cmul(cplx{k.kr, k.ki}, cplx{k.kr, k.ki});
-                            const cplx f4k2 = cdiv(cplx{0.0, 4.0}, kn2);  // 4i/k^2
-                            const cplx dQ = cadd(cmul(cplx{0.0, 1.0}, uv), cmul(f4k2, Aw));
-                            cplx sk = cadd(cmul(iRG, QL), cmul(G, dQ));
-                            sk = csub(sk, cmul(cmul(cplx{k.kr, k.ki}, G), tau));
-                            Sk = cadd(Sk, cscale(sk, ww));
-                            cplx Ve[3];
-                            for (int c = 0; c < 3; c++) Ve[c] = csub(cscale(Ae, rq[c]), Be[c]);
-                            const cplx uve =
-                                cadd(cadd(cscale(Ve[0], u[0]), cscale(Ve[1], u[1])), cscale(Ve[2], u[2]));
-                            Se = cadd(Se, cscale(cmul(G, csub(cmul(ik, uve), cmul(fik, Ae))), ww));
-                        }
+            for (int s = 0; s < 3; s++) as[s] = hb.n[s] >= 0 ? half_alpha(vb, hb.sign[s], hb.jf[s]) : 0.0;
+            for (int c = 0; c < 3; c++) v0[c] = vb[c], e1[c] = vb[3 + c] - vb[c], e2[c] = vb[6 + c] - vb[c];
+            cross3(e1, e2, nv);
+            const double2* const mats[4] = {a.W.WLe, a.W.WLi, a.W.WK, a.W.Weta};
+#pragma unroll
+            for (int t = 0; t < 3; t++) {
+                if (ha.n[t] < 0) continue;
+#pragma unroll
+                for (int m = 0; m < 4; m++) {
+                    cplx w[3] = {{0, 0}, {0, 0}, {0, 0}};
+#pragma unroll
+                    for (int s = 0; s < 3; s++) {
+                        if (hb.n[s] < 0) continue;
+                        const cplx c = cscale(c2(mats[m][(size_t)ha.n[t] * N + hb.n[s]]), s_alpha[t] * as[s]);
+                        const double f1 = hb.jf[s] == 1 ? 1.0 : 0.0, f2 = hb.jf[s] == 2 ? 1.0 : 0.0;
+                        w[0] = cadd(w[0], c);
+                        cfma(w[1], c, f1);
+                        cfma(w[2], c, f2);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 3; j++) {
+                        s_w[(t * GP_W + m * 6 + 2 * j) * GP_THREADS + tid] = w[j].re;
+                        s_w[(t * GP_W + m * 6 + 2 * j + 1) * GP_THREADS + tid] = w[j].im;
                     }
                 }
-                const double l1 = a.q.l1[p], l2 = a.q.l2[p], l0 = 1.0 - l1 - l2;
-                for (int c = 0; c < 3; c++) {
-                    gv[c] += l0 * grp[c];
-                    gv[3 + c] += l1 * grp[c];
-                    gv[6 + c] += l2 * grp[c];
+            }
+        }
+#pragma unroll 1
+        for (int p = 0; p < Nq; p++) {
+            double rho[3];
+            for (int c = 0; c < 3; c++) rho[c] = s_rp[p][c] - v0[c];
+            // moments: G and g of each medium, g'/R of both, R G of the interior
+            cplx G[2][3], g[2][6], h[6], rg[3];
+#pragma unroll
+            for (int j = 0; j < 6; j++) {
+                g[0][j] = g[1][j] = h[j] = {0, 0};
+                if (j < 3) G[0][j] = G[1][j] = rg[j] = {0, 0};
+            }
+#pragma unroll 1
+            for (int q = 0; q < Nq; q++) {
+                const double l1 = a.q.l1[q], l2 = a.q.l2[q];
+                const double m[6] = {1.0, l1, l2, l1 * l1, l1 * l2, l2 * l2};
+                double d[3];
+                for (int c = 0; c < 3; c++) d[c] = rho[c] - l1 * e1[c] - l2 * e2[c];
+                const double R2 = dot3(d, d);
+                const double invR = BOUNDED ? rsqrt_normal(R2) : rsqrt(R2), R = R2 * invR, invR2 = invR * invR;
+                const double f = a.q.w[p] * a.q.w[q] * INV4PI_D * invR;
+                cplx hs = {0, 0};
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const Medium k = med[e];
+                    double sn, cs, ea = f;
+                    if (BOUNDED)
+                        sincos_bounded(k.kr * R, &sn, &cs);
+                    else
+                        sincos(k.kr * R, &sn, &cs);
+                    if ((DAMP >> e) & 1) ea *= BOUNDED ? exp_decay_bounded(k.ki * R) : exp(-k.ki * R);
+                    const cplx Gq = {ea * cs, ea * sn};
+                    // g = G (ik - 1/R) / R, g' = -G (k^2 R^2 + 3 i k R - 3) / R^3
+                    const cplx gq = cscale(cmul(Gq, cplx{-k.ki - invR, k.kr}), invR);
+                    const cplx kk = cmul(cplx{k.kr, k.ki}, cplx{k.kr, k.ki});
+                    const cplx pg = {kk.re * R2 - 3.0 * k.ki * R - 3.0, kk.im * R2 + 3.0 * k.kr * R};
+                    hs = cadd(hs, cmul(Gq, pg));
+#pragma unroll
+                    for (int j = 0; j < 6; j++) {
+                        cfma(g[e][j], gq, m[j]);
+                        if (j < 3) cfma(G[e][j], Gq, m[j]);
+                        if (j < 3 && e == 1) cfma(rg[j], Gq, R * m[j]);
+                    }
                 }
+                hs = cscale(hs, -invR2 * invR2);
+#pragma unroll
+                for (int j = 0; j < 6; j++) cfma(h[j], hs, m[j]);
+            }
+            // moments times i k (the L form's scalar product) and 4 i / k (its charge term)
+            cplx gs[3], Gf[2], gf[2][3], kG[3], nu[3], ns;
+            {
+                const Medium k = med[1];
+                const cplx ik = {-k.ki, k.kr}, kc = {k.kr, k.ki};
+                const double kn = k.kr * k.kr + k.ki * k.ki;
+                const cplx fik = {4.0 * k.ki / kn, 4.0 * k.kr / kn}, f4k2 = cdiv(cplx{0.0, 4.0}, cmul(kc, kc));
+                // d/dk: dG/dk = i R G, dg/dk = -k G, and the factors i k and 4 i / k
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    gs[j] = cadd(g[0][j], g[1][j]);
+                    kG[j] = cmul(kc, G[1][j]);
+                    const cplx x = cadd(cmul(ik, rg[j]), G[1][j]);
+                    nu[j] = {-x.im, x.re};
+                }
+                const cplx y = cmul(fik, rg[0]);
+                ns = cadd(cmul(f4k2, G[1][0]), cplx{y.im, -y.re});
+            }
+#pragma unroll
+            for (int e = 0; e < 2; e++) {
+                const Medium k = med[e];
+                const cplx ik = {-k.ki, k.kr};
+                const double kn = k.kr * k.kr + k.ki * k.ki;
+                const cplx fik = {4.0 * k.ki / kn, 4.0 * k.kr / kn};
+                Gf[e] = cmul(fik, G[e][0]);
+#pragma unroll
+                for (int j = 0; j < 3; j++) {
+                    gf[e][j] = cmul(fik, g[e][j]);
+                    G[e][j] = cmul(ik, G[e][j]);
+                }
+#pragma unroll
+                for (int j = 0; j < 6; j++) g[e][j] = cmul(ik, g[e][j]);
+            }
+            double re1[3], re2[3], grp[3] = {0, 0, 0}, z[3] = {0, 0, 0};
+            cross3(rho, e1, re1);
+            cross3(rho, e2, re2);
+            constexpr int MI[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};  // moments of (1, l1, l2) times l_i
+#pragma unroll
+            for (int t = 0; t < 3; t++) {
+                if (ha.n[t] < 0) continue;
+                auto wt = [&](int i) -> cplx {
+                    const double* w = s_w + (t * GP_W + 2 * i) * GP_THREADS + tid;
+                    return {w[0], w[GP_THREADS]};
+                };
+                double u[3], e1u[3], e2u[3];
+                for (int c = 0; c < 3; c++) u[c] = s_rp[p][c] - s_va[3 * ha.jf[t] + c];
+                cross3(e1, u, e1u);
+                cross3(e2, u, e2u);
+                const double p1 = dot3(u, e1), p2 = dot3(u, e2), b1 = dot3(u, re1), b2 = dot3(u, re2), bn = dot3(u, nv);
+                double x1 = 0, x2 = 0, x3 = 0;
+#pragma unroll
+                for (int e = 0; e < 2; e++) {
+                    const cplx w0 = wt(3 * e), w1 = wt(3 * e + 1), w2 = wt(3 * e + 2);
+                    x1 += re_msub(w0, G[e][1], w1, G[e][0]);
+                    x2 += re_msub(w0, G[e][2], w2, G[e][0]);
+                    x3 += w0.re * Gf[e].re - w0.im * Gf[e].im;
+#pragma unroll
+                    for (int i = 0; i < 3; i++)
+                        z[i] += p1 * re_msub(w0, g[e][MI[i][1]], w1, g[e][MI[i][0]]) +
+                                p2 * re_msub(w0, g[e][MI[i][2]], w2, g[e][MI[i][0]]) -
+                                (w0.re * gf[e][i].re - w0.im * gf[e][i].im);
+                    if (e == 1) {
+                        const cplx s1 = cmsub(w0, nu[1], w1, nu[0]), s2 = cmsub(w0, nu[2], w2, nu[0]);
+                        Sk = cadd(Sk, cmul(w0, ns));
+                        cfma(Sk, s1, p1);
+                        cfma(Sk, s2, p2);
+                    }
+                }
+                const cplx k0 = wt(6), k1 = wt(7), k2 = wt(8);
+                const double y1 = re_msub(k0, gs[1], k1, gs[0]), y2 = re_msub(k0, gs[2], k2, gs[0]),
+                             y3 = re_msub(k2, gs[1], k1, gs[2]);
+#pragma unroll
+                for (int i = 0; i < 3; i++)
+                    z[i] += b1 * re_msub(k0, h[MI[i][1]], k1, h[MI[i][0]]) +
+                            b2 * re_msub(k0, h[MI[i][2]], k2, h[MI[i][0]]) + bn * re_msub(k2, h[MI[i][1]], k1, h[MI[i][2]]);
+                cfma(Sk, cmsub(k0, kG[1], k1, kG[0]), -b1);
+                cfma(Sk, cmsub(k0, kG[2], k2, kG[0]), -b2);
+                cfma(Sk, cmsub(k2, kG[1], k1, kG[2]), -bn);
+                const cplx n0 = wt(9), n1 = wt(10), n2 = wt(11);
+                cfma(Se, cmsub(n0, G[1][1], n1, G[1][0]), p1);
+                cfma(Se, cmsub(n0, G[1][2], n2, G[1][0]), p2);
+                Se = csub(Se, cmul(n0, Gf[1]));
+                gal[t] += p1 * x1 + p2 * x2 - x3 + b1 * y1 + b2 * y2 + bn * y3;
+#pragma unroll
+                for (int c = 0; c < 3; c++) {
+                    const double m = x1 * e1[c] + x2 * e2[c] + y1 * re1[c] + y2 * re2[c] + y3 * nv[c];
+                    gF[t][c] -= m;
+                    grp[c] += m + y1 * e1u[c] + y2 * e2u[c];
+                }
+            }
+            const double l1 = a.q.l1[p], l2 = a.q.l2[p], l0 = 1.0 - l1 - l2;
+            for (int c = 0; c < 3; c++) {
+                grp[c] += rho[c] * z[0] - e1[c] * z[1] - e2[c] * z[2];
+                gv[c] += l0 * grp[c];
+                gv[3 + c] += l1 * grp[c];
+                gv[6 + c] += l2 * grp[c];
             }
         }
     }
@@ -807,7 +907,13 @@ int adjoint_geometry(bem_ctx* ctx, const bem_geom* g, std::complex<double> kext,
     double* o_ff = o_rhs + (size_t)n * 9;
     const Medium ke{kext.real(), kext.imag()}, ki{kint.real(), kint.imag()};
     PairArgs pa{g->sing.tv, d_hinfo, nt, Nq, tq, ke, ki, gw, o_pair, o_skp, o_sep};
-    grad_pair_kernel<<<nt, 128, 0, st>>>(pa);
+    // the branch-free functions where no phase can leave their range
+    const double reach = 2.0 * g->rmax;
+    const bool bounded = std::max(std::abs(ke.kr), std::abs(ki.kr)) * reach < SINCOS_MAX && ke.ki == 0 && ki.ki >= 0;
+    auto pair = !bounded ? grad_pair_kernel<3, false> : ki.ki != 0 ? grad_pair_kernel<2, true> : grad_pair_kernel<0, true>;
+    const size_t pair_smem = (size_t)3 * GP_W * GP_THREADS * sizeof(double);
+    BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem));
+    pair<<<nt, GP_THREADS, pair_smem, st>>>(pa);
     BEM_LAUNCHED(ctx);
     SelfArgs sa{g->sing.tv, d_hinfo, nt, Nq, tq, ke, ki, flags, gw, o_self, o_sks, o_ses};
     grad_self_kernel<<<nblocks(nt, SELF_TRI), SELF_EVALS * SELF_TRI, 0, st>>>(sa);
