@@ -791,15 +791,17 @@ __global__ void permute_rows_kernel(const typename C2T<R>::type* __restrict__ B,
 // one launch, for the columns [c0, c1) of a right-hand side held row-major in
 // the factor itself (B_ROWMAJOR, the U12 step) or column-major (the solves).
 // One CTA owns RB columns; thread r holds row r of them in registers, so
-// warp s holds the 32-row sub-block s.  Step s: warp s substitutes through its
-// 32 x 32 diagonal block (in shared memory, [k][lane]), x_k going to the
-// other lanes by shuffles, and leaves the solved rows in shared memory; after
-// the one block barrier every later warp subtracts T's segment of its rows
-// times them.  The segment is loaded into registers before the barrier, under
-// the substitution of warp s, which bounds the kernel: 256 dependent steps of
-// ~60 cycles.  (Before: 16-row sub-blocks solved by one thread per column,
-// with T loaded from L2 in between: 84 us for a lower and 134 us for an upper
-// block in FP64, whatever the number of columns.)
+// warp s holds the 32-row sub-block s, and its 32 x 32 diagonal block of T as
+// well.  Step s: warp s substitutes through that block, x_k going to the other
+// lanes by shuffles, and leaves the solved rows in shared memory; after the
+// one block barrier every later warp subtracts T's segment of its rows times
+// them.  The segment comes by cp.async into the warp's 32 x 33 buffer while
+// warp s works, lanes along a row of T (a lane per row reads 32 lines per
+// load: 7 k cycles a step, twice the substitution).  Bound by 256 dependent
+// steps of a shuffle and two multiply-adds.  FP64, 32 columns: 19.9 us a lower
+// and 20.4 us an upper block; 32.7 and 30.1 us with the segments of T in
+// registers, loaded by a lane per row, the diagonal blocks in shared memory
+// and two columns a CTA.
 // An upper block's rows are scaled by their diagonal's reciprocal beforehand,
 // which takes the division out of the chain of steps.
 //
@@ -807,7 +809,7 @@ __global__ void permute_rows_kernel(const typename C2T<R>::type* __restrict__ B,
 // of an L D L^T factor), TRSM_UNIT makes an upper T unit-diagonal, and
 // TRSM_DIVDIAG divides the solution of a unit-lower T by T's diagonal (the D
 // of L D L^T) when it is stored.
-constexpr int TRSM_KB = 256, TRSM_TS = 32;
+constexpr int TRSM_KB = 256, TRSM_TS = 32, TRSM_PITCH = TRSM_TS + 1;
 static_assert(TRSM_KB == TRSM_BLOCK, "diagonal block rows");
 constexpr int TRSM_TRANS = 1, TRSM_UNIT = 2, TRSM_DIVDIAG = 4;
 
@@ -829,6 +831,13 @@ template <typename C2> __device__ __forceinline__ void csub_mul(C2& x, C2 a, C2 
     x = panel_msub(x, a, b);
 }
 
+__device__ __forceinline__ void cp_elem(double2* smem, const double2* gmem, bool valid) { dmma::cp16(smem, gmem, valid); }
+__device__ __forceinline__ void cp_elem(float2* smem, const float2* gmem, bool valid) {
+    const uint32_t d = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+    const int n = valid ? 8 : 0;  // 0: fill with zeros
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(gmem), "r"(n) : "memory");
+}
+
 template <typename R, bool UPPER, bool B_ROWMAJOR, int RB, int MODE = 0>
 __global__ void __launch_bounds__(TRSM_KB)
 trsm_block_kernel(const typename C2T<R>::type* __restrict__ T, int64_t ldt, int r0, int kb,
@@ -840,11 +849,7 @@ trsm_block_kernel(const typename C2T<R>::type* __restrict__ T, int64_t ldt, int 
                    DIVDIAG = (MODE & TRSM_DIVDIAG) != 0;
     using C2 = typename C2T<R>::type;
     constexpr int TS = TRSM_TS;
-    auto tel = [&](int i, int j) {  // element (i, j) of the triangle, block-relative
-        return TRANS ? T[(int64_t)(r0 + j) * ldt + r0 + i] : T[(int64_t)(r0 + i) * ldt + r0 + j];
-    };
     extern __shared__ __align__(16) unsigned char trsm_smem[];
-    C2* sD = reinterpret_cast<C2*>(trsm_smem);  // [warp][k][lane]: the diagonal blocks
     __shared__ __align__(16) C2 xs[2][TS][RB];
     const int r = threadIdx.x, lane = r & 31, warp = r >> 5, nsb = (int)blockDim.x >> 5;
     const int cb = c0 + blockIdx.x * RB, nc = min(RB, c1 - cb);
@@ -852,69 +857,75 @@ trsm_block_kernel(const typename C2T<R>::type* __restrict__ T, int64_t ldt, int 
     C2 zero;
     zero.x = 0;
     zero.y = 0;
-    C2* D = sD + (size_t)warp * TS * TS + lane;
-    C2 x[RB], inv = zero;
+    C2* buf = reinterpret_cast<C2*>(trsm_smem) + (size_t)warp * TS * TRSM_PITCH;  // [row][k] of one segment
+    // segment (warp, s) of T: rows of this warp, columns of sub-block s
+    auto fetch = [&](int s) {
+#pragma unroll 8
+        for (int e = lane; e < TS * TS; e += 32) {
+            const int i = TRANS ? e % TS : e / TS, k = TRANS ? e / TS : e % TS;
+            const int ti = warp * TS + i, tk = s * TS + k;
+            const bool ok = ti < kb && tk < kb;
+            const C2* src = TRANS ? T + (int64_t)(r0 + tk) * ldt + r0 + ti : T + (int64_t)(r0 + ti) * ldt + r0 + tk;
+            cp_elem(buf + i * TRSM_PITCH + k, ok ? src : T, ok);
+        }
+        dmma::cp_commit();
+    };
+    fetch(warp);
+    C2 x[RB], inv = zero, D[TS];
 #pragma unroll
     for (int c = 0; c < RB; c++) {
         x[c] = zero;
         if (row && c < nc) x[c] = B_ROWMAJOR ? B[(int64_t)(br0 + r) * ldb + cb + c] : B[(int64_t)(cb + c) * ldb + br0 + r];
     }
+    dmma::cp_wait<0>();
+    __syncwarp();
     if (UPPER && !UNIT && row) {
         C2 one = zero;
         one.x = 1;
-        inv = cdiv(one, tel(r, r));
+        inv = cdiv(one, buf[lane * TRSM_PITCH + lane]);
     }
-#pragma unroll 8
+#pragma unroll
     for (int k = 0; k < TS; k++) {
-        const int j = warp * TS + k;
-        C2 d = zero;
-        if (row && j < kb && (UPPER ? k > lane : k < lane)) d = tel(r, j);
-        if (UPPER && !UNIT) {
-            C2 e;
-            e.x = d.x * inv.x - d.y * inv.y;
-            e.y = d.x * inv.y + d.y * inv.x;
-            d = e;
-        }
-        D[k * TS] = d;
+        D[k] = zero;
+        if (UPPER ? k > lane : k < lane) D[k] = buf[lane * TRSM_PITCH + k];
+        if (UPPER && !UNIT) D[k] = panel_mul(D[k], inv);
     }
+    __syncwarp();
+    if (UPPER ? warp < nsb - 1 : warp > 0) fetch(UPPER ? nsb - 1 : 0);
     for (int step = 0; step < nsb; step++) {
         const int s = UPPER ? nsb - 1 - step : step, par = step & 1;
-        C2 t[TS];
         if (warp == s) {
             if (UPPER && !UNIT) {
 #pragma unroll
-                for (int c = 0; c < RB; c++) {
-                    C2 e;
-                    e.x = x[c].x * inv.x - x[c].y * inv.y;
-                    e.y = x[c].x * inv.y + x[c].y * inv.x;
-                    x[c] = e;
-                }
+                for (int c = 0; c < RB; c++) x[c] = panel_mul(x[c], inv);
             }
-#pragma unroll 8
+#pragma unroll
             for (int kk = 0; kk < TS; kk++) {
                 const int k = UPPER ? TS - 1 - kk : kk;
-                const C2 d = D[k * TS];
                 const bool open = UPPER ? lane < k : lane > k;
 #pragma unroll
                 for (int c = 0; c < RB; c++) {
                     const C2 xk = shfl_c(x[c], k);
-                    if (open) csub_mul(x[c], d, xk);
+                    if (open) csub_mul(x[c], D[k], xk);
                 }
             }
 #pragma unroll
             for (int c = 0; c < RB; c++) xs[par][lane][c] = x[c];
         }
         const bool later = UPPER ? warp < s : warp > s;
-        if (later) {
-#pragma unroll
-            for (int k = 0; k < TS; k++) t[k] = (row && s * TS + k < kb) ? tel(r, s * TS + k) : zero;
-        }
+        if (later) dmma::cp_wait<0>();
         __syncthreads();
         if (later) {
+            const C2* t = buf + lane * TRSM_PITCH;
+#pragma unroll 8
+            for (int k = 0; k < TS; k++) {
+                const C2 tk = t[k];
 #pragma unroll
-            for (int k = 0; k < TS; k++)
-#pragma unroll
-                for (int c = 0; c < RB; c++) csub_mul(x[c], t[k], xs[par][k][c]);
+                for (int c = 0; c < RB; c++) csub_mul(x[c], tk, xs[par][k][c]);
+            }
+            __syncwarp();
+            const int next = UPPER ? s - 1 : s + 1;
+            if (UPPER ? warp < next : warp > next) fetch(next);
         }
     }
     if (!row) return;
@@ -940,19 +951,19 @@ static int launch_trsm_block(bem_ctx* ctx, const typename C2T<R>::type* T, int64
     if (!(attr_set.load() & bit)) {
         BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(trsm_block_kernel<R, UPPER, B_ROWMAJOR, RB, MODE>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)(TRSM_KB * TRSM_TS * sizeof(C2))));
+                                               (int)(TRSM_KB * TRSM_PITCH * sizeof(C2))));
         attr_set.fetch_or(bit);
     }
     const int threads = (kb + TRSM_TS - 1) / TRSM_TS * TRSM_TS;
     const dim3 grid((c1 - c0 + RB - 1) / RB, batch);
-    trsm_block_kernel<R, UPPER, B_ROWMAJOR, RB, MODE><<<grid, threads, (size_t)threads * TRSM_TS * sizeof(C2), ctx->stream>>>(
+    trsm_block_kernel<R, UPPER, B_ROWMAJOR, RB, MODE><<<grid, threads, (size_t)threads * TRSM_PITCH * sizeof(C2), ctx->stream>>>(
         T, ldt, r0, kb, B, ldb, br0, c0, c1, sT, sB);
     return BEM_OK;
 }
 
 // B's rows of the block start at br0 (at r0, the block's own rows, when br0 < 0).
-// Columns per CTA: two while that gives no more CTAs than SMs (the
-// substitution's chain is the time, whatever the columns), else eight, whose
+// Columns per CTA: one while that gives no more CTAs than SMs, then two (the
+// substitution's chain is the time: 20, 22 to 24 us), else eight, whose
 // registers still hold the rows of T.
 template <typename R, bool UPPER, bool B_ROWMAJOR, int MODE = 0>
 int trsm_block(bem_ctx* ctx, const typename C2T<R>::type* T, int64_t ldt, int r0, int kb,
@@ -963,7 +974,9 @@ int trsm_block(bem_ctx* ctx, const typename C2T<R>::type* T, int64_t ldt, int r0
     if (c1 <= c0 || kb <= 0) return BEM_OK;
     if (kb > TRSM_KB) return fail(ctx, BEM_ERR_INVALID, "block TRSM: %d rows > %d", kb, TRSM_KB);
     cudaEvent_t ev = ctx->prof_begin(PROF_TRSM);
-    if ((int64_t)(c1 - c0 + 1) / 2 * batch <= ctx->sm_count)
+    if ((int64_t)(c1 - c0) * batch <= ctx->sm_count)
+        BEM_TRY((launch_trsm_block<R, UPPER, B_ROWMAJOR, 1, MODE>(ctx, T, ldt, r0, kb, B, ldb, c0, c1, br0, batch, sT, sB)));
+    else if ((int64_t)(c1 - c0 + 1) / 2 * batch <= ctx->sm_count)
         BEM_TRY((launch_trsm_block<R, UPPER, B_ROWMAJOR, 2, MODE>(ctx, T, ldt, r0, kb, B, ldb, c0, c1, br0, batch, sT, sB)));
     else
         BEM_TRY((launch_trsm_block<R, UPPER, B_ROWMAJOR, 8, MODE>(ctx, T, ldt, r0, kb, B, ldb, c0, c1, br0, batch, sT, sB)));
