@@ -55,17 +55,18 @@ int cgemm(bem_ctx* ctx, int M, int N, int K, const typename C2T<R>::type* A, int
     }
     if (batch > 1 && sizeof(R) != 8) return fail(ctx, BEM_ERR_INVALID, "batched GEMM is FP64 only");
     dim3 grid((N + 63) / 64, (M + 63) / 64, batch);
-    // the 3M kernel's tile: the least time of its rounds over the SMs.  A
-    // tile's time goes with its outputs; the smaller tiles reach about 0.8 and
-    // 0.5 of the big one's rate.
+    // the 3M kernel's tile: the least time of the SM with the most tiles.  Per
+    // K = 256 and SM, measured (us): 64 x 64 34 alone, 32 each of more; 32 x 32
+    // 10.7 and 9; 32 x 8 4.1 and 2.75 (3.5 with an N-major B).
     int tile = 0;
     if (sizeof(R) == 8 && ctx->dmma_3m) {
         const int bm[3] = {64, 32, 32}, bn[3] = {64, 32, 8};
-        const double rate[3] = {1.0, 0.8, 0.5};
+        const double one[3] = {34.0, 10.7, 4.1}, each[3] = {32.0, 9.0, b_kmajor ? 2.75 : 3.5};
         double best = 0.0;
         for (int t = 0; t < 3; t++) {
             const int64_t tiles = (int64_t)((M + bm[t] - 1) / bm[t]) * ((N + bn[t] - 1) / bn[t]) * batch;
-            const double cost = (double)((tiles + ctx->sm_count - 1) / ctx->sm_count) * bm[t] * bn[t] / rate[t];
+            const int64_t per_sm = (tiles + ctx->sm_count - 1) / ctx->sm_count;
+            const double cost = std::max(one[t], each[t] * (double)per_sm);
             if (t == 0 || (cost < best && (M + 31) / 32 <= 65535)) best = cost, tile = t;
         }
         grid = dim3((N + bn[tile] - 1) / bn[tile], (M + bm[tile] - 1) / bm[tile], batch);
@@ -81,32 +82,33 @@ int cgemm(bem_ctx* ctx, int M, int N, int K, const typename C2T<R>::type* A, int
         const double2* Bd = reinterpret_cast<const double2*>(B);
         double2* Cd = reinterpret_cast<double2*>(C);
         double2 al = make_double2(alpha.x, alpha.y), be = make_double2(beta.x, beta.y);
-        auto go = [&](auto kern, int slot, int threads, int smem) -> int {
+        auto go = [&](auto kern, int slot, int threads, int smem, int smem_max) -> int {
             const unsigned long long bit = 1ull << (ctx->device & 63);
             if (!(attr[slot].load() & bit)) {
-                BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+                BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max));
                 attr[slot].fetch_or(bit);
             }
             kern<<<grid, threads, smem, ctx->stream>>>(M, N, K, Ad, lda, Bd, ldb, Cd, ldc, al, be, sA, sB, sC);
             return BEM_OK;
         };
+        const int nst = (K + dmma::BKC - 1) / dmma::BKC;
         auto go3 = [&](auto tl, int slot) -> int {
             using T = decltype(tl);
             if (b_kmajor)
-                return c_colmajor ? go(dmma::zgemm3m_kernel<T, true, true>, slot, T::THREADS, T::SMEM_BYTES)
-                                  : go(dmma::zgemm3m_kernel<T, true, false>, slot + 1, T::THREADS, T::SMEM_BYTES);
-            return c_colmajor ? go(dmma::zgemm3m_kernel<T, false, true>, slot + 2, T::THREADS, T::SMEM_BYTES)
-                              : go(dmma::zgemm3m_kernel<T, false, false>, slot + 3, T::THREADS, T::SMEM_BYTES);
+                return c_colmajor ? go(dmma::zgemm3m_kernel<T, true, true>, slot, T::THREADS, T::smem_bytes(true, nst), T::smem_bytes(true, 1 << 20))
+                                  : go(dmma::zgemm3m_kernel<T, true, false>, slot + 1, T::THREADS, T::smem_bytes(true, nst), T::smem_bytes(true, 1 << 20));
+            return c_colmajor ? go(dmma::zgemm3m_kernel<T, false, true>, slot + 2, T::THREADS, T::smem_bytes(false, nst), T::smem_bytes(false, 1 << 20))
+                              : go(dmma::zgemm3m_kernel<T, false, false>, slot + 3, T::THREADS, T::smem_bytes(false, nst), T::smem_bytes(false, 1 << 20));
         };
         const int t4 = 128, s4 = dmma::SMEM_BYTES;
         int s;
         if (ctx->dmma_3m) {
             s = tile == 0 ? go3(dmma::M3Big{}, 4) : tile == 1 ? go3(dmma::M3Small{}, 8) : go3(dmma::M3Thin{}, 12);
         } else if (b_kmajor) {
-            s = c_colmajor ? go(dmma::zgemm_kernel<true, true>, 0, t4, s4) : go(dmma::zgemm_kernel<true, false>, 1, t4, s4);
+            s = c_colmajor ? go(dmma::zgemm_kernel<true, true>, 0, t4, s4, s4) : go(dmma::zgemm_kernel<true, false>, 1, t4, s4, s4);
         } else {
-            s = c_colmajor ? go(dmma::zgemm_kernel<false, true>, 2, t4, s4)
-                           : go(dmma::zgemm_kernel<false, false>, 3, t4, s4);
+            s = c_colmajor ? go(dmma::zgemm_kernel<false, true>, 2, t4, s4, s4)
+                           : go(dmma::zgemm_kernel<false, false>, 3, t4, s4, s4);
         }
         BEM_TRY(s);
     } else if (b_kmajor) {

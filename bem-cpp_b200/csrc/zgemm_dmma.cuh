@@ -196,26 +196,37 @@ zgemm_kernel(int M, int N, int K, const double2* __restrict__ A, int64_t lda, co
 
 // ----------------------------------------------------------------- 3M form
 // Tile of the 3M kernel: BM x BN complex outputs, WM x WN warps (each
-// BM / WM x BN / WN).  An SM gives ~125 G FP64 multiply-adds a second, so a
-// 64 x 64 tile of K = 256 takes 50 us on it: products with fewer such tiles
-// than SMs (the block updates of a solve with few right-hand sides) run on
-// smaller tiles that reach every SM.  An output's sums run over k in the same
-// order in every tile, so the tiles give the same bits.
-template <int BM_, int BN_, int WM_, int WN_, int MINB_> struct M3Tile {
+// BM / WM x BN / WN), STK / STN stages of K for a K-major / N-major B.  An SM
+// takes 34 us for a 64 x 64 tile of K = 256, alone or not: products with fewer
+// such tiles than SMs (the block updates of a solve with few right-hand sides)
+// run on smaller tiles that reach every SM.  A warp alone on its scheduler
+// issues a DMMA every 40 cycles, several one every 21, and one stage of a
+// small tile is 10 to 20 KB: so the small tiles keep more warps than their
+// outputs need and more stages in flight.  Solves of n = 3840 with 32 columns
+// (K = 256): 32 x 8 tiles 15.1 -> 7.5 us a product, the 32 x 32 ones and the
+// products with Z 34.1 -> 27 us, against two stages, four warps and the values
+// of C read one by one in the epilogue.  More stages cost co-resident CTAs (32 x 8, M = 4096: 15.0 us
+// with 4, 16.9 us with 5 to 8).  An output's sums run over k in the same order
+// in every tile, so the tiles give the same bits.
+template <int BM_, int BN_, int WM_, int WN_, int MINB_, int STK_, int STN_> struct M3Tile {
     static constexpr int BM = BM_, BN = BN_, WM = WM_, WN = WN_, MINB = MINB_;
     static constexpr int THREADS = 32 * WM * WN, IM = BM / WM / 8, NJ = BN / WN / 8;
     static constexpr int AROW = 2 * BKC + 8;    // doubles: 20 16-byte units, 4 mod 8 (conflict-free 128-bit reads)
     static constexpr int BROW_K = 2 * BKC + 8;
     static constexpr int BROW_N = 2 * BN + 4;   // 2 mod 8 16-byte units
     static constexpr int A_STAGE = BM * AROW;
-    static constexpr int B_STAGE = BN * BROW_K > BKC * BROW_N ? BN * BROW_K : BKC * BROW_N;
-    static constexpr int SMEM_BYTES = STAGES * (A_STAGE + B_STAGE) * 8;
+    static constexpr int stages(bool b_kmajor) { return b_kmajor ? STK_ : STN_; }
+    static constexpr int stage(bool b_kmajor) { return A_STAGE + (b_kmajor ? BN * BROW_K : BKC * BROW_N); }
+    // dynamic shared memory: no more stages than K has
+    static constexpr int smem_bytes(bool b_kmajor, int nst) {
+        return (nst < stages(b_kmajor) ? nst : stages(b_kmajor)) * stage(b_kmajor) * 8;
+    }
     static_assert(BM % (8 * WM) == 0 && BN % (8 * WN) == 0, "3M tile");
     static_assert(BM * BKC % THREADS == 0 && BN * BKC % THREADS == 0, "3M tile loads");
 };
-using M3Big = M3Tile<64, 64, 2, 4, 2>;
-using M3Small = M3Tile<32, 32, 2, 2, 4>;
-using M3Thin = M3Tile<32, 8, 4, 1, 4>;
+using M3Big = M3Tile<64, 64, 2, 4, 2, 2, 2>;
+using M3Small = M3Tile<32, 32, 4, 2, 3, 3, 3>;
+using M3Thin = M3Tile<32, 8, 4, 1, 4, 4, 4>;
 
 template <class T, bool B_KMAJOR, bool C_COLMAJOR>
 __global__ void __launch_bounds__(T::THREADS, T::MINB)
@@ -227,8 +238,7 @@ zgemm3m_kernel(int M, int N, int K, const double2* __restrict__ A, int64_t lda, 
     B += blockIdx.z * sB;
     C += blockIdx.z * sC;
     extern __shared__ __align__(16) double sm[];
-    double* As = sm;                          // STAGES x A_STAGE
-    double* Bs = sm + STAGES * T::A_STAGE;    // STAGES x B_STAGE
+    constexpr int ST = T::stages(B_KMAJOR), STAGE = T::stage(B_KMAJOR);  // stage: A_STAGE doubles of A, then B's
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int wm = (warp / T::WN) * 8 * IM, wn = (warp % T::WN) * 8 * NJ;  // warp tile origin (complex)
     const int m0 = blockIdx.y * T::BM, n0 = blockIdx.x * T::BN;
@@ -236,8 +246,8 @@ zgemm3m_kernel(int M, int N, int K, const double2* __restrict__ A, int64_t lda, 
 
     auto load_stage = [&](int st, int buf) {
         const int k0 = st * BKC;
-        double* as = As + buf * T::A_STAGE;
-        double* bs = Bs + buf * T::B_STAGE;
+        double* as = sm + buf * STAGE;
+        double* bs = as + T::A_STAGE;
 #pragma unroll
         for (int l = 0; l < T::BM * BKC / T::THREADS; l++) {
             const int e = tid + T::THREADS * l;
@@ -272,22 +282,22 @@ zgemm3m_kernel(int M, int N, int K, const double2* __restrict__ A, int64_t lda, 
             for (int h = 0; h < 2; h++) t1[i][j][h] = t2[i][j][h] = t3[i][j][h] = 0.0;
 
 #pragma unroll
-    for (int s = 0; s < STAGES - 1; s++) {
+    for (int s = 0; s < ST - 1; s++) {
         if (s < nst) load_stage(s, s);
         cp_commit();
     }
     const int fr = lane >> 2, fk = lane & 3;  // fragment row (A) / column (B), k within the m8n8k4 step
     for (int st = 0; st < nst; st++) {
-        cp_wait<STAGES - 2>();
+        cp_wait<ST - 2>();
         __syncthreads();
         {
-            const int nx = st + STAGES - 1;
-            if (nx < nst) load_stage(nx, nx % STAGES);
+            const int nx = st + ST - 1;
+            if (nx < nst) load_stage(nx, nx % ST);
             cp_commit();
         }
-        const int buf = st % STAGES;
-        const double* as = As + buf * T::A_STAGE;
-        const double* bs = Bs + buf * T::B_STAGE;
+        const int buf = st % ST;
+        const double* as = sm + buf * STAGE;
+        const double* bs = as + T::A_STAGE;
 #pragma unroll
         for (int kk = 0; kk < BKC / 4; kk++) {  // complex K steps of 4
             const int kc = 4 * kk + fk;
@@ -325,6 +335,16 @@ zgemm3m_kernel(int M, int N, int K, const double2* __restrict__ A, int64_t lda, 
     for (int i = 0; i < IM; i++) {
         const int gi = m0 + wm + 8 * i + fr;
         if (gi >= M) continue;
+        // the row's values of C first: their loads are in flight together
+        double2 c[NJ][2];
+#pragma unroll
+        for (int j = 0; j < NJ; j++)
+#pragma unroll
+            for (int h = 0; h < 2; h++) {
+                const int gj = n0 + wn + 8 * j + 2 * fk + h;
+                c[j][h] = make_double2(0.0, 0.0);
+                if (has_beta && gj < N) c[j][h] = C[C_COLMAJOR ? (int64_t)gj * ldc + gi : (int64_t)gi * ldc + gj];
+            }
 #pragma unroll
         for (int j = 0; j < NJ; j++)
 #pragma unroll
@@ -334,13 +354,11 @@ zgemm3m_kernel(int M, int N, int K, const double2* __restrict__ A, int64_t lda, 
                 const double ar = t1[i][j][h] - t2[i][j][h];
                 const double ai = t3[i][j][h] - t1[i][j][h] - t2[i][j][h];
                 double2 v = make_double2(alpha.x * ar - alpha.y * ai, alpha.x * ai + alpha.y * ar);
-                const int64_t idx = C_COLMAJOR ? (int64_t)gj * ldc + gi : (int64_t)gi * ldc + gj;
                 if (has_beta) {
-                    const double2 c = C[idx];
-                    v.x += beta.x * c.x - beta.y * c.y;
-                    v.y += beta.x * c.y + beta.y * c.x;
+                    v.x += beta.x * c[j][h].x - beta.y * c[j][h].y;
+                    v.y += beta.x * c[j][h].y + beta.y * c[j][h].x;
                 }
-                C[idx] = v;
+                C[C_COLMAJOR ? (int64_t)gj * ldc + gi : (int64_t)gi * ldc + gj] = v;
             }
     }
 }
