@@ -380,21 +380,25 @@ panel_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int r0, int nro
 // interchanging rows jj and p only exchanges their positions (one integer per
 // thread, which is also the tie break), and each row is written to its final
 // position at the end.  Per column jj:
-//   1. every warp finds its largest |re| + |im| of column jj among rows not
-//      yet taken (smallest position on ties); the winning lane leaves its
-//      columns jj.. in shared memory; block barrier;
-//   2. warp k reduces the CTA's candidates, forms 1 / pivot and writes value,
-//      position, reciprocal and row into CTA k's shared memory; cluster
-//      barrier;
-//   3. every warp reduces the C candidates from its own shared memory, and
-//      every row still active is scaled and takes the rank-1 update
-//      x -= l u, u read as a broadcast.
-// So a column costs one block and one cluster barrier and no load from
-// another SM: 60 us per 16 columns at 2300 rows with the rows in shared
-// memory, their interchange there and the candidates gathered from the
-// peers after the barrier.  Buffers alternate between two parities: a CTA
-// writing a peer's buffer in column jj + 2 has passed the barrier of jj + 1,
-// which that peer reaches after its reads of column jj.
+//   1. every warp has its largest |re| + |im| of column jj among rows not yet
+//      taken (smallest position on ties), searched with the row's reciprocal
+//      while the columns after jj were updated; the winning lane leaves both
+//      and its columns jj.. in shared memory; block barrier;
+//   2. every warp k < C reduces the CTA's candidates and sends the best one to
+//      CTA k's shared memory (st.async, counted on an mbarrier there);
+//   3. every thread waits for its CTA's C messages, every warp reduces the C
+//      candidates from its own shared memory, and every row still active is
+//      scaled and takes the rank-1 update x -= l u, u read as a broadcast,
+//      column jj + 1 first.
+// So a column costs one block barrier and one message's way to another SM.
+// 16 columns, us, now and with stores, a cluster barrier and the reciprocal
+// after it: 256 rows (1 CTA) 18.7 and 18.7, 2048 (8) 25.7 and 28.9, 4096 (16)
+// 26.8 and 37.0 (on 8 CTAs), 4608 (16) 28.9 and 39.0.  Of ~2600 cycles a
+// column on 8 CTAs the row's way into shared memory takes 430, the message 820,
+// the reductions 250 to 300 each and the updates 650.
+// Buffers alternate between two parities: a CTA sending to a peer in column
+// jj + 2 has that peer's message of jj + 1, sent after the block barrier that
+// follows the peer's reads of column jj.
 // Same pivot rule and per-element arithmetic (panel_mul, panel_msub) as
 // panel_kernel, so the same pivots and factors.
 // moves (2 n integers per matrix): for the w top positions k of the panel,
@@ -404,50 +408,81 @@ template <typename R> struct PanelW { static constexpr int v = 64 / (2 * (int)si
 constexpr int PR_THREADS = 512, PR_WARPS = PR_THREADS / 32, PR_CLUSTER = 16, PG = 4;
 constexpr int PR_PITCH = 256 + 16;  // bytes of a row in shared memory
 
-// The warp's largest bv, the smallest br among the lanes holding it and that
-// lane's bk, in every lane.  bv >= 0 (a lane without a candidate holds 0 with
-// br = INT_MAX): the bit patterns of non-negative floating-point numbers
-// order like unsigned integers, so integer warp reductions find it.
-__device__ __forceinline__ void warp_argmax_bits(unsigned hi, unsigned lo, int& br, int& bk, unsigned& mhi,
-                                                 unsigned& mlo) {
-    mhi = __reduce_max_sync(0xffffffffu, hi);
-    unsigned win = __ballot_sync(0xffffffffu, hi == mhi);
+// A pivot candidate: |v| as its bit pattern (v >= 0, 0 for none: the bits of
+// non-negative floating-point numbers order like unsigned integers, so integer
+// warp reductions compare them) and its row's position.
+__device__ __forceinline__ uint4 cand_bits(double v, int pos) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+    return make_uint4((unsigned)(b >> 32), (unsigned)b, (unsigned)pos, 0u);
+}
+__device__ __forceinline__ uint4 cand_bits(float v, int pos) { return make_uint4(__float_as_uint(v), 0u, (unsigned)pos, 0u); }
+// The lane with the warp's largest candidate, the smallest position on ties,
+// -1 where there is none; mhi is the largest upper word of all lanes.
+__device__ __forceinline__ int cand_lane(uint4 c, unsigned mhi) {
+    unsigned win = __ballot_sync(0xffffffffu, c.x == mhi);
     if (win & (win - 1)) {  // several lanes share the upper word: the lower one and the row decide
-        mlo = __reduce_max_sync(0xffffffffu, hi == mhi ? lo : 0u);
-        const bool top = hi == mhi && lo == mlo;
-        const unsigned mrow = __reduce_min_sync(0xffffffffu, top ? (unsigned)br : 0xffffffffu);
-        win = __ballot_sync(0xffffffffu, top && (unsigned)br == mrow);
+        const unsigned mlo = __reduce_max_sync(0xffffffffu, c.x == mhi ? c.y : 0u);
+        if ((mhi | mlo) == 0u) return -1;
+        const bool top = c.x == mhi && c.y == mlo;
+        const unsigned mrow = __reduce_min_sync(0xffffffffu, top ? c.z : 0xffffffffu);
+        win = __ballot_sync(0xffffffffu, top && c.z == mrow);
     }
-    const int w = __ffs(win) - 1;
-    mlo = __shfl_sync(0xffffffffu, lo, w);
-    br = __shfl_sync(0xffffffffu, br, w);
-    bk = __shfl_sync(0xffffffffu, bk, w);
+    return __ffs(win) - 1;
 }
-__device__ __forceinline__ void warp_argmax(double& bv, int& br, int& bk) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(bv);
-    unsigned mhi, mlo;
-    warp_argmax_bits((unsigned)(b >> 32), (unsigned)b, br, bk, mhi, mlo);
-    bv = __longlong_as_double((long long)(((unsigned long long)mhi << 32) | mlo));
+
+// A value into a peer's shared memory, counted on the peer's mbarrier.
+__device__ __forceinline__ void st_async(uint32_t dst, uint32_t bar, uint4 v) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(dst),
+                 "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(bar)
+                 : "memory");
 }
-__device__ __forceinline__ void warp_argmax(float& bv, int& br, int& bk) {
-    unsigned mhi, mlo;
-    warp_argmax_bits(__float_as_uint(bv), 0u, br, bk, mhi, mlo);
-    bv = __uint_as_float(mhi);
+__device__ __forceinline__ void st_async(uint32_t dst, uint32_t bar, double2 v) {
+    const unsigned long long x = (unsigned long long)__double_as_longlong(v.x), y = (unsigned long long)__double_as_longlong(v.y);
+    st_async(dst, bar, make_uint4((unsigned)x, (unsigned)(x >> 32), (unsigned)y, (unsigned)(y >> 32)));
+}
+__device__ __forceinline__ void st_async(uint32_t dst, uint32_t bar, float2 v) {
+    asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];" ::"r"(dst),
+                 "r"(__float_as_uint(v.x)), "r"(__float_as_uint(v.y)), "r"(bar)
+                 : "memory");
+}
+__device__ __forceinline__ uint32_t map_rank(uint32_t smem, int rank) {
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem), "r"(rank));
+    return r;
+}
+// Waits until the phase of this parity is complete, ~1 s of clock cycles at most.
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity) {
+    long long t0 = 0;
+    for (int i = 0;; i++) {
+        uint32_t ok;
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+            "selp.u32 %0, 1, 0, p;\n\t}"
+            : "=r"(ok)
+            : "r"(bar), "r"(parity)
+            : "memory");
+        if (ok) return true;
+        if (i == 0) t0 = clock64();
+        if (clock64() - t0 > 2000000000ll) return false;
+    }
 }
 
 template <typename R>
 __global__ void __launch_bounds__(PR_THREADS, 1)
 panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int r0, int nrows, int w,
-                 int* __restrict__ ipiv, int* __restrict__ info, int* __restrict__ moves, int64_t sA) {
+                 int* __restrict__ ipiv, int* __restrict__ info, int* __restrict__ moves, int64_t sA,
+                 int* __restrict__ status) {
     using C2 = typename C2T<R>::type;
     namespace cg = cooperative_groups;
     constexpr int W = PanelW<R>::v;
     cg::cluster_group cluster = cg::this_cluster();
     __shared__ __align__(16) C2 s_row[2][PR_WARPS][W];    // a warp's candidate row
     __shared__ __align__(16) C2 r_row[2][PR_CLUSTER][W];  // a CTA's candidate row (written by the peers)
-    __shared__ C2 r_inv[2][PR_CLUSTER];
-    __shared__ R s_v[2][PR_WARPS], r_v[2][PR_CLUSTER];
-    __shared__ int s_pos[2][PR_WARPS], r_pos[2][PR_CLUSTER], s_at[PR_THREADS];
+    __shared__ __align__(16) C2 s_inv[2][PR_WARPS], r_inv[2][PR_CLUSTER];
+    __shared__ __align__(16) uint4 s_cand[2][PR_WARPS], r_cand[2][PR_CLUSTER];
+    __shared__ __align__(8) unsigned long long r_bar[2];
+    __shared__ int s_at[PR_THREADS];
     // the rows on their way in and out, 256 B each: 16 lanes a row in global
     // memory, a thread a row here (an odd number of 16-byte units apart)
     extern __shared__ __align__(16) unsigned char pr_smem[];
@@ -458,6 +493,12 @@ panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int 
     ipiv += (int64_t)mi * n;
     info += mi;
     moves += (int64_t)mi * 2 * n;
+    const uint32_t bar0 = static_cast<uint32_t>(__cvta_generic_to_shared(&r_bar[0]));
+    if (C > 1 && tid == 0) {
+        for (int k = 0; k < 2; k++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8 * k) : "memory");
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    bool late = false;  // a wait ran out
     const int gr = b * T + tid;
     const bool valid = gr < nrows;
     bool act = valid;
@@ -489,6 +530,24 @@ panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int 
     // finished ones; the row rotates left by PG after each group, so W / PG
     // groups bring it back.  One loop over the groups instead of W unrolled
     // columns: those were 13 k instructions that every launch fetched anew.
+    // this thread's candidate of a column, the warp's largest upper word and
+    // the reciprocal that the row needs if it wins: all under the update of
+    // the columns after it
+    uint4 cand;
+    unsigned mhi;
+    C2 rinv;
+    auto search = [&](C2 xv) {
+        R v = act ? cabs1<R>(xv) : (R)0;
+        if (!(v > (R)0)) {  // a NaN is no candidate either
+            v = (R)0;
+            xv.x = 1, xv.y = 0;
+        }
+        cand = cand_bits(v, pos);
+        mhi = __reduce_max_sync(0xffffffffu, cand.x);
+        rinv = pivot_recip(xv);
+    };
+    const uint4 none = make_uint4(0u, 0u, 0x7fffffffu, 0u);
+    search(x[0]);
     for (int g0 = 0; g0 < W; g0 += PG) {
       const int rem = W - g0;
 #pragma unroll
@@ -496,54 +555,63 @@ panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int 
         const int jj = g0 + q;
         if (jj >= w) break;
         const int par = q & 1;  // PG is even: the parity of jj
-        // 1. this warp's candidate (v = 0: none; a NaN is none either)
-        R v = act ? cabs1<R>(x[q]) : (R)0;
-        if (!(v > (R)0)) v = (R)0;
-        int br = v > (R)0 ? pos : 0x7fffffff, bk = lane;
-        warp_argmax(v, br, bk);
-        if (lane == bk && v > (R)0) {
+        // 1. this warp's candidate
+        const int wl = cand_lane(cand, mhi);
+        if (lane == max(wl, 0)) {
+            s_cand[par][warp] = wl < 0 ? none : cand;
+            s_inv[par][warp] = rinv;
 #pragma unroll
-            for (int c = q; c < W; c++)
-                if (c < rem) s_row[par][warp][c] = x[c];
+            for (int c0 = 0; c0 < W; c0 += PG)
+                if (c0 < rem) {
+#pragma unroll
+                    for (int c = c0; c < c0 + PG; c++)
+                        if (c >= q) s_row[par][warp][c] = x[c];
+                }
         }
-        if (lane == 0) s_v[par][warp] = v, s_pos[par][warp] = br;
         __syncthreads();
+        uint4 rec = lane < nw ? s_cand[par][lane] : none;
         const C2* u;
         C2 inv;
         if (C > 1) {
             // 2. the CTA's candidate into every CTA of the cluster
-            for (int k = warp; k < C; k += nw) {
-                R cv = lane < nw ? s_v[par][lane] : (R)0;
-                int cr = lane < nw ? s_pos[par][lane] : 0x7fffffff, ck = lane;
-                warp_argmax(cv, cr, ck);
-                if (cv > (R)0) {
-                    const C2 iv = pivot_recip(s_row[par][ck][q]);
-                    if (lane >= q && lane < rem) cluster.map_shared_rank(&r_row[par][b][0], k)[lane] = s_row[par][ck][lane];
-                    if (lane == 0) *cluster.map_shared_rank(&r_inv[par][b], k) = iv;
-                }
-                if (lane == 0) {
-                    *cluster.map_shared_rank(&r_v[par][b], k) = cv;
-                    *cluster.map_shared_rank(&r_pos[par][b], k) = cv > (R)0 ? cr : 0x7fffffff;
+            const uint32_t bar = bar0 + 8 * par;
+            if (tid == 0) {
+                const int bytes = C * ((rem - q + 1) * (int)sizeof(C2) + (int)sizeof(uint4));
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+            }
+            if (warp < C) {
+                const int ck = cand_lane(rec, __reduce_max_sync(0xffffffffu, rec.x)), cw = max(ck, 0);
+                const C2 e = s_row[par][cw][lane < W ? lane : 0], iv = s_inv[par][cw];
+                const uint4 cc = ck < 0 ? none : s_cand[par][cw];
+                const uint32_t row = static_cast<uint32_t>(__cvta_generic_to_shared(&r_row[par][b][lane < W ? lane : 0])),
+                               to = static_cast<uint32_t>(__cvta_generic_to_shared(&r_cand[par][b])),
+                               rcp = static_cast<uint32_t>(__cvta_generic_to_shared(&r_inv[par][b]));
+                for (int k = warp; k < C; k += nw) {
+                    const uint32_t kb = map_rank(bar, k);
+                    if (lane >= q && lane < rem) st_async(map_rank(row, k), kb, e);
+                    if (lane == 0) {
+                        st_async(map_rank(to, k), kb, cc);
+                        st_async(map_rank(rcp, k), kb, iv);
+                    }
                 }
             }
-            cluster.sync();
-            v = lane < C ? r_v[par][lane] : (R)0;
-            br = lane < C ? r_pos[par][lane] : 0x7fffffff;
-            bk = lane;
-            warp_argmax(v, br, bk);
-            u = r_row[par][bk];
-            inv = r_inv[par][bk];
-        } else {
-            v = lane < nw ? s_v[par][lane] : (R)0;
-            br = lane < nw ? s_pos[par][lane] : 0x7fffffff;
-            bk = lane;
-            warp_argmax(v, br, bk);
-            u = s_row[par][bk];
-            inv = pivot_recip(u[q]);
+            if (!late) late = !mbar_wait_cluster(bar, (uint32_t)(jj >> 1) & 1u);
+            rec = lane < C ? r_cand[par][lane] : none;
         }
-        // 3. v = 0: a zero column, no interchange and no scaling (LAPACK records it)
-        const bool zp = !(v > (R)0);
-        const int piv = zp ? jj : br;
+        const int bk = cand_lane(rec, __reduce_max_sync(0xffffffffu, rec.x)), bw = max(bk, 0);
+        int piv;
+        if (C > 1) {
+            u = r_row[par][bw];
+            inv = r_inv[par][bw];
+            piv = (int)r_cand[par][bw].z;
+        } else {
+            u = s_row[par][bw];
+            inv = s_inv[par][bw];
+            piv = (int)s_cand[par][bw].z;
+        }
+        // 3. no candidate: a zero column, no interchange and no scaling (LAPACK records it)
+        const bool zp = bk < 0;
+        if (zp) piv = jj;
         if (b == 0 && tid == 0) {
             ipiv[r0 + jj] = r0 + piv;
             if (zp) atomicCAS(info, 0, r0 + jj + 1);
@@ -554,15 +622,21 @@ panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int 
         } else if (pos == jj) {
             pos = piv;
         }
-        if (act && !zp) {
-            const C2 l = panel_mul(x[q], inv);
-            x[q] = l;
+        const bool on = act && !zp;
+        const C2 l = panel_mul(x[q], inv);
+        if (on) x[q] = l;
+        // the next column first: its candidates are searched under the others' update
+        if (q + 1 < W && q + 1 < rem) {
+            if (on) x[q + 1] = panel_msub(x[q + 1], l, u[q + 1]);
+            search(x[q + 1]);
+        }
+        if (on) {
 #pragma unroll
             for (int c0 = 0; c0 < W; c0 += PG)
                 if (c0 < rem) {
 #pragma unroll
                     for (int c = c0; c < c0 + PG; c++)
-                        if (c > q) x[c] = panel_msub(x[c], l, u[c]);
+                        if (c > q + 1) x[c] = panel_msub(x[c], l, u[c]);
                 }
         }
       }
@@ -574,6 +648,10 @@ panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int 
 #pragma unroll
       for (int c = 0; c < PG; c++) x[W - PG + c] = done[c];
     }
+    if (late) *status = BEM_ERR_TIMEOUT;
+    __syncwarp();
+    // no CTA ends while a peer may still write to it (the wait is at the end)
+    if (C > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     // rows to their positions (every row of the panel was read before the first barrier)
     if (valid) {
 #pragma unroll
@@ -595,20 +673,24 @@ panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int 
         if (pos < w) moves[r0 + pos] = r0 + gr;
         if (gr < w) moves[n + r0 + gr] = r0 + pos;
     }
+    __syncwarp();
+    if (C > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// CTAs per cluster and threads per CTA for a sub-panel of nrows rows, 0 when
-// it does not fit one cluster (panel_kernel takes it): 256 rows a CTA up to 8
-// CTAs (the portable size), then up to 512 rows a CTA, then 16 CTAs -- 8192
-// rows.  Few rows a CTA keep the rank-1 update short (64 registers a row, the
-// FP64 pipe of one SM), few CTAs the cluster barrier.
+// CTAs per cluster and threads per CTA for a sub-panel of nrows rows of
+// `batch` matrices, 0 when it does not fit one cluster (panel_kernel takes
+// it): 256 rows a CTA up to 16 CTAs, then up to 512 rows a CTA -- 8192 rows.
+// Few rows a CTA keep the rank-1 update short (64 registers a row, the FP64
+// pipe of one SM).  Clusters of more than 8 CTAs fit about one to a GPC, so
+// more matrices than that take 8 CTAs while their rows fit.
 struct PanelShape {
     int C = 0, T = 0;
 };
-static PanelShape panel_reg_shape(int nrows) {
+static PanelShape panel_reg_shape(int nrows, int batch) {
     PanelShape p;
     if (nrows > PR_CLUSTER * PR_THREADS) return p;
-    p.C = nrows <= 8 * PR_THREADS ? std::min(8, (nrows + 255) / 256) : PR_CLUSTER;
+    const int most = batch > 8 && nrows <= 8 * PR_THREADS ? 8 : PR_CLUSTER;
+    p.C = std::min(most, (nrows + 255) / 256);
     p.T = ((nrows + p.C - 1) / p.C + 31) / 32 * 32;
     return p;
 }
@@ -616,10 +698,10 @@ static PanelShape panel_reg_shape(int nrows) {
 // panel_reg_shape, kept only where a cluster of that shape can be resident on
 // this device (asked once per shape and remembered).
 template <typename R>
-static PanelShape panel_reg_choice(bem_ctx* ctx, int nrows, int iw) {
+static PanelShape panel_reg_choice(bem_ctx* ctx, int nrows, int iw, int batch) {
     PanelShape p;
     if (!ctx->panel_clusters || iw > PanelW<R>::v) return p;
-    p = panel_reg_shape(nrows);
+    p = panel_reg_shape(nrows, batch);
     if (p.C == 0) return p;
     static std::mutex mu;
     static std::map<std::tuple<int, int, int>, bool> ok;
@@ -670,7 +752,8 @@ static int launch_panel_reg(bem_ctx* ctx, typename C2T<R>::type* A, int64_t lda,
     cfg.attrs = at;
     cfg.numAttrs = 1;
     cudaEvent_t ev = ctx->prof_begin(PROF_PANEL);
-    BEM_TRY_CUDA(ctx, cudaLaunchKernelEx(&cfg, panel_reg_kernel<R>, A, lda, n, i0, nrows, iw, d_ipiv, d_info, d_moves, sA));
+    BEM_TRY_CUDA(ctx, cudaLaunchKernelEx(&cfg, panel_reg_kernel<R>, A, lda, n, i0, nrows, iw, d_ipiv, d_info, d_moves, sA,
+                                         ctx->d_status));
     BEM_LAUNCHED(ctx);
     if (ev)
         ctx->prof_end(PROF_PANEL, ev, 8.0 * (double)nrows * iw * iw / 2 * batch,
@@ -1069,7 +1152,7 @@ int getrf(bem_ctx* ctx, typename C2T<R>::type* A, int64_t lda, int n, int* d_ipi
         for (int i0 = j0; i0 < j0 + jb; i0 += W) {
             const int iw = std::min(W, j0 + jb - i0);
             const int nrows = n - i0;
-            const PanelShape ps = panel_reg_choice<R>(ctx, nrows, iw);
+            const PanelShape ps = panel_reg_choice<R>(ctx, nrows, iw, 1);
             if (ps.C > 0) {
                 BEM_TRY(launch_panel_reg<R>(ctx, A, lda, n, i0, nrows, iw, d_ipiv, d_info, d_moves, 1, 0, ps));
             } else {
@@ -1200,7 +1283,7 @@ int getrf_batched(bem_ctx* ctx, double2* A, int64_t lda, int64_t sA, int n, int 
     const size_t smem_max = 220 * 1024;
     // every sub-panel fits one cluster (the first is the tallest): no
     // cooperative grid, no chunking of the batch
-    const bool all_clusters = panel_reg_choice<R>(ctx, n, W).C > 0;
+    const bool all_clusters = panel_reg_choice<R>(ctx, n, W, batch).C > 0;
     const int Rp_max = (int)std::min<int64_t>(n, ((int64_t)smem_max / (int64_t)sizeof(C2) - W) / W);
     if (Rp_max < 2 * W) return fail(ctx, BEM_ERR_INVALID, "batched LU: panel does not fit");
     const int Gm_min = (n + Rp_max - 1) / Rp_max;
@@ -1256,7 +1339,7 @@ int getrf_batched(bem_ctx* ctx, double2* A, int64_t lda, int64_t sA, int n, int 
         for (int i0 = j0; i0 < j0 + jb; i0 += W) {
             const int iw = std::min(W, j0 + jb - i0);
             const int nrows = n - i0;
-            const PanelShape ps = panel_reg_choice<R>(ctx, nrows, iw);
+            const PanelShape ps = panel_reg_choice<R>(ctx, nrows, iw, batch);
             if (ps.C > 0) {
                 BEM_TRY(launch_panel_reg<R>(ctx, A, lda, n, i0, nrows, iw, d_ipiv, d_info, d_moves, batch, sA, ps));
             } else {
