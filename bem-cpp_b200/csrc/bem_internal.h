@@ -139,8 +139,8 @@ void devmem_cache_enable(int device, bool on);
 bool devmem_cache_enabled(int device);
 
 // Triangle-pair assembly: per-triangle quadrature data relative to the
-// centroid, and the RWGs in tiles of ASM_TILE grown over shared triangles along a Morton curve of
-// their triangles' centroids, so that the RWGs of a tile share triangles.
+// centroid, and the RWGs in tiles of ASM_TILE grown over shared triangles,
+// started along a Morton curve of the centroids.
 constexpr int ASM_TRI_MAX = 32;  // distinct triangles of one tile (2 halves x 16 RWGs at most)
 struct DevTriAsm {
     double* c = nullptr;          // (nt, 3) centroids
@@ -189,7 +189,7 @@ struct bem_ctx {
     size_t tc_bytes = 0;
     bool tc_attr = false;
     int ff_kernel = 0;           // far field: 0 by triangles (shared phases), 1 per RWG-half point
-    int asm_kernel = 0;          // assembly: 0 triangle-pair moments (Morton tiles), 1 per RWG pair
+    int asm_kernel = 0;          // assembly: 0 triangle-pair moments (tiles of patches), 1 per RWG pair
     int tc_group_m = 16;         // row tiles per raster group of the persistent tensor-core GEMM
     bool tc_persistent = true;  // persistent tensor-core GEMM (else one CTA per tile)
     bool tc_pair = true;        // FP16-part GEMM on CTA pairs (cta_group::2, 256-row tiles)
@@ -208,8 +208,8 @@ struct bem_ctx {
     int gmres_digits = 0;        // GMRES products with Z: 0 FP64 DMMA GEMM, 2..8 int8 Ozaki digits
     bool batch_buckets = true;   // bem_batch_run: FP64 particles of one size batched (else one at a time)
     bool lu_autotune = true;     // batched LU shape from the autotuner (else NB 256, W 16)
-    bool panel_clusters = true;  // LU sub-panels that fit one thread-block cluster run on it (cluster
-                                 // barrier per column) instead of the cooperative grid
+    bool panel_clusters = true;  // LU sub-panels that fit one thread-block cluster run in its registers
+                                 // instead of on the cooperative grid
     int grad_method = 0;         // adjoint gradients: 0 contraction kernels (grad_geom.cu), 1 central
                                  // differences of reassembled operators
     int verify_cols = 64;        // refinement: columns whose error is measured with an FP64 residual
@@ -251,7 +251,7 @@ struct bem_geom {
     bem::DevSingular sing{};
     double* sing_coef = nullptr;  // (2N) sign*l/(2A) per half
     double* sing_free = nullptr;  // (3*2N) free vertex per half, x | y | z blocks
-    bem::DevTriAsm tri{};         // triangle-pair assembly data (Morton-ordered tiles)
+    bem::DevTriAsm tri{};         // triangle-pair assembly data (tiles of patches)
     void* dmem = nullptr;  // one allocation backing every device array (devmem_alloc)
     size_t dmem_bytes = 0;
 };

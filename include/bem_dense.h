@@ -109,10 +109,13 @@ int bem_ctx_set_symmetric(bem_ctx* ctx, int mode);
  * operator, right-hand-side and geometry buffers are cached the same way, and
  * bem_batch_run turns the cache on for its duration), "gemm_group_m" (16,
  * default: row tiles per raster group of the persistent tensor-core GEMM),
- * "assembly_kernel" (0, default: triangle-pair moments over Morton-ordered
- * tiles; 1: one thread per RWG pair, the reference's organisation),
+ * "assembly_kernel" (0, default: triangle-pair moments over tiles of RWGs that
+ * share triangles, while every phase k |r - r'| is below 2^20; 1, or beyond
+ * that: one thread per RWG pair, the reference's organisation),
  * "farfield_kernel" (0, default: phases shared by the RWG halves of a
- * triangle; 1: per RWG-half point), "batch_buckets" (1, default: bem_batch_run batches FP64 particles of one
+ * triangle, the Mueller matrices of real k at the particle's band limit and
+ * interpolated from there where that takes fewer directions; 1: per RWG-half
+ * point), "batch_buckets" (1, default: bem_batch_run batches FP64 particles of one
  * system size -- one assembly pass, one batched LU and one batched solve per
  * size; 0: one particle at a time), "lu_autotune" (1, default: the batched
  * LU's block and panel widths are chosen by timing the candidates once per
@@ -120,11 +123,11 @@ int bem_ctx_set_symmetric(bem_ctx* ctx, int mode);
  * factors are bitwise those of bem_lu_factor_dev), "gradient_method" (0,
  * default: the adjoint gradients contract the operator's derivative in
  * kernels; 1: central differences of reassembled operators, for checking),
- * "panel_clusters" (1, default: the sub-panels of the pivoted LU that fit the
- * shared memory of one cluster of at most 8 CTAs -- all of them up to order
- * ~6000 -- are factored by one thread-block cluster per matrix, one cluster
- * barrier per column; 0: every sub-panel on the cooperative grid, one grid
- * barrier per column; both give the same pivots and factors),
+ * "panel_clusters" (1, default: the sub-panels of the pivoted LU of at most
+ * 8192 rows are factored in the registers of one thread-block cluster per
+ * matrix, up to 16 CTAs, one exchange of candidates per column; 0: every
+ * sub-panel on the cooperative grid, one grid barrier per column; both give
+ * the same pivots and factors),
  * "fp64_gemm_3m" (1, default: the complex FP64 GEMMs of the pivoted LU, its
  * solves and the FP64 residual take three real products per complex product,
  * Re = Ar Br - Ai Bi, Im = (Ar + Ai)(Br + Bi) - Ar Br - Ai Bi, on the FP64
@@ -145,10 +148,11 @@ int bem_ctx_set_symmetric(bem_ctx* ctx, int mode);
  * the FP64 tensor path -- the same substitution regrouped, three quarters
  * of its flops in the GEMM; 0: one block triangular solve of 256 rows),
  * "solve_block_inverse" (1, default: the FP32 L D L^T factorisation also
- * keeps -L11^-1 of each 256-row diagonal block (n^2 / 256 complex64, 8 n^2 /
- * 256 bytes), and its solves apply the diagonal blocks as tensor-core
- * products with them; 0, or without memory for them: block triangular
- * solves; set before the factorisation),
+ * keeps -L11^-1 of each diagonal block of 256 "solve_superblock" rows (n x
+ * 256 solve_superblock complex64: 8 KB per row with the default 4), and its
+ * solves apply the diagonal blocks as tensor-core products with them; 0, or
+ * without memory for them: block triangular solves; set before the
+ * factorisation),
  * "ldlt_cluster_diag" (1, default: the FP32 L D L^T factors each 256 x 256
  * diagonal block on one cluster of 8 CTAs that holds the block in
  * distributed shared memory, 32 rows per CTA; 0, or where such a cluster
