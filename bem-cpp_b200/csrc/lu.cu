@@ -1701,9 +1701,9 @@ ldlt_diag_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int j0, int
 // 32q..32q+31, columns 0..32q+31, so no entry makes a round trip through
 // L2 between sub-panels.  Per 32-column sub-panel p:
 //   A. CTA p factors the 32 x 32 diagonal sub-block, column by column with
-//      a block barrier each: its 8 warps hold four rows each, a lane per
-//      column, so a column is one multiply-add per row and lane instead of 31 (277 us per block with one warp holding a row per lane,
-//      here and in B); the unscaled column entries go to U;
+//      a block barrier each: a lane per row, its 8 warps hold four columns
+//      each; the warp of a column leaves its unscaled entries in U, one store
+//      and one load a lane, and the scaling waits for the end;
 //   cluster barrier;
 //   B. every CTA q > p copies U and the pivots from CTA p and eliminates
 //      the sub-panel columns of its own rows (four rows per warp, a lane per
@@ -1711,17 +1711,23 @@ ldlt_diag_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int j0, int
 //   cluster barrier;
 //   C. every CTA q > p updates its rows' lower triangle right of the
 //      sub-panel: T = D L^T of block rows 32(p+1)..32q+31 is gathered from
-//      CTAs p+1..q, then each thread accumulates 4 rows x 7 column groups.
+//      CTAs p+1..q, 14 loads in flight per thread, then each thread
+//      accumulates 4 rows of one column group after the other: CTA p + 1, on
+//      which the next sub-panel waits, has one group.
 // Every entry goes through the same operations, in the same order, as in
 // ldlt_diag_kernel (the same pivot reciprocal, rank-1 updates in column
 // order, T = d_k l_c, the trailing sums in k order).  2 np + 1 cluster
 // barriers for np sub-panels, each at the top level of the kernel so that
 // every thread of the cluster reaches it; no spin loop.  *info: first zero
 // pivot (1-based).
+// Bound by the chain A, C of CTA p + 1, B: 107 us per block; 148 us with four
+// rows a warp and a lane per column in A (480 cycles a column, U stored and
+// scaled on the way), four gathers in flight and all column groups at once in
+// C; 277 us with one warp and a lane per row.
 constexpr int LDC_CTAS = 8, LDC_ROWS = 32, LDC_PITCH = 8 * LDC_ROWS + 1, LDC_UP = LDC_ROWS + 1,
               LDC_TP = 7 * LDC_ROWS + 1;
 constexpr size_t ldlt_cluster_smem_bytes() {
-    return ((size_t)LDC_ROWS * LDC_PITCH + 2 * (size_t)LDC_ROWS * LDC_UP + (size_t)LDC_ROWS * LDC_TP + 4 * LDC_ROWS) *
+    return ((size_t)LDC_ROWS * LDC_PITCH + 2 * (size_t)LDC_ROWS * LDC_UP + (size_t)LDC_ROWS * LDC_TP + 2 * LDC_ROWS) *
            sizeof(float2);
 }
 
@@ -1731,12 +1737,11 @@ ldlt_diag_cluster_kernel(float2* __restrict__ A, int64_t lda, int j0, int jb, in
     cg::cluster_group cluster = cg::this_cluster();
     extern __shared__ __align__(16) unsigned char ldc_smem[];
     float2* S = reinterpret_cast<float2*>(ldc_smem);  // [32][LDC_PITCH]: this CTA's block rows
-    float2* U = S + LDC_ROWS * LDC_PITCH;              // [32][LDC_UP]: unscaled sub-block entries (phase A)
-    float2* UL = U + LDC_ROWS * LDC_UP;                // [32][LDC_UP]: CTA p's U (phase B)
+    float2* U = S + LDC_ROWS * LDC_PITCH;              // [column][LDC_UP rows]: unscaled sub-block entries (phase A)
+    float2* UL = U + LDC_ROWS * LDC_UP;                // the same, CTA p's U (phase B)
     float2* T = UL + LDC_ROWS * LDC_UP;                // [32][LDC_TP]: d_k L[c][k] (phase C)
     float2* dk = T + LDC_ROWS * LDC_TP;                // [32]: the sub-panel's pivots
     float2* dinv = dk + LDC_ROWS;                      // [32]: their reciprocals (0 for a zero pivot)
-    float2* s_col = dinv + LDC_ROWS;                   // [2][32]: column entries of phase A, by parity
     const int q = (int)cluster.block_rank(), tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int r0 = q * LDC_ROWS;                       // this CTA's first block row
     const int nr = max(0, min(LDC_ROWS, jb - r0));     // its rows inside the block
@@ -1762,45 +1767,44 @@ ldlt_diag_cluster_kernel(float2* __restrict__ A, int64_t lda, int j0, int jb, in
     for (int p = 0; p < np; p++) {
         const int c0 = p * LDC_ROWS, w = min(LDC_ROWS, jb - c0);
         // A. the diagonal sub-block (rows c0.. of the block are this CTA's rows 0..w-1):
-        // warp: four rows, lane: column (the lower triangle counts); a column's
-        // unscaled entries are published by the lane that holds it
+        // lane: row, warp: four columns (the lower triangle counts); the warp that
+        // holds a column publishes its unscaled entries
         if (q == p) {
             float2 x[4];
 #pragma unroll
             for (int r = 0; r < 4; r++) {
-                const int i = wid * 4 + r;
-                x[r] = zero;
-                if (i < w && lane <= i) x[r] = S[i * LDC_PITCH + c0 + lane];
+                const int c = wid * 4 + r;
+                x[r] = (lane < w && c <= lane) ? S[lane * LDC_PITCH + c0 + c] : zero;
             }
-            for (int jj = 0; jj < w; jj++) {
-                float2* col = s_col + (jj & 1) * LDC_ROWS;
-                if (lane == jj) {
+            for (int j4 = 0; j4 < w; j4 += 4) {
 #pragma unroll
-                    for (int r = 0; r < 4; r++) col[wid * 4 + r] = x[r];
-                }
-                __syncthreads();
-                const float2 d = col[jj], u = col[lane];
-                const bool zp = (d.x == 0 && d.y == 0);
-                if (zp && tid == 0) atomicCAS(info, 0, j0 + c0 + jj + 1);
-                const float2 inv = zp ? zero : cdiv(one, d);
-#pragma unroll
-                for (int r = 0; r < 4; r++) {
-                    const int i = wid * 4 + r;
-                    const float2 a = col[i];
-                    const float2 l = panel_mul(a, inv);
-                    if (i > jj) {
-                        if (lane > jj) csub_mul(x[r], l, u);
-                        if (lane == jj) {
-                            U[i * LDC_UP + jj] = a;
-                            x[r] = l;
+                for (int r4 = 0; r4 < 4; r4++) {
+                    const int jj = j4 + r4;
+                    if (jj >= w) break;
+                    float2* col = U + jj * LDC_UP;
+                    if (wid * 4 == j4) col[lane] = x[r4];
+                    __syncthreads();
+                    if (wid * 4 + 3 > jj || wid == 0) {  // else this warp's columns are done
+                        const float2 d = col[jj];
+                        const bool zp = (d.x == 0 && d.y == 0);
+                        const float2 inv = zp ? zero : cdiv(one, d);
+                        if (tid == 0) {
+                            dinv[jj] = inv;
+                            if (zp) atomicCAS(info, 0, j0 + c0 + jj + 1);
                         }
+                        // rows above the column take part in what lies above the diagonal, which nothing reads
+                        const float2 l = panel_mul(col[lane], inv);
+#pragma unroll
+                        for (int r = 0; r < 4; r++)
+                            if (wid * 4 + r > jj) csub_mul(x[r], l, col[wid * 4 + r]);
                     }
                 }
             }
+            __syncthreads();
 #pragma unroll
             for (int r = 0; r < 4; r++) {
-                const int i = wid * 4 + r;
-                if (i < w && lane <= i) S[i * LDC_PITCH + c0 + lane] = x[r];
+                const int c = wid * 4 + r;
+                if (lane < w && c <= lane) S[lane * LDC_PITCH + c0 + c] = c < lane ? panel_mul(x[r], dinv[c]) : x[r];
             }
         }
         cluster.sync();
@@ -1808,10 +1812,10 @@ ldlt_diag_cluster_kernel(float2* __restrict__ A, int64_t lda, int j0, int jb, in
         if (q > p && nr > 0) {
             const float2* Up = cluster.map_shared_rank(U, p);
             const float2* Sp = cluster.map_shared_rank(S, p);
-            for (int e = tid; e < w * w; e += LDLT_THREADS) {
-                const int r = e / w, c = e % w;
-                if (c < r) UL[r * LDC_UP + c] = Up[r * LDC_UP + c];
-            }
+            // rows below: the sub-panel is whole, w = 32
+#pragma unroll
+            for (int e = tid; e < LDC_ROWS * LDC_ROWS; e += LDLT_THREADS)
+                UL[(e >> 5) * LDC_UP + (e & 31)] = Up[(e >> 5) * LDC_UP + (e & 31)];
             if (tid < w) {
                 const float2 d = Sp[tid * LDC_PITCH + c0 + tid];
                 dk[tid] = d;
@@ -1827,73 +1831,61 @@ ldlt_diag_cluster_kernel(float2* __restrict__ A, int64_t lda, int j0, int jb, in
             }
 #pragma unroll 4
             for (int jj = 0; jj < w; jj++) {
-                const float2 inv = dinv[jj], u = UL[lane * LDC_UP + jj];
+                const float2 inv = dinv[jj], u = UL[jj * LDC_UP + lane];
 #pragma unroll
                 for (int r = 0; r < 4; r++) {
-                    const float2 a = shfl_c(x[r], jj);
-                    const float2 l = panel_mul(a, inv);
+                    const float2 l = panel_mul(shfl_c(x[r], jj), inv);
                     if (lane > jj) csub_mul(x[r], l, u);
-                    if (lane == jj) x[r] = l;
                 }
             }
 #pragma unroll
             for (int r = 0; r < 4; r++) {
                 const int i = wid * 4 + r;
-                if (i < nr && lane < w) S[i * LDC_PITCH + c0 + lane] = x[r];
+                if (i < nr && lane < w) S[i * LDC_PITCH + c0 + lane] = panel_mul(x[r], dinv[lane]);
             }
         }
         cluster.sync();
         // C. this CTA's rows, columns cs..r0+31 of the lower triangle
         if (q > p && nr > 0) {
             const int cs = c0 + w, nc = r0 + LDC_ROWS - cs, ng = nc / 32;  // ng = q - p <= 7
-            // four independent remote loads in flight per thread
-            for (int e0 = 0; e0 < w * nc; e0 += 4 * LDLT_THREADS) {
-                float2 lc[4];
+            // 14 independent remote loads in flight per thread (w = 32 here)
+            for (int e0 = 0; e0 < LDC_ROWS * nc; e0 += 14 * LDLT_THREADS) {
+                float2 lc[14];
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int e = e0 + u * LDLT_THREADS + tid, c = e / w, k = e % w, row = cs + c;
+                for (int u = 0; u < 14; u++) {
+                    const int e = e0 + u * LDLT_THREADS + tid, row = cs + (e >> 5);
                     lc[u] = zero;
-                    if (e < w * nc && row < jb)
-                        lc[u] = cluster.map_shared_rank(S, row / LDC_ROWS)[(row % LDC_ROWS) * LDC_PITCH + c0 + k];
+                    if (e < LDC_ROWS * nc && row < jb)
+                        lc[u] = cluster.map_shared_rank(S, row / LDC_ROWS)[(row % LDC_ROWS) * LDC_PITCH + c0 + (e & 31)];
                 }
 #pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int e = e0 + u * LDLT_THREADS + tid, c = e / w, k = e % w;
-                    if (e < w * nc) {
-                        const float2 d = dk[k];
-                        T[k * LDC_TP + c] = panel_mul(d, lc[u]);
-                    }
+                for (int u = 0; u < 14; u++) {
+                    const int e = e0 + u * LDLT_THREADS + tid;
+                    if (e < LDC_ROWS * nc) T[(e & 31) * LDC_TP + (e >> 5)] = panel_mul(dk[e & 31], lc[u]);
                 }
             }
             __syncthreads();
-            float2 acc[4][7];
-            bool ok[4][7];
+            // a column group at a time: the next sub-panel waits for the CTA with one group
+            for (int g = 0; g < ng; g++) {
+                const int col = cs + lane + 32 * g;
+                float2 acc[4];
 #pragma unroll
-            for (int r = 0; r < 4; r++)
-#pragma unroll
-                for (int g = 0; g < 7; g++) {
-                    const int i = wid * 4 + r, col = cs + lane + 32 * g;
-                    ok[r][g] = g < ng && i < nr && col <= r0 + i;
-                    acc[r][g] = ok[r][g] ? S[i * LDC_PITCH + col] : zero;
+                for (int r = 0; r < 4; r++) {
+                    const int i = wid * 4 + r;
+                    acc[r] = (i < nr && col <= r0 + i) ? S[i * LDC_PITCH + col] : zero;
                 }
-#pragma unroll 2
-            for (int k = 0; k < w; k++) {
-                float2 a[4];
+#pragma unroll 8
+                for (int k = 0; k < LDC_ROWS; k++) {
+                    const float2 b = T[k * LDC_TP + lane + 32 * g];
 #pragma unroll
-                for (int r = 0; r < 4; r++) a[r] = S[(wid * 4 + r) * LDC_PITCH + c0 + k];
+                    for (int r = 0; r < 4; r++) csub_mul(acc[r], S[(wid * 4 + r) * LDC_PITCH + c0 + k], b);
+                }
 #pragma unroll
-                for (int g = 0; g < 7; g++)
-                    if (g < ng) {  // the column groups this CTA has at this sub-panel
-                        const float2 b = T[k * LDC_TP + lane + 32 * g];
-#pragma unroll
-                        for (int r = 0; r < 4; r++) csub_mul(acc[r][g], a[r], b);
-                    }
+                for (int r = 0; r < 4; r++) {
+                    const int i = wid * 4 + r;
+                    if (i < nr && col <= r0 + i) S[i * LDC_PITCH + col] = acc[r];
+                }
             }
-#pragma unroll
-            for (int r = 0; r < 4; r++)
-#pragma unroll
-                for (int g = 0; g < 7; g++)
-                    if (ok[r][g]) S[(wid * 4 + r) * LDC_PITCH + cs + lane + 32 * g] = acc[r][g];
             __syncthreads();
         }
     }
