@@ -210,6 +210,7 @@ struct bem_ctx {
     bool lu_autotune = true;     // batched LU shape from the autotuner (else NB 256, W 16)
     bool panel_clusters = true;  // LU sub-panels that fit one thread-block cluster run in its registers
                                  // instead of on the cooperative grid
+    int64_t panel_wait = 2000000000;  // clock cycles after which a wait of those clusters gives up
     int grad_method = 0;         // adjoint gradients: 0 contraction kernels (grad_geom.cu), 1 central
                                  // differences of reassembled operators
     int verify_cols = 64;        // refinement: columns whose error is measured with an FP64 residual

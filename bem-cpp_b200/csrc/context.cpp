@@ -285,6 +285,9 @@ int bem_ctx_set_option(bem_ctx* ctx, const char* name, int value) {
         ctx->oz_pace_lead = value;
     } else if (!std::strcmp(name, "panel_clusters")) {
         ctx->panel_clusters = value != 0;
+    } else if (!std::strcmp(name, "panel_wait_mcycles")) {
+        if (value < 0 || value > 4000) return bem::fail(ctx, BEM_ERR_INVALID, "panel_wait_mcycles must be 0..4000");
+        ctx->panel_wait = (int64_t)value * 1000000;
     } else if (!std::strcmp(name, "gmres_digits")) {
         if (value != 0 && (value < 2 || value > bem::oz::S_MAX))
             return bem::fail(ctx, BEM_ERR_INVALID, "gmres_digits must be 0 or 2..%d", bem::oz::S_MAX);

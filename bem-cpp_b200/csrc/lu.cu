@@ -401,6 +401,12 @@ panel_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int r0, int nro
 // follows the peer's reads of column jj.
 // Same pivot rule and per-element arithmetic (panel_mul, panel_msub) as
 // panel_kernel, so the same pivots and factors.
+// A wait that runs out (wait_cycles: ~1 s of a peer that does not send) ends
+// the columns: the warp takes nothing from the messages it lacks, so every
+// position stays one of the panel, and its CTA leaves at the next block barrier
+// (s_stop, by column parity: a column writes the next one's word) before it
+// sends again, stores no row and records BEM_ERR_TIMEOUT.  The kernels queued
+// behind it read that word before they follow `moves`.
 // moves (2 n integers per matrix): for the w top positions k of the panel,
 // moves[r0 + k] is the row now at position k and moves[n + r0 + k] the
 // position of the row formerly there: the interchanges as one gather.
@@ -450,8 +456,9 @@ __device__ __forceinline__ uint32_t map_rank(uint32_t smem, int rank) {
     asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem), "r"(rank));
     return r;
 }
-// Waits until the phase of this parity is complete, ~1 s of clock cycles at most.
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity) {
+// Waits until the phase of this parity is complete, `limit` clock cycles at most (0: gives up at once).
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, long long limit) {
+    if (limit <= 0) return false;
     long long t0 = 0;
     for (int i = 0;; i++) {
         uint32_t ok;
@@ -464,7 +471,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity)
             : "memory");
         if (ok) return true;
         if (i == 0) t0 = clock64();
-        if (clock64() - t0 > 2000000000ll) return false;
+        if (clock64() - t0 > limit) return false;
     }
 }
 
@@ -472,7 +479,7 @@ template <typename R>
 __global__ void __launch_bounds__(PR_THREADS, 1)
 panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int r0, int nrows, int w,
                  int* __restrict__ ipiv, int* __restrict__ info, int* __restrict__ moves, int64_t sA,
-                 int* __restrict__ status) {
+                 int* __restrict__ status, long long wait_cycles) {
     using C2 = typename C2T<R>::type;
     namespace cg = cooperative_groups;
     constexpr int W = PanelW<R>::v;
@@ -482,7 +489,7 @@ panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int 
     __shared__ __align__(16) C2 s_inv[2][PR_WARPS], r_inv[2][PR_CLUSTER];
     __shared__ __align__(16) uint4 s_cand[2][PR_WARPS], r_cand[2][PR_CLUSTER];
     __shared__ __align__(8) unsigned long long r_bar[2];
-    __shared__ int s_at[PR_THREADS];
+    __shared__ int s_at[PR_THREADS], s_stop[2];
     // the rows on their way in and out, 256 B each: 16 lanes a row in global
     // memory, a thread a row here (an odd number of 16-byte units apart)
     extern __shared__ __align__(16) unsigned char pr_smem[];
@@ -498,7 +505,7 @@ panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int 
         for (int k = 0; k < 2; k++) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0 + 8 * k) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    bool late = false;  // a wait ran out
+    if (tid < 2) s_stop[tid] = 0;
     const int gr = b * T + tid;
     const bool valid = gr < nrows;
     bool act = valid;
@@ -548,7 +555,8 @@ panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int 
     };
     const uint4 none = make_uint4(0u, 0u, 0x7fffffffu, 0u);
     search(x[0]);
-    for (int g0 = 0; g0 < W; g0 += PG) {
+    bool stop = false;
+    for (int g0 = 0; g0 < W && !stop; g0 += PG) {
       const int rem = W - g0;
 #pragma unroll
       for (int q = 0; q < PG; q++) {
@@ -570,6 +578,11 @@ panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int 
         }
         __syncthreads();
         uint4 rec = lane < nw ? s_cand[par][lane] : none;
+        if (C > 1 && s_stop[par]) {  // a warp's wait of the column before ran out
+            stop = true;
+            break;
+        }
+        bool late = false;
         const C2* u;
         C2 inv;
         if (C > 1) {
@@ -595,8 +608,9 @@ panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int 
                     }
                 }
             }
-            if (!late) late = !mbar_wait_cluster(bar, (uint32_t)(jj >> 1) & 1u);
-            rec = lane < C ? r_cand[par][lane] : none;
+            late = __any_sync(0xffffffffu, !mbar_wait_cluster(bar, (uint32_t)(jj >> 1) & 1u, wait_cycles));
+            if (late && lane == 0) s_stop[par ^ 1] = 1;
+            rec = lane < C && !late ? r_cand[par][lane] : none;
         }
         const int bk = cand_lane(rec, __reduce_max_sync(0xffffffffu, rec.x)), bw = max(bk, 0);
         int piv;
@@ -614,7 +628,7 @@ panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int 
         if (zp) piv = jj;
         if (b == 0 && tid == 0) {
             ipiv[r0 + jj] = r0 + piv;
-            if (zp) atomicCAS(info, 0, r0 + jj + 1);
+            if (zp && !late) atomicCAS(info, 0, r0 + jj + 1);
         }
         if (pos == piv) {
             pos = jj;
@@ -648,10 +662,18 @@ panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int 
 #pragma unroll
       for (int c = 0; c < PG; c++) x[W - PG + c] = done[c];
     }
-    if (late) *status = BEM_ERR_TIMEOUT;
+    __syncthreads();  // a late warp of the last column
+    const bool lost = C > 1 && (s_stop[0] | s_stop[1]) != 0;
+    if (lost && tid == 0) *status = BEM_ERR_TIMEOUT;
     __syncwarp();
     // no CTA ends while a peer may still write to it (the wait is at the end)
     if (C > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    if (lost) {
+        // messages sent before the peers arrived may still be on their way: ~0.1 ms, a hundred times what one takes
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        for (const long long t0 = clock64(); clock64() - t0 < 200000;) __nanosleep(1000);
+        return;
+    }
     // rows to their positions (every row of the panel was read before the first barrier)
     if (valid) {
 #pragma unroll
@@ -753,7 +775,7 @@ static int launch_panel_reg(bem_ctx* ctx, typename C2T<R>::type* A, int64_t lda,
     cfg.numAttrs = 1;
     cudaEvent_t ev = ctx->prof_begin(PROF_PANEL);
     BEM_TRY_CUDA(ctx, cudaLaunchKernelEx(&cfg, panel_reg_kernel<R>, A, lda, n, i0, nrows, iw, d_ipiv, d_info, d_moves, sA,
-                                         ctx->d_status));
+                                         ctx->d_status, ctx->panel_wait));
     BEM_LAUNCHED(ctx);
     if (ev)
         ctx->prof_end(PROF_PANEL, ev, 8.0 * (double)nrows * iw * iw / 2 * batch,
@@ -762,10 +784,12 @@ static int launch_panel_reg(bem_ctx* ctx, typename C2T<R>::type* A, int64_t lda,
 }
 
 // moves of a sub-panel (see panel_reg_kernel) from its interchanges, for the
-// panels of panel_kernel.  One thread per matrix: w <= 32 steps.
-__global__ void moves_kernel(const int* __restrict__ ipiv, int n, int r0, int w, int* __restrict__ moves, int batch) {
+// panels of panel_kernel.  One thread per matrix: w <= 32 steps.  A panel whose
+// barrier gave up (status) has left no pivots to follow.
+__global__ void moves_kernel(const int* __restrict__ ipiv, int n, int r0, int w, int* __restrict__ moves, int batch,
+                             const int* __restrict__ status) {
     const int mi = blockIdx.x * blockDim.x + threadIdx.x;
-    if (mi >= batch) return;
+    if (mi >= batch || *status != 0) return;
     ipiv += (int64_t)mi * n;
     moves += (int64_t)mi * 2 * n;
     // a position below the top is only ever exchanged with a top row, and only top rows go there
@@ -803,10 +827,12 @@ __global__ void moves_kernel(const int* __restrict__ ipiv, int n, int r0, int w,
 // block column before.  SOLVE (one sub-panel): the columns of the second
 // range are then solved with the panel's unit lower triangle (U12 of the
 // sub-panel), saving that kernel's launch and its pass over the rows.
+// A non-zero status word (a panel's wait ran out) leaves the rows where they
+// are: `moves` is then not all written.
 template <typename R, bool SOLVE>
 __global__ void __launch_bounds__(64)
 move_rows_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, const int* __restrict__ moves, int n, int k0,
-                 int k1, int w, int c0a, int c1a, int c0b, int c1b, int64_t sA = 0) {
+                 int k1, int w, int c0a, int c1a, int c0b, int c1b, const int* __restrict__ status, int64_t sA = 0) {
     using C2 = typename C2T<R>::type;
     constexpr int W = PanelW<R>::v;
     A += blockIdx.y * sA;  // batched: blockIdx.y selects the matrix
@@ -816,6 +842,7 @@ move_rows_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, const int* 
     const int t = blockIdx.x * blockDim.x + threadIdx.x, na = c1a - c0a;
     const bool in = t < na + (c1b - c0b), second = t >= na;
     const int c = second ? c0b + (t - na) : c0a + t;
+    const int gave_up = *status;  // used after the first loads of `moves`
     for (int r0 = k0; r0 < k1; r0 += w) {
         const int iw = min(w, k1 - r0);
         __syncthreads();
@@ -827,6 +854,7 @@ move_rows_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, const int* 
             for (int e = threadIdx.x; e < iw * iw; e += blockDim.x)
                 sT[e / iw][e % iw] = A[(int64_t)(r0 + e / iw) * lda + r0 + e % iw];
         __syncthreads();
+        if (gave_up != 0) return;
         if (!in) continue;
         C2 x[W], y[W];
 #pragma unroll
@@ -1174,7 +1202,7 @@ int getrf(bem_ctx* ctx, typename C2T<R>::type* A, int64_t lda, int n, int* d_ipi
                 if (ev)
                     ctx->prof_end(PROF_PANEL, ev, 8.0 * (double)nrows * iw * iw / 2,
                                   (double)nrows * iw * 2 * sizeof(C2));
-                moves_kernel<<<1, 32, 0, ctx->stream>>>(d_ipiv, n, i0, iw, d_moves, 1);
+                moves_kernel<<<1, 32, 0, ctx->stream>>>(d_ipiv, n, i0, iw, d_moves, 1, ctx->d_status);
                 BEM_LAUNCHED(ctx);
             }
             // interchanges on the rest of this block column, and the sub-panel's U12
@@ -1183,7 +1211,7 @@ int getrf(bem_ctx* ctx, typename C2T<R>::type* A, int64_t lda, int n, int* d_ipi
             if (ncol > 0) {
                 cudaEvent_t ev = ctx->prof_begin(PROF_PIVOT);
                 move_rows_kernel<R, true><<<(ncol + 63) / 64, 64, 0, ctx->stream>>>(A, lda, d_moves, n, i0, i0 + iw, iw,
-                                                                                  ca0, ca1, cb0, cb1);
+                                                                                  ca0, ca1, cb0, cb1, ctx->d_status);
                 BEM_LAUNCHED(ctx);
                 if (ev) ctx->prof_end(PROF_PIVOT, ev, 0.0, 4.0 * sizeof(C2) * iw * (double)ncol);
             }
@@ -1199,7 +1227,7 @@ int getrf(bem_ctx* ctx, typename C2T<R>::type* A, int64_t lda, int n, int* d_ipi
         if (ncol > 0) {
             cudaEvent_t ev = ctx->prof_begin(PROF_PIVOT);
             move_rows_kernel<R, false><<<(ncol + 63) / 64, 64, 0, ctx->stream>>>(A, lda, d_moves, n, j0, j0 + jb, W, 0, j0,
-                                                                               j0 + jb, n);
+                                                                               j0 + jb, n, ctx->d_status);
             BEM_LAUNCHED(ctx);
             if (ev) ctx->prof_end(PROF_PIVOT, ev, 0.0, 4.0 * sizeof(C2) * jb * (double)ncol);
         }
@@ -1359,7 +1387,7 @@ int getrf_batched(bem_ctx* ctx, double2* A, int64_t lda, int64_t sA, int n, int 
                 if (ev)
                     ctx->prof_end(PROF_PANEL, ev, 8.0 * (double)nrows * iw * iw / 2 * batch,
                                   (double)nrows * iw * 2 * sizeof(C2) * batch);
-                moves_kernel<<<(batch + 31) / 32, 32, 0, ctx->stream>>>(d_ipiv, n, i0, iw, d_moves, batch);
+                moves_kernel<<<(batch + 31) / 32, 32, 0, ctx->stream>>>(d_ipiv, n, i0, iw, d_moves, batch, ctx->d_status);
                 BEM_LAUNCHED(ctx);
             }
             const int ca0 = j0, ca1 = i0, cb0 = i0 + iw, cb1 = j0 + jb;
@@ -1367,7 +1395,7 @@ int getrf_batched(bem_ctx* ctx, double2* A, int64_t lda, int64_t sA, int n, int 
             if (ncol > 0) {
                 cudaEvent_t ev = ctx->prof_begin(PROF_PIVOT);
                 move_rows_kernel<R, true><<<dim3((ncol + 63) / 64, batch), 64, 0, ctx->stream>>>(
-                    A, lda, d_moves, n, i0, i0 + iw, iw, ca0, ca1, cb0, cb1, sA);
+                    A, lda, d_moves, n, i0, i0 + iw, iw, ca0, ca1, cb0, cb1, ctx->d_status, sA);
                 BEM_LAUNCHED(ctx);
                 if (ev) ctx->prof_end(PROF_PIVOT, ev, 0.0, 4.0 * sizeof(C2) * iw * (double)ncol * batch);
             }
@@ -1381,7 +1409,7 @@ int getrf_batched(bem_ctx* ctx, double2* A, int64_t lda, int64_t sA, int n, int 
         if (ncol > 0) {
             cudaEvent_t ev = ctx->prof_begin(PROF_PIVOT);
             move_rows_kernel<R, false><<<dim3((ncol + 63) / 64, batch), 64, 0, ctx->stream>>>(A, lda, d_moves, n, j0, j0 + jb,
-                                                                                            W, 0, j0, j0 + jb, n, sA);
+                                                                                            W, 0, j0, j0 + jb, n, ctx->d_status, sA);
             BEM_LAUNCHED(ctx);
             if (ev) ctx->prof_end(PROF_PIVOT, ev, 0.0, 4.0 * sizeof(C2) * jb * (double)ncol * batch);
         }

@@ -128,6 +128,9 @@ int bem_ctx_set_symmetric(bem_ctx* ctx, int mode);
  * matrix, up to 16 CTAs, one exchange of candidates per column; 0: every
  * sub-panel on the cooperative grid, one grid barrier per column; both give
  * the same pivots and factors),
+ * "panel_wait_mcycles" (2000, default: millions of SM clock cycles, about one
+ * second, after which a CTA of those clusters stops waiting for its peers'
+ * candidates and the factorisation returns BEM_ERR_TIMEOUT; 0: at once),
  * "fp64_gemm_3m" (1, default: the complex FP64 GEMMs of the pivoted LU, its
  * solves and the FP64 residual take three real products per complex product,
  * Re = Ar Br - Ai Bi, Im = (Ar + Ai)(Br + Bi) - Ar Br - Ai Bi, on the FP64
