@@ -647,7 +647,8 @@ farfield_nodes_kernel(FFArgs a, DevTriAsm ta, int nt, const double* __restrict__
 // W[j][d] of the trigonometric interpolation from the 2 H nodes t_j = pi j / H
 // to t_d = pi d / (ndir - 1): sin(H x) cot(x / 2) / (2 H) with x = t_d - t_j =
 // pi m / (H (ndir - 1)), m an integer, so both arguments reduce exactly
-// (2 H (ndir - 1) < 2^31: H is at most ndir and its sums fit shared memory).
+// (2 H ndir <= FF_MAX_WEIGHTS, so the integers fit 32 bits).
+constexpr int FF_MAX_WEIGHTS = 1 << 27;
 __global__ void ff_weights_kernel(int H, int ndir, double* __restrict__ W) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= 2 * H * ndir) return;
@@ -719,8 +720,9 @@ static int ff_node_pairs(double x, int limit) {
 
 // Plan of the band-limited far field of a call, H = 0 where the direct kernel
 // takes it: a complex k (no conjugate nodes), directions of the caller,
-// arguments beyond the sine's range, or so few directions that H node pairs
-// and the interpolation cost more (operations per direction: Nq 33 + 96 per
+// arguments beyond the sine's range, so many directions that their weights
+// would take more than 1 GB (and the indices 32 bits), or so few that H node
+// pairs and the interpolation cost more (operations per direction: Nq 33 + 96 per
 // triangle either way; per node pair and direction 48 of interpolation).
 // RT (host) need not be orthonormal: |rhat(t).r| <= smax |r| with smax the
 // largest singular value of (R^T x, R^T z).
@@ -744,6 +746,7 @@ static FFPlan plan_ff(const bem_ctx* ctx, const bem_geom* g, const double* RT, i
     if (!(x < SINCOS_MAX)) return p;
     const int H = ff_node_pairs(x, ndir);
     const double per_dir = (g->Nq * 33.0 + 96.0) * g->nt;
+    if ((int64_t)2 * H * ndir > FF_MAX_WEIGHTS) return p;
     // the interpolation's shared memory bounds H as well
     if (H < 1 || H * (per_dir + 48.0 * ndir) > per_dir * ndir || (size_t)2 * H * 24 * 8 > 200 * 1024) return p;
     p.H = H;
