@@ -300,6 +300,7 @@ void pivots_to_perm(const std::vector<int>& ipiv, std::vector<int>& perm);
 // null) receives dloss/dv; dpsi_dk (host, 4 doubles) the complex
 // contractions sum S . d(Z D)/dRe k_int and sum S . d(Z D)/dIm k_int,
 // dpsi_deta (2 doubles) sum S . d(Z D)/deta_int.
+constexpr int ADJ_MAX_ANGLES = 1706;  // scattering angles of a gradient: 80 B of shared memory each
 int adjoint_geometry(bem_ctx* ctx, const bem_geom* g, std::complex<double> kext, std::complex<double> kint,
                      double eta_e, double eta_i, unsigned flags, const void* X, const void* Lam, int ncols,
                      const double* RT_dev, int n_orient, const void* ab_dev, int ntheta,

@@ -926,7 +926,8 @@ int adjoint_geometry(bem_ctx* ctx, const bem_geom* g, std::complex<double> kext,
     FFArgs2 fa{g->sing.tv, d_hinfo, nt, N, Nq, tq, kext.real(), kext.imag(), eta_e, RT_dev, n_orient, ntheta,
                (const double2*)ab_dev, (const double2*)X, n, d_part};
     const size_t smem = std::max((size_t)ntheta * 5 * 16, (size_t)GFF_THREADS * 13 * 8);
-    BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(grad_ff_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(grad_ff_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           ADJ_MAX_ANGLES * 5 * 16));  // the largest size: the limit is the device's
     grad_ff_kernel<<<dim3(nblocks(nt, GFF_THREADS / Nq), ff_parts), GFF_THREADS, smem, st>>>(fa);
     BEM_LAUNCHED(ctx);
     part_sum_kernel<<<nblocks(9 * (int64_t)nt, 256), 256, 0, st>>>(d_part, ff_parts, 9 * nt, o_ff);

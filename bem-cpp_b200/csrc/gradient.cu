@@ -332,13 +332,12 @@ static int adjoint_core(bem_ctx* ctx, const bem_problem* p, const double* target
     aa.ab = (const double2*)dAB.p;
     aa.G = (double2*)dY.p;  // g
     aa.ldg = n;
-    // ntheta x (1 + 4) complex, reused by the 25 values of a thread.  The
-    // limit on ntheta is that of the reassembly path's buffers of old (120 B an angle).
-    if ((size_t)((3 * nt + 1) & ~1) * 8 + (size_t)nt * 6 * 16 > 200 * 1024)
-        return fail(ctx, BEM_ERR_INVALID, "ntheta %d too large for the adjoint far field", nt);
+    // ntheta x (1 + 4) complex, reused by the 25 values of a thread
+    if (nt > ADJ_MAX_ANGLES) return fail(ctx, BEM_ERR_INVALID, "ntheta %d too large for the adjoint far field", nt);
     const size_t smem = std::max((size_t)nt * 5 * 16, (size_t)AFF_THREADS * 25 * 8);
+    // the limit is the device's, shared with other host threads' contexts: always the largest size
     BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(farfield_adjoint_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem));
+                                           ADJ_MAX_ANGLES * 5 * 16));
     BEM_TRY_CUDA(ctx, cudaMemsetAsync(dY.p, 0, xb, ctx->stream));
     const int per = AFF_THREADS / g->Nq;
     farfield_adjoint_kernel<<<dim3((g->nt + per - 1) / per, no), AFF_THREADS, smem, ctx->stream>>>(aa);

@@ -243,6 +243,10 @@ __device__ __forceinline__ void panel_eliminate(typename C2T<R>::type* tile, int
     }
 }
 
+// Dynamic shared memory that panel_kernel may take, always set as its limit:
+// the limit is the device's, and other host threads' contexts launch it too.
+constexpr int PANEL_SMEM = 220 * 1024;
+
 // Factors the sub-panel rows [r0, n), columns [r0, r0+w) of the row-major
 // matrix A.  CTA b owns panel rows [b*Rp, min((b+1)*Rp, nrows)) (relative
 // to r0) in shared memory; Rp >= w so the w pivot rows live in CTA 0.
@@ -1147,10 +1151,9 @@ int getrf(bem_ctx* ctx, typename C2T<R>::type* A, int64_t lda, int n, int* d_ipi
     int G0 = std::min(Gmax_sm, std::max(1, n / W));
     int Rp0 = std::max((n + G0 - 1) / G0, 2 * W);
     size_t smem0 = ((size_t)Rp0 * W + W) * sizeof(C2);
-    if (smem0 > 220 * 1024)
+    if (smem0 > PANEL_SMEM)
         return fail(ctx, BEM_ERR_INVALID, "n=%d too large for the panel kernel (%zu B smem)", n, smem0);
-    BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(panel_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)smem0));
+    BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(panel_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, PANEL_SMEM));
     BEM_TRY_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, panel_kernel<R>, 256, smem0));
     if (occ < 1) return fail(ctx, BEM_ERR_INVALID, "panel kernel does not fit on an SM");
     const int Gcap = occ * ctx->sm_count;
@@ -1308,7 +1311,7 @@ int getrf_batched(bem_ctx* ctx, double2* A, int64_t lda, int64_t sA, int n, int 
     if (n < 1 || batch < 1) return fail(ctx, BEM_ERR_INVALID, "batched LU: n=%d batch=%d", n, batch);
     if (W < 1 || W > PanelW<R>::v || NB < W || NB > TRSM_KB || NB % W != 0)
         return fail(ctx, BEM_ERR_INVALID, "batched LU shape NB=%d W=%d", NB, W);
-    const size_t smem_max = 220 * 1024;
+    const size_t smem_max = PANEL_SMEM;
     // every sub-panel fits one cluster (the first is the tallest): no
     // cooperative grid, no chunking of the batch
     const bool all_clusters = panel_reg_choice<R>(ctx, n, W, batch).C > 0;

@@ -21,6 +21,11 @@ namespace bem {
 
 #define INV4PI_FF 0.079577471545947667884
 
+// The dynamic shared-memory limit of a kernel belongs to the device, not to a
+// context, and contexts of other host threads launch the same kernels: every
+// launch here sets the largest size that the kernel can need, never its own.
+constexpr int FF_MAXQ = 13;
+
 struct RhsArgs {
     DevTriAsm ta;
     const double* coef;  // 2N: sign l / (2A) of a half
@@ -192,9 +197,13 @@ int rhs_dev(bem_ctx* ctx, const bem_geom* g, double k_re, double k_im, double et
     // about four waves of blocks (two a SM), each taking several groups of orientations
     const int groups = (a.n_orient + RHS_ORI - 1) / RHS_ORI;
     const int gy = std::max(1, std::min(groups, (int)((8LL * ctx->sm_count + g->tri.ntile - 1) / g->tri.ntile)));
-    const size_t smem = ((size_t)ASM_TRI_MAX * (g->Nq * 4 + 3) + RHS_ORI * RHS_FLD + (size_t)ASM_TRI_MAX * RHS_TRI) * 8;
+    auto smem_bytes = [](int nq) {
+        return ((size_t)ASM_TRI_MAX * (nq * 4 + 3) + RHS_ORI * RHS_FLD + (size_t)ASM_TRI_MAX * RHS_TRI) * 8;
+    };
+    const size_t smem = smem_bytes(g->Nq);
     auto kern = general ? rhs_kernel<true, 0> : g->Nq == 7 ? rhs_kernel<false, 7> : g->Nq == 4 ? rhs_kernel<false, 4> : rhs_kernel<false, 0>;
-    BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    if (g->Nq > FF_MAXQ) return fail(ctx, BEM_ERR_INVALID, "quadrature of %d points (at most %d)", g->Nq, FF_MAXQ);
+    BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes(FF_MAXQ)));
     kern<<<dim3(g->tri.ntile, gy), RHS_THREADS, smem, ctx->stream>>>(a);
     BEM_LAUNCHED(ctx);
     // the workspace is reused by later calls: finish before returning
@@ -417,7 +426,6 @@ __global__ void __launch_bounds__(256) farfield_kernel(FFArgs a, int dpb) {
 // independent, formed once per block and staged chunk).  One sincos per
 // triangle point instead of per RWG-half point, ~4x fewer operations.
 constexpr int FT_CHUNK = 64;  // triangles staged per step
-constexpr int FF_MAXQ = 13;
 
 __global__ void __launch_bounds__(256) farfield_tri_kernel(FFArgs a, DevTriAsm ta, int nt, const double* coef,
                                                            int dpb) {
@@ -675,6 +683,7 @@ __global__ void ff_weights_kernel(int H, int ndir, double* __restrict__ W) {
 
 // Thread: one direction of the orientation blockIdx.x; the node sums (all
 // parts, in order) in shared memory.
+constexpr int FF_INTERP_SMEM = 200 * 1024;
 __global__ void __launch_bounds__(192) farfield_interp_kernel(FFArgs a, const double* __restrict__ nodes, int parts,
                                                               int H, const double* __restrict__ W) {
     extern __shared__ __align__(16) double sm[];  // 2 H x 24
@@ -748,7 +757,7 @@ static FFPlan plan_ff(const bem_ctx* ctx, const bem_geom* g, const double* RT, i
     const double per_dir = (g->Nq * 33.0 + 96.0) * g->nt;
     if ((int64_t)2 * H * ndir > FF_MAX_WEIGHTS) return p;
     // the interpolation's shared memory bounds H as well
-    if (H < 1 || H * (per_dir + 48.0 * ndir) > per_dir * ndir || (size_t)2 * H * 24 * 8 > 200 * 1024) return p;
+    if (H < 1 || H * (per_dir + 48.0 * ndir) > per_dir * ndir || (size_t)2 * H * 24 * 8 > FF_INTERP_SMEM) return p;
     p.H = H;
     const int chunks = (H + FN_PAIRS - 1) / FN_PAIRS, tchunks = (g->nt + FN_CHUNK - 1) / FN_CHUNK;
     // three blocks of 128 threads fit an SM: enough parts for about four waves
@@ -766,13 +775,14 @@ static int launch_ff_nodes(bem_ctx* ctx, const bem_geom* g, const FFArgs& a, con
     BEM_LAUNCHED(ctx);
     auto kern = g->Nq == 7 ? farfield_nodes_kernel<7> : g->Nq == 4 ? farfield_nodes_kernel<4> : farfield_nodes_kernel<0>;
     const size_t smem = (size_t)FN_CHUNK * (g->Nq * 3 + FN_REC) * 16;
-    BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           FN_CHUNK * (FF_MAXQ * 3 + FN_REC) * 16));
     kern<<<dim3((p.H + FN_PAIRS - 1) / FN_PAIRS, a.n_orient, p.parts), FN_PAIRS * FN_LANES, smem, ctx->stream>>>(
         a, g->tri, g->nt, g->sing_coef, p.H, nodes);
     BEM_LAUNCHED(ctx);
     const size_t ismem = (size_t)2 * p.H * 24 * 8;
     BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(farfield_interp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           (int)ismem));
+                                           FF_INTERP_SMEM));
     farfield_interp_kernel<<<dim3(a.n_orient, (a.ndir + 191) / 192), 192, ismem, ctx->stream>>>(a, nodes, p.parts, p.H,
                                                                                              weights);
     BEM_LAUNCHED(ctx);
@@ -797,20 +807,20 @@ __global__ void mueller_sum_kernel(const double* __restrict__ Mo, int n_orient, 
 static int launch_ff(bem_ctx* ctx, const bem_geom* g, FFArgs& a) {
     int nchunk = (a.ndir + 63) / 64;
     int dpb = (a.ndir + nchunk - 1) / nchunk;
-    int threads = dpb * FF_LANES;
+    int threads = dpb * FF_LANES;  // 256 at most: no kernel here takes more than 48 KB
+    static_assert(64 * FF_LANES * 24 * 8 <= 48 * 1024 &&
+                      FT_CHUNK * (3 + FF_MAXQ * 4) * 8 + FT_CHUNK * 16 * 16 <= 48 * 1024 &&
+                      FF_CHUNK * (6 * 8 + 4 * 16) <= 48 * 1024,
+                  "far field shared memory");
     dim3 grid(nchunk, a.n_orient);
     cudaEvent_t ev = ctx->prof_begin(PROF_FARFIELD);
     if (ctx->ff_kernel == 0) {
         if (g->Nq > FF_MAXQ) return fail(ctx, BEM_ERR_INVALID, "quadrature of %d points (at most %d)", g->Nq, FF_MAXQ);
         size_t smem = std::max((size_t)FT_CHUNK * (3 + FF_MAXQ * 4) * 8 + (size_t)FT_CHUNK * 16 * 16,
                                (size_t)threads * 24 * 8);
-        BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(farfield_tri_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem));
         farfield_tri_kernel<<<grid, threads, smem, ctx->stream>>>(a, g->tri, g->nt, g->sing_coef, dpb);
     } else {
         size_t smem = std::max((size_t)FF_CHUNK * (6 * 8 + 4 * 16), (size_t)threads * 24 * 8);
-        BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(farfield_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               (int)smem));
         farfield_kernel<<<grid, threads, smem, ctx->stream>>>(a, dpb);
     }
     BEM_LAUNCHED(ctx);
