@@ -6,6 +6,8 @@
 
 #include <cmath>
 
+#include "math_device.cuh"
+
 namespace bem {
 
 #define INV4PI_D 0.079577471545947667884
@@ -22,85 +24,11 @@ struct Medium {
     double kr, ki;  // k = kr + i ki
 };
 
-// sin and cos without a branch, for |x| below SINCOS_MAX: n = round(2 x / pi),
-// the remainder x - n pi/2 in two fused steps (the first is exact: both
-// operands are multiples of the remainder's last place), the Taylor
-// polynomials of degree 15 and 16 on [-pi/4, pi/4] (their first omitted terms
-// are below 5e-17 and 3e-18) and the quadrant's exchange and signs.  Within
-// 2e-16 of the exact values (tests).  The library's function takes a branch
-// for large arguments at every call, which keeps the compiler from
-// interleaving the independent evaluations of a quadrature loop: the kernels
-// here are bound by the latency of these chains at 8 to 16 warps per SM.
-constexpr double SINCOS_MAX = 1048576.0;
-__device__ __forceinline__ void sincos_bounded(double x, double* sn, double* cs) {
-    const double shift = 6755399441055744.0;  // 1.5 * 2^52: the sum's low bits are the rounded integer
-    const double t = __fma_rn(x, 0.63661977236758134308, shift);
-    const int n = __double2loint(t);
-    const double fn = t - shift;
-    double r = __fma_rn(-fn, 1.5707963267948965580, x);
-    r = __fma_rn(-fn, 6.1232339957367660359e-17, r);
-    const double z = r * r;
-    double p = __fma_rn(z, -1.0 / 1307674368000.0, 1.0 / 6227020800.0);
-    p = __fma_rn(z, p, -1.0 / 39916800.0);
-    p = __fma_rn(z, p, 1.0 / 362880.0);
-    p = __fma_rn(z, p, -1.0 / 5040.0);
-    p = __fma_rn(z, p, 1.0 / 120.0);
-    p = __fma_rn(z, p, -1.0 / 6.0);
-    const double s = __fma_rn(r * z, p, r);
-    double q = __fma_rn(z, 1.0 / 20922789888000.0, -1.0 / 87178291200.0);
-    q = __fma_rn(z, q, 1.0 / 479001600.0);
-    q = __fma_rn(z, q, -1.0 / 3628800.0);
-    q = __fma_rn(z, q, 1.0 / 40320.0);
-    q = __fma_rn(z, q, -1.0 / 720.0);
-    q = __fma_rn(z, q, 1.0 / 24.0);
-    q = __fma_rn(z, q, -0.5);
-    const double c = __fma_rn(z, q, 1.0);
-    const double a = (n & 1) ? c : s, b = (n & 1) ? s : c;
-    *sn = __hiloint2double(__double2hiint(a) ^ (int)((unsigned)(n & 2) << 30), __double2loint(a));
-    *cs = __hiloint2double(__double2hiint(b) ^ (int)((unsigned)((n + 1) & 2) << 30), __double2loint(b));
-}
-
 // e^-x for x >= 0.  Below 2^-54 the correctly rounded value is exactly 1;
 // the literal G_smooth at coincident points (R_s = 1e-15) subtracts
 // 1/(4 pi R_s) from e^-x cos(k R_s)/(4 pi R_s), so one unit in the last
 // place of e^-x there would become 0.0156 in G.
 __device__ __forceinline__ double exp_decay(double x) { return x < 5.551115123125783e-17 ? 1.0 : exp(-x); }
-
-// e^-x without a branch, x clamped to [0, 708] (e^-0 = 1 exactly; below e^-708
-// the value does not count): x = -(n ln 2 + r), |r| <= ln 2 / 2, in two fused
-// steps, the Taylor polynomial of degree 13 (first omitted term below 5e-18)
-// and 2^n added to the exponent.
-__device__ __forceinline__ double exp_decay_bounded(double x) {
-    x = fmin(fmax(x, 0.0), 708.0);
-    const double shift = 6755399441055744.0;
-    const double t = __fma_rn(x, -1.4426950408889634074, shift);
-    const double fn = t - shift;
-    double r = __fma_rn(fn, -0.69314718055994530942, -x);
-    r = __fma_rn(fn, -2.3190468138462995585e-17, r);
-    double p = __fma_rn(r, 1.0 / 6227020800.0, 1.0 / 479001600.0);
-    p = __fma_rn(r, p, 1.0 / 39916800.0);
-    p = __fma_rn(r, p, 1.0 / 3628800.0);
-    p = __fma_rn(r, p, 1.0 / 362880.0);
-    p = __fma_rn(r, p, 1.0 / 40320.0);
-    p = __fma_rn(r, p, 1.0 / 5040.0);
-    p = __fma_rn(r, p, 1.0 / 720.0);
-    p = __fma_rn(r, p, 1.0 / 120.0);
-    p = __fma_rn(r, p, 1.0 / 24.0);
-    p = __fma_rn(r, p, 1.0 / 6.0);
-    p = __fma_rn(r, p, 0.5);
-    p = __fma_rn(r, p, 1.0);
-    p = __fma_rn(r, p, 1.0);
-    return __hiloint2double(__double2hiint(p) + (int)((unsigned)__double2loint(t) << 20), __double2loint(p));
-}
-
-// 1 / sqrt(x) for a normal x > 0: the hardware's approximation (about 2^-20)
-// and one cubically convergent step, y (1 + e / 2 + 3 e^2 / 8) with e = 1 - x y^2.
-__device__ __forceinline__ double rsqrt_normal(double x) {
-    double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = __fma_rn(-x * y, y, 1.0);
-    return __fma_rn(y * e, __fma_rn(e, 0.375, 0.5), y);
-}
 
 // G_smooth = (exp(ikR) - 1)/(4 pi R) without cancellation (limit ik/(4 pi)).
 __device__ __forceinline__ cplx g_smooth_exact(Medium k, double R) {

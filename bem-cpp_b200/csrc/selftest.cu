@@ -1,3 +1,5 @@
+// Entry points that the tests use to see parts of the library on their own.
+//
 // The failure path of a bounded device-side wait, exercised without a fault.
 //
 // Every wait in this library's kernels (the tensor-core pipelines' mbarriers,
@@ -12,9 +14,28 @@
 #include <cstdint>
 
 #include "bem_internal.h"
+#include "math_device.cuh"
 
 namespace bem {
 namespace {
+
+// own[i], ref[i] (two values a point for fn 0): the branch-free function of
+// math_device.cuh and the library's at x[i].
+__global__ void math_kernel(int fn, const double* __restrict__ x, int n, double* __restrict__ own,
+                            double* __restrict__ ref) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    if (fn == 0) {
+        sincos_bounded(x[i], &own[2 * i], &own[2 * i + 1]);
+        sincos(x[i], &ref[2 * i], &ref[2 * i + 1]);
+    } else if (fn == 1) {
+        own[i] = exp_decay_bounded(x[i]);
+        ref[i] = exp(-x[i]);
+    } else {
+        own[i] = rsqrt_normal(x[i]);
+        ref[i] = rsqrt(x[i]);
+    }
+}
 
 __global__ void bounded_wait_kernel(const volatile int* flag, long long cycles, int* status) {
     const long long t0 = clock64();
@@ -29,6 +50,25 @@ __global__ void bounded_wait_kernel(const volatile int* flag, long long cycles, 
 
 }  // namespace
 }  // namespace bem
+
+extern "C" int bem_selftest_math(bem_ctx* ctx, int fn, const double* x, int n, double* own, double* ref) {
+    if (!ctx || !x || !own || !ref || n < 1 || n > (1 << 26) || fn < 0 || fn > 2) return BEM_ERR_INVALID;
+    BEM_TRY_CUDA(ctx, cudaSetDevice(ctx->device));
+    const size_t out = (size_t)n * (fn == 0 ? 2 : 1);
+    double* d = nullptr;
+    BEM_TRY_CUDA(ctx, cudaMalloc(&d, ((size_t)n + 2 * out) * sizeof(double)));
+    cudaError_t e = cudaMemcpyAsync(d, x, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess) {
+        bem::math_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(fn, d, n, d + n, d + n + out);
+        ctx->launches++;
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpyAsync(own, d + n, out * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(ref, d + n + out, out * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    cudaFree(d);
+    return e == cudaSuccess ? BEM_OK : bem::fail(ctx, BEM_ERR_CUDA, "elementary functions: %s", cudaGetErrorString(e));
+}
 
 extern "C" int bem_selftest_bounded_wait(bem_ctx* ctx, int64_t cycles, int set_flag) {
     if (!ctx || cycles < 0 || cycles > 4000000000LL) return BEM_ERR_INVALID;

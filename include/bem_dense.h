@@ -184,6 +184,11 @@ const char* bem_version(void);
  * call returns BEM_ERR_TIMEOUT with the context still usable; set_flag = 1:
  * BEM_OK.  No counterpart in the reference (its CUDA errors exit). */
 int bem_selftest_bounded_wait(bem_ctx* ctx, int64_t cycles, int set_flag);
+/* The branch-free elementary functions of the quadrature kernels beside CUDA's
+ * own, at n points x (host arrays, n at most 2^26): fn 0: sine and cosine
+ * interleaved (own and ref hold 2 n), |x| < 2^20; 1: exp(-x), x >= 0; 2:
+ * 1/sqrt(x), x > 0 normal.  No counterpart in the reference. */
+int bem_selftest_math(bem_ctx* ctx, int fn, const double* x, int n, double* own, double* ref);
 
 /* ----------------------------------------------------- geometry (host) */
 /* Meshes are returned through caller buffers.  Pass NULL buffers to query
