@@ -37,6 +37,7 @@
 #include "bem_internal.h"
 #include "cgemm_simt.cuh"
 #include "lu_internal.h"
+#include "math_device.cuh"
 #include "zgemm_dmma.cuh"
 
 namespace bem {
@@ -171,19 +172,6 @@ template <typename R> __device__ __forceinline__ R cabs1(typename C2T<R>::type v
 }
 
 // ------------------------------------------------------------ panel kernel
-// 1 / p of a pivot: conj(p) times the reciprocal of |p|^2, which the hardware
-// approximates to about 2^-20 and two Newton steps finish (the division's
-// branches were ~100 cycles of every panel column); conj(p) / |p|^2 by
-// divisions outside that approximation's range.
-__device__ __forceinline__ double2 pivot_recip(double2 p) {
-    const double den = p.x * p.x + p.y * p.y;
-    if (!(den > 1e-290 && den < 1e290)) return make_double2(p.x / den, -p.y / den);
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(den));
-    y = __fma_rn(y, __fma_rn(-den, y, 1.0), y);
-    y = __fma_rn(y, __fma_rn(-den, y, 1.0), y);
-    return make_double2(p.x * y, -p.y * y);
-}
 __device__ __forceinline__ float2 pivot_recip(float2 p) {
     const float den = p.x * p.x + p.y * p.y;
     return make_float2(p.x / den, -p.y / den);

@@ -19,8 +19,8 @@
 namespace bem {
 namespace {
 
-// own[i], ref[i] (two values a point for fn 0): the branch-free function of
-// math_device.cuh and the library's at x[i].
+// own[i], ref[i] (two values a point for fn 0 and 3): the branch-free function
+// of math_device.cuh and CUDA's at x[i] (fn 3: x[2i] + i x[2i + 1], by divisions).
 __global__ void math_kernel(int fn, const double* __restrict__ x, int n, double* __restrict__ own,
                             double* __restrict__ ref) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -31,9 +31,14 @@ __global__ void math_kernel(int fn, const double* __restrict__ x, int n, double*
     } else if (fn == 1) {
         own[i] = exp_decay_bounded(x[i]);
         ref[i] = exp(-x[i]);
-    } else {
+    } else if (fn == 2) {
         own[i] = rsqrt_normal(x[i]);
         ref[i] = rsqrt(x[i]);
+    } else {
+        const double2 p = make_double2(x[2 * i], x[2 * i + 1]), r = pivot_recip(p);
+        const double den = p.x * p.x + p.y * p.y;
+        own[2 * i] = r.x, own[2 * i + 1] = r.y;
+        ref[2 * i] = p.x / den, ref[2 * i + 1] = -p.y / den;
     }
 }
 
@@ -52,19 +57,19 @@ __global__ void bounded_wait_kernel(const volatile int* flag, long long cycles, 
 }  // namespace bem
 
 extern "C" int bem_selftest_math(bem_ctx* ctx, int fn, const double* x, int n, double* own, double* ref) {
-    if (!ctx || !x || !own || !ref || n < 1 || n > (1 << 26) || fn < 0 || fn > 2) return BEM_ERR_INVALID;
+    if (!ctx || !x || !own || !ref || n < 1 || n > (1 << 26) || fn < 0 || fn > 3) return BEM_ERR_INVALID;
     BEM_TRY_CUDA(ctx, cudaSetDevice(ctx->device));
-    const size_t out = (size_t)n * (fn == 0 ? 2 : 1);
+    const size_t in = (size_t)n * (fn == 3 ? 2 : 1), out = (size_t)n * (fn == 0 || fn == 3 ? 2 : 1);
     double* d = nullptr;
-    BEM_TRY_CUDA(ctx, cudaMalloc(&d, ((size_t)n + 2 * out) * sizeof(double)));
-    cudaError_t e = cudaMemcpyAsync(d, x, (size_t)n * sizeof(double), cudaMemcpyHostToDevice, ctx->stream);
+    BEM_TRY_CUDA(ctx, cudaMalloc(&d, (in + 2 * out) * sizeof(double)));
+    cudaError_t e = cudaMemcpyAsync(d, x, in * sizeof(double), cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) {
-        bem::math_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(fn, d, n, d + n, d + n + out);
+        bem::math_kernel<<<(n + 255) / 256, 256, 0, ctx->stream>>>(fn, d, n, d + in, d + in + out);
         ctx->launches++;
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = cudaMemcpyAsync(own, d + n, out * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(ref, d + n + out, out * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(own, d + in, out * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(ref, d + in + out, out * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     cudaFree(d);
     return e == cudaSuccess ? BEM_OK : bem::fail(ctx, BEM_ERR_CUDA, "elementary functions: %s", cudaGetErrorString(e));
