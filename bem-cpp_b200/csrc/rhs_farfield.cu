@@ -37,6 +37,19 @@ struct RhsArgs {
     int64_t ldb;
 };
 
+// a . b = h + l: the products with their roundings (fused multiply-add), their
+// sums with theirs (Knuth's two-sum).
+__device__ __forceinline__ void dot_two(const double* a, const double* b, double* h, double* l) {
+    double s = __dmul_rn(a[0], b[0]), e = __fma_rn(a[0], b[0], -s);
+#pragma unroll
+    for (int i = 1; i < 3; i++) {
+        const double p = __dmul_rn(a[i], b[i]), t = __dadd_rn(s, p), bb = t - s;  // no contraction
+        e += __fma_rn(a[i], b[i], -p) + ((s - (t - bb)) + (p - bb));
+        s = t;
+    }
+    *h = s, *l = e;
+}
+
 // Both polarisations of RHS_ORI orientations at a time for the 16 RWGs of an
 // assembly tile, by triangles: the phase at a quadrature point is shared by
 // the RWG halves of its triangle, f_h = s_h (u - pi_h), so the tile's ~16
@@ -46,6 +59,11 @@ struct RhsArgs {
 // vectors e (thread: RWG and orientation).  2 x fewer exponentials than per
 // RWG half, and the fields are dotted once per half instead of per point.
 // Bound by the FP64 pipe; the output is 4 x 16 B per (RWG, orientation).
+// The phase k k_hat.r takes the triangle's centroid in two doubles and adds what
+// lies between it and the point, which is short, so k_hat.r is rounded once at
+// its own size: error against 64 bits 1.004 of that of the sums per RWG half at
+// 2N = 15360, k rmax = 10 (1.10 with the centroids dotted plainly), for 19 of
+// ~330 operations a triangle and orientation (510 -> 519 us).
 // GENERAL: complex k or arguments beyond sincos_bounded (library functions).
 constexpr int RHS_ORI = 16, RHS_THREADS = 288;  // 18 triangles x 16 orientations a pass
 constexpr int RHS_FLD = 15;                     // k_hat and (E, H) of two polarisations
@@ -105,13 +123,14 @@ __global__ void __launch_bounds__(RHS_THREADS, 3) rhs_kernel(RhsArgs a) {
             const double* kh = s_f + ol * RHS_FLD;
             const double kx = kh[0], ky = kh[1], kz = kh[2];
             const double* c = s_c + 3 * li;
-            const double sc = kx * c[0] + ky * c[1] + kz * c[2];
+            double s0, sc;
+            dot_two(kh, c, &s0, &sc);
             double E[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll
             for (int q = 0; q < Nq; q++) {
                 const double2 uxy = *(const double2*)(s_pt + 4 * (li * Nq + q)),
                               uzw = *(const double2*)(s_pt + 4 * (li * Nq + q) + 2);
-                const double sq = sc + (kx * uxy.x + ky * uxy.y + kz * uzw.x);
+                const double sq = s0 + __fma_rn(kx, uxy.x, __fma_rn(ky, uxy.y, __fma_rn(kz, uzw.x, sc)));
                 double sn, cs;
                 if constexpr (GENERAL) {
                     sincos(a.kr * sq, &sn, &cs);
