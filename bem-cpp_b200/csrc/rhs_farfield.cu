@@ -50,6 +50,49 @@ __device__ __forceinline__ void dot_two(const double* a, const double* b, double
     *h = s, *l = e;
 }
 
+// Sums and products in two doubles h + l (Knuth's two-sum, Dekker's product by a
+// fused multiply-add), good to about 2^-100 of the largest term.
+struct Two {
+    double h, l;
+};
+__device__ __forceinline__ Two two_sum(double a, double b) {
+    const double s = __dadd_rn(a, b), v = s - a;
+    return {s, (a - (s - v)) + (b - v)};
+}
+__device__ __forceinline__ Two two_add(Two a, Two b) {
+    const Two s = two_sum(a.h, b.h);
+    return two_sum(s.h, s.l + (a.l + b.l));
+}
+__device__ __forceinline__ Two two_mul(Two a, Two b) {
+    const double p = __dmul_rn(a.h, b.h);
+    return two_sum(p, __fma_rn(a.h, b.h, -p) + (a.h * b.l + a.l * b.h));
+}
+
+// sin and cos of pi num / den, |num| <= 2 den, to about 2^-63: the nearest multiple
+// of pi / 2 off as an integer, then the Taylor polynomials of degree 19 and 18
+// with their first two terms in two doubles.
+__device__ void sincospi_two(int num, int den, Two* sn, Two* cs) {
+    const long long q = (4LL * num + (num >= 0 ? den : -den)) / (2LL * den);  // 2 num / den, rounded
+    const double rem = (double)(2LL * num - q * den), dd = (double)den, a = rem / dd;
+    const Two r = two_mul(Two{a, __fma_rn(-a, dd, rem) / dd}, Two{1.5707963267948965580, 6.1232339957367660359e-17});
+    const Two z = two_mul(r, r);
+    const double x = z.h;
+    double p = 1.0 / 120.0 + x * (-1.0 / 5040.0 + x * (1.0 / 362880.0 + x * (-1.0 / 39916800.0 + x * (1.0 / 6227020800.0 +
+               x * (-1.0 / 1307674368000.0 + x * (1.0 / 355687428096000.0 + x * (-1.0 / 121645100408832000.0)))))));
+    double c = -1.0 / 720.0 + x * (1.0 / 40320.0 + x * (-1.0 / 3628800.0 + x * (1.0 / 479001600.0 +
+               x * (-1.0 / 87178291200.0 + x * (1.0 / 20922789888000.0 + x * (-1.0 / 6402373705728000.0))))));
+    // 1/6 and 1/24 in two doubles: 1/3 is 0.333.. + 1.85e-17
+    const Two sixth = {-1.0 / 6.0, -9.2518585385429706566e-18}, t24 = {1.0 / 24.0, 2.3129646346357426642e-18};
+    const Two s = two_add(r, two_mul(two_mul(r, z), two_add(sixth, Two{x * p, 0.0})));
+    const Two u = two_add(two_add(Two{1.0, 0.0}, Two{-0.5 * z.h, -0.5 * z.l}),
+                          two_mul(two_mul(z, z), two_add(t24, Two{x * c, 0.0})));
+    const bool odd = q & 1;
+    const double fs = ((q & 2) != 0) ? -1.0 : 1.0, fc = (((q + 1) & 2) != 0) ? -1.0 : 1.0;
+    const Two vs = odd ? u : s, vc = odd ? s : u;
+    *sn = {fs * vs.h, fs * vs.l};
+    *cs = {fc * vc.h, fc * vc.l};
+}
+
 // Both polarisations of RHS_ORI orientations at a time for the 16 RWGs of an
 // assembly tile, by triangles: the phase at a quadrature point is shared by
 // the RWG halves of its triangle, f_h = s_h (u - pi_h), so the tile's ~16
@@ -563,13 +606,20 @@ __global__ void __launch_bounds__(256) farfield_tri_kernel(FFArgs a, DevTriAsm t
 // Im, the two nodes are P + iQ and P - iQ.  H phases per point instead of
 // ntheta: 47 instead of 181 at k rmax = 16, 18 at k rmax = 1.
 //
+// An error of a node's angle is the same for every triangle and orientation and
+// does not average out, so the node's sine and cosine and a centroid's
+// projections are held in two doubles and the centroid's phase is summed in
+// two.  With the weights rounded once and the nodes taken from far to near, the
+// Mueller matrices are 2.7e-16 to 3.2e-16 off 80-bit sums (k rmax = 1 to 15), the
+// kernel per direction 3.5e-16 to 4.3e-16.
+//
 // farfield_nodes_kernel is bound by the FP64 pipe: per (node pair, triangle)
-// Nq (23 for the sine and cosine, 10) + 96 operations.  Block: FN_PAIRS node
+// Nq (24 for the sine and cosine, 11) + 18 for the centroid + 96 operations.  Block: FN_PAIRS node
 // pairs x FN_LANES triangle lanes of one orientation, and every gridDim.z-th
 // chunk of FN_CHUNK triangles; the parts are added in order by
 // farfield_interp_kernel.
 constexpr int FN_PAIRS = 16, FN_LANES = 8, FN_CHUNK = 64;
-constexpr int FN_REC = 17;  // a triangle's 4 alpha and 12 gamma, padded: odd, so the lanes' records do not conflict
+constexpr int FN_REC = 19;  // a triangle's 4 alpha and 12 gamma and its centroid's two projections, padded: odd, so the lanes' records do not conflict
 
 template <int NQ>
 __global__ void __launch_bounds__(FN_PAIRS* FN_LANES, 3)
@@ -577,15 +627,16 @@ farfield_nodes_kernel(FFArgs a, DevTriAsm ta, int nt, const double* __restrict__
                       double* __restrict__ nodes) {
     extern __shared__ __align__(16) double sm[];
     const int Nq = NQ > 0 ? NQ : a.Nq;
-    double2* s_p = (double2*)sm;                      // FN_CHUNK * Nq * 3: (x1, x2) (w, w u_x) (w u_y, w u_z)
-    double2* s_ag = s_p + FN_CHUNK * Nq * 3;          // FN_CHUNK * FN_REC: per column k alpha, gamma
+    double2* s_p = (double2*)sm;                      // FN_CHUNK * Nq * 3: (x1, x2) of u, (w, w u_x) (w u_y, w u_z)
+    double2* s_ag = s_p + FN_CHUNK * Nq * 3;          // FN_CHUNK * FN_REC: per column k alpha, gamma; the centroid's x1, x2
     const int o = blockIdx.y, tid = threadIdx.x, lane = tid % FN_LANES;
     const int j = blockIdx.x * FN_PAIRS + tid / FN_LANES;  // node pair: t_j = pi j / H and t_j + pi
     const int c0 = 2 * o, c1 = 2 * o + 1, N = a.N;
     const double* R = a.RT + 9 * (size_t)o;
-    double st, ct;
-    sincospi((double)j / H, &st, &ct);
-    st *= a.kr, ct *= a.kr;
+    Two kst, kct;  // k times the node's sine and cosine
+    sincospi_two(j, H, &kst, &kct);
+    kst = two_mul(kst, Two{a.kr, 0.0}), kct = two_mul(kct, Two{a.kr, 0.0});
+    const double st = kst.h, ct = kct.h;
     double P[12][2], Q[12][2];
 #pragma unroll
     for (int i = 0; i < 12; i++) P[i][0] = P[i][1] = Q[i][0] = Q[i][1] = 0.0;
@@ -594,14 +645,18 @@ farfield_nodes_kernel(FFArgs a, DevTriAsm ta, int nt, const double* __restrict__
         __syncthreads();
         for (int e = tid; e < cnt * Nq; e += FN_PAIRS * FN_LANES) {
             const size_t src = (size_t)t0 * Nq + e;
-            const double* c = ta.c + 3 * (size_t)(t0 + e / Nq);
             const double ux = ta.u[src * 3], uy = ta.u[src * 3 + 1], uz = ta.u[src * 3 + 2], w = ta.jw[src];
-            // R^T x . r and R^T z . r, the centroid's part first
-            const double x1 = (R[0] * c[0] + R[3] * c[1] + R[6] * c[2]) + (R[0] * ux + R[3] * uy + R[6] * uz);
-            const double x2 = (R[2] * c[0] + R[5] * c[1] + R[8] * c[2]) + (R[2] * ux + R[5] * uy + R[8] * uz);
-            s_p[3 * e] = make_double2(x1, x2);
+            // R^T x . u and R^T z . u
+            s_p[3 * e] = make_double2(R[0] * ux + R[3] * uy + R[6] * uz, R[2] * ux + R[5] * uy + R[8] * uz);
             s_p[3 * e + 1] = make_double2(w, w * ux);
             s_p[3 * e + 2] = make_double2(w * uy, w * uz);
+        }
+        for (int e = tid; e < cnt * 2; e += FN_PAIRS * FN_LANES) {
+            const int k = e % 2 * 2;  // R^T x . c and R^T z . c
+            const double ax[3] = {R[k], R[3 + k], R[6 + k]};
+            double h, l;
+            dot_two(ax, ta.c + 3 * (size_t)(t0 + e / 2), &h, &l);
+            s_ag[e / 2 * FN_REC + 16 + e % 2] = make_double2(h, l);
         }
         for (int e = tid; e < cnt * 4; e += FN_PAIRS * FN_LANES) {
             const int tt = e / 4, k = e % 4;  // k: J0 M0 J1 M1
@@ -626,11 +681,17 @@ farfield_nodes_kernel(FFArgs a, DevTriAsm ta, int nt, const double* __restrict__
         for (int tt = lane; tt < cnt; tt += FN_LANES) {
             double E0r = 0, E0i = 0, Eu[3][2] = {{0, 0}, {0, 0}, {0, 0}};
             const double2* pt = s_p + (size_t)tt * Nq * 3;
+            // the centroid's phase x0 + x0l
+            const double2 c1 = s_ag[tt * FN_REC + 16], c2 = s_ag[tt * FN_REC + 17];
+            const double p1 = __dmul_rn(st, c1.x), p2 = __dmul_rn(ct, c2.x);
+            const Two ph = two_sum(p1, p2);
+            const double x0 = ph.h, x0l = ph.l + ((__fma_rn(st, c1.x, -p1) + __fma_rn(ct, c2.x, -p2)) +
+                                                  (st * c1.y + ct * c2.y + kst.l * c1.x + kct.l * c2.x));
 #pragma unroll
             for (int q = 0; q < Nq; q++) {
                 const double2 x = pt[3 * q], wx = pt[3 * q + 1], yz = pt[3 * q + 2];
                 double sn, cs;
-                sincos_bounded(st * x.x + ct * x.y, &sn, &cs);
+                sincos_bounded(x0 + __fma_rn(st, x.x, __fma_rn(ct, x.y, x0l)), &sn, &cs);
                 // exp(-i k rhat.r) = cs - i sn
                 E0r += cs * wx.x, E0i -= sn * wx.x;
                 Eu[0][0] += cs * wx.y, Eu[0][1] -= sn * wx.y;
@@ -671,46 +732,66 @@ farfield_nodes_kernel(FFArgs a, DevTriAsm ta, int nt, const double* __restrict__
     }
 }
 
-// W[j][d] of the trigonometric interpolation from the 2 H nodes t_j = pi j / H
-// to t_d = pi d / (ndir - 1): sin(H x) cot(x / 2) / (2 H) with x = t_d - t_j =
-// pi m / (H (ndir - 1)), m an integer, so both arguments reduce exactly
-// (2 H ndir <= FF_MAX_WEIGHTS, so the integers fit 32 bits).
+// The nodes in the order in which a direction's sums take them, from the
+// farthest to the nearest: e = 0 .. 2 H - 1 -> node jc + H, then jc +- (H - 1)
+// and so on to jc, the node nearest to t_d.  The weights fall off as the
+// cotangent of the distance, so the partial sums stay small until the last few
+// terms, and those alone round at the result's size: 0.72 of 2^-53 in the 2-norm
+// against 2 (H = 17) to 3.6 (H = 48) in the order of the nodes (restated in NumPy).
+__device__ __forceinline__ int ff_node(int e, int jc, int H) {
+    const int k = e == 0 ? H : H - (e + 1) / 2;
+    int j = (e & 1) ? jc + k : jc - k;
+    if (j < 0) j += 2 * H;
+    if (j >= 2 * H) j -= 2 * H;
+    return j;
+}
+__device__ __forceinline__ int ff_nearest(int d, int H, int nd) { return (2 * d * H + nd) / (2 * nd); }
+
+// W[e][d] of the trigonometric interpolation from the 2 H nodes t_j = pi j / H
+// to the call's theta_d, j = ff_node(e, ..): sin(H x) cot(x / 2) / (2 H), x =
+// theta_d - t_j.  theta_d is pi d / (ndir - 1) rounded: the weight is formed for the
+// exact fraction, where x = pi m / (H (ndir - 1)) with an integer m and sin(H x) =
+// +-sin(pi m / (ndir - 1)) (2 H ndir <= FF_MAX_WEIGHTS, so the integers fit 32
+// bits), and corrected to first order for the rounding of theta_d.  A weight's
+// error is the same for every orientation, so it is rounded once.
 constexpr int FF_MAX_WEIGHTS = 1 << 27;
-__global__ void ff_weights_kernel(int H, int ndir, double* __restrict__ W) {
+__global__ void ff_weights_kernel(int H, int ndir, const double* __restrict__ theta, double* __restrict__ W) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= 2 * H * ndir) return;
-    const int j = i / ndir, d = i % ndir, nd = ndir - 1;
-    // x modulo 2 pi in (-pi, pi], and sin(H x) = sin(pi m / nd) from the
-    // fraction nearest to its zeros: quotients near 0 keep their relative accuracy
+    const int d = i % ndir, nd = ndir - 1, j = ff_node(i / ndir, ff_nearest(d, H, nd), H);
     const int per = 2 * H * nd;
-    int m = (int)(((long long)d * H - (long long)j * nd) % per);
+    int m = (int)(((long long)d * H - (long long)j * nd) % per);  // x modulo 2 pi in (-pi, pi]
     if (m > per / 2) m -= per;
     if (m <= -per / 2) m += per;
     double w = 1.0;
     if (m != 0) {
-        double s, c;
-        sincospi((double)m / (double)per, &s, &c);  // x / 2
-        int k = m % (2 * nd);
-        if (k > nd) k -= 2 * nd;
-        if (k < -nd) k += 2 * nd;
-        if (2 * k > nd) k = nd - k;
-        if (2 * k < -nd) k = -nd - k;
-        w = sinpi((double)k / nd) * c / (s * 2.0 * H);
+        Two s, c, sh, ch;
+        sincospi_two(m, per, &s, &c);              // x / 2
+        sincospi_two(m % (2 * nd), nd, &sh, &ch);  // H x
+        const Two num = two_mul(sh, c), den = two_mul(s, Two{2.0 * H, 0.0});
+        const double q = num.h / den.h;
+        // theta_d - pi d / nd = -(pi d - theta_d nd) / nd, and the weight's slope there
+        const double th = theta[d], pd = __dmul_rn(3.1415926535897931160, (double)d);
+        const double off = -((__fma_rn(-th, (double)nd, pd) + __fma_rn(3.1415926535897931160, (double)d, -pd)) +
+                             1.2246467991473532072e-16 * d) / nd;
+        const double slope = (ch.h * c.h * H - sh.h / (2.0 * s.h)) / den.h;
+        w = q + ((__fma_rn(-q, den.h, num.h) + (num.l - q * den.l)) / den.h + off * slope);
     }
     W[i] = w;
 }
 
 // Thread: one direction of the orientation blockIdx.x; the node sums (all
-// parts, in order) in shared memory.
-constexpr int FF_INTERP_SMEM = 200 * 1024;
+// parts, in order) in shared memory, an odd number of 16-byte units apart: the
+// lanes of a warp are at up to 16 neighbouring nodes.
+constexpr int FF_NODE = 26, FF_MAX_H = 533, FF_INTERP_SMEM = 2 * FF_MAX_H * FF_NODE * 8;
 __global__ void __launch_bounds__(192) farfield_interp_kernel(FFArgs a, const double* __restrict__ nodes, int parts,
                                                               int H, const double* __restrict__ W) {
-    extern __shared__ __align__(16) double sm[];  // 2 H x 24
+    extern __shared__ __align__(16) double sm[];  // 2 H x FF_NODE
     const int o = blockIdx.x, cnt = 2 * H * 24;
     for (int e = threadIdx.x; e < cnt; e += blockDim.x) {
         double s = 0.0;
         for (int z = 0; z < parts; z++) s += nodes[((size_t)z * a.n_orient + o) * cnt + e];
-        sm[e] = s;
+        sm[e / 24 * FF_NODE + e % 24] = s;
     }
     __syncthreads();
     const int d = blockIdx.y * blockDim.x + threadIdx.x;
@@ -718,9 +799,10 @@ __global__ void __launch_bounds__(192) farfield_interp_kernel(FFArgs a, const do
     double acc[12][2];
 #pragma unroll
     for (int i = 0; i < 12; i++) acc[i][0] = acc[i][1] = 0.0;
-    for (int j = 0; j < 2 * H; j++) {
-        const double w = W[(size_t)j * a.ndir + d];
-        const double2* v = (const double2*)(sm + (size_t)j * 24);
+    const int jc = ff_nearest(d, H, a.ndir - 1);
+    for (int e = 0; e < 2 * H; e++) {
+        const double w = W[(size_t)e * a.ndir + d];
+        const double2* v = (const double2*)(sm + (size_t)ff_node(e, jc, H) * FF_NODE);
 #pragma unroll
         for (int i = 0; i < 12; i++) {
             const double2 x = v[i];
@@ -776,7 +858,7 @@ static FFPlan plan_ff(const bem_ctx* ctx, const bem_geom* g, const double* RT, i
     const double per_dir = (g->Nq * 33.0 + 96.0) * g->nt;
     if ((int64_t)2 * H * ndir > FF_MAX_WEIGHTS) return p;
     // the interpolation's shared memory bounds H as well
-    if (H < 1 || H * (per_dir + 48.0 * ndir) > per_dir * ndir || (size_t)2 * H * 24 * 8 > FF_INTERP_SMEM) return p;
+    if (H < 1 || H * (per_dir + 48.0 * ndir) > per_dir * ndir || H > FF_MAX_H) return p;
     p.H = H;
     const int chunks = (H + FN_PAIRS - 1) / FN_PAIRS, tchunks = (g->nt + FN_CHUNK - 1) / FN_CHUNK;
     // three blocks of 128 threads fit an SM: enough parts for about four waves
@@ -790,7 +872,7 @@ static FFPlan plan_ff(const bem_ctx* ctx, const bem_geom* g, const double* RT, i
 static int launch_ff_nodes(bem_ctx* ctx, const bem_geom* g, const FFArgs& a, const FFPlan& p, double* nodes,
                            double* weights) {
     cudaEvent_t ev = ctx->prof_begin(PROF_FARFIELD);
-    ff_weights_kernel<<<(2 * p.H * a.ndir + 255) / 256, 256, 0, ctx->stream>>>(p.H, a.ndir, weights);
+    ff_weights_kernel<<<(2 * p.H * a.ndir + 255) / 256, 256, 0, ctx->stream>>>(p.H, a.ndir, a.theta, weights);
     BEM_LAUNCHED(ctx);
     auto kern = g->Nq == 7 ? farfield_nodes_kernel<7> : g->Nq == 4 ? farfield_nodes_kernel<4> : farfield_nodes_kernel<0>;
     const size_t smem = (size_t)FN_CHUNK * (g->Nq * 3 + FN_REC) * 16;
@@ -799,7 +881,7 @@ static int launch_ff_nodes(bem_ctx* ctx, const bem_geom* g, const FFArgs& a, con
     kern<<<dim3((p.H + FN_PAIRS - 1) / FN_PAIRS, a.n_orient, p.parts), FN_PAIRS * FN_LANES, smem, ctx->stream>>>(
         a, g->tri, g->nt, g->sing_coef, p.H, nodes);
     BEM_LAUNCHED(ctx);
-    const size_t ismem = (size_t)2 * p.H * 24 * 8;
+    const size_t ismem = (size_t)2 * p.H * FF_NODE * 8;
     BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(farfield_interp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            FF_INTERP_SMEM));
     farfield_interp_kernel<<<dim3(a.n_orient, (a.ndir + 191) / 192), 192, ismem, ctx->stream>>>(a, nodes, p.parts, p.H,
