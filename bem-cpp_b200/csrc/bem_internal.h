@@ -208,8 +208,8 @@ struct bem_ctx {
     int gmres_digits = 0;        // GMRES products with Z: 0 FP64 DMMA GEMM, 2..8 int8 Ozaki digits
     bool batch_buckets = true;   // bem_batch_run: FP64 particles of one size batched (else one at a time)
     bool lu_autotune = true;     // batched LU shape from the autotuner (else NB 256, W 16)
-    bool panel_clusters = true;  // LU sub-panels that fit one thread-block cluster run in its registers
-                                 // instead of on the cooperative grid
+    int panel_clusters = 1;      // LU sub-panels that fit one thread-block cluster run in its registers
+                                 // instead of on the cooperative grid: 0 none, 1 up to 16 CTAs, else that many
     int64_t panel_wait = 2000000000;  // clock cycles after which a wait of those clusters gives up
     int grad_method = 0;         // adjoint gradients: 0 contraction kernels (grad_geom.cu), 1 central
                                  // differences of reassembled operators

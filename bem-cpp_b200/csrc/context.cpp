@@ -284,7 +284,7 @@ int bem_ctx_set_option(bem_ctx* ctx, const char* name, int value) {
         if (value < 0) return bem::fail(ctx, BEM_ERR_INVALID, "residual_pace_lead must be >= 0");
         ctx->oz_pace_lead = value;
     } else if (!std::strcmp(name, "panel_clusters")) {
-        ctx->panel_clusters = value != 0;
+        ctx->panel_clusters = value < 0 ? 1 : value;
     } else if (!std::strcmp(name, "panel_wait_mcycles")) {
         if (value < 0 || value > 4000) return bem::fail(ctx, BEM_ERR_INVALID, "panel_wait_mcycles must be 0..4000");
         ctx->panel_wait = (int64_t)value * 1000000;

@@ -699,38 +699,30 @@ panel_reg_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int n, int 
     if (C > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// CTAs per cluster and threads per CTA for a sub-panel of nrows rows of
-// `batch` matrices, 0 when it does not fit one cluster (panel_kernel takes
-// it): 256 rows a CTA up to 16 CTAs, then up to 512 rows a CTA -- 8192 rows.
-// Few rows a CTA keep the rank-1 update short (64 registers a row, the FP64
-// pipe of one SM).  Clusters of more than 8 CTAs fit about one to a GPC, so
-// more matrices than that take 8 CTAs while their rows fit.
+// CTAs per cluster (`most` at most) and threads per CTA for a sub-panel of
+// nrows rows, 0 when it does not fit: 256 rows a CTA up to `most` CTAs, then up
+// to 512 rows a CTA -- 8192 rows on 16 CTAs, 4096 on 8.  Few rows a CTA keep the
+// rank-1 update short (64 registers a row, the FP64 pipe of one SM).
 struct PanelShape {
     int C = 0, T = 0;
 };
-static PanelShape panel_reg_shape(int nrows, int batch) {
+static PanelShape panel_reg_shape(int nrows, int most) {
     PanelShape p;
-    if (nrows > PR_CLUSTER * PR_THREADS) return p;
-    const int most = batch > 8 && nrows <= 8 * PR_THREADS ? 8 : PR_CLUSTER;
+    if (nrows > most * PR_THREADS) return p;
     p.C = std::min(most, (nrows + 255) / 256);
     p.T = ((nrows + p.C - 1) / p.C + 31) / 32 * 32;
     return p;
 }
 
-// panel_reg_shape, kept only where a cluster of that shape can be resident on
-// this device (asked once per shape and remembered).
-template <typename R>
-static PanelShape panel_reg_choice(bem_ctx* ctx, int nrows, int iw, int batch) {
-    PanelShape p;
-    if (!ctx->panel_clusters || iw > PanelW<R>::v) return p;
-    p = panel_reg_shape(nrows, batch);
-    if (p.C == 0) return p;
+// Clusters of a shape that this device holds at a time (asked once per shape
+// and remembered).
+template <typename R> static int panel_resident(bem_ctx* ctx, PanelShape p) {
     static std::mutex mu;
-    static std::map<std::tuple<int, int, int>, bool> ok;
+    static std::map<std::tuple<int, int, int>, int> known;
     const auto key = std::make_tuple(ctx->device, p.C, p.T);
     std::lock_guard<std::mutex> lk(mu);
-    auto it = ok.find(key);
-    if (it == ok.end()) {
+    auto it = known.find(key);
+    if (it == known.end()) {
         auto kern = panel_reg_kernel<R>;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)p.C);
@@ -749,10 +741,23 @@ static PanelShape panel_reg_choice(bem_ctx* ctx, int nrows, int iw, int batch) {
             (p.C <= 8 || cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) &&
             cudaOccupancyMaxActiveClusters(&ncl, (const void*)kern, &cfg) == cudaSuccess && ncl >= 1;
         if (!fits) cudaGetLastError();
-        it = ok.emplace(key, fits).first;
+        it = known.emplace(key, fits ? ncl : 0).first;
     }
-    if (!it->second) p = PanelShape{};
-    return p;
+    return it->second;
+}
+
+// The shape for a sub-panel of `batch` matrices: up to 16 CTAs, or up to 8
+// where the rows fit 8 and fewer such clusters than matrices can be resident
+// (the rest would wait for a second round; none on a device that holds no
+// cluster of more than 8).  C = 0: panel_kernel takes it.
+template <typename R>
+static PanelShape panel_reg_choice(bem_ctx* ctx, int nrows, int iw, int batch) {
+    if (!ctx->panel_clusters || iw > PanelW<R>::v) return PanelShape{};
+    const int most = ctx->panel_clusters == 1 ? PR_CLUSTER : std::min(ctx->panel_clusters, PR_CLUSTER);
+    const PanelShape wide = panel_reg_shape(nrows, most), narrow = panel_reg_shape(nrows, std::min(most, 8));
+    const int nw = wide.C > 0 ? panel_resident<R>(ctx, wide) : 0;
+    if (narrow.C > 0 && narrow.C < wide.C && nw < batch && panel_resident<R>(ctx, narrow) > 0) return narrow;
+    return nw > 0 ? wide : PanelShape{};
 }
 
 // One launch of panel_reg_kernel: `batch` matrices (A + i sA, pivots

@@ -125,7 +125,8 @@ int bem_ctx_set_symmetric(bem_ctx* ctx, int mode);
  * kernels; 1: central differences of reassembled operators, for checking),
  * "panel_clusters" (1, default: the sub-panels of the pivoted LU of at most
  * 8192 rows are factored in the registers of one thread-block cluster per
- * matrix, up to 16 CTAs, one exchange of candidates per column; 0: every
+ * matrix, up to 16 CTAs, one exchange of candidates per column; 2..16: at
+ * most so many CTAs, 512 rows each; 0: every
  * sub-panel on the cooperative grid, one grid barrier per column; both give
  * the same pivots and factors),
  * "panel_wait_mcycles" (2000, default: millions of SM clock cycles, about one
