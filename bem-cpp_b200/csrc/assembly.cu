@@ -124,10 +124,19 @@ static void position_arrays(const bem_geom* g, PosArrays& A) {
         }
 }
 
-static double largest_vertex(const HostMesh& m) {
-    double r2 = 0.0;
-    for (const V3& v : m.verts) r2 = std::max(r2, v.x * v.x + v.y * v.y + v.z * v.z);
-    return std::sqrt(r2);
+// g->rmax and g->extent: the largest |r| and a bound of |r - r'| (the diagonal
+// of the bounding box, which unlike 2 rmax does not grow with the distance from
+// the origin) over the vertices and so over all quadrature points.
+static void mesh_bounds(bem_geom* g) {
+    double r2 = 0.0, lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
+    for (const V3& v : g->mesh.verts) {
+        const double x[3] = {v.x, v.y, v.z};
+        r2 = std::max(r2, x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
+        for (int i = 0; i < 3; i++) lo[i] = std::min(lo[i], x[i]), hi[i] = std::max(hi[i], x[i]);
+    }
+    g->rmax = std::sqrt(r2);
+    g->extent = std::sqrt((hi[0] - lo[0]) * (hi[0] - lo[0]) + (hi[1] - lo[1]) * (hi[1] - lo[1]) +
+                          (hi[2] - lo[2]) * (hi[2] - lo[2]));
 }
 
 // RWG order of the assembly tiles (ASM_TILE consecutive ones each): patches
@@ -207,7 +216,7 @@ static std::vector<int> patch_order(const HostRWG& r, int nt, const std::vector<
 
 int geom_upload(bem_ctx* ctx, bem_geom* g) {
     const HostMesh& m = g->mesh;
-    g->rmax = largest_vertex(m);
+    mesh_bounds(g);
     const HostRWG& r = g->rwg;
     const Quad& q = g->quad;
     const int N = r.N, Nq = q.n, nt = m.nt();
@@ -419,7 +428,7 @@ int geom_set_vertices(bem_ctx* ctx, bem_geom* g, const double* verts) {
         return fail(ctx, BEM_ERR_INVALID, "vertex update needs a geometry built from its mesh");
     for (int i = 0; i < m.nv(); i++) m.verts[i] = {verts[3 * i], verts[3 * i + 1], verts[3 * i + 2]};
     rwg_refresh(m, r);
-    g->rmax = largest_vertex(m);
+    mesh_bounds(g);
     PosArrays A;
     position_arrays(g, A);
     const int N = r.N;
@@ -1162,9 +1171,9 @@ int assemble_dev(bem_ctx* ctx, const bem_geom* g, double ke_re, double ke_im, do
     a.coef = g->sing_coef;
     a.tile_flag = nullptr;
     // triangle pairs, unless a phase could leave the range of sincos_bounded
-    // (|r - r'| <= 2 rmax): then the per-RWG kernel with the library's sine and cosine
+    // (|r - r'| <= extent): then the per-RWG kernel with the library's sine and cosine
     const double kmax = std::max(std::fabs(ke_re), mode == 2 ? std::fabs(ki_re) : 0.0);
-    const bool tri = ctx->asm_kernel == 0 && kmax * 2.0 * g->rmax < SINCOS_MAX;
+    const bool tri = ctx->asm_kernel == 0 && kmax * g->extent < SINCOS_MAX;
     const unsigned char* rec = nullptr;
     if (rwg_mask) {
         // tiles holding a flagged RWG, and the RWGs of those tiles

@@ -245,6 +245,7 @@ struct bem_geom {
     int device = 0;
     int N = 0, Nq = 0, nv = 0, nt = 0, quad_order = 7;
     double rmax = 0.0;     // largest |vertex|: bounds every quadrature point's
+    double extent = 0.0;   // bound of the distance of two points
     bem::HostMesh mesh;
     bem::HostRWG rwg;
     bem::Quad quad;

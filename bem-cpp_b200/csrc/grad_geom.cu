@@ -908,8 +908,7 @@ int adjoint_geometry(bem_ctx* ctx, const bem_geom* g, std::complex<double> kext,
     const Medium ke{kext.real(), kext.imag()}, ki{kint.real(), kint.imag()};
     PairArgs pa{g->sing.tv, d_hinfo, nt, Nq, tq, ke, ki, gw, o_pair, o_skp, o_sep};
     // the branch-free functions where no phase can leave their range
-    const double reach = 2.0 * g->rmax;
-    const bool bounded = std::max(std::abs(ke.kr), std::abs(ki.kr)) * reach < SINCOS_MAX && ke.ki == 0 && ki.ki >= 0;
+    const bool bounded = std::max(std::abs(ke.kr), std::abs(ki.kr)) * g->extent < SINCOS_MAX && ke.ki == 0 && ki.ki >= 0;
     auto pair = !bounded ? grad_pair_kernel<3, false> : ki.ki != 0 ? grad_pair_kernel<2, true> : grad_pair_kernel<0, true>;
     const size_t pair_smem = (size_t)3 * GP_W * GP_THREADS * sizeof(double);
     BEM_TRY_CUDA(ctx, cudaFuncSetAttribute(pair, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pair_smem));
