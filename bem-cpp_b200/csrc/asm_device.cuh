@@ -24,11 +24,12 @@ struct Medium {
     double kr, ki;  // k = kr + i ki
 };
 
-// e^-x for x >= 0.  Below 2^-54 the correctly rounded value is exactly 1;
+// e^-x (growth for a medium with gain, x < 0).  For |x| below 2^-54 the
+// correctly rounded value is exactly 1;
 // the literal G_smooth at coincident points (R_s = 1e-15) subtracts
 // 1/(4 pi R_s) from e^-x cos(k R_s)/(4 pi R_s), so one unit in the last
 // place of e^-x there would become 0.0156 in G.
-__device__ __forceinline__ double exp_decay(double x) { return x < 5.551115123125783e-17 ? 1.0 : exp(-x); }
+__device__ __forceinline__ double exp_decay(double x) { return fabs(x) < 5.551115123125783e-17 ? 1.0 : exp(-x); }
 
 // G_smooth = (exp(ikR) - 1)/(4 pi R) without cancellation (limit ik/(4 pi)).
 __device__ __forceinline__ cplx g_smooth_exact(Medium k, double R) {

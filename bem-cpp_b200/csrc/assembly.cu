@@ -1173,7 +1173,9 @@ int assemble_dev(bem_ctx* ctx, const bem_geom* g, double ke_re, double ke_im, do
     // triangle pairs, unless a phase could leave the range of sincos_bounded
     // (|r - r'| <= extent): then the per-RWG kernel with the library's sine and cosine
     const double kmax = std::max(std::fabs(ke_re), mode == 2 ? std::fabs(ki_re) : 0.0);
-    const bool tri = ctx->asm_kernel == 0 && kmax * g->extent < SINCOS_MAX;
+    // or a medium's gain the range of exp_decay_bounded
+    const double gain = std::max(-ke_im, mode == 2 ? -ki_im : 0.0);
+    const bool tri = ctx->asm_kernel == 0 && kmax * g->extent < SINCOS_MAX && !(gain * g->extent > 700.0);
     const unsigned char* rec = nullptr;
     if (rwg_mask) {
         // tiles holding a flagged RWG, and the RWGs of those tiles

@@ -46,13 +46,13 @@ __device__ __forceinline__ void sincos_bounded(double x, double* sn, double* cs)
     *cs = __hiloint2double(__double2hiint(b) ^ (int)((unsigned)((n + 1) & 2) << 30), __double2loint(b));
 }
 
-// e^-x without a branch, x clamped to [0, 708] (e^-0 = 1 exactly; below e^-708
-// the value does not count): x = -(n ln 2 + r), |r| <= ln 2 / 2, in two fused
+// e^-x without a branch, x clamped to [-708, 708] (e^-0 = 1 exactly; below
+// e^-708 the value does not count, above e^708 the callers do not come): x = -(n ln 2 + r), |r| <= ln 2 / 2, in two fused
 // steps (Cody and Waite's reduction), the Taylor polynomial of degree 13 (first
 // omitted term below 5e-18) and 2^n added to the exponent.  Largest relative
 // error measured 1.24 of 2^-53, CUDA's exp 1.24 on the same arguments.
 __device__ __forceinline__ double exp_decay_bounded(double x) {
-    x = fmin(fmax(x, 0.0), 708.0);
+    x = fmin(fmax(x, -708.0), 708.0);
     const double shift = 6755399441055744.0;
     const double t = __fma_rn(x, -1.4426950408889634074, shift);
     const double fn = t - shift;

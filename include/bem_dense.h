@@ -187,7 +187,7 @@ const char* bem_version(void);
 int bem_selftest_bounded_wait(bem_ctx* ctx, int64_t cycles, int set_flag);
 /* The branch-free elementary functions of the quadrature kernels beside CUDA's
  * own, at n points x (host arrays, n at most 2^26): fn 0: sine and cosine
- * interleaved (own and ref hold 2 n), |x| < 2^20; 1: exp(-x), x >= 0; 2:
+ * interleaved (own and ref hold 2 n), |x| < 2^20; 1: exp(-x), |x| <= 708; 2:
  * 1/sqrt(x), x > 0 normal; 3: 1/p of p = x[2i] + i x[2i+1] (x, own and ref
  * hold 2 n), ref by divisions.  No counterpart in the reference. */
 int bem_selftest_math(bem_ctx* ctx, int fn, const double* x, int n, double* own, double* ref);
