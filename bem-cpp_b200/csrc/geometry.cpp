@@ -102,8 +102,8 @@ HostMesh make_hex_prism(double ar, int refinements) {
 }
 
 // Edge j of triangle t: key vertices lo < hi, sorted by (lo, hi) and, for one
-// edge, in the order of the triangles.  A bucket per lower vertex (a handful
-// of edges each) and an insertion sort in it.
+// edge, in the order of the triangles.  A bucket per lower vertex: a handful of
+// edges each, inserted in place, or a fan's many, sorted afterwards.
 namespace {
 struct TriEdge {
     int lo, hi, tri, opp;
@@ -114,6 +114,7 @@ std::vector<TriEdge> sorted_edges(const HostMesh& m) {
     for (int t = 0; t < nt; t++)
         for (int j = 0; j < 3; j++) first[std::min(m.tris[3 * t + j], m.tris[3 * t + (j + 1) % 3]) + 1]++;
     for (int v = 0; v < nv; v++) first[v + 1] += first[v];
+    constexpr int FEW = 64;  // an insertion sort's steps are the bucket's length squared
     std::vector<int> at(first.begin(), first.end() - 1);
     std::vector<TriEdge> e(3 * (size_t)nt);
     for (int t = 0; t < nt; t++)
@@ -121,9 +122,14 @@ std::vector<TriEdge> sorted_edges(const HostMesh& m) {
             const int a = m.tris[3 * t + j], b = m.tris[3 * t + (j + 1) % 3];
             const TriEdge x{std::min(a, b), std::max(a, b), t, m.tris[3 * t + (j + 2) % 3]};
             int i = at[x.lo]++;
-            for (; i > first[x.lo] && e[i - 1].hi > x.hi; i--) e[i] = e[i - 1];
+            if (first[x.lo + 1] - first[x.lo] <= FEW)
+                for (; i > first[x.lo] && e[i - 1].hi > x.hi; i--) e[i] = e[i - 1];
             e[i] = x;
         }
+    for (int v = 0; v < nv; v++)
+        if (first[v + 1] - first[v] > FEW)
+            std::stable_sort(e.begin() + first[v], e.begin() + first[v + 1],
+                             [](const TriEdge& a, const TriEdge& b) { return a.hi < b.hi; });
     return e;
 }
 }  // namespace
