@@ -284,7 +284,7 @@ struct LuShape {
     int NB = 256, W = 16;
 };
 int getrf_batched(bem_ctx* ctx, double2* A, int64_t lda, int64_t sA, int n, int batch, int* d_ipiv, int* d_info,
-                  LuShape shape);
+                  LuShape shape, bool clear_status = true);
 // The batched LU's shape for (n, batch), chosen by timing the candidates
 // once on test matrices of order n and kept for the process.
 int tune_lu_shape(bem_ctx* ctx, int n, int batch, LuShape* out);

@@ -1302,7 +1302,7 @@ int getrs(bem_ctx* ctx, const typename C2T<R>::type* LU, int64_t lda, int n, con
 // as fit co-resident next to the other matrices' (one cooperative grid);
 // batches larger than that are factored in chunks.
 int getrf_batched(bem_ctx* ctx, double2* A, int64_t lda, int64_t sA, int n, int batch, int* d_ipiv, int* d_info,
-                  LuShape shape) {
+                  LuShape shape, bool clear_status) {
     using R = double;
     using C2 = double2;
     const int NB = shape.NB, W = shape.W;
@@ -1338,7 +1338,7 @@ int getrf_batched(bem_ctx* ctx, double2* A, int64_t lda, int64_t sA, int n, int 
         for (int b0 = 0; b0 < batch; b0 += chunk) {
             const int nb = std::min(chunk, batch - b0);
             BEM_TRY(getrf_batched(ctx, A + (int64_t)b0 * sA, lda, sA, n, nb, d_ipiv + (int64_t)b0 * n, d_info + b0,
-                                  shape));
+                                  shape, clear_status && b0 == 0));
         }
         return BEM_OK;
     }
@@ -1359,7 +1359,8 @@ int getrf_batched(bem_ctx* ctx, double2* A, int64_t lda, int64_t sA, int n, int 
     pw.status = ctx->d_status;
     int* d_moves = (int*)(ws + o_mv);
     BEM_TRY_CUDA(ctx, cudaMemsetAsync(d_info, 0, batch * sizeof(int), ctx->stream));
-    BEM_TRY_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
+    // the chunks of a batch keep one status word: a wait that ran out in an earlier one is not forgotten
+    if (clear_status) BEM_TRY_CUDA(ctx, cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream));
     const C2 m1 = mk<C2>(-1, 0), p1 = mk<C2>(1, 0);
     // U12 by 64-row slabs, as in getrf (the same arithmetic per matrix)
     const bool u12b = ctx->lu_u12_slabs;
