@@ -687,10 +687,11 @@ __global__ void __launch_bounds__(256) assemble_kernel(AsmArgs a) {
 // Bound by the FP64 pipe, ~100 operations per point pair for two lossless
 // media, ~120 with one absorbing, which is 58 % busy: the 52 accumulators of a
 // thread leave room for two blocks of four warps an SM.  2N = 18432, one
-// medium absorbing: 28.6 ms, 64.3 ms before (moments per point pair and medium,
-// 17.1 triangles a tile).  Measured against it: three blocks of 128 at 168
-// registers 31.2 ms, 96 threads 37.9 ms, 160 threads 36.8 ms, the inner loop
-// unrolled 7 times 29.3 ms, not at all 32.0 ms.  A tile pair's ~240 triangle
+// medium absorbing: 29.3 ms, 64.3 ms before (moments per point pair and medium,
+// 17.1 triangles a tile).  Measured against it, at 28.6 ms with a sine of three
+// operations less: three blocks of 128 at 168 registers 31.2 ms, 96 threads
+// 37.9 ms, 160 threads 36.8 ms, the inner loop unrolled 7 times 29.3 ms, not at
+// all 32.0 ms.  A tile pair's ~240 triangle
 // pairs are two rounds of 128 threads.
 constexpr int ASM_THREADS = 128;
 // points of a triangle in shared memory: Nq x (u, weight), padded to an odd

@@ -141,7 +141,8 @@ __device__ void block_sum(double* vals, double* smem, double* out) {
 // Bound by the FP64 pipe: ~10 k operations of point pairs and ~8 k of
 // contractions a triangle pair (~100 k with three evaluations of both
 // Green's functions and six complex cross products per point pair).
-// 1280 triangles, 7 points, an absorbing interior: 8.94 -> 3.09 ms.
+// 1280 triangles, 7 points, an absorbing interior: 8.94 -> 3.17 ms, the pipe 56 %
+// busy.
 // DAMP: bit e, Im k_e != 0; BOUNDED: a real exterior k, Im k >= 0 inside and
 // phases below SINCOS_MAX, the range of the branch-free functions (else the
 // library's functions).

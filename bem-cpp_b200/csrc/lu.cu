@@ -11,7 +11,7 @@
 //                        (pivot search, swap, scale, rank-1 update); panels
 //                        of up to 8192 rows run panel_reg_kernel instead,
 //                        rows in registers, on one cluster of at most 16
-//                        CTAs with a cluster barrier per column
+//                        CTAs with one exchange of candidates per column
 //       interchanges + U12 + thin GEMM for the rest of the block column
 //     interchanges of the block's pivots on the other columns
 //     U12 = L11^-1 A12  (blocked TRSM)
@@ -392,8 +392,9 @@ panel_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int r0, int nro
 //      column jj + 1 first.
 // So a column costs one block barrier and one message's way to another SM.
 // 16 columns, us, now and with stores, a cluster barrier and the reciprocal
-// after it: 256 rows (1 CTA) 18.7 and 18.7, 2048 (8) 25.7 and 28.9, 4096 (16)
-// 26.8 and 37.0 (on 8 CTAs), 4608 (16) 28.9 and 39.0.  Of ~2600 cycles a
+// after it: 256 rows (1 CTA) 18.7 and 18.7, 2048 (8) 26.7 and 28.9, 4096 (16)
+// 28.3 and 37.0 (on 8 CTAs), 4608 (16) 30.1 and 39.0; 1 to 1.5 us of them are the
+// bound of the waits and the corrected reciprocal.  Of ~2600 cycles a
 // column on 8 CTAs the row's way into shared memory takes 430, the message 820,
 // the reductions 250 to 300 each and the updates 650.
 // Buffers alternate between two parities: a CTA sending to a peer in column
@@ -916,8 +917,8 @@ __global__ void permute_rows_kernel(const typename C2T<R>::type* __restrict__ B,
 // them.  The segment comes by cp.async into the warp's 32 x 33 buffer while
 // warp s works, lanes along a row of T (a lane per row reads 32 lines per
 // load: 7 k cycles a step, twice the substitution).  Bound by 256 dependent
-// steps of a shuffle and two multiply-adds.  FP64, 32 columns: 19.9 us a lower
-// and 20.4 us an upper block; 32.7 and 30.1 us with the segments of T in
+// steps of a shuffle, a product and a subtraction.  FP64, 32 columns: 19.8 us a
+// lower and 21.3 us an upper block; 32.7 and 30.1 us with the segments of T in
 // registers, loaded by a lane per row, the diagonal blocks in shared memory
 // and two columns a CTA.
 // An upper block's rows are scaled by their diagonal's reciprocal beforehand,
@@ -1750,7 +1751,9 @@ ldlt_diag_kernel(typename C2T<R>::type* __restrict__ A, int64_t lda, int j0, int
 // barriers for np sub-panels, each at the top level of the kernel so that
 // every thread of the cluster reaches it; no spin loop.  *info: first zero
 // pivot (1-based).
-// Bound by the chain A, C of CTA p + 1, B: 107 us per block; 148 us with four
+// Bound by the chain A, C of CTA p + 1, B: 108 us per block alone (ncu, 1.9 GHz),
+// 123 to 148 us in factorisations of 2N = 15360 and 29040, between tensor-core
+// GEMMs at the power cap.  Alone as well: 148 us with four
 // rows a warp and a lane per column in A (480 cycles a column, U stored and
 // scaled on the way), four gathers in flight and all column groups at once in
 // C; 277 us with one warp and a lane per row.
@@ -2013,11 +2016,6 @@ __global__ void neg_eye_kernel(float2* __restrict__ W, int jb) {
     W[t] = make_float2(r == c ? -1.f : 0.f, 0.f);
 }
 
-// Blocked right-looking L D L^T of the row-major complex64 S (lower triangle).
-// Per 256-column block: the diagonal block is factored in one CTA; its
-// inverse factor W = L11^-T D^-1 comes from a block TRSM on -I; the panel
-// below becomes L21 = S21 W in one tensor-core GEMM (in place: the operands
-// are packed before the product is written); then the lower-triangle update.
 // L[c * ldl + r] = W[c * 256 + r] d_r for c <= r < jb (W = -L11^-1 D^-1 of the
 // diagonal block at j0, d_r its pivots): -L11^-1 itself.  The rest of L is zero already.
 __global__ void linv_from_w_kernel(const float2* __restrict__ W, const float2* __restrict__ A, int64_t lda, int j0,
@@ -2032,6 +2030,13 @@ __global__ void linv_from_w_kernel(const float2* __restrict__ W, const float2* _
     }
 }
 
+// Blocked right-looking L D L^T of the row-major complex64 S (lower triangle).
+// Per 256-column block: the diagonal block is factored on one cluster of 8 CTAs
+// (or, where that cannot be resident, in one CTA); its inverse factor W = L11^-T
+// D^-1 comes from a block TRSM on -I; the panel below becomes L21 = S21 W in one
+// tensor-core GEMM (in place: the operands are packed before the product is
+// written); then the lower-triangle update.  With Linv the inverse blocks of
+// linv_sb diagonal blocks are put together from W on the way.
 int sytrf_nopiv(bem_ctx* ctx, float2* A, int64_t lda, int n, int* d_info, float2* Linv, int linv_sb) {
     using C2 = float2;
     const int NB = TRSM_KB;
