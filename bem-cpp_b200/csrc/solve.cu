@@ -335,14 +335,8 @@ int lu_factor_ex(bem_ctx* ctx, void* Z, int n, int64_t ldz, int precision, bool 
             if (lu->ldlt) {
                 if (ctx->solve_inv) {
                     // inverses of the diagonal blocks for the solves (without
-                    // room for them the solves keep block triangular solves).
-                    // Three 256-row blocks at most: composed inverses contract the
-                    // refinement a little less than single ones, and what the last
-                    // sweep leaves grows with that.  Against single inverses with K =
-                    // 256 updates the error of 16 systems of 2N = 720 to 4608 is 1.009
-                    // with four blocks, 0.995 with three; 2790 columns at 2N = 15360
-                    // take 150 ms with four or three, 165 with one
-                    lu->linv_sb = std::max(1, std::min(3, ctx->solve_sb));
+                    // room for them the solves keep block triangular solves)
+                    lu->linv_sb = std::max(1, std::min(4, ctx->solve_sb));
                     lu->linv_bytes = linv_count(n, lu->linv_sb) * sizeof(float2);
                     lu->Linv = (float2*)devmem_alloc(ctx->device, lu->linv_bytes, ctx);
                 }

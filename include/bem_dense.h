@@ -152,8 +152,8 @@ int bem_ctx_set_symmetric(bem_ctx* ctx, int mode);
  * the FP64 tensor path -- the same substitution regrouped, three quarters
  * of its flops in the GEMM; 0: one block triangular solve of 256 rows),
  * "solve_block_inverse" (1, default: the FP32 L D L^T factorisation also
- * keeps -L11^-1 of each diagonal block of 256 "solve_superblock" rows, 768 at
- * most (as many complex64 per row of Z: 6 KB with the default 4), and its
+ * keeps -L11^-1 of each diagonal block of 256 "solve_superblock" rows (n x
+ * 256 solve_superblock complex64: 8 KB per row with the default 4), and its
  * solves apply the diagonal blocks as tensor-core products with them; 0, or
  * without memory for them: block triangular solves; set before the
  * factorisation),
